@@ -1,0 +1,1000 @@
+// Translations without atomics: the FP64 matvec, its float-float form (FMM_FLOAT2) and the
+// deterministic mixed matvec.
+//
+// Every translation is rotation - coaxial - rotation (transMatsVecsMul_SR_rcr, reference
+// translation.cu:1864-1961).  A pass's translations are grouped by operator class: the M2L
+// directions of equal (dz, dx^2 + dy^2) have one polar angle and one length, so they share the
+// rotation block and the coaxial block and differ only by azimuthal phases (61 classes of the
+// 316 directions; two polar angles for the octants of M2M and L2L).  A CTA takes TC
+// translations of one class as columns and applies the three stages in shared memory; a lane
+// owns one column (and one of 32/TC row groups), so that every rotation or coaxial entry is one
+// load for all columns and no lane idles on a short row.  The result of a translation goes to
+// its own slot of a scratch buffer (slots in destination order), and own_reduce_kernel adds
+// each destination's slots in list order: no atomics, results repeat bit for bit.  Passes whose
+// results exceed the scratch run in chunks of consecutive destination boxes.
+//
+// FP64 and float-float keep the expansions between P2M and L2P in the basis x+_m = x_m + x_-m,
+// x-_m = x_m - x_-m (m > 0; x+_0 = x_0).  The rotation block is centrally symmetric,
+// H_{-m',-m} = H_{m',m}, so it splits into one block for x+ and one for x-: half the multiply-adds
+// of the rotations; the coaxial block is the same for +m and -m and does not see the basis; and
+// the phases cost 4 instead of 6 operations per entry and side.  The FP32 instantiation keeps the
+// plain basis and the order of operations of the mixed tiles' predecessor, so that deterministic
+// results stay what they were bit for bit.
+//
+// What bounds it: the FP64 pipe (2 multiply-adds per clock and SM; the fine levels run at 75-80 %
+// of it), in float-float the FP32 pipes (15 instructions per multiply-add): 16 p^3 / 3
+// multiply-adds per translation against 8 p^3 with the whole rotation block.  Measured against one
+// CTA per destination box, which took its translations one after another with a lane per
+// output: FP64 matvec on the 81,920-triangle sphere (p = 40 .. 10) 69.7 -> 27.3 ms (level-6 M2L
+// 23.5 -> 8.4), float-float on the 200,000-triangle head (p = 40 .. 8) 30.1 -> 15.1 ms,
+// deterministic mixed on the 20,480-triangle sphere 2.36 -> 1.26 ms.
+#include "plan.h"
+#include "ff.cuh"
+#include <algorithm>
+#include <type_traits>
+#include <vector>
+
+namespace fmm {
+
+namespace {
+
+// folded rotation table: degree n holds (n+1) x (2n+1) entries [m][j], m = 0..n, row j <= n the
+// x+ row m' = j, row j > n the x- row m' = j - n (its m = 0 entry is zero)
+__host__ __device__ __forceinline__ int fold_off(int n) { return n * (4 * n * n + 3 * n - 1) / 6; }
+__host__ __device__ __forceinline__ int fold_size(int p) { return fold_off(p); }
+
+// ---- arithmetic of one type: V a complex number (one 8- or 16-byte value in memory), X the same
+// prepared for multiply-adds, S a real table entry, K a complex one, E a phase; V accumulates
+// real and CA complex products, value() is the finished sum.
+template <typename T> struct Ops;
+
+template <> struct Ops<double> {
+    typedef double2 V;
+    typedef double S;
+    typedef double2 K;
+    typedef double2 E, X, CA;
+    static constexpr bool FOLD = true;
+    static constexpr int NORM = 4;
+    static constexpr int R = 1;  // rows per lane
+    static __device__ __forceinline__ V load(const V *p) { return *p; }
+    static __device__ __forceinline__ void store(V *p, V v) { *p = v; }
+    static __device__ __forceinline__ V zero() { return make_double2(0.0, 0.0); }
+    static __device__ __forceinline__ CA czero() { return zero(); }
+    static __device__ __forceinline__ S table(const S *p) { return __ldg(p); }
+    static __device__ __forceinline__ K table(const K *p) { return __ldg(p); }
+    static __device__ __forceinline__ X prep(V v) { return v; }
+    static __device__ __forceinline__ V add(V a, V b) { return make_double2(a.x + b.x, a.y + b.y); }
+    static __device__ __forceinline__ void mac(V &a, S h, X x)
+    {
+        a.x = fma(h, x.x, a.x);
+        a.y = fma(h, x.y, a.y);
+    }
+    static __device__ __forceinline__ void cmac(CA &a, K c, X x)
+    {
+        a.x = fma(c.x, x.x, a.x);
+        a.x = fma(-c.y, x.y, a.x);
+        a.y = fma(c.x, x.y, a.y);
+        a.y = fma(c.y, x.x, a.y);
+    }
+    static __device__ __forceinline__ V value(V a) { return a; }
+    static __device__ __forceinline__ V norm(V a) { return a; }
+    // cos x + i sin y, the phases in the folded basis; e = (cos, sin)
+    static __device__ __forceinline__ V phase(E e, V x, V y)
+    {
+        return make_double2(fma(-e.y, y.y, e.x * x.x), fma(e.y, y.x, e.x * x.y));
+    }
+    static __device__ __forceinline__ E conj(E e) { return make_double2(e.x, -e.y); }
+};
+
+// Float-float: the pairs (re, im) of the high and of the low parts side by side, so that the packed
+// FP32 instructions (two FP32 operations each, at the FP32 pipes' rate but half the issue slots)
+// work on re and im together.  Each operation rounds as its scalar form: ff_mac is ff_fma
+// (ff.cuh) on both parts.
+typedef unsigned long long f2;
+struct __align__(16) ffv {
+    f2 hi, lo;
+};
+__device__ __forceinline__ f2 f2_pack(float a, float b)
+{
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 f2_parts(f2 a)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
+{
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a - b
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) { return f2_fma(b, 0xbf800000bf800000ull, a); }
+
+// a table entry with both halves equal, so that a 16-byte load gives the operands of the packed
+// instructions
+struct __align__(16) ffs {
+    f2 hi, lo;
+};
+struct __align__(16) ffk {
+    ffs x, y;
+};
+
+template <> struct Ops<ff> {
+    typedef ffv V;
+    typedef ffs S;
+    typedef ffk K;
+    typedef float4 E;  // (cos hi, cos lo, sin hi, sin lo)
+    struct X {
+        f2 hi, nhi, lo;  // nhi = -hi
+    };
+    struct CA {
+        V x, y;  // sums of re(c) v and of im(c) v
+    };
+    static constexpr bool FOLD = true;
+    static constexpr int R = 2;
+    static constexpr int NORM = 1;  // products between two norm()
+    static __device__ __forceinline__ V load(const V *p)
+    {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
+        return V{v.x, v.y};
+    }
+    static __device__ __forceinline__ void store(V *p, V v) { *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(v.hi, v.lo); }
+    static __device__ __forceinline__ S table(const S *p)
+    {
+        const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(p));
+        return S{v.x, v.y};
+    }
+    static __device__ __forceinline__ K table(const K *p) { return K{table(&p->x), table(&p->y)}; }
+    static __device__ __forceinline__ V zero() { return V{0ull, 0ull}; }
+    static __device__ __forceinline__ CA czero() { return CA{zero(), zero()}; }
+    static __device__ __forceinline__ X prep(V v) { return X{v.hi, v.hi ^ 0x8000000080000000ull, v.lo}; }
+    static __device__ __forceinline__ V add(V a, V b)
+    {
+        const float2 ah = f2_parts(a.hi), al = f2_parts(a.lo), bh = f2_parts(b.hi), bl = f2_parts(b.lo);
+        const ff x = ff(ah.x, al.x) + ff(bh.x, bl.x), y = ff(ah.y, al.y) + ff(bh.y, bl.y);
+        return V{f2_pack(x.hi, y.hi), f2_pack(x.lo, y.lo)};
+    }
+    static __device__ __forceinline__ V norm(V a)
+    {
+        const f2 h = f2_add(a.hi, a.lo);
+        return V{h, f2_sub(a.lo, f2_sub(h, a.hi))};
+    }
+    static __device__ __forceinline__ CA norm(CA a) { return CA{norm(a.x), norm(a.y)}; }
+    // a += h x: the product of the high parts as p + e exactly (TwoProd), a.hi + p as s + t exactly
+    // (TwoSum); e, t and the cross products go to the low part, which norm() brings back under the
+    // high one (FastTwoSum) after every product: a sum of n products is accurate to about n 2^-47 of
+    // the sum of their magnitudes, the same form of bound as FP64 summation (n 2^-53).  A norm()
+    // after every second product only measured 4 % faster and 10 % further from FP64; none until
+    // the end, twice as far.
+    static __device__ __forceinline__ void mac(V &a, S h, X x)
+    {
+        const f2 np = f2_mul(h.hi, x.nhi);  // -p
+        const f2 e = f2_fma(h.hi, x.hi, np);
+        const f2 s = f2_sub(a.hi, np), bb = f2_sub(s, a.hi), d = f2_sub(a.hi, f2_sub(s, bb));
+        const f2 t = f2_sub(d, f2_add(np, bb));
+        a.lo = f2_fma(h.hi, x.lo, a.lo);
+        a.lo = f2_fma(h.lo, x.hi, a.lo);
+        a.lo = f2_add(a.lo, f2_add(e, t));
+        a.hi = s;
+    }
+    static __device__ __forceinline__ void cmac(CA &a, K c, X x)
+    {
+        mac(a.x, c.x, x);
+        mac(a.y, c.y, x);
+    }
+    static __device__ __forceinline__ V times_i(V v)
+    {
+        const float2 h = f2_parts(v.hi), l = f2_parts(v.lo);
+        return V{f2_pack(-h.y, h.x), f2_pack(-l.y, l.x)};
+    }
+    static __device__ __forceinline__ V value(V a) { return norm(a); }
+    static __device__ __forceinline__ V value(CA a) { return add(norm(a.x), times_i(norm(a.y))); }
+    static __device__ __forceinline__ V phase(E e, V x, V y)
+    {
+        V r = zero();
+        mac(r, S{f2_pack(e.x, e.x), f2_pack(e.y, e.y)}, prep(x));
+        mac(r, S{f2_pack(e.z, e.z), f2_pack(e.w, e.w)}, prep(times_i(y)));
+        return norm(r);
+    }
+    static __device__ __forceinline__ E conj(E e) { return make_float4(e.x, e.y, -e.z, -e.w); }
+};
+
+// FP32 (deterministic mixed plans): the plain basis; every product and sum rounds in one fixed
+// way, spelled out so that no compilation of it can contract them differently.
+template <> struct Ops<float> {
+    typedef float2 V;
+    typedef float S;
+    typedef float2 K;
+    typedef float2 E, X, CA;
+    static constexpr bool FOLD = false;
+    static constexpr int NORM = 4;
+    static constexpr int R = 4;
+    static __device__ __forceinline__ V load(const V *p) { return *p; }
+    static __device__ __forceinline__ void store(V *p, V v) { *p = v; }
+    static __device__ __forceinline__ V zero() { return make_float2(0.f, 0.f); }
+    static __device__ __forceinline__ CA czero() { return zero(); }
+    static __device__ __forceinline__ S table(const S *p) { return __ldg(p); }
+    static __device__ __forceinline__ K table(const K *p) { return __ldg(p); }
+    static __device__ __forceinline__ X prep(V v) { return v; }
+    static __device__ __forceinline__ V add(V a, V b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
+    static __device__ __forceinline__ void mac(V &a, S h, X x)
+    {
+        a.x = __fmaf_rn(h, x.x, a.x);
+        a.y = __fmaf_rn(h, x.y, a.y);
+    }
+    // c x
+    static __device__ __forceinline__ V mul(V c, V x)
+    {
+        return make_float2(__fmaf_rn(c.x, x.x, -__fmul_rn(c.y, x.y)), __fmaf_rn(c.y, x.x, __fmul_rn(c.x, x.y)));
+    }
+    // conj(e) x
+    static __device__ __forceinline__ V cjmul(V e, V x)
+    {
+        return make_float2(__fmaf_rn(e.x, x.x, __fmul_rn(e.y, x.y)), __fmaf_rn(e.x, x.y, -__fmul_rn(e.y, x.x)));
+    }
+    static __device__ __forceinline__ void cmac(CA &a, K c, X x) { a = add(a, mul(c, x)); }
+    static __device__ __forceinline__ V value(V a) { return a; }
+    static __device__ __forceinline__ V norm(V a) { return a; }
+};
+
+// pair index q -> (n, m), 0 <= m <= n, q = n (n + 1) / 2 + m
+__device__ __forceinline__ void pair_nm(int q, int &n, int &m)
+{
+    int k = (int)((sqrtf(8.f * q + 1.f) - 1.f) * 0.5f);
+    while (k * (k + 1) / 2 > q) k--;
+    while ((k + 1) * (k + 2) / 2 <= q) k++;
+    n = k;
+    m = q - k * (k + 1) / 2;
+}
+
+template <typename T> struct OwnArgs {
+    typedef typename Ops<T>::V V;
+    typedef typename Ops<T>::S S;
+    typedef typename Ops<T>::K K;
+    int p, nin, nq, pin, pout, pmax;  // RCR order; degrees used of the source and of the result
+    int rows;                         // rows of each of the two shared-memory tiles
+    const int4 *items;                // (rotation table row, first translation, count, coaxial block)
+    const int *slot;                  // translations in class order -> slot
+    const int *src;                   // per slot: source box and phase row
+    const short *key;
+    const S *rot;
+    size_t rot_stride;
+    const typename Ops<T>::E *ph;     // [row][m + pmax - 1]
+    const K *Cc;
+    const V *in;
+    V *out;
+    int slot0;                        // slot of out[0]
+    const int *u1, *u2, *u3;          // work units of the three stages
+    int n1, n2, n3;
+};
+
+// One rotation stage.  The rows of degree n are taken in groups of R rows of one sign (x+ or x-;
+// FP32: any rows); unit = n | first group << 8, a lane takes one group of its column.
+template <typename T, int TC>
+__device__ __forceinline__ void rot_stage(const typename Ops<T>::S *__restrict__ rot, const typename Ops<T>::V *X,
+                                          typename Ops<T>::V *Y, const int *__restrict__ units, int nu)
+{
+    typedef Ops<T> O;
+    constexpr int R = O::R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int c = lane % TC, rl = lane / TC;
+    for (int u = warp; u < nu; u += nw) {
+        const int info = __ldg(units + u), n = info & 255, w = 2 * n + 1, r0 = n * n + n;
+        const int np = O::FOLD ? (n + R) / R : (w + R - 1) / R, nm = O::FOLD ? (n + R - 1) / R : 0;
+        const int g = min((info >> 8) + rl, np + nm - 1), minus = O::FOLD && g >= np;
+        const int first = minus ? 1 + (g - np) * R : g * R;         // m' (FP32: row) of the first row
+        const int last = O::FOLD ? n : w - 1;
+        const int steps = O::FOLD ? n + 1 : w;
+        const typename O::S *h = rot + (O::FOLD ? fold_off(n) : rot_off(n)) + (minus ? n : 0) + first;
+        const typename O::V *x = X + (O::FOLD ? r0 : n * n) * TC + c;
+        const int dx = minus ? -TC : TC;
+        typename O::V acc[R];
+        typename O::S hn[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            acc[k] = O::zero();
+            hn[k] = O::table(h + k);  // rows past the last read the next entry; their sums are dropped
+        }
+#pragma unroll 4
+        for (int m = 0; m < steps; m++) {
+            typename O::S hc[R];
+            if (m + 1 < steps) h += w;  // the last step loads its own entries again
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                hc[k] = hn[k];
+                hn[k] = O::table(h + k);
+            }
+            const typename O::X xv = O::prep(O::load(x));
+            x += dx;
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                O::mac(acc[k], hc[k], xv);
+                if ((m & (O::NORM - 1)) == O::NORM - 1) acc[k] = O::norm(acc[k]);
+            }
+        }
+        if ((info >> 8) + rl < np + nm) {
+#pragma unroll
+            for (int k = 0; k < R; k++)
+                if (first + k <= last) {
+                    const int q = O::FOLD ? (minus ? r0 - first - k : r0 + first + k) : n * n + first + k;
+                    O::store(Y + q * TC + c, O::value(acc[k]));
+                }
+        }
+    }
+}
+
+// The coaxial stage: rows n' of +m then of -m in groups of R; unit = |m| | first group << 8.
+template <typename T, int TC>
+__device__ __forceinline__ void coax_stage(int p, int nin, int nq, const typename Ops<T>::K *__restrict__ Cc,
+                                           const typename Ops<T>::V *X, typename Ops<T>::V *Y,
+                                           const int *__restrict__ units, int nu)
+{
+    typedef Ops<T> O;
+    constexpr int R = O::R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int c = lane % TC, rl = lane / TC;
+    for (int u = warp; u < nu; u += nw) {
+        const int info = __ldg(units + u), am = info & 255, sz = p - am, nrow = nq - am;
+        const int np = (nrow + R - 1) / R, nm = am > 0 ? np : 0;
+        const int g = min((info >> 8) + rl, np + nm - 1), minus = g >= np;
+        const int first = (minus ? g - np : g) * R, sm = minus ? -am : am;
+        const typename O::K *cb = Cc + coax_off(p, am) + first;
+        const typename O::V *x = X + (am * am + am + sm) * TC + c;
+        int dx = (2 * am + 2) * TC;
+        typename O::CA acc[R];
+        typename O::K cn[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            acc[k] = O::czero();
+            cn[k] = O::table(cb + k);
+        }
+#pragma unroll 4
+        for (int n = 0; n < nin - am; n++) {
+            typename O::K cc[R];
+            if (n + 1 < nin - am) cb += sz;
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                cc[k] = cn[k];
+                cn[k] = O::table(cb + k);
+            }
+            const typename O::X xv = O::prep(O::load(x));
+            x += dx;
+            dx += 2 * TC;
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                O::cmac(acc[k], cc[k], xv);
+                if ((n & (O::NORM - 1)) == O::NORM - 1) acc[k] = O::norm(acc[k]);
+            }
+        }
+        if ((info >> 8) + rl < np + nm) {
+#pragma unroll
+            for (int k = 0; k < R; k++)
+                if (first + k < nrow) {
+                    const int nn = am + first + k;
+                    O::store(Y + (nn * nn + nn + sm) * TC + c, O::value(acc[k]));
+                }
+        }
+    }
+}
+
+template <typename T, int TC>
+__global__ void __launch_bounds__(512, 1) own_tile_kernel(OwnArgs<T> a)
+{
+    typedef Ops<T> O;
+    typedef typename O::V V;
+    typedef typename O::E E;
+    constexpr int GI = 32 / TC;  // gather / scatter: TC columns x GI pairs (n, m >= 0) per warp
+    extern __shared__ double2 own_smem[];
+    __shared__ int s_src[TC], s_key[TC], s_out[TC];
+    V *X = reinterpret_cast<V *>(own_smem), *W = X + (size_t)a.rows * TC;
+    const int4 it = a.items[blockIdx.x];
+    const int cnt = it.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (threadIdx.x < TC) {
+        const int s = a.slot[it.y + min((int)threadIdx.x, cnt - 1)];
+        s_src[threadIdx.x] = a.src[s];
+        s_key[threadIdx.x] = a.key[s];
+        s_out[threadIdx.x] = s - a.slot0;
+    }
+    __syncthreads();
+    const int c = lane % TC, gi = lane / TC, w = 2 * a.pmax - 1, off = a.pmax - 1;
+    const E *ph = a.ph + (size_t)s_key[c] * w + off;
+    // gather with the phases e^{i m phi}
+    {
+        const int np = a.nin * (a.nin + 1) / 2;
+        const V *src = a.in + (size_t)s_src[c] * a.pin * a.pin;
+        for (int q = warp * GI + gi; q < np; q += nw * GI) {
+            int n, m;
+            pair_nm(q, n, m);
+            const int r0 = n * n + n;
+            V xp = O::zero(), xm = xp;
+            if (c < cnt) {
+                const V *in = src + r0;
+                xp = O::load(in + m);
+                if constexpr (O::FOLD) {
+                    if (m > 0) {
+                        const V vp = xp, vm = O::load(in - m);
+                        const E e = __ldg(ph + m);
+                        xp = O::phase(e, vp, vm);
+                        xm = O::phase(e, vm, vp);
+                    }
+                } else {
+                    xp = O::mul(xp, __ldg(ph + m));
+                    if (m > 0) xm = O::mul(O::load(in - m), __ldg(ph - m));
+                }
+            }
+            O::store(X + (r0 + m) * TC + c, xp);
+            if (m > 0) O::store(X + (r0 - m) * TC + c, xm);
+        }
+    }
+    __syncthreads();
+    const typename O::S *rot = a.rot + (size_t)it.x * a.rot_stride;
+    rot_stage<T, TC>(rot, X, W, a.u1, a.n1);
+    __syncthreads();
+    coax_stage<T, TC>(a.p, a.nin, a.nq, a.Cc + (size_t)it.w * coax_size(a.p), W, X, a.u2, a.n2);
+    __syncthreads();
+    rot_stage<T, TC>(rot, X, W, a.u3, a.n3);
+    __syncthreads();
+    // results with the phases e^{-i m phi}
+    if (c < cnt) {
+        const int np = a.nq * (a.nq + 1) / 2;
+        V *dst = a.out + (size_t)s_out[c] * a.pout * a.pout;
+        for (int q = warp * GI + gi; q < np; q += nw * GI) {
+            int n, m;
+            pair_nm(q, n, m);
+            const int r0 = n * n + n;
+            V *out = dst + r0;
+            const V yp = O::load(W + (r0 + m) * TC + c);
+            if constexpr (O::FOLD) {
+                if (m > 0) {
+                    const V ym = O::load(W + (r0 - m) * TC + c);
+                    const E e = O::conj(__ldg(ph + m));
+                    O::store(out + m, O::phase(e, yp, ym));
+                    O::store(out - m, O::phase(e, ym, yp));
+                } else {
+                    O::store(out, yp);
+                }
+            } else {
+                O::store(out + m, O::cjmul(__ldg(ph + m), yp));
+                if (m > 0) O::store(out - m, O::cjmul(__ldg(ph - m), O::load(W + (r0 - m) * TC + c)));
+            }
+        }
+    }
+}
+
+// Dst[b] = (add ? Dst[b] : 0) + the slots beg[b] .. beg[b+1]-1 of part (slot s at s - slot0), n2
+// entries each, in order; with S > 1 in S runs whose sums are added in order
+template <typename T>
+__global__ void own_reduce_kernel(int b0, int b1, int n2, int S, int add, int slot0, const int *__restrict__ beg,
+                                  const typename Ops<T>::V *__restrict__ part, typename Ops<T>::V *__restrict__ Dst)
+{
+    typedef Ops<T> O;
+    const size_t n = (size_t)(b1 - b0) * n2;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+        const int b = b0 + (int)(t / n2), i = (int)(t % n2), s0 = beg[b], ns = beg[b + 1] - s0;
+        const typename O::V *q = part + (size_t)(s0 - slot0) * n2 + i;
+        typename O::V *d = Dst + (size_t)b * n2 + i, tot = O::zero();
+        for (int c = 0; c < S; c++) {
+            const int sa = (int)((long long)ns * c / S), sb = (int)((long long)ns * (c + 1) / S);
+            typename O::V acc = c == 0 && add ? O::load(d) : O::zero();
+#pragma unroll 4
+            for (int s = sa; s < sb; s++) acc = O::add(acc, O::load(q + (size_t)s * n2));
+            tot = c == 0 ? acc : O::add(tot, acc);
+        }
+        O::store(d, tot);
+    }
+}
+
+// in place: plain -> x+/x- (fwd), or back
+__global__ void own_fold_kernel(double2 *x, size_t nb, int p, int fwd)
+{
+    const int np = p * (p + 1) / 2;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nb * np; t += (size_t)gridDim.x * blockDim.x) {
+        int n, m;
+        pair_nm((int)(t % np), n, m);
+        if (m == 0) continue;
+        double2 *q = x + (t / np) * (size_t)p * p + n * n + n;
+        const double2 a = q[m], b = q[-m];
+        const double f = fwd ? 1.0 : 0.5;
+        q[m] = make_double2(f * (a.x + b.x), f * (a.y + b.y));
+        q[-m] = make_double2(f * (a.x - b.x), f * (a.y - b.y));
+    }
+}
+
+// FP64 plain -> float-float x+/x- (times ds[n] where given), and back
+__global__ void own_fold_ff_kernel(const double2 *__restrict__ in, ffv *__restrict__ out, size_t nb, int p,
+                                   const double *__restrict__ ds)
+{
+    const int np = p * (p + 1) / 2;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nb * np; t += (size_t)gridDim.x * blockDim.x) {
+        int n, m;
+        pair_nm((int)(t % np), n, m);
+        const size_t base = (t / np) * (size_t)p * p + n * n + n;
+        const double f = ds ? ds[n] : 1.0;
+        auto put = [&](size_t i, double re, double im) {
+            const ff a = ff_from(re * f), b = ff_from(im * f);
+            Ops<ff>::store(out + i, ffv{f2_pack(a.hi, b.hi), f2_pack(a.lo, b.lo)});
+        };
+        const double2 a = in[base + m];
+        if (m == 0) {
+            put(base, a.x, a.y);
+        } else {
+            const double2 b = in[base - m];
+            put(base + m, a.x + b.x, a.y + b.y);
+            put(base - m, a.x - b.x, a.y - b.y);
+        }
+    }
+}
+__global__ void own_unfold_ff_kernel(const ffv *__restrict__ in, double2 *__restrict__ out, size_t nb, int p,
+                                     const double *__restrict__ ds)
+{
+    const int np = p * (p + 1) / 2;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nb * np; t += (size_t)gridDim.x * blockDim.x) {
+        int n, m;
+        pair_nm((int)(t % np), n, m);
+        const size_t base = (t / np) * (size_t)p * p + n * n + n;
+        const double f = (ds ? ds[n] : 1.0) * (m ? 0.5 : 1.0);
+        auto get = [&](size_t i) {
+            const ffv v = Ops<ff>::load(in + i);
+            const float2 h = f2_parts(v.hi), l = f2_parts(v.lo);
+            return make_double2((double)h.x + (double)l.x, (double)h.y + (double)l.y);
+        };
+        const double2 a = get(base + m);
+        if (m == 0) {
+            out[base] = make_double2(f * a.x, f * a.y);
+        } else {
+            const double2 b = get(base - m);
+            out[base + m] = make_double2(f * (a.x + b.x), f * (a.y + b.y));
+            out[base - m] = make_double2(f * (a.x - b.x), f * (a.y - b.y));
+        }
+    }
+}
+
+// folded rotation tables of the classes' representative rows rep[k] of H (see fold_off)
+__global__ void own_fold_table_kernel(int pmax, const int *__restrict__ rep, const double *__restrict__ H,
+                                      double *__restrict__ o64, ffs *__restrict__ off2)
+{
+    const int n = blockIdx.x, k = blockIdx.y, w = 2 * n + 1;
+    const double *Hn = H + (size_t)rep[k] * rot_size(pmax) + rot_off(n);
+    const size_t base = (size_t)k * fold_size(pmax) + fold_off(n);
+    for (int t = threadIdx.x; t < (n + 1) * w; t += blockDim.x) {
+        const int m = t / w, j = t % w, mp = j <= n ? j : j - n;
+        const double a = Hn[(n + m) * w + n + mp], b = Hn[(n - m) * w + n + mp];
+        double v;
+        if (j > n)
+            v = m ? a - b : 0.0;
+        else if (m)
+            v = mp ? a + b : 0.5 * (a + b);
+        else
+            v = mp ? a + Hn[n * w + n - mp] : a;
+        if (o64) o64[base + t] = v;
+        if (off2) {
+            const ff f = ff_from(v);
+            off2[base + t] = ffs{f2_pack(f.hi, f.hi), f2_pack(f.lo, f.lo)};
+        }
+    }
+}
+
+// ---- lists
+// per slot of M2M (children in the parents' order) and L2L (boxes): source box and phase row
+__global__ void own_m2m_slots_kernel(int nb, const int *child_list, const unsigned char *octant, int *src, short *key)
+{
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nb; s += gridDim.x * blockDim.x) {
+        src[s] = child_list[s];
+        key[s] = (short)(NDIR + octant[child_list[s]]);
+    }
+}
+__global__ void own_l2l_slots_kernel(int nb, const unsigned char *octant, short *key)
+{
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nb; s += gridDim.x * blockDim.x)
+        key[s] = (short)(NDIR + 8 + octant[s]);
+}
+// class order: bin (chunk of the slot) * ncls + class; counts (list null), then positions
+__global__ void own_bin_kernel(int n, const short *__restrict__ key, const int *__restrict__ cls_of_key,
+                               const int *__restrict__ chunk_slot, int nchunk, int ncls, int *bins, int *list)
+{
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        int c = 0;
+        while (c + 1 < nchunk && s >= chunk_slot[c + 1]) c++;
+        const int pos = atomicAdd(bins + c * ncls + cls_of_key[key[s]], 1);
+        if (list) list[pos] = s;
+    }
+}
+
+unsigned ew_grid(size_t n) { return (unsigned)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 152 * 16)); }
+
+// Columns of a tile: two tiles of `rows` rows in shared memory, at most TWO_CTA bytes where two
+// CTAs (of 256 threads) are to share an SM, so that one computes while the other gathers or waits
+// at a barrier; else one CTA of 512 threads.  Most columns first: a table entry then serves more
+// multiply-adds (M2L of the head in float-float, 8 / 16 / 32 columns: p = 8 8.2 / 6.8 / 5.9 ms,
+// p = 10 4.0 / 3.3 / 3.1); where only 8 columns leave room for two CTAs (p = 20) 16 columns in one
+// CTA measured the same (FP64 5.08 against 5.02 ms), and 4 columns in one of two CTAs as 8 in one
+// (p = 30: 3.86 against 3.91).
+constexpr size_t TWO_CTA = 112 * 1024 + 512, ONE_CTA = 226 * 1024;
+
+int pick_cols(int rows, size_t elem)
+{
+    for (int tc : {32, 16, 8})
+        if (2 * elem * rows * tc <= TWO_CTA) return tc;
+    for (int tc : {8, 4, 2})
+        if (2 * elem * rows * tc <= ONE_CTA) return tc;
+    return 0;
+}
+
+// bytes of the scratch that holds one chunk of translated expansions
+constexpr size_t PART_CAP = 128u << 20;
+
+template <typename T, int TC>
+int launch_tc(const OwnArgs<T> &a, int n_items, cudaStream_t st)
+{
+    static size_t attr = 0;
+    const size_t sm = 2 * sizeof(typename Ops<T>::V) * (size_t)a.rows * TC;
+    int e = raise_smem_limit((const void *)own_tile_kernel<T, TC>, sm, &attr);
+    if (e) return e;
+    own_tile_kernel<T, TC><<<n_items, sm > TWO_CTA ? 512 : 256, sm, st>>>(a);
+    FMM_CUDA_TRY(cudaGetLastError());
+    return FMM_OK;
+}
+
+// the lists and units of one pass (built on first use, on the plan's stream)
+template <typename T>
+int build_pass(Plan *P, int l, int which, OwnPass &O)
+{
+    typedef typename Ops<T>::V C;
+    LevelDev &L = P->lev[l];
+    cudaStream_t st = P->stream;
+    const int pp = which == PASS_M2L ? L.p : P->lev[l - 1].p;
+    O.p = pp;
+    O.pin = which == PASS_M2M ? L.p : pp;
+    O.pout = which == PASS_L2L ? L.p : pp;
+    const int nin = std::min(O.pin, pp), nq = std::min(O.pout, pp), ndst = which == PASS_M2M ? P->lev[l - 1].nb : L.nb;
+    O.rows = std::max(nin, nq) * std::max(nin, nq);
+    O.tc = pick_cols(O.rows, sizeof(C));
+    if (!O.tc) {
+        fmm_set_error("translation order %d above 60", pp);
+        return FMM_ERR_CUDA;
+    }
+    // slots: the destination's translations in list order
+    std::vector<int> beg;
+    const int *beg_dev = which == PASS_M2L ? L.sr_beg : which == PASS_M2M ? P->lev[l - 1].child_beg : nullptr;
+    const int n = which == PASS_M2L ? (int)L.num_sr : L.nb;
+    O.beg = beg_dev;
+    if (beg_dev) {
+        beg.resize(ndst + 1);
+        FMM_CUDA_TRY(cudaMemcpyAsync(beg.data(), beg_dev, sizeof(int) * (ndst + 1), cudaMemcpyDeviceToHost, st));
+    }
+    if (which == PASS_M2L) {
+        O.src = L.sr_src;
+        O.key = L.sr_dir;
+    } else {
+        FMM_CUDA_TRY(dev_alloc(P, (void **)&O.key_own, sizeof(short) * std::max(1, L.nb)));
+        O.key = O.key_own;
+        if (which == PASS_M2M) {
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&O.src_own, sizeof(int) * std::max(1, L.nb)));
+            O.src = O.src_own;
+            own_m2m_slots_kernel<<<ew_grid(L.nb), 256, 0, st>>>(L.nb, P->lev[l - 1].child_list, L.octant, O.src_own, O.key_own);
+        } else {
+            O.src = L.parent;
+            own_l2l_slots_kernel<<<ew_grid(L.nb), 256, 0, st>>>(L.nb, L.octant, O.key_own);
+        }
+    }
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    // chunks of destinations whose results fit the scratch
+    const size_t slot_bytes = sizeof(C) * O.pout * O.pout;
+    O.chunk_box.assign(1, 0);
+    std::vector<int> chunk_slot(1, 0);
+    size_t most = 0;
+    if (beg_dev) {
+        const int cap = (int)std::max<size_t>(1, PART_CAP / slot_bytes);
+        for (int b = 0; b < ndst;) {
+            int e = b + 1;
+            while (e < ndst && beg[e + 1] - beg[b] <= cap) e++;
+            most = std::max(most, (size_t)(beg[e] - beg[b]) * slot_bytes);
+            O.chunk_box.push_back(e);
+            chunk_slot.push_back(beg[e]);
+            b = e;
+        }
+    } else {
+        O.chunk_box.push_back(ndst);
+        chunk_slot.push_back(n);
+    }
+    O.part_bytes = most;
+    O.chunk_slot = chunk_slot;
+    const int nchunk = (int)chunk_slot.size() - 1;
+    // classes
+    std::vector<int> cls, rep;
+    const int nkeys = which == PASS_M2L ? NDIR : 8, key0 = which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8;
+    direction_classes(P, which, nkeys, cls, rep);
+    const int ncls = (int)rep.size(), cls0 = which == PASS_M2L ? 0 : which == PASS_M2M ? P->own_ncls : P->own_ncls + 2;
+    std::vector<int> cls_of_key(NDIR + 16, 0);
+    for (int d = 0; d < nkeys; d++) cls_of_key[key0 + d] = cls[d];
+    FMM_CUDA_TRY(dev_alloc(P, (void **)&O.slot, sizeof(int) * std::max(1, n)));
+    int *tmp = nullptr;  // class of key, chunk beginnings, bins
+    const size_t nbin = (size_t)nchunk * ncls;
+    FMM_CUDA_TRY(cudaMalloc(&tmp, sizeof(int) * (NDIR + 16 + chunk_slot.size() + nbin)));
+    int *d_cls = tmp, *d_chunk = tmp + NDIR + 16, *d_bins = d_chunk + chunk_slot.size();
+    std::vector<int> bins(nbin);
+    std::vector<int4> items;
+    cudaError_t ce = cudaMemcpyAsync(d_cls, cls_of_key.data(), sizeof(int) * cls_of_key.size(), cudaMemcpyHostToDevice, st);
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_chunk, chunk_slot.data(), sizeof(int) * chunk_slot.size(), cudaMemcpyHostToDevice, st);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(d_bins, 0, sizeof(int) * nbin, st);
+    if (ce == cudaSuccess) {
+        own_bin_kernel<<<ew_grid(n), 256, 0, st>>>(n, O.key, d_cls, d_chunk, nchunk, ncls, d_bins, nullptr);
+        ce = cudaMemcpyAsync(bins.data(), d_bins, sizeof(int) * nbin, cudaMemcpyDeviceToHost, st);
+    }
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+    if (ce == cudaSuccess) {
+        O.chunk_item.assign(1, 0);
+        int pos = 0;
+        for (int c = 0; c < nchunk; c++) {
+            for (int k = 0; k < ncls; k++) {
+                const int cnt = bins[(size_t)c * ncls + k];
+                bins[(size_t)c * ncls + k] = pos;
+                const int rrow = std::is_same<T, float>::value ? key0 + rep[k] : cls0 + k;
+                for (int a = 0; a < cnt; a += O.tc)
+                    items.push_back(make_int4(rrow, pos + a, std::min(O.tc, cnt - a), which == PASS_M2L ? P->dir_dist[rep[k]] : 0));
+                pos += cnt;
+            }
+            O.chunk_item.push_back((int)items.size());
+        }
+        ce = cudaMemcpyAsync(d_bins, bins.data(), sizeof(int) * nbin, cudaMemcpyHostToDevice, st);
+        own_bin_kernel<<<ew_grid(n), 256, 0, st>>>(n, O.key, d_cls, d_chunk, nchunk, ncls, d_bins, O.slot);
+    }
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+    cudaFree(tmp);
+    FMM_CUDA_TRY(ce);
+    // work units, longest first: groups of R rows of one sign, 32 / tc groups each
+    const int rl = 32 / O.tc, R = Ops<T>::R;
+    std::vector<int> un;
+    auto rot_units = [&](int deg) {
+        int k = 0;
+        for (int d = deg - 1; d >= 0; d--) {
+            const int ng = Ops<T>::FOLD ? (d + R) / R + (d + R - 1) / R : (2 * d + R) / R;
+            for (int g = 0; g < ng; g += rl, k++) un.push_back(d | g << 8);
+        }
+        return k;
+    };
+    O.n1 = rot_units(nin);
+    O.n2 = 0;
+    // orders m that the source does not reach (nq > nin) give rows of zeros
+    for (int am = 0; am < nq; am++) {
+        const int ng = (am ? 2 : 1) * ((nq - am + R - 1) / R);
+        for (int g = 0; g < ng; g += rl, O.n2++) un.push_back(am | g << 8);
+    }
+    O.n3 = rot_units(nq);
+    FMM_CUDA_TRY(dev_alloc(P, (void **)&O.items, sizeof(int4) * std::max<size_t>(1, items.size())));
+    FMM_CUDA_TRY(dev_alloc(P, (void **)&O.units, sizeof(int) * un.size()));
+    FMM_CUDA_TRY(cudaMemcpyAsync(O.items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, st));
+    FMM_CUDA_TRY(cudaMemcpyAsync(O.units, un.data(), sizeof(int) * un.size(), cudaMemcpyHostToDevice, st));
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    O.built = 1;
+    return FMM_OK;
+}
+
+template <typename T> int tables_of(Plan *P, OwnArgs<T> &a);
+template <> int tables_of<double>(Plan *P, OwnArgs<double> &a)
+{
+    a.rot = P->own_rot64;
+    a.rot_stride = fold_size(P->pmax);
+    a.ph = P->PHsr64;
+    return FMM_OK;
+}
+template <> int tables_of<ff>(Plan *P, OwnArgs<ff> &a)
+{
+    a.rot = reinterpret_cast<const ffs *>(P->own_rot_ff);
+    a.rot_stride = fold_size(P->pmax);
+    a.ph = P->PHall_ff;
+    return FMM_OK;
+}
+template <> int tables_of<float>(Plan *P, OwnArgs<float> &a)
+{
+    a.rot = P->Hsr32;
+    a.rot_stride = rot_size(P->pmax);
+    a.ph = P->PHsr32;
+    return FMM_OK;
+}
+
+template <typename T> struct LevelArrays {
+    typename Ops<T>::V *Cm, *Dl;
+    const typename Ops<T>::K *Csr, *Cup, *Cdown;
+};
+template <typename T> LevelArrays<T> arrays_of(LevelDev &L);
+template <> LevelArrays<double> arrays_of<double>(LevelDev &L) { return {L.Cm64, L.Dl64, L.Csr64, L.Crr64, L.Crr64}; }
+template <> LevelArrays<float> arrays_of<float>(LevelDev &L)
+{
+    return {L.Cm32, L.Dl32, L.Csr32, L.Crr32, L.Crr32L ? L.Crr32L : L.Crr32};
+}
+template <> LevelArrays<ff> arrays_of<ff>(LevelDev &L)
+{
+    return {reinterpret_cast<ffv *>(L.Cm_ff), reinterpret_cast<ffv *>(L.Dl_ff), reinterpret_cast<const ffk *>(L.Csr_ff),
+            reinterpret_cast<const ffk *>(L.Crr_ff), reinterpret_cast<const ffk *>(L.CrrL_ff ? L.CrrL_ff : L.Crr_ff)};
+}
+
+template <typename T>
+int run_pass(Plan *P, int l, int which, OwnPass &O)
+{
+    typedef typename Ops<T>::V C;
+    cudaStream_t st = P->stream;
+    LevelDev &L = P->lev[l];
+    LevelArrays<T> A = arrays_of<T>(L), U = l > P->lmin ? arrays_of<T>(P->lev[l - 1]) : A;
+    OwnArgs<T> a;
+    int e = tables_of<T>(P, a);
+    if (e) return e;
+    a.p = O.p;
+    a.pin = O.pin;
+    a.pout = O.pout;
+    a.nin = std::min(O.pin, O.p);
+    a.nq = std::min(O.pout, O.p);
+    a.pmax = P->pmax;
+    a.rows = O.rows;
+    a.slot = O.slot;
+    a.src = O.src;
+    a.key = O.key;
+    a.Cc = which == PASS_M2L ? A.Csr : which == PASS_M2M ? A.Cup : A.Cdown;
+    a.in = which == PASS_L2L ? U.Dl : A.Cm;
+    a.u1 = O.units;
+    a.u2 = O.units + O.n1;
+    a.u3 = O.units + O.n1 + O.n2;
+    a.n1 = O.n1;
+    a.n2 = O.n2;
+    a.n3 = O.n3;
+    C *dst = which == PASS_M2M ? U.Cm : A.Dl;
+    const int n2 = O.pout * O.pout;
+    // a parent of lower order than the child reaches the child's first degrees only
+    if (which == PASS_L2L && a.nq < O.pout)
+        FMM_CUDA_TRY(cudaMemsetAsync(dst, 0, sizeof(C) * (size_t)L.nb * n2, st));
+    for (size_t c = 0; c + 1 < O.chunk_box.size(); c++) {
+        const int n = O.chunk_item[c + 1] - O.chunk_item[c];
+        a.items = O.items + O.chunk_item[c];
+        a.slot0 = O.chunk_slot[c];
+        a.out = which == PASS_L2L ? dst : (C *)P->own_part;
+        if (n > 0) {
+            switch (O.tc) {
+            case 32: e = launch_tc<T, 32>(a, n, st); break;
+            case 16: e = launch_tc<T, 16>(a, n, st); break;
+            case 8: e = launch_tc<T, 8>(a, n, st); break;
+            case 4: e = launch_tc<T, 4>(a, n, st); break;
+            default: e = launch_tc<T, 2>(a, n, st); break;
+            }
+            if (e) return e;
+        }
+        if (which != PASS_L2L) {
+            const int b0 = O.chunk_box[c], b1 = O.chunk_box[c + 1];
+            const int S = which == PASS_M2L ? std::max(1, L.m2l_split) : 1;
+            own_reduce_kernel<T><<<ew_grid((size_t)(b1 - b0) * n2), 256, 0, st>>>(
+                b0, b1, n2, S, which == PASS_M2L && l > P->lmin, a.slot0, O.beg, (const C *)P->own_part, dst);
+            FMM_CUDA_TRY(cudaGetLastError());
+        }
+    }
+    return FMM_OK;
+}
+
+template <typename T> int slot_of_type() { return std::is_same<T, double>::value ? 0 : std::is_same<T, ff>::value ? 1 : 2; }
+
+// lists of every pass, folded tables and the scratch, on first use
+template <typename T>
+int ensure_own(Plan *P)
+{
+    const int ty = slot_of_type<T>();
+    if (P->own_ready[ty]) return FMM_OK;
+    if (!P->own_ncls) {
+        std::vector<int> cls, rep;
+        direction_classes(P, PASS_M2L, NDIR, cls, rep);
+        P->own_ncls = (int)rep.size();
+    }
+    if (Ops<T>::FOLD) {
+        const bool f64 = std::is_same<T, double>::value;
+        std::vector<int> reps, cls, rep;
+        for (int which : {PASS_M2L, PASS_M2M, PASS_L2L}) {
+            const int key0 = which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8;
+            direction_classes(P, which, which == PASS_M2L ? NDIR : 8, cls, rep);
+            for (int r : rep) reps.push_back(key0 + r);
+        }
+        const size_t n = reps.size() * (size_t)fold_size(P->pmax) + TABLE_PAD;
+        if (f64)
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot64, sizeof(double) * n));
+        else
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot_ff, sizeof(ffs) * n));
+        int *d_rep = nullptr;
+        FMM_CUDA_TRY(cudaMalloc(&d_rep, sizeof(int) * reps.size()));
+        cudaError_t ce = cudaMemcpyAsync(d_rep, reps.data(), sizeof(int) * reps.size(), cudaMemcpyHostToDevice, P->stream);
+        own_fold_table_kernel<<<dim3(P->pmax, (unsigned)reps.size()), 128, 0, P->stream>>>(
+            P->pmax, d_rep, P->Hsr64, f64 ? P->own_rot64 : nullptr, f64 ? nullptr : reinterpret_cast<ffs *>(P->own_rot_ff));
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(P->stream);
+        cudaFree(d_rep);
+        FMM_CUDA_TRY(ce);
+    }
+    size_t part = 0;
+    for (int l = P->lmin; l <= P->lmax; l++)
+        for (int which : {PASS_M2M, PASS_M2L, PASS_L2L}) {
+            if (which != PASS_M2L && l == P->lmin) continue;
+            OwnPass &O = P->own[ty][l][which];
+            int e = build_pass<T>(P, l, which, O);
+            if (e) return e;
+            part = std::max(part, O.part_bytes);
+        }
+    if (part > P->own_part_bytes) {
+        cudaFree(P->own_part);
+        P->own_part = nullptr;
+        P->device_bytes -= P->own_part_bytes;
+        P->own_part_bytes = 0;
+        FMM_CUDA_TRY(dev_alloc(P, &P->own_part, part));
+        P->own_part_bytes = part;
+    }
+    P->own_ready[ty] = 1;
+    return FMM_OK;
+}
+
+template <typename T>
+int translate(Plan *P, void (*beg)(Plan *, int, int), void (*end)(Plan *))
+{
+    const int ty = slot_of_type<T>();
+    int e = ensure_own<T>(P);
+    if (e) return e;
+    LevelDev &LL = P->lev[P->lmax];
+    cudaStream_t st = P->stream;
+    const size_t np = (size_t)LL.nb * LL.p * (LL.p + 1) / 2;
+    if (std::is_same<T, double>::value)
+        own_fold_kernel<<<ew_grid(np), 256, 0, st>>>(LL.Cm64, LL.nb, LL.p, 1);
+    else if (std::is_same<T, ff>::value)
+        own_fold_ff_kernel<<<ew_grid(np), 256, 0, st>>>(LL.Cm64, reinterpret_cast<ffv *>(LL.Cm_ff), LL.nb, LL.p, P->dsc_leaf_dev);
+    for (int l = P->lmax; l > P->lmin; l--) {
+        beg(P, PASS_M2M, l);
+        if ((e = run_pass<T>(P, l, PASS_M2M, P->own[ty][l][PASS_M2M]))) return e;
+        end(P);
+    }
+    for (int l = P->lmin; l <= P->lmax; l++) {
+        beg(P, PASS_M2L, l);
+        if (l > P->lmin && (e = run_pass<T>(P, l, PASS_L2L, P->own[ty][l][PASS_L2L]))) return e;
+        if ((e = run_pass<T>(P, l, PASS_M2L, P->own[ty][l][PASS_M2L]))) return e;
+        end(P);
+    }
+    if (std::is_same<T, double>::value)
+        own_fold_kernel<<<ew_grid(np), 256, 0, st>>>(LL.Dl64, LL.nb, LL.p, 0);
+    else if (std::is_same<T, ff>::value)
+        own_unfold_ff_kernel<<<ew_grid(np), 256, 0, st>>>(reinterpret_cast<const ffv *>(LL.Dl_ff), LL.Dl64, LL.nb, LL.p, P->dsc_leaf_dev);
+    FMM_CUDA_TRY(cudaGetLastError());
+    return FMM_OK;
+}
+
+} // namespace
+
+int translate_owner(Plan *P, int type, void (*beg)(Plan *, int, int), void (*end)(Plan *))
+{
+    return type == OWN_FP64 ? translate<double>(P, beg, end)
+                            : type == OWN_FF ? translate<ff>(P, beg, end) : translate<float>(P, beg, end);
+}
+
+void free_owner(Plan *P)
+{
+    for (auto &ty : P->own)
+        for (auto &lev : ty)
+            for (OwnPass &O : lev) {
+                cudaFree(O.items);
+                cudaFree(O.slot);
+                cudaFree(O.units);
+                cudaFree(O.src_own);
+                cudaFree(O.key_own);
+            }
+    cudaFree(P->own_part);
+    cudaFree(P->own_rot64);
+    cudaFree(P->own_rot_ff);
+}
+
+} // namespace fmm

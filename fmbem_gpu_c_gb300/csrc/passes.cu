@@ -1,18 +1,15 @@
-// The FMM matvec: P2M, M2M, M2L (+ fused L2L), L2P + near field.  Templated on the
-// arithmetic type: double for the plain path, float for the mixed-precision path, float-float
-// (ff.cuh) for the M2L of the FMM_FLOAT2 path.
+// The FMM matvec: P2M, translations, L2P + near field.  Templated on the arithmetic type: double
+// for the plain path, float for the mixed-precision path.
 //
 // Every translation is rotation - coaxial - rotation (RCR) as in the reference
 // (transMatsVecsMul_SR_rcr, translation.cu:1864-1961): rotate by (phi, theta, 0), apply the
 // coaxial blocks for |t|, rotate back by (0, theta, phi).  The rotation matrix is
 // e^{i m alpha} e^{-i m' gamma} H_n^{m'm}(beta) (translation.cu:1221-1235), so one real
 // table H per direction serves both rotations and the phases are applied elementwise.
-// The FP64 path is owner-computes: each destination box is owned by one CTA that accumulates
-// all its translations in shared memory and writes once (no atomics, bit-reproducible); on
-// levels with few boxes a box's sources are split over several CTAs whose partial sums are
-// added in a fixed order.
-// The mixed path runs the batched direction-grouped tiles of batched.cu, which add into the
-// expansions with FP32 atomics, so mixed results vary in the last bits from run to run.
+// The FP64 path, its float-float form (FMM_FLOAT2) and deterministic mixed plans run the
+// translations of owner.cu (no atomics, bit-reproducible).  The mixed path runs the batched
+// direction-grouped tiles of batched.cu, which add into the expansions with FP32 atomics, so
+// mixed results vary in the last bits from run to run.
 #include "plan.h"
 #include "ff.cuh"
 #include <algorithm>
@@ -22,12 +19,10 @@
 namespace fmm {
 
 __constant__ int c_dir_dist[NDIR];
-__constant__ int c_dir_hrep[NDIR]; // direction -> the direction whose (identical) rotation table it reads
 
 template <typename T> struct Cx;
 template <> struct Cx<double> { typedef double2 t; };
 template <> struct Cx<float> { typedef float2 t; };
-template <> struct Cx<ff> { typedef ff2 t; };
 
 __device__ __forceinline__ void decode_nm(int i, int &n, int &m)
 {
@@ -43,46 +38,33 @@ __device__ __forceinline__ double2 to_c(double2 v, double) { return v; }
 __device__ __forceinline__ double2 to_d(float2 v) { return make_double2(v.x, v.y); }
 __device__ __forceinline__ double2 to_d(double2 v) { return v; }
 
-// acc += a b: as written for FP32 and FP64 (contracted to an FMA), the fused float-float
-// multiply-add for ff
-template <typename T>
-__device__ __forceinline__ void mac(T &acc, T a, T b)
-{
-    if constexpr (std::is_same<T, ff>::value)
-        acc = ff_fma(a, b, acc);
-    else
-        acc += a * b;
-}
-
 // One RCR translation by a whole CTA.  x has pin^2 entries (zero padded to p); the result
 // for n < pout is accumulated into sY.  H and ph are the direction's real rotation table
 // (stride rot_size(pmax), prefix order p) and phases e^{i m phi} indexed m + pmax - 1.
-template <typename T>
-__device__ void rcr_block(int p, int pmax, const T *__restrict__ H, const typename Cx<T>::t *__restrict__ ph,
-                          const typename Cx<T>::t *__restrict__ Cc, const typename Cx<T>::t *__restrict__ xin, int pin,
-                          typename Cx<T>::t *sX, typename Cx<T>::t *sW1, typename Cx<T>::t *sW2,
-                          typename Cx<T>::t *sY, int pout)
+__device__ void rcr_block(int p, int pmax, const double *__restrict__ H, const double2 *__restrict__ ph,
+                          const double2 *__restrict__ Cc, const double2 *__restrict__ xin, int pin,
+                          double2 *sX, double2 *sW1, double2 *sW2,
+                          double2 *sY, int pout)
 {
-    typedef typename Cx<T>::t C;
     const int pp = p * p, pin2 = pin * pin, tid = threadIdx.x, nt = blockDim.x, off = pmax - 1;
     for (int i = tid; i < pp; i += nt) {
         int n, m;
         decode_nm(i, n, m);
-        C v = (i < pin2) ? xin[i] : mk2((T)0, (T)0);
+        double2 v = (i < pin2) ? xin[i] : mk2(0.0, 0.0);
         sX[i] = cmul(v, ph[m + off]);
     }
     __syncthreads();
     for (int i = tid; i < pp; i += nt) {
         int n, mp;
         decode_nm(i, n, mp);
-        const T *col = H + rot_off(n) + (mp + n);
+        const double *col = H + rot_off(n) + (mp + n);
         const int w = 2 * n + 1, base = n * n;
-        T ar = 0, ai = 0;
+        double ar = 0, ai = 0;
         for (int m = 0; m < w; m++) {
-            T h = col[m * w];
-            C v = sX[base + m];
-            mac(ar, h, v.x);
-            mac(ai, h, v.y);
+            double h = col[m * w];
+            double2 v = sX[base + m];
+            ar += h * v.x;
+            ai += h * v.y;
         }
         sW1[i] = mk2(ar, ai);
     }
@@ -91,20 +73,13 @@ __device__ void rcr_block(int p, int pmax, const T *__restrict__ H, const typena
         int np, m;
         decode_nm(i, np, m);
         int am = m < 0 ? -m : m, sz = p - am;
-        const C *col = Cc + coax_off(p, am) + (np - am);
-        T ar = 0, ai = 0;
+        const double2 *col = Cc + coax_off(p, am) + (np - am);
+        double ar = 0, ai = 0;
         for (int n = am; n < p; n++) {
-            C c = col[(n - am) * sz];
-            C v = sW1[n * n + n + m];
-            if constexpr (std::is_same<T, ff>::value) {
-                ar = ff_fma(c.x, v.x, ar);
-                ar = ff_fma(-c.y, v.y, ar);
-                ai = ff_fma(c.x, v.y, ai);
-                ai = ff_fma(c.y, v.x, ai);
-            } else {
-                ar += c.x * v.x - c.y * v.y;
-                ai += c.x * v.y + c.y * v.x;
-            }
+            double2 c = col[(n - am) * sz];
+            double2 v = sW1[n * n + n + m];
+            ar += c.x * v.x - c.y * v.y;
+            ai += c.x * v.y + c.y * v.x;
         }
         sW2[i] = mk2(ar, ai);
     }
@@ -113,18 +88,18 @@ __device__ void rcr_block(int p, int pmax, const T *__restrict__ H, const typena
     for (int i = tid; i < po2; i += nt) {
         int n, mp;
         decode_nm(i, n, mp);
-        const T *col = H + rot_off(n) + (mp + n);
+        const double *col = H + rot_off(n) + (mp + n);
         const int w = 2 * n + 1, base = n * n;
-        T ar = 0, ai = 0;
+        double ar = 0, ai = 0;
         for (int m = 0; m < w; m++) {
-            T h = col[m * w];
-            C v = sW2[base + m];
-            mac(ar, h, v.x);
-            mac(ai, h, v.y);
+            double h = col[m * w];
+            double2 v = sW2[base + m];
+            ar += h * v.x;
+            ai += h * v.y;
         }
-        C e = ph[mp + off];
+        double2 e = ph[mp + off];
         // conj(e) * (ar + i ai)
-        C y = sY[i];
+        double2 y = sY[i];
         y.x += e.x * ar + e.y * ai;
         y.y += e.x * ai - e.y * ar;
         sY[i] = y;
@@ -209,89 +184,11 @@ __global__ void p2m_kernel(int pl, const int *__restrict__ leaf_beg, const int *
     }
 }
 
-template <typename T>
-__global__ void m2m_kernel(int pp, int pc, int pmax, const int *__restrict__ child_beg, const int *__restrict__ child_list,
-                           const unsigned char *__restrict__ octant, const T *__restrict__ Hss,
-                           const typename Cx<T>::t *__restrict__ PHss, const typename Cx<T>::t *__restrict__ Crr,
-                           const typename Cx<T>::t *__restrict__ Cchild, typename Cx<T>::t *__restrict__ Cpar)
-{
-    typedef typename Cx<T>::t C;
-    extern __shared__ unsigned char smraw[];
-    C *sX = (C *)smraw;
-    int P2 = pp * pp;
-    C *sW1 = sX + P2, *sW2 = sW1 + P2, *sY = sW2 + P2;
-    int q = blockIdx.x, rs = rot_size(pmax), w = 2 * pmax - 1;
-    for (int i = threadIdx.x; i < P2; i += blockDim.x) sY[i] = mk2((T)0, (T)0);
-    __syncthreads();
-    for (int s = child_beg[q]; s < child_beg[q + 1]; s++) {
-        int ch = child_list[s], o = octant[ch];
-        rcr_block<T>(pp, pmax, Hss + (size_t)o * rs, PHss + (size_t)o * w, Crr, Cchild + (size_t)ch * pc * pc, pc,
-                     sX, sW1, sW2, sY, pp);
-    }
-    for (int i = threadIdx.x; i < P2; i += blockDim.x) Cpar[(size_t)q * P2 + i] = sY[i];
-}
-
 __global__ void to_float_kernel2(const double *in, float *out, size_t n)
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = (float)in[i];
 }
-
-template <typename T>
-__global__ void m2l_kernel(int p, int pmax, int pp, const int *__restrict__ sr_beg, const int *__restrict__ sr_src,
-                           const short *__restrict__ sr_dir, const T *__restrict__ Hsr,
-                           const typename Cx<T>::t *__restrict__ PHsr, const typename Cx<T>::t *__restrict__ Csr,
-                           const typename Cx<T>::t *__restrict__ Cm, const int *__restrict__ parent,
-                           const unsigned char *__restrict__ octant, const T *__restrict__ Hrr,
-                           const typename Cx<T>::t *__restrict__ PHrr, const typename Cx<T>::t *__restrict__ Crr,
-                           const typename Cx<T>::t *__restrict__ Dpar, typename Cx<T>::t *__restrict__ Dl,
-                           typename Cx<T>::t *__restrict__ part)
-{
-    typedef typename Cx<T>::t C;
-    extern __shared__ unsigned char smraw[];
-    int pe = pp > p ? pp : p, E2 = pe * pe, P2 = p * p;
-    C *sX = (C *)smraw;
-    C *sW1 = sX + E2, *sW2 = sW1 + E2, *sY = sW2 + E2;
-    int b = blockIdx.x, rs = rot_size(pmax), w = 2 * pmax - 1, cs = coax_size(p);
-    // owner-computes: the L2L from the parent and every M2L source, accumulated in shared
-    // memory and written once.  With gridDim.y = S > 1 (levels with few boxes), CTA (b, c)
-    // takes the c-th of S runs of box b's sources (run 0 also the L2L) and writes its partial
-    // sum to part[c][b]; m2l_reduce_kernel adds the runs in order.
-    const int S = gridDim.y, c = blockIdx.y, s0 = sr_beg[b], ns = sr_beg[b + 1] - s0;
-    const int sa = s0 + (int)((long long)ns * c / S), sb = s0 + (int)((long long)ns * (c + 1) / S);
-    for (int i = threadIdx.x; i < P2; i += blockDim.x) sY[i] = mk2((T)0, (T)0);
-    __syncthreads();
-    if (pp > 0 && c == 0) {
-        // L2L: parent local (order pp) translated to this box, truncated to p
-        int o = octant[b];
-        rcr_block<T>(pp, pmax, Hrr + (size_t)o * rs, PHrr + (size_t)o * w, Crr, Dpar + (size_t)parent[b] * pp * pp, pp,
-                     sX, sW1, sW2, sY, p);
-    }
-    for (int s = sa; s < sb; s++) {
-        int src = sr_src[s], dir = sr_dir[s];
-        rcr_block<T>(p, pmax, Hsr + (size_t)c_dir_hrep[dir] * rs, PHsr + (size_t)dir * w, Csr + (size_t)c_dir_dist[dir] * cs,
-                     Cm + (size_t)src * P2, p, sX, sW1, sW2, sY, p);
-    }
-    C *out = S > 1 ? part + ((size_t)c * gridDim.x + b) * P2 : Dl + (size_t)b * P2;
-    for (int i = threadIdx.x; i < P2; i += blockDim.x) out[i] = sY[i];
-}
-
-// Dl[b] = sum over c of part[c][b], c in order (the result does not depend on the schedule)
-template <typename T>
-__global__ void m2l_reduce_kernel(int S, size_t n, const typename Cx<T>::t *__restrict__ part, typename Cx<T>::t *__restrict__ Dl)
-{
-    typedef typename Cx<T>::t C;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        C a = part[i];
-        for (int c = 1; c < S; c++) {
-            C v = part[(size_t)c * n + i];
-            a.x += v.x;
-            a.y += v.y;
-        }
-        Dl[i] = a;
-    }
-}
-
 
 // L2P + near field + identity for element e (one warp) and a group of up to G right-hand sides
 // (blockIdx.y): the near row and the element's basis are loaded once for the group, the x
@@ -368,8 +265,6 @@ __global__ void l2p_near_kernel(int nf, int pl, const int *__restrict__ elem_lea
     }
 }
 
-static inline int block_for(int p) { return p >= 16 ? 256 : 128; }
-
 static void timer_begin(Plan *P, const char *name, cudaStream_t st = nullptr)
 {
     if (P->profiling != 1 || P->ntimers >= MAX_TIMERS) return;
@@ -384,65 +279,17 @@ static void timer_end(Plan *P, cudaStream_t st = nullptr)
     P->ntimers++;
 }
 
-// Raise the dynamic shared-memory limit of the owner-computes translation kernels to what
-// order pmax needs (4 p^2 complex for the CTA-level RCR).
-template <typename T>
-static int set_smem_attrs(int pmax)
-{
-    typedef typename Cx<T>::t C;
-    static size_t m2m_set = 0, m2l_set = 0;
-    size_t smax = 4 * (size_t)pmax * pmax * sizeof(C);
-    int st = raise_smem_limit((const void *)m2m_kernel<T>, smax, &m2m_set);
-    if (st) return st;
-    return raise_smem_limit((const void *)m2l_kernel<T>, smax, &m2l_set);
-}
+static const char *pass_names[3][14] = {
+    {"m2m_l0", "m2m_l1", "m2m_l2", "m2m_l3", "m2m_l4", "m2m_l5", "m2m_l6", "m2m_l7", "m2m_l8", "m2m_l9", "m2m_l10",
+     "m2m_l11", "m2m_l12", "m2m_l13"},
+    {"m2l_l0", "m2l_l1", "m2l_l2", "m2l_l3", "m2l_l4", "m2l_l5", "m2l_l6", "m2l_l7", "m2l_l8", "m2l_l9", "m2l_l10",
+     "m2l_l11", "m2l_l12", "m2l_l13"},
+    {"l2l_l0", "l2l_l1", "l2l_l2", "l2l_l3", "l2l_l4", "l2l_l5", "l2l_l6", "l2l_l7", "l2l_l8", "l2l_l9", "l2l_l10",
+     "l2l_l11", "l2l_l12", "l2l_l13"}};
+static void pass_begin(Plan *P, int which, int l) { timer_begin(P, pass_names[which][l]); }
+static void pass_end(Plan *P) { timer_end(P); }
 
-template <typename T>
-static int launch_m2l_level(Plan *P, int l, const char *tname)
-{
-    typedef typename Cx<T>::t C;
-    const bool f64 = sizeof(T) == 8;
-    int lmin = P->lmin, pmax = P->pmax;
-    cudaStream_t st = P->stream;
-    LevelDev &L = P->lev[l];
-    const T *Hsr = f64 ? (const T *)P->Hsr64 : (const T *)P->Hsr32;
-    const T *Hrr = f64 ? (const T *)P->Hrr64 : (const T *)P->Hrr32;
-    const C *PHsr = f64 ? (const C *)P->PHsr64 : (const C *)P->PHsr32;
-    const C *PHrr = f64 ? (const C *)P->PHrr64 : (const C *)P->PHrr32;
-    const C *Csr = f64 ? (const C *)L.Csr64 : (const C *)L.Csr32;
-    // the fused L2L: FP64, or the FP32 table scaled for L2L (plans with scaled expansions)
-    const C *Crr = l > lmin ? (f64 ? (const C *)L.Crr64 : (const C *)(L.Crr32L ? L.Crr32L : L.Crr32)) : nullptr;
-    const C *Cm = f64 ? (const C *)L.Cm64 : (const C *)L.Cm32;
-    C *Dl = f64 ? (C *)L.Dl64 : (C *)L.Dl32;
-    const C *Dpar = l > lmin ? (f64 ? (const C *)P->lev[l - 1].Dl64 : (const C *)P->lev[l - 1].Dl32) : nullptr;
-    int pp = l > lmin ? P->lev[l - 1].p : 0;
-    int pe = pp > L.p ? pp : L.p;
-    size_t sm = 4 * (size_t)pe * pe * sizeof(C);
-    timer_begin(P, tname);
-    // levels with few boxes split each box's sources over S CTAs (P->m2l_split, sized at plan
-    // creation so that the level fills the GPU) and add the runs in a second pass
-    const int S = std::max(1, L.m2l_split);
-    C *part = S > 1 ? (C *)P->m2l_part64 : nullptr;
-    m2l_kernel<T><<<dim3(L.nb, S), block_for(pe), sm, st>>>(L.p, pmax, pp, L.sr_beg, L.sr_src, L.sr_dir, Hsr, PHsr, Csr,
-                                                              Cm, L.parent, L.octant, Hrr, PHrr, Crr, Dpar, Dl, part);
-    if (S > 1) {
-        size_t n = (size_t)L.nb * L.p * L.p;
-        int blocks = (int)std::min<size_t>((n + 255) / 256, 152 * 8);
-        m2l_reduce_kernel<T><<<blocks, 256, 0, st>>>(S, n, part, Dl);
-    }
-    timer_end(P);
-    FMM_CUDA_TRY(cudaGetLastError());
-    return FMM_OK;
-}
-
-// ---------------------------------------------------------------- float-float M2L (FMM_FLOAT2)
-__global__ void ff_from_real_kernel(const double *__restrict__ in, float2 *__restrict__ out, size_t n)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const ff a = ff_from(in[i]);
-        out[i] = make_float2(a.hi, a.lo);
-    }
-}
+// ---------------------------------------------------------------- float-float tables (FMM_FLOAT2)
 __global__ void ff_from_cplx_kernel(const double2 *__restrict__ in, float4 *__restrict__ out, size_t n)
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -450,59 +297,27 @@ __global__ void ff_from_cplx_kernel(const double2 *__restrict__ in, float4 *__re
         out[i] = make_float4(a.hi, a.lo, b.hi, b.lo);
     }
 }
-__global__ void ff_to_cplx_kernel(const float4 *__restrict__ in, double2 *__restrict__ out, size_t n)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 v = in[i];
-        out[i] = make_double2(ff_to(ff(v.x, v.y)), ff_to(ff(v.z, v.w)));
-    }
-}
-// the same for expansions [box][p^2] kept scaled by degree: entry i times ds[degree of i % ppl]
-__global__ void ff_from_cplx_deg_kernel(const double2 *__restrict__ in, float4 *__restrict__ out, size_t n, int ppl,
-                                        const double *__restrict__ ds)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        int deg, m;
-        decode_nm((int)(i % ppl), deg, m);
-        const double f = ds[deg];
-        const ff a = ff_from(in[i].x * f), b = ff_from(in[i].y * f);
-        out[i] = make_float4(a.hi, a.lo, b.hi, b.lo);
-    }
-}
-__global__ void ff_to_cplx_deg_kernel(const float4 *__restrict__ in, double2 *__restrict__ out, size_t n, int ppl,
-                                      const double *__restrict__ ds)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        int deg, m;
-        decode_nm((int)(i % ppl), deg, m);
-        const double f = ds[deg];
-        const float4 v = in[i];
-        out[i] = make_double2(ff_to(ff(v.x, v.y)) * f, ff_to(ff(v.z, v.w)) * f);
-    }
-}
 static unsigned ew_grid(size_t n) { return (unsigned)std::min<size_t>((n + 255) / 256, 152 * 16); }
 
-// nmat coaxial tables of order p (the layout of coax_off: block m, entry (n', n) at
-// (n - m)(p - m) + n' - m) with rows times row[n'] and columns times col[n], in float-float
-static std::vector<float4> ff_scaled_coax(const std::vector<double2> &in, int p, int nmat, const std::vector<double> &row,
-                                          const std::vector<double> &col)
+// coaxial tables of order p (layout of coax_off; blockIdx.x = m, blockIdx.y = table) in
+// float-float, every part twice (the operands of the packed instructions in owner.cu): two
+// float4 per entry, (re hi, re hi, re lo, re lo) and the same of im; rows times row[n'] and
+// columns times col[n] where given
+__global__ void ff_coax_kernel(const double2 *__restrict__ in, float4 *__restrict__ out, int p, const double *__restrict__ row,
+                               const double *__restrict__ col)
 {
-    std::vector<float4> out(in.size());
-    const int cs = coax_size(p);
-    for (int q = 0; q < nmat; q++)
-        for (int m = 0; m < p; m++) {
-            const int sz = p - m, off = q * cs + coax_off(p, m);
-            for (int i = 0; i < sz * sz; i++) {
-                const int a = i % sz, b = i / sz;
-                const double f = row[m + a] * col[m + b], x = in[off + i].x * f, y = in[off + i].y * f;
-                const float xh = (float)x, yh = (float)y;
-                out[off + i] = make_float4(xh, (float)(x - (double)xh), yh, (float)(y - (double)yh));
-            }
-        }
-    return out;
+    const int m = blockIdx.x, sz = p - m;
+    const size_t off = (size_t)blockIdx.y * coax_size(p) + coax_off(p, m);
+    for (int i = threadIdx.x; i < sz * sz; i += blockDim.x) {
+        const double f = row ? row[m + i % sz] * col[m + i / sz] : 1.0;
+        const double2 c = in[off + i];
+        const ff x = ff_from(c.x * f), y = ff_from(c.y * f);
+        out[2 * (off + i)] = make_float4(x.hi, x.hi, x.lo, x.lo);
+        out[2 * (off + i) + 1] = make_float4(y.hi, y.hi, y.lo, y.lo);
+    }
 }
 
-// The float-float copies of the translation tables (rotations, phases, coaxial blocks) and
+// The float-float copies of the translation tables (phases, coaxial blocks; the rotations: owner.cu) and
 // the expansions, made on first use.  Where the FP32 mixed tables are built, the FP32 exponent
 // range holds them: plain, or scaled by degree as the FP32 ones (multipoles d_n M_n, locals
 // L_n / d_n, the coaxial tables scaled to match, the leaf expansions scaled on the way in and
@@ -514,49 +329,54 @@ static int ensure_ff(Plan *P)
         P->ff_ready = -1;
         return FMM_OK;
     }
-    const int pmax = P->pmax, rs = rot_size(pmax), w = 2 * pmax - 1;
-    const size_t nh = (size_t)(NDIR + 16) * rs, nph = (size_t)(NDIR + 16) * w;
-    FMM_CUDA_TRY(dev_alloc(P, (void **)&P->Hall_ff, sizeof(float2) * nh));
+    const size_t nph = (size_t)(NDIR + 16) * (2 * P->pmax - 1);
     FMM_CUDA_TRY(dev_alloc(P, (void **)&P->PHall_ff, sizeof(float4) * nph));
-    ff_from_real_kernel<<<ew_grid(nh), 256, 0, P->stream>>>(P->Hsr64, P->Hall_ff, nh);
     ff_from_cplx_kernel<<<ew_grid(nph), 256, 0, P->stream>>>(P->PHsr64, P->PHall_ff, nph);
-    for (int l = P->lmin; l <= P->lmax; l++) {
-        LevelDev &L = P->lev[l];
-        const size_t ncs = (size_t)NDIST * coax_size(L.p), ne = (size_t)L.nb * L.p * L.p;
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Csr_ff, sizeof(float4) * ncs));
-        if (l > P->lmin) FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Crr_ff, sizeof(float4) * coax_size(P->lev[l - 1].p)));
-        if (!P->scaled) {
-            ff_from_cplx_kernel<<<ew_grid(ncs), 256, 0, P->stream>>>(L.Csr64, L.Csr_ff, ncs);
-            if (l > P->lmin)
-                ff_from_cplx_kernel<<<ew_grid(coax_size(P->lev[l - 1].p)), 256, 0, P->stream>>>(
-                    L.Crr64, L.Crr_ff, coax_size(P->lev[l - 1].p));
-        } else {
-            // the scalings of the FP32 tables (gen_coax_tables): M2L 1/d^l both sides; M2M rows
-            // d^{l-1}, columns 1/d^l below the child order (0 above); L2L rows 1/d^l below the
-            // child order (0 above), columns d^{l-1}
-            const int pall = (int)P->dsc[l].size();
-            std::vector<double> inv(pall), up(pall, 0.0), down(pall, 0.0);
-            for (int n = 0; n < pall; n++) inv[n] = 1.0 / P->dsc[l][n];
-            for (int n = 0; n < L.p && n < pall; n++) up[n] = down[n] = inv[n];
-            std::vector<double2> h(ncs);
-            FMM_CUDA_TRY(cudaMemcpy(h.data(), L.Csr64, sizeof(double2) * ncs, cudaMemcpyDeviceToHost));
-            std::vector<float4> f = ff_scaled_coax(h, L.p, NDIST, inv, inv);
-            FMM_CUDA_TRY(cudaMemcpy(L.Csr_ff, f.data(), sizeof(float4) * ncs, cudaMemcpyHostToDevice));
+    // the scalings of the FP32 tables (gen_coax_tables): M2L 1/d^l both sides; M2M rows d^{l-1},
+    // columns 1/d^l below the child order (0 above); L2L rows 1/d^l below the child order (0
+    // above), columns d^{l-1}; per level on the device: d, 1/d, and 1/d below the level's order
+    std::vector<double> sc;
+    std::vector<size_t> sc_at(P->lmax + 1, 0);
+    double *dsc = nullptr;
+    if (P->scaled) {
+        for (int l = P->lmin; l <= P->lmax; l++) {
+            const std::vector<double> &d = P->dsc[l];
+            sc_at[l] = sc.size();
+            sc.insert(sc.end(), d.begin(), d.end());
+            for (double v : d) sc.push_back(1.0 / v);
+            for (int n = 0; n < (int)d.size(); n++) sc.push_back(n < P->lev[l].p ? 1.0 / d[n] : 0.0);
+        }
+        FMM_CUDA_TRY(cudaMalloc(&dsc, sizeof(double) * sc.size()));
+    }
+    auto tables = [&]() -> int {
+        if (dsc) FMM_CUDA_TRY(cudaMemcpyAsync(dsc, sc.data(), sizeof(double) * sc.size(), cudaMemcpyHostToDevice, P->stream));
+        for (int l = P->lmin; l <= P->lmax; l++) {
+            LevelDev &L = P->lev[l];
+            const size_t ne = (size_t)L.nb * L.p * L.p;
+            const double *d = dsc ? dsc + sc_at[l] : nullptr, *inv = dsc ? d + P->dsc[l].size() : nullptr;
+            const double *cut = dsc ? inv + P->dsc[l].size() : nullptr;
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Csr_ff, 2 * sizeof(float4) * (NDIST * coax_size(L.p) + TABLE_PAD)));
+            ff_coax_kernel<<<dim3(L.p, NDIST), 128, 0, P->stream>>>(L.Csr64, L.Csr_ff, L.p, inv, inv);
             if (l > P->lmin) {
                 const int pp = P->lev[l - 1].p;
-                const size_t nrr = coax_size(pp);
-                h.resize(nrr);
-                FMM_CUDA_TRY(cudaMemcpy(h.data(), L.Crr64, sizeof(double2) * nrr, cudaMemcpyDeviceToHost));
-                f = ff_scaled_coax(h, pp, 1, P->dsc[l - 1], up);
-                FMM_CUDA_TRY(cudaMemcpy(L.Crr_ff, f.data(), sizeof(float4) * nrr, cudaMemcpyHostToDevice));
-                f = ff_scaled_coax(h, pp, 1, down, P->dsc[l - 1]);
-                FMM_CUDA_TRY(dev_alloc(P, (void **)&L.CrrL_ff, sizeof(float4) * nrr));
-                FMM_CUDA_TRY(cudaMemcpy(L.CrrL_ff, f.data(), sizeof(float4) * nrr, cudaMemcpyHostToDevice));
+                const double *dp = dsc ? dsc + sc_at[l - 1] : nullptr;
+                FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Crr_ff, 2 * sizeof(float4) * (coax_size(pp) + TABLE_PAD)));
+                ff_coax_kernel<<<dim3(pp, 1), 128, 0, P->stream>>>(L.Crr64, L.Crr_ff, pp, dp, cut);
+                if (dsc) {
+                    FMM_CUDA_TRY(dev_alloc(P, (void **)&L.CrrL_ff, 2 * sizeof(float4) * (coax_size(pp) + TABLE_PAD)));
+                    ff_coax_kernel<<<dim3(pp, 1), 128, 0, P->stream>>>(L.Crr64, L.CrrL_ff, pp, cut, dp);
+                }
             }
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Cm_ff, sizeof(float4) * ne));
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Dl_ff, sizeof(float4) * ne));
         }
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Cm_ff, sizeof(float4) * ne));
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Dl_ff, sizeof(float4) * ne));
-    }
+        FMM_CUDA_TRY(cudaGetLastError());
+        FMM_CUDA_TRY(cudaStreamSynchronize(P->stream));
+        return FMM_OK;
+    };
+    const int rc = tables();
+    cudaFree(dsc);
+    if (rc) return rc;
     if (P->scaled) {
         const std::vector<double> &d = P->dsc[P->lmax];
         FMM_CUDA_TRY(dev_alloc(P, (void **)&P->dsc_leaf_dev, sizeof(double) * d.size()));
@@ -564,61 +384,6 @@ static int ensure_ff(Plan *P)
     }
     FMM_CUDA_TRY(cudaGetLastError());
     P->ff_ready = 1;
-    return FMM_OK;
-}
-
-// The M2M of level l into level l - 1 in float-float (the parent-owned m2m_kernel).
-static int launch_m2m_level_ff(Plan *P, int l, const char *tname)
-{
-    static size_t m2m_set = 0;
-    const int pmax = P->pmax, rs = rot_size(pmax), w = 2 * pmax - 1;
-    int e = raise_smem_limit((const void *)m2m_kernel<ff>, 4 * (size_t)pmax * pmax * sizeof(ff2), &m2m_set);
-    if (e) return e;
-    LevelDev &L = P->lev[l], &PL = P->lev[l - 1];
-    const ff *Hss = reinterpret_cast<const ff *>(P->Hall_ff) + (size_t)NDIR * rs;
-    const ff2 *PHss = reinterpret_cast<const ff2 *>(P->PHall_ff) + (size_t)NDIR * w;
-    const size_t sm = 4 * (size_t)PL.p * PL.p * sizeof(ff2);
-    timer_begin(P, tname);
-    m2m_kernel<ff><<<PL.nb, block_for(PL.p), sm, P->stream>>>(
-        PL.p, L.p, pmax, PL.child_beg, PL.child_list, L.octant, Hss, PHss, reinterpret_cast<const ff2 *>(L.Crr_ff),
-        reinterpret_cast<const ff2 *>(L.Cm_ff), reinterpret_cast<ff2 *>(PL.Cm_ff));
-    timer_end(P);
-    FMM_CUDA_TRY(cudaGetLastError());
-    return FMM_OK;
-}
-
-// The M2L (+ fused L2L) of level l in float-float: the owner-computes m2l_kernel on the
-// float-float tables and expansions.
-static int launch_m2l_level_ff(Plan *P, int l, const char *tname)
-{
-    static size_t m2l_set = 0;
-    const int lmin = P->lmin, pmax = P->pmax, rs = rot_size(pmax), w = 2 * pmax - 1;
-    int e = raise_smem_limit((const void *)m2l_kernel<ff>, 4 * (size_t)pmax * pmax * sizeof(ff2), &m2l_set);
-    if (e) return e;
-    cudaStream_t st = P->stream;
-    LevelDev &L = P->lev[l];
-    const ff *Hall = reinterpret_cast<const ff *>(P->Hall_ff);
-    const ff2 *PHall = reinterpret_cast<const ff2 *>(P->PHall_ff);
-    const ff *Hsr = Hall, *Hrr = Hall + (size_t)(NDIR + 8) * rs;
-    const ff2 *PHsr = PHall, *PHrr = PHall + (size_t)(NDIR + 8) * w;
-    const ff2 *Csr = reinterpret_cast<const ff2 *>(L.Csr_ff);
-    const ff2 *Crr = l > lmin ? reinterpret_cast<const ff2 *>(L.CrrL_ff ? L.CrrL_ff : L.Crr_ff) : nullptr;
-    const ff2 *Cm = reinterpret_cast<const ff2 *>(L.Cm_ff);
-    ff2 *Dl = reinterpret_cast<ff2 *>(L.Dl_ff);
-    const ff2 *Dpar = l > lmin ? reinterpret_cast<const ff2 *>(P->lev[l - 1].Dl_ff) : nullptr;
-    const int pp = l > lmin ? P->lev[l - 1].p : 0, pe = pp > L.p ? pp : L.p;
-    const size_t sm = 4 * (size_t)pe * pe * sizeof(ff2);
-    timer_begin(P, tname);
-    const int S = std::max(1, L.m2l_split);
-    ff2 *part = S > 1 ? reinterpret_cast<ff2 *>(P->m2l_part64) : nullptr;
-    m2l_kernel<ff><<<dim3(L.nb, S), block_for(pe), sm, st>>>(L.p, pmax, pp, L.sr_beg, L.sr_src, L.sr_dir, Hsr, PHsr, Csr,
-                                                               Cm, L.parent, L.octant, Hrr, PHrr, Crr, Dpar, Dl, part);
-    if (S > 1) {
-        const size_t n = (size_t)L.nb * L.p * L.p;
-        m2l_reduce_kernel<ff><<<(int)std::min<size_t>((n + 255) / 256, 152 * 8), 256, 0, st>>>(S, n, part, Dl);
-    }
-    timer_end(P);
-    FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
 
@@ -692,19 +457,13 @@ static int translate32_direct(Plan *P, int nrhs)
         cudaEventRecord(P->phase.beg, st);
         P->have_phase = 1;
     }
-    static const char *m2m_names[] = {"m2m_l0", "m2m_l1", "m2m_l2", "m2m_l3", "m2m_l4", "m2m_l5", "m2m_l6",
-                                      "m2m_l7", "m2m_l8", "m2m_l9", "m2m_l10", "m2m_l11", "m2m_l12", "m2m_l13"};
-    static const char *m2l_names[] = {"m2l_l0", "m2l_l1", "m2l_l2", "m2l_l3", "m2l_l4", "m2l_l5", "m2l_l6",
-                                      "m2l_l7", "m2l_l8", "m2l_l9", "m2l_l10", "m2l_l11", "m2l_l12", "m2l_l13"};
-    static const char *l2l_names[] = {"l2l_l0", "l2l_l1", "l2l_l2", "l2l_l3", "l2l_l4", "l2l_l5", "l2l_l6",
-                                      "l2l_l7", "l2l_l8", "l2l_l9", "l2l_l10", "l2l_l11", "l2l_l12", "l2l_l13"};
     for (int l = lmin; l <= lmax; l++) {
         size_t n = (size_t)P->lev[l].nb * P->lev[l].p * P->lev[l].p * sizeof(float2) * nrhs;
         if (l < lmax) FMM_CUDA_TRY(cudaMemsetAsync(P->lev[l].Cm32, 0, n, st));
         FMM_CUDA_TRY(cudaMemsetAsync(P->lev[l].Dl32, 0, n, st));
     }
     for (int l = lmax; l > lmin; l--) {
-        timer_begin(P, m2m_names[l]);
+        timer_begin(P, pass_names[PASS_M2M][l]);
         int e = launch_pass32(P, l, PASS_M2M, nrhs, st);
         if (e) return e;
         timer_end(P);
@@ -715,7 +474,7 @@ static int translate32_direct(Plan *P, int nrhs)
     for (int i = 0; i < P->nside; i++) FMM_CUDA_TRY(cudaStreamWaitEvent(P->side[i], P->fork_ev, 0));
     for (int l = lmin; l <= lmax; l++) {
         cudaStream_t sl = P->side[(l - lmin) % P->nside];
-        timer_begin(P, m2l_names[l], sl);
+        timer_begin(P, pass_names[PASS_M2L][l], sl);
         int e = launch_pass32(P, l, PASS_M2L, nrhs, sl);
         if (e) return e;
         timer_end(P, sl);
@@ -726,7 +485,7 @@ static int translate32_direct(Plan *P, int nrhs)
     FMM_CUDA_TRY(cudaStreamWaitEvent(st, P->m2l_ev[lmin], 0));
     for (int l = lmin + 1; l <= lmax; l++) {
         FMM_CUDA_TRY(cudaStreamWaitEvent(st, P->m2l_ev[l], 0));
-        timer_begin(P, l2l_names[l]);
+        timer_begin(P, pass_names[PASS_L2L][l]);
         int e = launch_pass32(P, l, PASS_L2L, nrhs, st);
         if (e) return e;
         timer_end(P);
@@ -787,7 +546,7 @@ static int translate32(Plan *P, int nrhs)
     return FMM_OK;
 }
 
-// ffm2l (T = double only): the M2L and its fused L2L in float-float (FMM_FLOAT2)
+// ffm2l (T = double only): the translations in float-float (FMM_FLOAT2)
 template <typename T>
 static int run_matvec_t(Plan *P, const double2 *x, double2 *y, int transpose, int nrhs, bool ffm2l = false)
 {
@@ -795,26 +554,14 @@ static int run_matvec_t(Plan *P, const double2 *x, double2 *y, int transpose, in
     const bool f64 = sizeof(T) == 8;
     // owner-computes translations: the FP64 path, and the mixed path of deterministic plans
     const bool owner = f64 || P->opt.deterministic;
-    int lmin = P->lmin, lmax = P->lmax, pmax = P->pmax;
+    const int lmax = P->lmax;
     cudaStream_t st = P->stream;
-    {
-        int st = set_smem_attrs<T>(pmax);
-        if (st) return st;
-    }
     P->ntimers = 0;
     P->have_total = 0;
     P->have_phase = 0;
     if (P->profiling) cudaEventRecord(P->total.beg, st);
-    const T *Hsr = f64 ? (const T *)P->Hsr64 : (const T *)P->Hsr32;
-    const T *Hss = f64 ? (const T *)P->Hss64 : (const T *)P->Hss32;
-    const T *Hrr = f64 ? (const T *)P->Hrr64 : (const T *)P->Hrr32;
-    const C *PHsr = f64 ? (const C *)P->PHsr64 : (const C *)P->PHsr32;
-    const C *PHss = f64 ? (const C *)P->PHss64 : (const C *)P->PHss32;
-    const C *PHrr = f64 ? (const C *)P->PHrr64 : (const C *)P->PHrr32;
     auto Cm = [&](int l) { return f64 ? (C *)P->lev[l].Cm64 : (C *)P->lev[l].Cm32; };
     auto Dl = [&](int l) { return f64 ? (C *)P->lev[l].Dl64 : (C *)P->lev[l].Dl32; };
-    auto Csr = [&](int l) { return f64 ? (const C *)P->lev[l].Csr64 : (const C *)P->lev[l].Csr32; };
-    auto Crr = [&](int l) { return f64 ? (const C *)P->lev[l].Crr64 : (const C *)P->lev[l].Crr32; };
     const C *U = f64 ? (const C *)P->U64 : (const C *)P->U32;
     const C *Rv = f64 ? (const C *)P->Rv64 : (const C *)P->Rv32;
     const C *nearv = f64 ? (const C *)P->near64 : (const C *)P->near32;
@@ -825,10 +572,6 @@ static int run_matvec_t(Plan *P, const double2 *x, double2 *y, int transpose, in
         return FMM_ERR_CUDA;
     }
 
-    static const char *m2m_names[] = {"m2m_l0", "m2m_l1", "m2m_l2", "m2m_l3", "m2m_l4", "m2m_l5", "m2m_l6",
-                                      "m2m_l7", "m2m_l8", "m2m_l9", "m2m_l10", "m2m_l11", "m2m_l12", "m2m_l13"};
-    static const char *m2l_names[] = {"m2l_l0", "m2l_l1", "m2l_l2", "m2l_l3", "m2l_l4", "m2l_l5", "m2l_l6",
-                                      "m2l_l7", "m2l_l8", "m2l_l9", "m2l_l10", "m2l_l11", "m2l_l12", "m2l_l13"};
     timer_begin(P, "p2m");
     // the transposed operator swaps the roles of the element moments and the centroid basis
     // (index-flipped), keeps every translation, and uses the transposed near-field matrix
@@ -839,45 +582,9 @@ static int run_matvec_t(Plan *P, const double2 *x, double2 *y, int transpose, in
         p2m_kernel<T, 8><<<dim3(LL.nb, (nrhs + 7) / 8), 128, 0, st>>>(LL.p, P->leaf_beg, P->leaf_elem, transpose ? Rv : U, x,
                                                                    P->opt.k, Cm(lmax), transpose, P->nf, LL.nb, nrhs, x32);
     timer_end(P);
-    if (!owner) {
-        int e = translate32(P, nrhs);
+    {
+        int e = owner ? translate_owner(P, ffm2l ? OWN_FF : f64 ? OWN_FP64 : OWN_FP32, pass_begin, pass_end) : translate32(P, nrhs);
         if (e) return e;
-    }
-    for (int l = lmax; l > lmin && owner && !ffm2l; l--) {
-        LevelDev &L = P->lev[l], &PL = P->lev[l - 1];
-        size_t sm = 4 * (size_t)PL.p * PL.p * sizeof(C);
-        timer_begin(P, m2m_names[l]);
-        m2m_kernel<T><<<PL.nb, block_for(PL.p), sm, st>>>(PL.p, L.p, pmax, PL.child_beg, PL.child_list, L.octant, Hss,
-                                                           PHss, Crr(l), Cm(l), Cm(l - 1));
-        timer_end(P);
-    }
-    if (f64 && ffm2l) {
-        // the leaf multipoles into float-float; M2M, M2L and L2L in float-float; the leaf locals
-        // back to FP64 for L2P
-        {
-            const size_t n = (size_t)LL.nb * LL.p * LL.p;
-            if (P->dsc_leaf_dev)
-                ff_from_cplx_deg_kernel<<<ew_grid(n), 256, 0, st>>>(LL.Cm64, LL.Cm_ff, n, LL.p * LL.p, P->dsc_leaf_dev);
-            else
-                ff_from_cplx_kernel<<<ew_grid(n), 256, 0, st>>>(LL.Cm64, LL.Cm_ff, n);
-        }
-        for (int l = lmax; l > lmin; l--) {
-            int st = launch_m2m_level_ff(P, l, m2m_names[l]);
-            if (st) return st;
-        }
-        for (int l = lmin; l <= lmax; l++) {
-            int st = launch_m2l_level_ff(P, l, m2l_names[l]);
-            if (st) return st;
-        }
-        const size_t n = (size_t)LL.nb * LL.p * LL.p;
-        if (P->dsc_leaf_dev)
-            ff_to_cplx_deg_kernel<<<ew_grid(n), 256, 0, st>>>(LL.Dl_ff, LL.Dl64, n, LL.p * LL.p, P->dsc_leaf_dev);
-        else
-            ff_to_cplx_kernel<<<ew_grid(n), 256, 0, st>>>(LL.Dl_ff, LL.Dl64, n);
-    }
-    for (int l = lmin; l <= lmax && owner && !ffm2l; l++) {
-        int st = launch_m2l_level<T>(P, l, m2l_names[l]);
-        if (st) return st;
     }
     timer_begin(P, "l2p_near");
     double2 a = make_double2(P->opt.a_re, P->opt.a_im);
@@ -923,7 +630,7 @@ __global__ void dense_rcr_kernel(int p, int pmax, int pin, int pout, const int *
     for (int i = threadIdx.x; i < w; i += blockDim.x) sOne[i] = make_double2(1.0, 0.0);
     __syncthreads();
     const double2 *cb = Cc + (coax_per_dir ? (size_t)c_dir_dist[d] * coax_size(p) : 0);
-    rcr_block<double>(p, pmax, H + (size_t)d * rs, PH ? PH + (size_t)d * w : sOne, cb, sE, pin, sX, sW1, sW2, sY, pout);
+    rcr_block(p, pmax, H + (size_t)d * rs, PH ? PH + (size_t)d * w : sOne, cb, sE, pin, sX, sW1, sW2, sY, pout);
     for (int i = threadIdx.x; i < po2; i += blockDim.x) T[((size_t)c * po2 + i) * pi2 + j] = sY[i];
 }
 
@@ -955,10 +662,9 @@ int gen_dense_rcr(Plan *P, int l, int which, const int *keys, int nkeys, double2
     return FMM_OK;
 }
 
-int set_dir_dist(const int *dd, const int *hrep)
+int set_dir_dist(const int *dd)
 {
     FMM_CUDA_TRY(cudaMemcpyToSymbol(c_dir_dist, dd, sizeof(int) * NDIR));
-    FMM_CUDA_TRY(cudaMemcpyToSymbol(c_dir_hrep, hrep, sizeof(int) * NDIR));
     return FMM_OK;
 }
 

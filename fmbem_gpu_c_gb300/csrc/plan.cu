@@ -15,7 +15,7 @@
 #include <thread>
 
 namespace fmm {
-int set_dir_dist(const int *dd, const int *hrep);
+int set_dir_dist(const int *dd);
 }
 
 using namespace fmm;
@@ -97,7 +97,7 @@ static void free_plan(Plan *P)
             F(R->td.B); F(R->td.items); F(R->td.src); F(R->td.dst); F(R->td.dir);
         }
     }
-    F(P->tc_err); F(P->tc_ones); F(P->hrep_dev); F(P->m2l_part64); F(P->Hall_ff); F(P->PHall_ff); F(P->dsc_leaf_dev);
+    F(P->tc_err); F(P->tc_ones); F(P->hrep_dev); F(P->PHall_ff); F(P->dsc_leaf_dev);
     F(P->Hsr64); F(P->PHsr64); F(P->Hsr32); F(P->PHsr32);
     F(P->V_dev); F(P->F_dev); F(P->elem_leaf); F(P->leaf_beg); F(P->leaf_elem);
     F(P->U64); F(P->Rv64); F(P->U32); F(P->Rv32); F(P->near_beg); F(P->near_col); F(P->near64); F(P->near32);
@@ -110,6 +110,7 @@ static void free_plan(Plan *P)
         cudaEventDestroy(P->total.beg); cudaEventDestroy(P->total.end);
         cudaEventDestroy(P->phase.beg); cudaEventDestroy(P->phase.end);
     }
+    free_owner(P);
     drop_graph(P);
     if (P->stream) cudaStreamDestroy(P->stream);
     for (int i = 0; i < NSIDE; i++) {
@@ -207,7 +208,7 @@ static int plan_create_impl(std::vector<double> &&V, std::vector<int> &&F, const
     CTRY(cudaMemcpy(P->F_dev, P->F.data(), sizeof(int) * P->F.size(), cudaMemcpyHostToDevice));
     CTRY(cudaMemcpy(P->elem_leaf, P->tree.elem_leaf.data(), sizeof(int) * nf, cudaMemcpyHostToDevice));
     TRY(gen_rotation_tables(P));
-    TRY(set_dir_dist(P->dir_dist, P->dir_hrep));
+    TRY(set_dir_dist(P->dir_dist));
     CTRY(dev_alloc(P, (void **)&P->hrep_dev, sizeof(int) * NDIR));
     CTRY(cudaMemcpy(P->hrep_dev, P->dir_hrep, sizeof(int) * NDIR, cudaMemcpyHostToDevice));
     TRY(build_lists(P));
@@ -223,21 +224,17 @@ static int plan_create_impl(std::vector<double> &&V, std::vector<int> &&F, const
         }
     }
     {
-        // FP64 M2L of levels with few boxes: split each box's sources over up to 16 CTAs so
-        // that the level has ~4 CTAs per SM (each run keeps >= 8 translations)
+        // runs a box's M2L sources are summed in by the translations without atomics: up to 16 on
+        // levels with few boxes (each run keeps >= 8 translations)
         int dev = 0, nsm = 152;
         CTRY(cudaGetDevice(&dev));
         CTRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        size_t part = 0;
         for (int l = P->lmin; l <= P->lmax; l++) {
             LevelDev &L = P->lev[l];
             long long target = 4LL * nsm, per_box = L.nb ? L.num_sr / L.nb : 0;
             int S = L.nb > 0 && L.nb < target ? (int)std::min<long long>(16, (target + L.nb - 1) / L.nb) : 1;
-            S = (int)std::max<long long>(1, std::min<long long>(S, per_box / 8));
-            L.m2l_split = S;
-            if (S > 1) part = std::max(part, (size_t)S * L.nb * L.p * L.p);
+            L.m2l_split = (int)std::max<long long>(1, std::min<long long>(S, per_box / 8));
         }
-        if (part) CTRY(dev_alloc(P, (void **)&P->m2l_part64, sizeof(double2) * part));
     }
     TRY(gen_element_tables(P));
     TRY(gen_near_field(P));

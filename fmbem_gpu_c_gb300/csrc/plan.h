@@ -9,6 +9,8 @@ namespace fmm {
 
 constexpr int NDIR = 316;      // M2L offsets (dx,dy,dz) in [-3,3]^3 with max |d| >= 2
 constexpr int NDIST = 15;      // distinct squared lengths of those offsets
+constexpr int TABLE_PAD = 4;   // entries readable past the last one of the rotation and coaxial tables of
+                               // owner.cu, whose lanes load rows in groups
 constexpr int MAX_TIMERS = 64;
 constexpr int NSIDE = 8;      // side streams for the independent M2L passes (at most)
 
@@ -87,6 +89,22 @@ struct RcrPass {
     const int *g_src, *g_dst;        // source and destination box of translation t
 };
 
+// One pass of the translations without atomics (owner.cu): translations ("slots", in destination
+// order) sorted by operator class inside chunks of consecutive destination boxes.
+struct OwnPass {
+    int built = 0, p = 0, pin = 0, pout = 0, rows = 0, tc = 0;
+    int4 *items = nullptr;        // (rotation table row, first, count, coaxial block)
+    int *slot = nullptr;          // slots in class order
+    const int *src = nullptr, *beg = nullptr;   // per slot: source box; per destination: its slots
+    const short *key = nullptr;   // per slot: phase row
+    int *src_own = nullptr;
+    short *key_own = nullptr;
+    int *units = nullptr;         // work units of the three stages
+    int n1 = 0, n2 = 0, n3 = 0;
+    std::vector<int> chunk_box, chunk_slot, chunk_item;
+    size_t part_bytes = 0;
+};
+
 struct LevelDev {
     int nb = 0, p = 0;
     int *parent = nullptr;        // [nb], index in level l-1 (l > lmin)
@@ -98,8 +116,8 @@ struct LevelDev {
     short *sr_dir = nullptr;      // direction index 0..315
     long long num_sr = 0;
     double2 *Cm64 = nullptr, *Dl64 = nullptr;
-    // float-float M2L of the FP64 path (FMM_FLOAT2): coaxial tables and expansions, each
-    // complex entry as (re hi, re lo, im hi, im lo)
+    // float-float form of the FP64 translations (FMM_FLOAT2): coaxial tables (two float4 per entry:
+    // re hi twice, re lo twice; the same of im) and expansions (re hi, im hi, re lo, im lo)
     float4 *Csr_ff = nullptr, *Crr_ff = nullptr, *Cm_ff = nullptr, *Dl_ff = nullptr;
     float4 *CrrL_ff = nullptr;    // the L2L's float-float table where the expansions are scaled
     float2 *Cm32 = nullptr, *Dl32 = nullptr;
@@ -111,7 +129,7 @@ struct LevelDev {
     // batched passes of the mixed path: M2L of this level, M2M (this level -> parents),
     // L2L (parents -> this level)
     RcrList m2l, m2m, l2l;
-    int m2l_split = 1;            // FP64 M2L: CTAs per box (source runs), > 1 on levels with few boxes
+    int m2l_split = 1;            // owner translations: runs a box's M2L sources are summed in
 };
 
 struct Timer {
@@ -168,11 +186,16 @@ struct Plan {
     int graph_nrhs = 0, graph_seen = 0;
     int *tc_err = nullptr;        // set by a tensor-core pass when one of its waits gives up
     float2 *tc_ones = nullptr;    // phases of the tensor-core passes without phases (all 1)
-    float2 *Hall_ff = nullptr;    // float-float rotation tables (as the FP64 ones, (hi, lo) each)
     float4 *PHall_ff = nullptr;   // float-float phases
     int ff_ready = 0;             // 1 once the float-float tables exist, -1 where they cannot
     double *dsc_leaf_dev = nullptr; // degree scales d_n of the leaf level (plans with scaled expansions)
-    double2 *m2l_part64 = nullptr; // FP64 M2L partial sums of split levels [run][box][p^2]
+    // translations without atomics (owner.cu), per type (OWN_*), level and pass
+    OwnPass own[3][FMM_MAX_LEVEL + 2][3];
+    int own_ready[3] = {0, 0, 0}, own_ncls = 0;
+    double *own_rot64 = nullptr;  // folded rotation tables per class, FP64 and float-float
+    float4 *own_rot_ff = nullptr; // (hi, hi, lo, lo) per entry
+    void *own_part = nullptr;     // translated expansions of one chunk, before their sums
+    size_t own_part_bytes = 0;
     size_t device_bytes = 0;
     char mixed_note[160] = "plan was created without build_mixed";
     // FP32 expansions scaled by degree (low k t): multipole d_n M_n, local L_n / d_n per level
@@ -228,6 +251,12 @@ enum { PASS_M2M = 0, PASS_M2L = 1, PASS_L2L = 2 };
 int launch_pass32(Plan *P, int l, int which, int nrhs, cudaStream_t st);
 // the list and descriptor of a batched SIMT pass (items not set), or null where the level has none
 RcrList *pass32_desc(Plan *P, int l, int which, int nrhs, RcrPass &ps);
+
+// owner.cu: the translations without atomics, from the leaf multipoles to the leaf locals
+// (OWN_FF: from Cm64 to Dl64 through the float-float expansions); beg / end time a pass of a level
+enum { OWN_FP64 = 0, OWN_FF = 1, OWN_FP32 = 2 };
+int translate_owner(Plan *P, int type, void (*beg)(Plan *, int, int), void (*end)(Plan *));
+void free_owner(Plan *P);
 
 // plan.cu: y = a x + b y over n entries
 void launch_axpby(double a, const double2 *x, double b, double2 *y, size_t n, cudaStream_t st);

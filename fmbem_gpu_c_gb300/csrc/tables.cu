@@ -250,7 +250,7 @@ int gen_rotation_tables(Plan *P)
     if (P->opt.build_mixed) {
         float *H32 = nullptr;
         float2 *PH32 = nullptr;
-        FMM_CUDA_TRY(cudaMalloc(&H32, sizeof(float) * (size_t)(NDIR + 16) * rs));
+        FMM_CUDA_TRY(cudaMalloc(&H32, sizeof(float) * ((size_t)(NDIR + 16) * rs + TABLE_PAD)));
         FMM_CUDA_TRY(cudaMalloc(&PH32, sizeof(float2) * (size_t)(NDIR + 16) * w));
         to_float(Hall, H32, (size_t)(NDIR + 16) * rs, P->stream);
         to_float((const double *)PHall, (float *)PH32, (size_t)(NDIR + 16) * w * 2, P->stream);
@@ -455,7 +455,7 @@ int gen_coax_tables(Plan *P)
         double mx;
         std::vector<float2> f = scaled_coax(hsr[l], p, NDIST, inv, inv, &mx);
         scaled_max = std::max(scaled_max, mx);
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Csr32, sizeof(float2) * f.size()));
+        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Csr32, sizeof(float2) * (f.size() + TABLE_PAD)));
         FMM_CUDA_TRY(cudaMemcpy(L.Csr32, f.data(), sizeof(float2) * f.size(), cudaMemcpyHostToDevice));
         if (l > P->lmin) {
             int pp = P->lev[l - 1].p;
@@ -466,12 +466,12 @@ int gen_coax_tables(Plan *P)
             for (int n = 0; n < p && n < pall; n++) up_col[n] = down_row[n] = inv[n];
             f = scaled_coax(hrr[l], pp, 1, P->dsc[l - 1], up_col, &mx);
             scaled_max = std::max(scaled_max, mx);
-            FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Crr32, sizeof(float2) * f.size()));
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Crr32, sizeof(float2) * (f.size() + TABLE_PAD)));
             FMM_CUDA_TRY(cudaMemcpy(L.Crr32, f.data(), sizeof(float2) * f.size(), cudaMemcpyHostToDevice));
             if (P->scaled) {
                 f = scaled_coax(hrr[l], pp, 1, down_row, P->dsc[l - 1], &mx);
                 scaled_max = std::max(scaled_max, mx);
-                FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Crr32L, sizeof(float2) * f.size()));
+                FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Crr32L, sizeof(float2) * (f.size() + TABLE_PAD)));
                 FMM_CUDA_TRY(cudaMemcpy(L.Crr32L, f.data(), sizeof(float2) * f.size(), cudaMemcpyHostToDevice));
             }
         }
