@@ -14,10 +14,19 @@
 //   far pairs, source j   sum_i mu_i A_ij = sum_nm Psi_j[nm] U_j[n,-m] with Psi the leaf local
 //                         of the transposed pass on mu (U_j[n,-m] integrates R_n^m over T_j):
 //                         differentiate the integral over T_j in its vertices.
-// Every local derivative is exact to rounding: forward-mode dual numbers through the same
-// quadrature rules, Green's function and regular basis.  The basis is evaluated through
-// u = (x + i y)/r and polynomials in z/r (Q_n^m = st^m q_n^m), which stays smooth on the
-// z-axis where (theta, phi) do not.
+// Every local derivative is exact to rounding, and taken in reverse: the objective's weight is known
+// before a quadrature point is evaluated, so a point adds real vectors to the gradients by the
+// source's vertices, normal and area and the target's centroid and normal (a few operations more
+// than its value), and the vertices follow by the chain rule once per pair.  The basis is
+// evaluated through u = (x + i y)/r and polynomials in z/r (Q_n^m = st^m q_n^m), which stays
+// smooth on the z-axis where (theta, phi) do not.
+//
+// What bounds it: the FP64 pipe (per point a sincos, a reciprocal square root and some 40
+// multiply-adds; the near pairs of a Burton-Miller plan have 24 edge points per segment beside 7
+// or 9 on the face).  On the 5,120-triangle head (498,000 near pairs, admittance, Burton-Miller)
+// against forward-mode dual numbers with 9 to 18 slots: near pairs 111 -> 5.5 ms, source side
+// of the far pairs 22 -> 0.9, far points 7.8 -> 0.3, target side 2.1 -> 0.3, the whole fmm_vjp
+// with its adjoint solve 163 -> 27 ms.
 #include "plan.h"
 #include <algorithm>
 #include <vector>
@@ -31,6 +40,8 @@ __constant__ int v_rule_n[2];
 // the 8-point Gauss rule on [-1, 1] of the Burton-Miller edge integrals (tables.cu)
 constexpr int V_LINE_PTS = 8;
 __constant__ double v_line_x[V_LINE_PTS], v_line_w[V_LINE_PTS];
+
+static int upload_legendre();
 
 static int upload_vjp_rules()
 {
@@ -48,393 +59,330 @@ static int upload_vjp_rules()
     line_rule(V_LINE_PTS, lx, lw);
     FMM_CUDA_TRY(cudaMemcpyToSymbol(v_line_x, lx, sizeof(lx)));
     FMM_CUDA_TRY(cudaMemcpyToSymbol(v_line_w, lw, sizeof(lw)));
+    int st = upload_legendre();
+    if (st) return st;
     dev_done = dev;
     return FMM_OK;
 }
 
-// ----------------------------------------------------------------------------- dual numbers
-template <int N> struct Dn {
-    double v, d[N];
-};
-
-template <int N> __device__ __forceinline__ Dn<N> dconst(double a)
-{
-    Dn<N> r;
-    r.v = a;
-#pragma unroll
-    for (int i = 0; i < N; i++) r.d[i] = 0.0;
-    return r;
-}
-template <int N> __device__ __forceinline__ Dn<N> dvar(double a, int slot)
-{
-    Dn<N> r = dconst<N>(a);
-    r.d[slot] = 1.0;
-    return r;
-}
-template <int N> __device__ __forceinline__ Dn<N> operator+(const Dn<N> &a, const Dn<N> &b)
-{
-    Dn<N> r;
-    r.v = a.v + b.v;
-#pragma unroll
-    for (int i = 0; i < N; i++) r.d[i] = a.d[i] + b.d[i];
-    return r;
-}
-template <int N> __device__ __forceinline__ Dn<N> operator-(const Dn<N> &a, const Dn<N> &b)
-{
-    Dn<N> r;
-    r.v = a.v - b.v;
-#pragma unroll
-    for (int i = 0; i < N; i++) r.d[i] = a.d[i] - b.d[i];
-    return r;
-}
-template <int N> __device__ __forceinline__ Dn<N> operator-(const Dn<N> &a)
-{
-    Dn<N> r;
-    r.v = -a.v;
-#pragma unroll
-    for (int i = 0; i < N; i++) r.d[i] = -a.d[i];
-    return r;
-}
-template <int N> __device__ __forceinline__ Dn<N> operator*(const Dn<N> &a, const Dn<N> &b)
-{
-    Dn<N> r;
-    r.v = a.v * b.v;
-#pragma unroll
-    for (int i = 0; i < N; i++) r.d[i] = a.d[i] * b.v + a.v * b.d[i];
-    return r;
-}
-template <int N> __device__ __forceinline__ Dn<N> operator*(double s, const Dn<N> &a)
-{
-    Dn<N> r;
-    r.v = s * a.v;
-#pragma unroll
-    for (int i = 0; i < N; i++) r.d[i] = s * a.d[i];
-    return r;
-}
-template <int N> __device__ __forceinline__ Dn<N> operator/(const Dn<N> &a, const Dn<N> &b)
-{
-    Dn<N> r;
-    double inv = 1.0 / b.v;
-    r.v = a.v * inv;
-#pragma unroll
-    for (int i = 0; i < N; i++) r.d[i] = (a.d[i] - r.v * b.d[i]) * inv;
-    return r;
-}
-template <int N> __device__ __forceinline__ Dn<N> dsqrt(const Dn<N> &a)
-{
-    Dn<N> r;
-    r.v = sqrt(a.v);
-    double h = 0.5 / r.v;
-#pragma unroll
-    for (int i = 0; i < N; i++) r.d[i] = a.d[i] * h;
-    return r;
-}
-template <int N> __device__ __forceinline__ void dsincos(const Dn<N> &a, Dn<N> &s, Dn<N> &c)
-{
-    double sv, cv;
-    sincos(a.v, &sv, &cv);
-    s.v = sv;
-    c.v = cv;
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        s.d[i] = cv * a.d[i];
-        c.d[i] = -sv * a.d[i];
-    }
-}
-
-// complex dual
-template <int N> struct CDn {
-    Dn<N> re, im;
-};
-template <int N> __device__ __forceinline__ CDn<N> cdzero()
-{
-    CDn<N> r;
-    r.re = dconst<N>(0.0);
-    r.im = dconst<N>(0.0);
-    return r;
-}
-template <int N> __device__ __forceinline__ CDn<N> cdmul(const CDn<N> &a, const CDn<N> &b)
-{
-    CDn<N> r;
-    r.re = a.re * b.re - a.im * b.im;
-    r.im = a.re * b.im + a.im * b.re;
-    return r;
-}
-// acc += c * a  (c a plain complex constant)
-template <int N> __device__ __forceinline__ void cdmac(CDn<N> &acc, double2 c, const CDn<N> &a)
-{
-    acc.re.v += c.x * a.re.v - c.y * a.im.v;
-    acc.im.v += c.x * a.im.v + c.y * a.re.v;
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        acc.re.d[i] += c.x * a.re.d[i] - c.y * a.im.d[i];
-        acc.im.d[i] += c.x * a.im.d[i] + c.y * a.re.d[i];
-    }
-}
-// derivative of Re(w * z) for a plain complex w, one slot
-template <int N> __device__ __forceinline__ double re_wd(double2 w, const CDn<N> &z, int i)
-{
-    return w.x * z.re.d[i] - w.y * z.im.d[i];
-}
-
-// ----------------------------------------------------------------------------- kernels in duals
-template <int N>
-__device__ void tri_normal_d(const Dn<N> *nod, Dn<N> *nc, Dn<N> &J)
-{
-    Dn<N> u0 = nod[0] - nod[6], u1 = nod[1] - nod[7], u2 = nod[2] - nod[8];
-    Dn<N> v0 = nod[3] - nod[6], v1 = nod[4] - nod[7], v2 = nod[5] - nod[8];
-    nc[0] = u1 * v2 - u2 * v1;
-    nc[1] = u2 * v0 - u0 * v2;
-    nc[2] = u0 * v1 - u1 * v0;
-    J = dsqrt(nc[0] * nc[0] + nc[1] * nc[1] + nc[2] * nc[2]);
-}
-
-// G(x, y) = exp(ikr)/(4 pi r) (kern 0) or dG/dn_x = G (ik - 1/r) (x - y).nh / r (kern 1); the
-// caller passes the unit normal
-template <int N>
-__device__ CDn<N> green_d(double k, const Dn<N> *x, const Dn<N> *y, const Dn<N> *nh, int kern)
-{
-    Dn<N> d0 = x[0] - y[0], d1 = x[1] - y[1], d2 = x[2] - y[2];
-    Dn<N> r = dsqrt(d0 * d0 + d1 * d1 + d2 * d2);
-    Dn<N> s, c;
-    dsincos(k * r, s, c);
-    Dn<N> inv = dconst<N>(1.0 / (4.0 * FMM_PI)) / r;
-    CDn<N> g;
-    g.re = c * inv;
-    g.im = s * inv;
-    if (!kern) return g;
-    Dn<N> dn = (d0 * nh[0] + d1 * nh[1] + d2 * nh[2]) / r;
-    Dn<N> ar = -(dconst<N>(1.0) / r);
-    CDn<N> f;
-    f.re = ar * dn;
-    f.im = k * dn;
-    return cdmul(g, f);
-}
-
-template <int N>
-__device__ CDn<N> elem_integral_d(double k, const Dn<N> *nod, const Dn<N> *y, int rule, int kern)
-{
-    Dn<N> nc[3], J;
-    tri_normal_d(nod, nc, J);
-    Dn<N> nh[3] = {nc[0] / J, nc[1] / J, nc[2] / J};
-    CDn<N> acc = cdzero<N>();
-    int nq = v_rule_n[rule];
-    for (int q = 0; q < nq; q++) {
-        const double *b = &v_rule_bary[rule][3 * q];
-        Dn<N> x[3];
-        for (int a = 0; a < 3; a++) x[a] = b[0] * nod[a] + b[1] * nod[3 + a] + b[2] * nod[6 + a];
-        CDn<N> g = green_d(k, x, y, nh, kern);
-        Dn<N> wq = v_rule_w[rule][q] * J;
-        acc.re = acc.re + wq * g.re;
-        acc.im = acc.im + wq * g.im;
-    }
-    return acc;
-}
-
-template <int N>
-__device__ void centroid_d(const Dn<N> *nod, Dn<N> *y)
-{
-    for (int a = 0; a < 3; a++) {
-        Dn<N> c23 = 0.5 * (nod[3 + a] + nod[6 + a]);
-        y[a] = nod[a] + (2.0 / 3.0) * (c23 - nod[a]);
-    }
-}
-
-// self term: centroid split into three sub-triangles with the collapsed rule
-template <int N>
-__device__ CDn<N> elem_integral_sgl_d(double k, const Dn<N> *nod, int kern)
-{
-    Dn<N> y[3];
-    centroid_d(nod, y);
-    CDn<N> acc = cdzero<N>();
-    for (int s = 0; s < 3; s++) {
-        Dn<N> sub[9];
-        int a0 = 3 * s, b0 = 3 * ((s + 1) % 3);
-        for (int t = 0; t < 3; t++) {
-            sub[t] = nod[a0 + t];
-            sub[3 + t] = nod[b0 + t];
-            sub[6 + t] = y[t];
-        }
-        CDn<N> part = elem_integral_d(k, sub, y, 0, kern);
-        acc.re = acc.re + part.re;
-        acc.im = acc.im + part.im;
-    }
-    return acc;
-}
-
-// ---------------------------------------------------------------- Burton-Miller terms in duals
-// The same forms as tables.cu (elem_integrals_fused, hyper_edges, elem_hyper_self); the numbers of
-// edge segments follow from the values, as there, and are held fixed by the derivative.
+// Number of equal segments of an edge of length len seen from distance dist, as in tables.cu; the
+// numbers follow from the values and are held fixed by the derivative.
 __device__ __forceinline__ int edge_segments_v(double len, double dist)
 {
     double m = ceil(len / fmax(dist, 1e-12 * len));
     return m > 64.0 ? 64 : (int)m;
 }
 
-// int_T dG(x, y)/dn_y dS_x, ny the unit normal at y
-template <int N>
-__device__ CDn<N> elem_dGdny_d(double k, const Dn<N> *nod, const Dn<N> *y, const Dn<N> *ny, int rule)
-{
-    Dn<N> nc[3], J;
-    tri_normal_d(nod, nc, J);
-    CDn<N> acc = cdzero<N>();
-    int nq = v_rule_n[rule];
-    for (int q = 0; q < nq; q++) {
-        const double *b = &v_rule_bary[rule][3 * q];
-        Dn<N> x[3];
-        for (int a = 0; a < 3; a++) x[a] = b[0] * nod[a] + b[1] * nod[3 + a] + b[2] * nod[6 + a];
-        CDn<N> g = green_d(k, x, y, ny, 1);   // G (ik - 1/r) (x - y).ny / r
-        Dn<N> wq = v_rule_w[rule][q] * J;
-        acc.re = acc.re - wq * g.re;
-        acc.im = acc.im - wq * g.im;
-    }
-    return acc;
-}
-
-// int_T d2G/dn_x dn_y dS_x at y off T: k^2 (ny.nT) int_T G - oint (ny x grad_y G) . dl
-template <int N>
-__device__ CDn<N> elem_hyper_near_d(double k, const Dn<N> *nod, const Dn<N> *y, const Dn<N> *ny, int rule)
-{
-    Dn<N> nc[3], J;
-    tri_normal_d(nod, nc, J);
-    CDn<N> S = elem_integral_d(k, nod, y, rule, 0);
-    Dn<N> dn = (ny[0] * nc[0] + ny[1] * nc[1] + ny[2] * nc[2]) / J;
-    CDn<N> line = cdzero<N>();
-    for (int e = 0; e < 3; e++) {
-        const Dn<N> *va = nod + 3 * e, *vb = nod + 3 * ((e + 1) % 3);
-        Dn<N> t[3] = {vb[0] - va[0], vb[1] - va[1], vb[2] - va[2]}, a[3] = {y[0] - va[0], y[1] - va[1], y[2] - va[2]};
-        double tt = t[0].v * t[0].v + t[1].v * t[1].v + t[2].v * t[2].v, len = sqrt(tt);
-        double sc = fmin(fmax((a[0].v * t[0].v + a[1].v * t[1].v + a[2].v * t[2].v) / tt, 0.0), 1.0);
-        double e0 = a[0].v - sc * t[0].v, e1 = a[1].v - sc * t[1].v, e2 = a[2].v - sc * t[2].v;
-        int nseg = edge_segments_v(len, sqrt(e0 * e0 + e1 * e1 + e2 * e2));
-        Dn<N> tn0 = t[1] * ny[2] - t[2] * ny[1], tn1 = t[2] * ny[0] - t[0] * ny[2], tn2 = t[0] * ny[1] - t[1] * ny[0];
-        for (int g = 0; g < nseg; g++)
-            for (int q = 0; q < V_LINE_PTS; q++) {
-                double s = (g + 0.5 + 0.5 * v_line_x[q]) / nseg, w = 0.5 * v_line_w[q] / nseg;
-                Dn<N> d0 = a[0] - s * t[0], d1 = a[1] - s * t[1], d2 = a[2] - s * t[2];
-                Dn<N> r2 = d0 * d0 + d1 * d1 + d2 * d2, r = dsqrt(r2);
-                Dn<N> sn, cs;
-                dsincos(k * r, sn, cs);
-                Dn<N> f = (w / (4.0 * FMM_PI)) * (d0 * tn0 + d1 * tn1 + d2 * tn2) / r2;
-                Dn<N> ar = -(dconst<N>(1.0) / r);
-                // e^{ikr} (ik - 1/r) f
-                line.re = line.re + f * (cs * ar - k * sn);
-                line.im = line.im + f * (k * cs + sn * ar);
-            }
-    }
-    Dn<N> kk = (k * k) * dn;
-    CDn<N> out;
-    out.re = kk * S.re - line.re;
-    out.im = kk * S.im - line.im;
-    return out;
-}
-
-// Hadamard finite part of int_T d2G/dn_x dn_y at the centroid of the flat element T
-template <int N>
-__device__ CDn<N> elem_hyper_self_d(double k, const Dn<N> *nod)
-{
-    Dn<N> c[3];
-    centroid_d(nod, c);
-    CDn<N> ang = cdzero<N>();
-    for (int e = 0; e < 3; e++) {
-        const Dn<N> *va = nod + 3 * e, *vb = nod + 3 * ((e + 1) % 3);
-        Dn<N> t[3] = {vb[0] - va[0], vb[1] - va[1], vb[2] - va[2]}, u[3] = {va[0] - c[0], va[1] - c[1], va[2] - c[2]};
-        Dn<N> c0 = u[1] * t[2] - u[2] * t[1], c1 = u[2] * t[0] - u[0] * t[2], c2 = u[0] * t[1] - u[1] * t[0];
-        Dn<N> hL = dsqrt(c0 * c0 + c1 * c1 + c2 * c2);
-        double len = sqrt(t[0].v * t[0].v + t[1].v * t[1].v + t[2].v * t[2].v);
-        int nseg = edge_segments_v(len, hL.v / len);
-        for (int g = 0; g < nseg; g++)
-            for (int q = 0; q < V_LINE_PTS; q++) {
-                double s = (g + 0.5 + 0.5 * v_line_x[q]) / nseg, w = 0.5 * v_line_w[q] / nseg;
-                Dn<N> d0 = u[0] + s * t[0], d1 = u[1] + s * t[1], d2 = u[2] + s * t[2];
-                Dn<N> r = dsqrt(d0 * d0 + d1 * d1 + d2 * d2);
-                Dn<N> sn, cs;
-                dsincos(k * r, sn, cs);
-                Dn<N> f = w * hL / (r * r * r);
-                ang.re = ang.re + f * cs;
-                ang.im = ang.im + f * sn;
-            }
-    }
-    CDn<N> out;
-    out.re = (-1.0 / (4.0 * FMM_PI)) * ang.re;
-    out.im = (-1.0 / (4.0 * FMM_PI)) * ang.im + dconst<N>(2.0 * FMM_PI * k / (4.0 * FMM_PI));
-    return out;
-}
-
-// spherical Bessel j_n(x), n < NB, Miller's backward recurrence normalised by j0 or j1, in duals
-template <int N>
-__device__ void sph_jn_d(int NB, const Dn<N> &x, Dn<N> *j)
-{
-    Dn<N> s, c;
-    dsincos(x, s, c);
-    Dn<N> j0 = s / x, j1 = s / (x * x) - c / x;
-    int big = NB > (int)x.v ? NB : (int)x.v;
-    int start = big + 40 + (int)(4.0 * sqrt((double)big + 1.0));
-    Dn<N> fp1 = dconst<N>(0.0), f = dconst<N>(1e-300), f1 = dconst<N>(0.0);
-    for (int n = start; n >= 1; n--) {
-        Dn<N> fm1 = ((2.0 * n + 1.0) * f) / x - fp1;
-        fp1 = f;
-        f = fm1;
-        if (n - 1 < NB) j[n - 1] = f;
-        if (n - 1 == 1) f1 = f;
-        if (fabs(f.v) > 1e250) {
-            f = 1e-250 * f;
-            fp1 = 1e-250 * fp1;
-            f1 = 1e-250 * f1;
-            for (int q = (n - 1 < NB ? n - 1 : NB); q < NB; q++) j[q] = 1e-250 * j[q];
-        }
-    }
-    Dn<N> scale = (fabs(j0.v) > fabs(j1.v)) ? j0 / f : j1 / f1;
-    for (int n = 0; n < NB; n++) j[n] = j[n] * scale;
-}
-
 constexpr int VJP_PMAX = 24; // largest leaf order (plus one for gradient expansions) handled here
 
-// out[e] = sum_{n < P, |m| <= n} coef[e][n^2+n+m] R_n^m(v), R_n^m = j_n(kr) q_n^|m|(z/r) u^m
-// (u^{-m} read as conj(u)^m), for NE expansions at one dual point v
-template <int N, int NE>
-__device__ void eval_expansions_d(int P, double k, const Dn<N> *v, const double2 *const *coef, CDn<N> *out)
+// factors of the recurrence in degree of q_n^m (Q_n^m = st^m q_n^m): q_n = a (ct q_{n-1} - b q_{n-2});
+// q_m^m and the factor of q_{m+1}^m = sqrt(2m+3) ct q_m^m
+__constant__ double v_leg_a[VJP_PMAX * VJP_PMAX], v_leg_b[VJP_PMAX * VJP_PMAX];
+__constant__ double v_leg_mm[VJP_PMAX], v_leg_s[VJP_PMAX];
+
+static int upload_legendre()
 {
-    Dn<N> r = dsqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-    Dn<N> ct = v[2] / r;
-    CDn<N> u;
-    u.re = v[0] / r;
-    u.im = v[1] / r;
-    Dn<N> jn[VJP_PMAX];
-    sph_jn_d(P, k * r, jn);
-    for (int e = 0; e < NE; e++) out[e] = cdzero<N>();
-    CDn<N> um = cdzero<N>();
-    um.re = dconst<N>(1.0);
+    double la[VJP_PMAX * VJP_PMAX] = {}, lb[VJP_PMAX * VJP_PMAX] = {}, mm[VJP_PMAX], ls[VJP_PMAX];
     double cmm = 0.28209479177387814; // q_0^0 = 1/sqrt(4 pi)
+    for (int m = 0; m < VJP_PMAX; m++) {
+        if (m > 0) cmm *= sqrt((2.0 * m + 1.0) / (2.0 * m));
+        mm[m] = cmm;
+        ls[m] = sqrt(2.0 * m + 3.0);
+        for (int n = m + 2; n < VJP_PMAX; n++) {
+            la[n * VJP_PMAX + m] = sqrt((4.0 * n * n - 1.0) / ((double)n * n - (double)m * m));
+            lb[n * VJP_PMAX + m] = sqrt(((n - 1.0) * (n - 1.0) - (double)m * m) / (4.0 * (n - 1.0) * (n - 1.0) - 1.0));
+        }
+    }
+    FMM_CUDA_TRY(cudaMemcpyToSymbol(v_leg_a, la, sizeof(la)));
+    FMM_CUDA_TRY(cudaMemcpyToSymbol(v_leg_b, lb, sizeof(lb)));
+    FMM_CUDA_TRY(cudaMemcpyToSymbol(v_leg_mm, mm, sizeof(mm)));
+    FMM_CUDA_TRY(cudaMemcpyToSymbol(v_leg_s, ls, sizeof(ls)));
+    return FMM_OK;
+}
+
+// f_e(v) = sum_{n < P, |m| <= n} coef[e][n^2+n+m] R_n^m(v), R_n^m = j_n(kr) q_n^|m|(z/r) u^m
+// (u^{-m} read as conj(u)^m), and (GRAD) its gradient, for NE expansions at one point.  The sums over
+// n are taken at fixed m for the value and its derivatives by r and by z/r; the derivative by u
+// follows from the powers of u.
+template <int NE, bool GRAD>
+__device__ void eval_expansions(int P, double k, const double *v, const double2 *const *coef, double2 *val,
+                                double2 (*grd)[3])
+{
+    const double r = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]), ri = 1.0 / r, ct = v[2] * ri;
+    const double2 u = make_double2(v[0] * ri, v[1] * ri);
+    double jn[VJP_PMAX + 1];
+    sph_jn_array(P + 1, k * r, jn);
+    double2 F[NE], Fr[NE], Fc[NE], Gp[NE], Gm[NE];
+#pragma unroll
+    for (int e = 0; e < NE; e++) F[e] = Fr[e] = Fc[e] = Gp[e] = Gm[e] = make_double2(0.0, 0.0);
+    double2 um = make_double2(1.0, 0.0), um1 = make_double2(0.0, 0.0);
+    auto add = [](double2 &a, double f, double2 c) {
+        a.x = fma(f, c.x, a.x);
+        a.y = fma(f, c.y, a.y);
+    };
     for (int m = 0; m < P; m++) {
         if (m > 0) {
-            cmm *= sqrt((2.0 * m + 1.0) / (2.0 * m));
-            um = cdmul(um, u);
+            um1 = um;
+            um = cmul(um, u);
         }
-        Dn<N> q2 = dconst<N>(0.0), q1 = dconst<N>(0.0);
+        double2 Ap[NE], Am[NE], Arp[NE], Arm[NE], Acp[NE], Acm[NE];
+#pragma unroll
+        for (int e = 0; e < NE; e++) Ap[e] = Am[e] = Arp[e] = Arm[e] = Acp[e] = Acm[e] = make_double2(0.0, 0.0);
+        double q2 = 0.0, q1 = 0.0, d2 = 0.0, d1 = 0.0;
         for (int n = m; n < P; n++) {
-            Dn<N> q;
-            if (n == m) q = dconst<N>(cmm);
-            else if (n == m + 1) q = (sqrt(2.0 * m + 3.0) * cmm) * ct;
-            else {
-                double a = sqrt((4.0 * n * n - 1.0) / ((double)n * n - (double)m * m));
-                double b = sqrt(((n - 1.0) * (n - 1.0) - (double)m * m) / (4.0 * (n - 1.0) * (n - 1.0) - 1.0));
+            double q, d;
+            if (n == m) {
+                q = v_leg_mm[m];
+                d = 0.0;
+            } else if (n == m + 1) {
+                d = v_leg_s[m] * q1;
+                q = d * ct;
+            } else {
+                const double a = v_leg_a[n * VJP_PMAX + m], b = v_leg_b[n * VJP_PMAX + m];
                 q = a * (ct * q1 - b * q2);
+                d = a * (q1 + ct * d1 - b * d2);
             }
             q2 = q1;
             q1 = q;
-            Dn<N> base = jn[n] * q;
-            CDn<N> Rp, Rm;
-            Rp.re = base * um.re;
-            Rp.im = base * um.im;
-            Rm.re = Rp.re;
-            Rm.im = -Rp.im;
+            d2 = d1;
+            d1 = d;
+            const double t0 = jn[n] * q;
+            const double tr = GRAD ? (n * ri * jn[n] - k * jn[n + 1]) * q : 0.0, tc = GRAD ? jn[n] * d : 0.0;
+#pragma unroll
             for (int e = 0; e < NE; e++) {
-                cdmac(out[e], coef[e][n * n + n + m], Rp);
-                if (m > 0) cdmac(out[e], coef[e][n * n + n - m], Rm);
+                const double2 cp = coef[e][n * n + n + m];
+                add(Ap[e], t0, cp);
+                if (GRAD) {
+                    add(Arp[e], tr, cp);
+                    add(Acp[e], tc, cp);
+                }
+                if (m > 0) {
+                    const double2 cm = coef[e][n * n + n - m];
+                    add(Am[e], t0, cm);
+                    if (GRAD) {
+                        add(Arm[e], tr, cm);
+                        add(Acm[e], tc, cm);
+                    }
+                }
+            }
+        }
+        // a u^m + b conj(u)^m
+        auto both = [&](double2 &s, double2 a, double2 b) {
+            s.x += (a.x + b.x) * um.x - (a.y - b.y) * um.y;
+            s.y += (a.x - b.x) * um.y + (a.y + b.y) * um.x;
+        };
+#pragma unroll
+        for (int e = 0; e < NE; e++) {
+            both(F[e], Ap[e], Am[e]);
+            if (GRAD) {
+                both(Fr[e], Arp[e], Arm[e]);
+                both(Fc[e], Acp[e], Acm[e]);
+                add(Gp[e], m, cmul(Ap[e], um1));
+                add(Gm[e], m, cconjmul(um1, Am[e]));
             }
         }
     }
+#pragma unroll
+    for (int e = 0; e < NE; e++) {
+        val[e] = F[e];
+        if (GRAD) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                const double ra = v[a] * ri, ca = ((a == 2 ? 1.0 : 0.0) - ct * ra) * ri;
+                // d u / d v_a and its conjugate
+                const double2 ua = make_double2(((a == 0 ? 1.0 : 0.0) - u.x * ra) * ri, ((a == 1 ? 1.0 : 0.0) - u.y * ra) * ri);
+                double2 g = cadd(cscale(Fr[e], ra), cscale(Fc[e], ca));
+                g = cadd(g, cmul(Gp[e], ua));
+                grd[e][a] = cadd(g, cconjmul(ua, Gm[e]));
+            }
+        }
+    }
+}
+
+// grad phi and its derivatives H[b][a] = d_a d_b phi from the values and gradients of the
+// derivative expansions d/dz, d+ and d- (d/dx +- i d/dy)
+__device__ __forceinline__ void cartesian(const double2 *val, const double2 (*grd)[3], double2 *g, double2 (*H)[3])
+{
+    auto xy = [](double2 p, double2 m, double2 &x, double2 &y) {
+        x = make_double2(0.5 * (p.x + m.x), 0.5 * (p.y + m.y));
+        y = make_double2(0.5 * (p.y - m.y), -0.5 * (p.x - m.x));
+    };
+    xy(val[1], val[2], g[0], g[1]);
+    g[2] = val[0];
+    for (int a = 0; a < 3; a++) {
+        xy(grd[1][a], grd[2][a], H[0][a], H[1][a]);
+        H[2][a] = grd[0][a];
+    }
+}
+
+// ----------------------------------------------------------------------------- pairs, in reverse
+__device__ __forceinline__ double re_mul(double2 a, double2 b) { return a.x * b.x - a.y * b.y; }
+
+// G = exp(ikr)/(4 pi r), h = G'/r (grad G = h d) and e = h'/r (grad h = e d) at distance r: the
+// phase (c, s), the factors of r and kr, from which only real parts of products with complex
+// weights are taken: w exp(ikr) first, then the polynomials in ikr.
+struct Radial {
+    double c, s, kr, f, fh, fe;
+};
+__device__ __forceinline__ Radial radial(double k, double r2)
+{
+    Radial o;
+    const double ri = rsqrt(r2), ri2 = ri * ri;
+    o.kr = k * (r2 * ri);
+    sincos(o.kr, &o.s, &o.c);
+    o.f = ri * (1.0 / (4.0 * FMM_PI));
+    o.fh = o.f * ri2;
+    o.fe = o.fh * ri2;
+    return o;
+}
+// w exp(ikr), and Re(w G), Re(w h), Re(w e) from it
+__device__ __forceinline__ double2 turned(const Radial &o, double2 w)
+{
+    return make_double2(w.x * o.c - w.y * o.s, w.x * o.s + w.y * o.c);
+}
+__device__ __forceinline__ double re_g(const Radial &o, double2 z) { return o.f * z.x; }
+__device__ __forceinline__ double re_h(const Radial &o, double2 z) { return -o.fh * (z.x + o.kr * z.y); }
+__device__ __forceinline__ double re_e(const Radial &o, double2 z)
+{
+    return o.fe * ((3.0 - o.kr * o.kr) * z.x + 3.0 * o.kr * z.y);
+}
+
+// the unnormalised normal N = u x v of a triangle (u = v0 - v2, v = v1 - v2) and its length
+struct Tri {
+    double u[3], v[3], N[3], J;
+};
+__device__ __forceinline__ Tri tri_of(const double *nd)
+{
+    Tri t;
+    for (int a = 0; a < 3; a++) {
+        t.u[a] = nd[a] - nd[6 + a];
+        t.v[a] = nd[3 + a] - nd[6 + a];
+    }
+    t.N[0] = t.u[1] * t.v[2] - t.u[2] * t.v[1];
+    t.N[1] = t.u[2] * t.v[0] - t.u[0] * t.v[2];
+    t.N[2] = t.u[0] * t.v[1] - t.u[1] * t.v[0];
+    t.J = sqrt(t.N[0] * t.N[0] + t.N[1] * t.N[1] + t.N[2] * t.N[2]);
+    return t;
+}
+__device__ __forceinline__ double dot3(const double *a, const double *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
+// s += f (a x b)
+__device__ __forceinline__ void cross_add(double *s, double f, const double *a, const double *b)
+{
+    s[0] += f * (a[1] * b[2] - a[2] * b[1]);
+    s[1] += f * (a[2] * b[0] - a[0] * b[2]);
+    s[2] += f * (a[0] * b[1] - a[1] * b[0]);
+}
+// gradients by N and J to the vertices
+__device__ __forceinline__ void normal_to_nodes(const Tri &t, double *gN, double gJ, double *gs)
+{
+    for (int a = 0; a < 3; a++) gN[a] += gJ / t.J * t.N[a];
+    double gu[3] = {0, 0, 0}, gv[3] = {0, 0, 0};
+    cross_add(gu, 1.0, t.v, gN);
+    cross_add(gv, 1.0, gN, t.u);
+    for (int a = 0; a < 3; a++) {
+        gs[a] += gu[a];
+        gs[3 + a] += gv[a];
+        gs[6 + a] -= gu[a] + gv[a];
+    }
+}
+
+// The gradient of Re[ w0 (b I0 + c I1) + w1 (b I2 + c (k^2 (ny.nh) I0 - L)) ] over the element nd:
+// I0, I1, I2 the integrals of G, dG/dn_x and dG/dn_y by the regular rule, L the edge integral
+// of the regularised hypersingular kernel (tables.cu: elem_integrals_fused, hyper_edges; the numbers
+// of edge segments follow from the values, as there, and are held fixed).  w0b = w0 b etc.; BM:
+// with the w1 terms.  gs: by the vertices; gy, gny: by the target's point and unit normal (added).
+template <bool BM>
+__device__ __forceinline__ void pair_grad(double k, const double *nd, const double *y, const double *ny, int rule,
+                                          double2 w0b, double2 w0c, double2 w1b, double2 w1c, double *gs, double *gy,
+                                          double *gny)
+{
+    const Tri t = tri_of(nd);
+    const double dn = BM ? dot3(ny, t.N) / t.J : 0.0;
+    const double2 A0 = BM ? make_double2(w0b.x + k * k * dn * w1c.x, w0b.y + k * k * dn * w1c.y) : w0b;
+    double gN[3] = {0, 0, 0}, gJ = 0.0, gdn = 0.0;
+    for (int i = 0; i < 9; i++) gs[i] = 0.0;
+    const int nq = v_rule_n[rule];
+    for (int q = 0; q < nq; q++) {
+        const double *bb = &v_rule_bary[rule][3 * q], wq = v_rule_w[rule][q];
+        double d[3];
+        for (int a = 0; a < 3; a++) d[a] = bb[0] * nd[a] + bb[1] * nd[3 + a] + bb[2] * nd[6 + a] - y[a];
+        const Radial f = radial(k, dot3(d, d));
+        const double2 z0 = turned(f, A0), z1 = turned(f, w0c);
+        const double dN = dot3(d, t.N), a1h = re_h(f, z1);
+        // by d: along d, along N and (BM) along ny
+        double along = t.J * re_h(f, z0) + re_e(f, z1) * dN, a2h = 0.0, dny = 0.0;
+        if (BM) {
+            const double2 z2 = turned(f, w1b);
+            dny = dot3(d, ny);
+            a2h = -re_h(f, z2);
+            along -= t.J * re_e(f, z2) * dny;
+            gdn += wq * re_g(f, turned(f, w1c));
+        }
+        gJ += wq * (re_g(f, z0) + a2h * dny);
+        for (int a = 0; a < 3; a++) {
+            double D = along * d[a] + a1h * t.N[a];
+            if (BM) {
+                D += t.J * a2h * ny[a];
+                gny[a] += wq * t.J * a2h * d[a];
+            }
+            D *= wq;
+            gN[a] += wq * a1h * d[a];
+            gs[a] += bb[0] * D;
+            gs[3 + a] += bb[1] * D;
+            gs[6 + a] += bb[2] * D;
+        }
+    }
+    for (int a = 0; a < 3; a++) gy[a] -= gs[a] + gs[3 + a] + gs[6 + a];
+    if (BM) {
+        if (w1c.x != 0.0 || w1c.y != 0.0) {
+            // -w1 c L: along an edge d = a - s t, and d . (t x ny) = a . (t x ny)
+            for (int e = 0; e < 3; e++) {
+                const double *va = nd + 3 * e, *vb = nd + 3 * ((e + 1) % 3);
+                double tt[3], av[3], tn[3] = {0, 0, 0};
+                for (int a = 0; a < 3; a++) {
+                    tt[a] = vb[a] - va[a];
+                    av[a] = y[a] - va[a];
+                }
+                cross_add(tn, 1.0, tt, ny);
+                const double t2 = dot3(tt, tt), at = dot3(av, tt), len = sqrt(t2);
+                const double sc = fmin(fmax(at / t2, 0.0), 1.0);
+                const double e0 = av[0] - sc * tt[0], e1 = av[1] - sc * tt[1], e2 = av[2] - sc * tt[2];
+                const int nseg = edge_segments_v(len, sqrt(e0 * e0 + e1 * e1 + e2 * e2));
+                double hs = 0.0, es = 0.0, ess = 0.0, esss = 0.0;  // sums of -Re(w1c h), -Re(w1c e) s^0, s^1, s^2
+                const double inv = 1.0 / nseg;
+                for (int g = 0; g < nseg; g++)
+                    for (int q = 0; q < V_LINE_PTS; q++) {
+                        const double s = (g + 0.5 + 0.5 * v_line_x[q]) * inv, w = -0.5 * v_line_w[q] * inv;
+                        const double d0 = av[0] - s * tt[0], d1 = av[1] - s * tt[1], d2 = av[2] - s * tt[2];
+                        const Radial f = radial(k, d0 * d0 + d1 * d1 + d2 * d2);
+                        const double2 z = turned(f, w1c);
+                        const double he = w * re_e(f, z), hes = s * he;
+                        hs += w * re_h(f, z);
+                        es += he;
+                        ess += hes;
+                        esss += s * hes;
+                    }
+                const double an = dot3(av, tn);
+                double ga[3], gt[3] = {0, 0, 0};
+                for (int a = 0; a < 3; a++) ga[a] = hs * tn[a] + an * (es * av[a] - ess * tt[a]);
+                cross_add(gt, hs, ny, av);
+                cross_add(gny, hs, av, tt);
+                for (int a = 0; a < 3; a++) {
+                    gt[a] -= an * (ess * av[a] - esss * tt[a]);
+                    gy[a] += ga[a];
+                    gs[3 * e + a] -= ga[a] + gt[a];
+                    gs[3 * ((e + 1) % 3) + a] += gt[a];
+                }
+            }
+        }
+        gdn *= k * k * t.J;
+        for (int a = 0; a < 3; a++) {
+            gny[a] += gdn / t.J * t.N[a];
+            gN[a] += gdn / t.J * ny[a];
+        }
+        gJ -= gdn * dn / t.J;
+    }
+    normal_to_nodes(t, gN, gJ, gs);
 }
 
 __device__ __forceinline__ void load_tri_d(const double *V, const int *F, int e, double *nod)
@@ -450,62 +398,67 @@ __device__ __forceinline__ void add_vertex_grad(double *grad, const int *F, int 
 }
 
 // ----------------------------------------------------------------------------- VJP kernels
-// the far-field operator F_kj = -int_{T_j} (b G + c dG/dn_x)(x, p_k) dS (fmm_far_field) with
-// dual-number vertex derivatives
-template <int N>
-__device__ __forceinline__ CDn<N> far_entry_d(double k, const Dn<N> *nod, const Dn<N> *y, int rule, double2 nb, double2 nc)
+// The far-field operator F_kj = -int_{T_j} (b G + c dG/dn_x)(x, p_k) dS (fmm_far_field); a group of
+// `grp` lanes (a power of two, at most a warp) takes an element and shares its points.
+__device__ __forceinline__ double group_sum(double v, int grp)
 {
-    CDn<N> f = cdzero<N>();
-    if (nb.x != 0.0 || nb.y != 0.0) cdmac(f, nb, elem_integral_d(k, nod, y, rule, 0));
-    if (nc.x != 0.0 || nc.y != 0.0) cdmac(f, nc, elem_integral_d(k, nod, y, rule, 1));
-    return f;
+    for (int o = grp / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// 2 Re[ sum_k conj(pbar_k) x_j dF_kj/dV_j ] for the vertices of element j; nb = -b, nc = -c
+__global__ void vjp_farpts_kernel(const double *V, const int *F, int nf, double k, int rule, double2 nb, double2 nc,
+                                  const double *pts, int npts, const double2 *pbar, const double2 *x, double *grad, int grp)
+{
+    const int id = blockIdx.x * blockDim.x + threadIdx.x, j = id / grp, l = id % grp;
+    double g9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (j < nf) {
+        double nd[9];
+        load_tri_d(V, F, j, nd);
+        const double2 xj = x[j], z = make_double2(0.0, 0.0);
+        for (int t = l; t < npts; t += grp) {
+            const double2 pb = pbar[t];
+            // w = 2 conj(pbar) x_j
+            const double2 w = make_double2(2.0 * (pb.x * xj.x + pb.y * xj.y), 2.0 * (pb.x * xj.y - pb.y * xj.x));
+            double gs[9], gy[3] = {0, 0, 0};
+            pair_grad<false>(k, nd, pts + 3 * t, nullptr, rule, cmul(w, nb), cmul(w, nc), z, z, gs, gy, nullptr);
+            for (int i = 0; i < 9; i++) g9[i] += gs[i];
+        }
+    }
+    for (int i = 0; i < 9; i++) g9[i] = group_sum(g9[i], grp);
+    if (j < nf && l == 0) add_vertex_grad(grad, F, j, g9);
 }
 
 // right-hand side of the conjugated adjoint system: rhs_j = sum_k F_kj conj(pbar_k)
 __global__ void vjp_adjoint_rhs_kernel(const double *V, const int *F, int nf, double k, int rule, double2 nb, double2 nc,
-                                       const double *pts, int npts, const double2 *pbar, double2 *rhs);
-
-// 2 Re[ sum_k conj(pbar_k) x_j dF_kj/dV_j ] for the vertices of element j; nb = -b, nc = -c
-__global__ void vjp_farpts_kernel(const double *V, const int *F, int nf, double k, int rule, double2 nb, double2 nc,
-                                  const double *pts, int npts, const double2 *pbar, const double2 *x, double *grad)
+                                       const double *pts, int npts, const double2 *pbar, double2 *rhs, int grp)
 {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nf; j += gridDim.x * blockDim.x) {
+    const int id = blockIdx.x * blockDim.x + threadIdx.x, j = id / grp, l = id % grp;
+    double2 acc = make_double2(0.0, 0.0);
+    if (j < nf) {
         double nd[9];
         load_tri_d(V, F, j, nd);
-        Dn<9> nod[9];
-        for (int i = 0; i < 9; i++) nod[i] = dvar<9>(nd[i], i);
-        double g9[9] = {0};
-        double2 xj = x[j];
-        for (int t = 0; t < npts; t++) {
-            Dn<9> y[3] = {dconst<9>(pts[3 * t]), dconst<9>(pts[3 * t + 1]), dconst<9>(pts[3 * t + 2])};
-            CDn<9> f = far_entry_d(k, nod, y, rule, nb, nc);
-            double2 pb = pbar[t];
-            // w = conj(pbar) x_j
-            double2 w = make_double2(pb.x * xj.x + pb.y * xj.y, pb.x * xj.y - pb.y * xj.x);
-            for (int i = 0; i < 9; i++) g9[i] += 2.0 * re_wd(w, f, i);
+        const Tri tr = tri_of(nd);
+        const int nq = v_rule_n[rule];
+        for (int t = l; t < npts; t += grp) {
+            const double *y = pts + 3 * t;
+            double2 I0 = make_double2(0.0, 0.0), I1 = I0;
+            for (int q = 0; q < nq; q++) {
+                const double *bb = &v_rule_bary[rule][3 * q], wq = v_rule_w[rule][q];
+                double d[3];
+                for (int a = 0; a < 3; a++) d[a] = bb[0] * nd[a] + bb[1] * nd[3 + a] + bb[2] * nd[6 + a] - y[a];
+                const Radial f = radial(k, dot3(d, d));
+                // G and h = -(1 - ikr) exp(ikr) / (4 pi r^3)
+                I0 = cadd(I0, cscale(make_double2(f.c, f.s), wq * tr.J * f.f));
+                I1 = cadd(I1, cscale(make_double2(f.c + f.kr * f.s, f.s - f.kr * f.c), -wq * dot3(d, tr.N) * f.fh));
+            }
+            const double2 f = cadd(cmul(nb, I0), cmul(nc, I1));
+            acc = cadd(acc, cconjmul(pbar[t], f));
         }
-        add_vertex_grad(grad, F, j, g9);
     }
-}
-
-__global__ void vjp_adjoint_rhs_kernel(const double *V, const int *F, int nf, double k, int rule, double2 nb, double2 nc,
-                                       const double *pts, int npts, const double2 *pbar, double2 *rhs)
-{
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nf; j += gridDim.x * blockDim.x) {
-        double nd[9];
-        load_tri_d(V, F, j, nd);
-        Dn<1> nod[9];
-        for (int i = 0; i < 9; i++) nod[i] = dconst<1>(nd[i]);
-        double2 acc = make_double2(0.0, 0.0);
-        for (int t = 0; t < npts; t++) {
-            Dn<1> y[3] = {dconst<1>(pts[3 * t]), dconst<1>(pts[3 * t + 1]), dconst<1>(pts[3 * t + 2])};
-            CDn<1> f = far_entry_d(k, nod, y, rule, nb, nc);
-            double2 pb = pbar[t];
-            acc.x += f.re.v * pb.x + f.im.v * pb.y; // F conj(pbar)
-            acc.y += f.im.v * pb.x - f.re.v * pb.y;
-        }
-        rhs[j] = acc;
-    }
+    acc.x = group_sum(acc.x, grp);
+    acc.y = group_sum(acc.y, grp);
+    if (j < nf && l == 0) rhs[j] = acc;
 }
 
 // 2 Re[ mu_i db_i/dV ] with b_i = exp(i k dir.c_i), c_i the centroid (1/3 per vertex)
@@ -528,53 +481,139 @@ __global__ void vjp_rhs_kernel(const double *V, const int *F, int nf, double k, 
     }
 }
 
-// near pairs: -2 Re[ mu_i x_j dA_ij ], A_ij = b int_Tj G(., c_i) + c int_Tj dG/dn(., c_i);
-// slots 0..8 the vertices of T_j, 9..11 the centroid c_i (1/3 to each vertex of T_i)
-__global__ void vjp_near_kernel(const double *V, const int *F, int nf, const int *near_beg, const int *near_col,
-                                double k, double2 bco, double2 cco, int rule, const double2 *mu, const double2 *x,
-                                double *grad)
+// near pairs i != j: -2 Re[ mu_i x_j dA_ij ], A_ij = b I0 + c I1 and (BM) alpha (b K'_ij + c N_ij), one
+// thread per entry of the near-field matrix.  The source's vertices take their share at once; by
+// the target's centroid and unit normal the sums over its row go to tgt[i][6].
+template <bool BM>
+__global__ void __launch_bounds__(128)
+vjp_near_kernel(const double *V, const int *F, int nf, long long nnz, const int *__restrict__ near_beg,
+                const int *__restrict__ near_col, double k, double2 bco, double2 cco, double2 alpha, int rule,
+                const double2 *mu, const double2 *x, double *grad, double *tgt)
 {
-    int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int nwt = (gridDim.x * blockDim.x) >> 5;
-    for (int i = warp; i < nf; i += nwt) {
-        double ndi[9], ci[3];
-        load_tri_d(V, F, i, ndi);
-        for (int a = 0; a < 3; a++) ci[a] = ndi[a] + (2.0 / 3.0) * (0.5 * (ndi[3 + a] + ndi[6 + a]) - ndi[a]);
-        double2 mi = mu[i];
-        double gi[9] = {0};
-        for (int s = near_beg[i] + lane; s < near_beg[i + 1]; s += 32) {
-            int j = near_col[s];
-            double nd[9];
-            load_tri_d(V, F, j, nd);
-            double2 xj = x[j];
-            // w = -(mu_i x_j)
-            double2 w = make_double2(-(mi.x * xj.x - mi.y * xj.y), -(mi.x * xj.y + mi.y * xj.x));
-            double g9[9];
-            if (i == j) {
-                Dn<9> nod[9];
-                for (int q = 0; q < 9; q++) nod[q] = dvar<9>(nd[q], q);
-                CDn<9> v = cdzero<9>();
-                if (bco.x != 0.0 || bco.y != 0.0) cdmac(v, bco, elem_integral_sgl_d(k, nod, 0));
-                if (cco.x != 0.0 || cco.y != 0.0) cdmac(v, cco, elem_integral_sgl_d(k, nod, 1));
-                for (int q = 0; q < 9; q++) g9[q] = 2.0 * re_wd(w, v, q);
-                add_vertex_grad(grad, F, j, g9);
-            } else {
-                Dn<12> nod[9], y[3];
-                for (int q = 0; q < 9; q++) nod[q] = dvar<12>(nd[q], q);
-                for (int a = 0; a < 3; a++) y[a] = dvar<12>(ci[a], 9 + a);
-                CDn<12> v = cdzero<12>();
-                if (bco.x != 0.0 || bco.y != 0.0) cdmac(v, bco, elem_integral_d(k, nod, y, rule, 0));
-                if (cco.x != 0.0 || cco.y != 0.0) cdmac(v, cco, elem_integral_d(k, nod, y, rule, 1));
-                for (int q = 0; q < 9; q++) g9[q] = 2.0 * re_wd(w, v, q);
-                add_vertex_grad(grad, F, j, g9);
-                for (int a = 0; a < 3; a++) {
-                    double gc = 2.0 * re_wd(w, v, 9 + a) / 3.0;
-                    for (int t = 0; t < 3; t++) gi[3 * t + a] += gc;
-                }
-            }
+    const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const bool on = s < nnz;
+    int i = 0;
+    double t6[6] = {0, 0, 0, 0, 0, 0};
+    if (on) {
+        // row of entry s: the last i with near_beg[i] <= s
+        int hi = nf;
+        while (hi - i > 1) {
+            const int mid = (i + hi) >> 1;
+            if (near_beg[mid] <= s) i = mid; else hi = mid;
         }
-        add_vertex_grad(grad, F, i, gi);
+        const int j = near_col[s];
+        if (i != j) {
+            double ndi[9], nd[9], y[3], ny[3];
+            load_tri_d(V, F, i, ndi);
+            load_tri_d(V, F, j, nd);
+            for (int a = 0; a < 3; a++) y[a] = ndi[a] + (2.0 / 3.0) * (0.5 * (ndi[3 + a] + ndi[6 + a]) - ndi[a]);
+            if (BM) {
+                const Tri ti = tri_of(ndi);
+                for (int a = 0; a < 3; a++) ny[a] = ti.N[a] / ti.J;
+            }
+            const double2 w = cscale(cmul(mu[i], x[j]), -2.0), w1 = BM ? cmul(w, alpha) : w;
+            double gs[9];
+            pair_grad<BM>(k, nd, y, ny, rule, cmul(w, bco), cmul(w, cco), cmul(w1, bco), cmul(w1, cco), gs, t6, t6 + 3);
+            add_vertex_grad(grad, F, j, gs);
+        }
     }
+    // rows are longer than a warp's 32 entries on most meshes: one addition per warp and row
+    constexpr int NT = BM ? 6 : 3;
+    const int i0 = __shfl_sync(0xffffffffu, i, 0);
+    if (__all_sync(0xffffffffu, !on || i == i0)) {
+        for (int a = 0; a < NT; a++) t6[a] = group_sum(t6[a], 32);
+        if ((threadIdx.x & 31) == 0 && on)
+            for (int a = 0; a < NT; a++) atomicAdd(&tgt[6 * (size_t)i + a], t6[a]);
+    } else if (on) {
+        for (int a = 0; a < NT; a++) atomicAdd(&tgt[6 * (size_t)i + a], t6[a]);
+    }
+}
+
+// The target sides of the near pairs (tgt: gradients by centroid and unit normal) to the vertices,
+// and the self terms: b G (three sub-triangles at the centroid by the collapsed rule; dG/dn
+// vanishes on the element's own plane, wherever its vertices are) and (BM) alpha c N_ii
+// (K'_ii = 0), the Hadamard finite part -(1/4 pi) [sum over edges of hL int exp(ikr)/r^3 - 2 pi i k],
+// hL = |u x t| with u from the centroid to the edge and t along it.  One thread per element and
+// sub-triangle / edge.
+__global__ void vjp_near_self_kernel(const double *V, const int *F, int nf, double k, double2 bco, double2 cco,
+                                     double2 alpha, const double2 *mu, const double2 *x, const double *tgt, double *grad)
+{
+    const int id = blockIdx.x * blockDim.x + threadIdx.x, i = id / 3, e = id % 3, e1 = (e + 1) % 3;
+    if (i >= nf) return;
+    const bool hb = bco.x != 0.0 || bco.y != 0.0;
+    const bool hn = (cco.x != 0.0 || cco.y != 0.0) && (alpha.x != 0.0 || alpha.y != 0.0);
+    double nd[9], g9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, gc[3] = {0, 0, 0}, c[3];
+    load_tri_d(V, F, i, nd);
+    if (e == 0) {
+        const double *g = tgt + 6 * (size_t)i;
+        const Tri tr = tri_of(nd);
+        // unit normal n = N / J: dJ/dN = n, so by N: (g - (g.n) n) / J
+        double n[3], gN[3];
+        for (int a = 0; a < 3; a++) n[a] = tr.N[a] / tr.J;
+        const double gn = dot3(g + 3, n);
+        for (int a = 0; a < 3; a++) {
+            gN[a] = (g[3 + a] - gn * n[a]) / tr.J;
+            gc[a] = g[a];
+        }
+        normal_to_nodes(tr, gN, 0.0, g9);
+    }
+    const double2 w = cscale(cmul(mu[i], x[i]), -2.0), z = make_double2(0.0, 0.0);
+    double va[3], vb[3], ga[3] = {0, 0, 0}, gb[3] = {0, 0, 0};
+    for (int a = 0; a < 3; a++) {
+        c[a] = nd[a] + (2.0 / 3.0) * (0.5 * (nd[3 + a] + nd[6 + a]) - nd[a]);
+        va[a] = nd[3 * e + a];
+        vb[a] = nd[3 * e1 + a];
+    }
+    if (hb) {
+        const double sub[9] = {va[0], va[1], va[2], vb[0], vb[1], vb[2], c[0], c[1], c[2]};
+        double gs[9], gy[3] = {0, 0, 0};
+        pair_grad<false>(k, sub, c, nullptr, 0, cmul(w, bco), z, z, z, gs, gy, nullptr);
+        for (int a = 0; a < 3; a++) {
+            ga[a] += gs[a];
+            gb[a] += gs[3 + a];
+            gc[a] += gs[6 + a] + gy[a];
+        }
+    }
+    if (hn) {
+        const double2 w1 = cscale(cmul(cmul(w, alpha), cco), -1.0 / (4.0 * FMM_PI));
+        double u[3], t[3], uc[3] = {0, 0, 0}, gu[3] = {0, 0, 0}, gt[3] = {0, 0, 0};
+        for (int a = 0; a < 3; a++) {
+            u[a] = va[a] - c[a];
+            t[a] = vb[a] - va[a];
+        }
+        cross_add(uc, 1.0, u, t);
+        const double hL = sqrt(dot3(uc, uc)), len = sqrt(dot3(t, t));
+        const int nseg = edge_segments_v(len, hL / len);
+        // p = exp(ikr)/r^3, p'/r = exp(ikr) (ikr - 3)/r^5
+        double ps = 0.0, es = 0.0, ess = 0.0, esss = 0.0;
+        for (int g = 0; g < nseg; g++)
+            for (int q = 0; q < V_LINE_PTS; q++) {
+                const double s = (g + 0.5 + 0.5 * v_line_x[q]) / nseg, wl = 0.5 * v_line_w[q] / nseg;
+                double d[3];
+                for (int a = 0; a < 3; a++) d[a] = u[a] + s * t[a];
+                const Radial f = radial(k, dot3(d, d));
+                const double2 zw = turned(f, w1);
+                const double f3 = wl * (4.0 * FMM_PI) * f.fh, f5 = wl * (4.0 * FMM_PI) * f.fe;
+                const double pe = -f5 * (3.0 * zw.x + f.kr * zw.y);
+                ps += f3 * zw.x;
+                es += pe;
+                ess += s * pe;
+                esss += s * s * pe;
+            }
+        cross_add(gu, ps / hL, t, uc);
+        cross_add(gt, ps / hL, uc, u);
+        for (int a = 0; a < 3; a++) {
+            gu[a] += hL * (es * u[a] + ess * t[a]);
+            gt[a] += hL * (ess * u[a] + esss * t[a]);
+            ga[a] += gu[a] - gt[a];
+            gb[a] += gt[a];
+            gc[a] -= gu[a];
+        }
+    }
+    for (int t = 0; t < 3; t++)
+        for (int a = 0; a < 3; a++)
+            g9[3 * t + a] += gc[a] / 3.0 + (t == e ? ga[a] : 0.0) + (t == e1 ? gb[a] : 0.0);
+    add_vertex_grad(grad, F, i, g9);
 }
 
 // far pairs, target side: -2 Re[ mu_i d/dc_i sum_nm D_i[nm] R_n^m(c_i - C) ], 1/3 per vertex
@@ -585,75 +624,21 @@ __global__ void vjp_far_target_kernel(const double *V, const int *F, int nf, int
         double nd[9];
         load_tri_d(V, F, i, nd);
         int b = elem_leaf[i];
-        Dn<3> v[3];
+        double v[3];
         for (int a = 0; a < 3; a++) {
             double c = nd[a] + (2.0 / 3.0) * (0.5 * (nd[3 + a] + nd[6 + a]) - nd[a]);
-            v[a] = dvar<3>(c - box_ctr[3 * b + a], a);
+            v[a] = c - box_ctr[3 * b + a];
         }
         const double2 *coef[1] = {D + (size_t)b * pl * pl};
-        CDn<3> t[1];
-        eval_expansions_d<3, 1>(pl, k, v, coef, t);
+        double2 f[1], g[1][3];
+        eval_expansions<1, true>(pl, k, v, coef, f, g);
         double2 m = mu[i], w = make_double2(-m.x, -m.y);
         double g9[9];
         for (int a = 0; a < 3; a++) {
-            double gc = 2.0 * re_wd(w, t[0], a) / 3.0;
+            double gc = 2.0 * re_mul(w, g[0][a]) / 3.0;
             for (int q = 0; q < 3; q++) g9[3 * q + a] = gc;
         }
         add_vertex_grad(grad, F, i, g9);
-    }
-}
-
-// Burton-Miller near pairs: -2 Re[ mu_i x_j d/dV alpha (b K'_ij + c N_ij) ], both elements'
-// vertices as dual slots (0..8 source j, 9..17 target i: its centroid and unit normal); the
-// self term N_ii (K'_ii = 0) in the element's own 9 slots
-__global__ void vjp_near_bm_kernel(const double *V, const int *F, int nf, const int *near_beg, const int *near_col,
-                                   double k, double2 bco, double2 cco, double2 alpha, int rule, const double2 *mu,
-                                   const double2 *x, double *grad)
-{
-    int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int nwt = (gridDim.x * blockDim.x) >> 5;
-    const bool hb = bco.x != 0.0 || bco.y != 0.0, hc = cco.x != 0.0 || cco.y != 0.0;
-    for (int i = warp; i < nf; i += nwt) {
-        double ndi[9];
-        load_tri_d(V, F, i, ndi);
-        double2 mi = mu[i];
-        double gi[9] = {0};
-        for (int s = near_beg[i] + lane; s < near_beg[i + 1]; s += 32) {
-            int j = near_col[s];
-            double2 xj = x[j];
-            // w = -(mu_i x_j alpha)
-            double2 mx = make_double2(mi.x * xj.x - mi.y * xj.y, mi.x * xj.y + mi.y * xj.x);
-            double2 w = make_double2(-(mx.x * alpha.x - mx.y * alpha.y), -(mx.x * alpha.y + mx.y * alpha.x));
-            if (i == j) {
-                if (!hc) continue;
-                Dn<9> nod[9];
-                for (int q = 0; q < 9; q++) nod[q] = dvar<9>(ndi[q], q);
-                CDn<9> v = cdzero<9>();
-                cdmac(v, cco, elem_hyper_self_d(k, nod));
-                double g9[9];
-                for (int q = 0; q < 9; q++) g9[q] = 2.0 * re_wd(w, v, q);
-                add_vertex_grad(grad, F, j, g9);
-            } else {
-                double nd[9];
-                load_tri_d(V, F, j, nd);
-                Dn<18> nod[9], tgt[9], y[3], ncy[3], Jy;
-                for (int q = 0; q < 9; q++) {
-                    nod[q] = dvar<18>(nd[q], q);
-                    tgt[q] = dvar<18>(ndi[q], 9 + q);
-                }
-                centroid_d(tgt, y);
-                tri_normal_d(tgt, ncy, Jy);
-                Dn<18> ny[3] = {ncy[0] / Jy, ncy[1] / Jy, ncy[2] / Jy};
-                CDn<18> v = cdzero<18>();
-                if (hb) cdmac(v, bco, elem_dGdny_d(k, nod, y, ny, rule));
-                if (hc) cdmac(v, cco, elem_hyper_near_d(k, nod, y, ny, rule));
-                double g9[9];
-                for (int q = 0; q < 9; q++) g9[q] = 2.0 * re_wd(w, v, q);
-                add_vertex_grad(grad, F, j, g9);
-                for (int q = 0; q < 9; q++) gi[q] += 2.0 * re_wd(w, v, 9 + q);
-            }
-        }
-        add_vertex_grad(grad, F, i, gi);
     }
 }
 
@@ -665,30 +650,30 @@ __global__ void vjp_far_target_bm_kernel(const double *V, const int *F, int nf, 
 {
     const int po = pl + 1;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x) {
-        double nd[9];
+        double nd[9], v[3], n[3], gc[3], gn[3], gN[3], g9[9];
         load_tri_d(V, F, i, nd);
         int b = elem_leaf[i];
-        Dn<9> nod[9], c[3], nc[3], J;
-        for (int q = 0; q < 9; q++) nod[q] = dvar<9>(nd[q], q);
-        centroid_d(nod, c);
-        tri_normal_d(nod, nc, J);
-        Dn<9> v[3];
-        for (int a = 0; a < 3; a++) v[a] = c[a] - dconst<9>(box_ctr[3 * b + a]);
+        const Tri tr = tri_of(nd);
+        for (int a = 0; a < 3; a++) {
+            v[a] = nd[a] + (2.0 / 3.0) * (0.5 * (nd[3 + a] + nd[6 + a]) - nd[a]) - box_ctr[3 * b + a];
+            n[a] = tr.N[a] / tr.J;
+        }
         const double2 *coef[3] = {Dz + (size_t)b * po * po, Dp + (size_t)b * po * po, Dm + (size_t)b * po * po};
-        CDn<9> e[3];
-        eval_expansions_d<9, 3>(po, k, v, coef, e);
-        CDn<9> gx, gy;
-        gx.re = 0.5 * (e[1].re + e[2].re);
-        gx.im = 0.5 * (e[1].im + e[2].im);
-        gy.re = 0.5 * (e[1].im - e[2].im);
-        gy.im = -0.5 * (e[1].re - e[2].re);
-        CDn<9> f;
-        f.re = (gx.re * nc[0] + gy.re * nc[1] + e[0].re * nc[2]) / J;
-        f.im = (gx.im * nc[0] + gy.im * nc[1] + e[0].im * nc[2]) / J;
-        double2 m = mu[i];
-        double2 w = make_double2(-(m.x * alpha.x - m.y * alpha.y), -(m.x * alpha.y + m.y * alpha.x));
-        double g9[9];
-        for (int q = 0; q < 9; q++) g9[q] = 2.0 * re_wd(w, f, q);
+        double2 e[3], de[3][3], g[3], H[3][3];
+        eval_expansions<3, true>(po, k, v, coef, e, de);
+        cartesian(e, de, g, H);
+        // f = n . grad phi(c)
+        const double2 w = cscale(cmul(mu[i], alpha), -2.0);
+        for (int a = 0; a < 3; a++) {
+            gc[a] = re_mul(w, H[0][a]) * n[0] + re_mul(w, H[1][a]) * n[1] + re_mul(w, H[2][a]) * n[2];
+            gn[a] = re_mul(w, g[a]);
+        }
+        const double q = dot3(gn, n);
+        for (int a = 0; a < 3; a++) {
+            gN[a] = (gn[a] - q * n[a]) / tr.J;
+            for (int t = 0; t < 3; t++) g9[3 * t + a] = gc[a] / 3.0;
+        }
+        normal_to_nodes(tr, gN, 0.0, g9);
         add_vertex_grad(grad, F, i, g9);
     }
 }
@@ -699,25 +684,24 @@ __global__ void vjp_rhs_bm_kernel(const double *V, const int *F, int nf, double 
                                   double2 alpha, const double2 *mu, double *grad)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x) {
-        double nd[9];
+        double nd[9], c[3], n[3], gN[3], g9[9];
+        const double dv[3] = {dx, dy, dz};
         load_tri_d(V, F, i, nd);
-        Dn<9> nod[9], c[3], nc[3], J;
-        for (int q = 0; q < 9; q++) nod[q] = dvar<9>(nd[q], q);
-        centroid_d(nod, c);
-        tri_normal_d(nod, nc, J);
-        Dn<9> ph = k * (dx * c[0] + dy * c[1] + dz * c[2]);
-        Dn<9> kd = k * ((dx * nc[0] + dy * nc[1] + dz * nc[2]) / J);
-        Dn<9> sn, cs;
-        dsincos(ph, sn, cs);
-        // alpha i kd (cs + i sn) = alpha kd (-sn + i cs)
-        CDn<9> t;
-        t.re = -(kd * sn);
-        t.im = kd * cs;
-        CDn<9> f = cdzero<9>();
-        cdmac(f, alpha, t);
-        double2 m = mu[i];
-        double g9[9];
-        for (int q = 0; q < 9; q++) g9[q] = 2.0 * re_wd(m, f, q);
+        const Tri tr = tri_of(nd);
+        for (int a = 0; a < 3; a++) {
+            c[a] = nd[a] + (2.0 / 3.0) * (0.5 * (nd[3 + a] + nd[6 + a]) - nd[a]);
+            n[a] = tr.N[a] / tr.J;
+        }
+        double sn, cs;
+        sincos(k * dot3(dv, c), &sn, &cs);
+        // b = i k alpha (d.n) e^{ik d.c}: by n i k alpha e d, by c i k b d
+        const double2 z = cmul(cscale(cmul(mu[i], alpha), 2.0 * k), make_double2(-sn, cs));  // 2 mu alpha i k e
+        const double dn = dot3(dv, n), gc = -k * dn * z.y, gn = z.x, gq = gn * dn;
+        for (int a = 0; a < 3; a++) {
+            gN[a] = (gn * dv[a] - gq * n[a]) / tr.J;
+            for (int t = 0; t < 3; t++) g9[3 * t + a] = gc * dv[a] / 3.0;
+        }
+        normal_to_nodes(tr, gN, 0.0, g9);
         add_vertex_grad(grad, F, i, g9);
     }
 }
@@ -753,59 +737,41 @@ __global__ void deriv_coef_kernel(int nb, int pl, double k, const double2 *Psi, 
     }
 }
 
-// far pairs, source side: -2 Re[ x_j d/dV_j sum_q w_q (b phi(y_q) J + c grad phi(y_q) . Nc) ]
-// with phi = sum_nm Psi_j[nm] R_n^m(. - C) and Nc = J nh the unnormalised normal
-__global__ void vjp_far_source_kernel(const double *V, const int *F, int nf, int pl, double k, int rule, double2 bco,
-                                      double2 cco, const int *elem_leaf, const double *box_ctr, const double2 *Psi,
-                                      const double2 *Dz, const double2 *Dp, const double2 *Dm, const double2 *x,
-                                      double *grad)
+// far pairs, source side: -2 Re[ x_j d/dV_j sum_q w_q (b phi(y_q) J + c grad phi(y_q) . N) ] with
+// phi = sum_nm Psi_j[nm] R_n^m(. - C), grad phi and its gradient from its derivative expansions, and
+// N = J nh the unnormalised normal; one thread per element and quadrature point
+__global__ void __launch_bounds__(128)
+vjp_far_source_kernel(const double *V, const int *F, int nf, int pl, double k, int rule, double2 bco, double2 cco,
+                      const int *elem_leaf, const double *box_ctr, const double2 *Psi, const double2 *Dz,
+                      const double2 *Dp, const double2 *Dm, const double2 *x, double *grad)
 {
-    const int po = pl + 1;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nf; j += gridDim.x * blockDim.x) {
-        double nd[9];
-        load_tri_d(V, F, j, nd);
-        int b = elem_leaf[j];
-        Dn<9> nod[9];
-        for (int i = 0; i < 9; i++) nod[i] = dvar<9>(nd[i], i);
-        Dn<9> nc[3], J;
-        tri_normal_d(nod, nc, J);
-        // the order pl expansion zero-padded to pl + 1 shares the evaluation with its derivatives
-        const double2 *coef[4] = {nullptr, Dz + (size_t)b * po * po, Dp + (size_t)b * po * po, Dm + (size_t)b * po * po};
-        CDn<9> S = cdzero<9>();
-        int nq = v_rule_n[rule];
-        for (int q = 0; q < nq; q++) {
-            const double *bb = &v_rule_bary[rule][3 * q];
-            Dn<9> v[3];
-            for (int a = 0; a < 3; a++)
-                v[a] = bb[0] * nod[a] + bb[1] * nod[3 + a] + bb[2] * nod[6 + a] - dconst<9>(box_ctr[3 * b + a]);
-            CDn<9> e[4];
-            const double2 *c1[1] = {Psi + (size_t)b * pl * pl};
-            eval_expansions_d<9, 1>(pl, k, v, c1, e);
-            eval_expansions_d<9, 3>(po, k, v, coef + 1, e + 1);
-            // grad phi: dx = (d+ + d-)/2, dy = (d+ - d-)/(2i), dz
-            CDn<9> gx, gy;
-            gx.re = 0.5 * (e[2].re + e[3].re);
-            gx.im = 0.5 * (e[2].im + e[3].im);
-            gy.re = 0.5 * (e[2].im - e[3].im);
-            gy.im = -0.5 * (e[2].re - e[3].re);
-            CDn<9> dn;
-            dn.re = gx.re * nc[0] + gy.re * nc[1] + e[1].re * nc[2];
-            dn.im = gx.im * nc[0] + gy.im * nc[1] + e[1].im * nc[2];
-            CDn<9> phiJ;
-            phiJ.re = e[0].re * J;
-            phiJ.im = e[0].im * J;
-            double wq = v_rule_w[rule][q];
-            CDn<9> t = cdzero<9>();
-            cdmac(t, bco, phiJ);
-            cdmac(t, cco, dn);
-            S.re = S.re + wq * t.re;
-            S.im = S.im + wq * t.im;
-        }
-        double2 xj = x[j], w = make_double2(-xj.x, -xj.y);
-        double g9[9];
-        for (int i = 0; i < 9; i++) g9[i] = 2.0 * re_wd(w, S, i);
-        add_vertex_grad(grad, F, j, g9);
+    const int po = pl + 1, nq = v_rule_n[rule], id = blockIdx.x * blockDim.x + threadIdx.x, q = id / nf, j = id % nf;
+    if (q >= nq) return;
+    double nd[9], v[3], gs[9], gN[3], gJ = 0.0;
+    load_tri_d(V, F, j, nd);
+    const int b = elem_leaf[j];
+    const Tri tr = tri_of(nd);
+    const double *bb = &v_rule_bary[rule][3 * q], wq = v_rule_w[rule][q];
+    for (int a = 0; a < 3; a++) v[a] = bb[0] * nd[a] + bb[1] * nd[3 + a] + bb[2] * nd[6 + a] - box_ctr[3 * b + a];
+    const double2 w = cscale(x[j], -2.0 * wq), wb = cmul(w, bco), wc = cmul(w, cco);
+    const double2 *coef[3] = {Dz + (size_t)b * po * po, Dp + (size_t)b * po * po, Dm + (size_t)b * po * po};
+    double2 e[3], de[3][3], g[3], H[3][3];
+    eval_expansions<3, true>(po, k, v, coef, e, de);
+    cartesian(e, de, g, H);
+    if (bco.x != 0.0 || bco.y != 0.0) {
+        const double2 *c1[1] = {Psi + (size_t)b * pl * pl};
+        double2 phi[1];
+        eval_expansions<1, false>(pl, k, v, c1, phi, nullptr);
+        gJ = re_mul(wb, phi[0]);
     }
+    for (int a = 0; a < 3; a++) {
+        const double gy = tr.J * re_mul(wb, g[a]) + re_mul(wc, H[0][a]) * tr.N[0] + re_mul(wc, H[1][a]) * tr.N[1] +
+                          re_mul(wc, H[2][a]) * tr.N[2];
+        gN[a] = re_mul(wc, g[a]);
+        for (int t = 0; t < 3; t++) gs[3 * t + a] = bb[t] * gy;
+    }
+    normal_to_nodes(tr, gN, gJ, gs);
+    add_vertex_grad(grad, F, j, gs);
 }
 
 // g_beta[j] = i k ( (w_j - z_j) x_j - (alpha/2) mu_j x_j ): the admittance derivative per
@@ -824,6 +790,14 @@ __global__ void vjp_admittance_kernel(int nf, double k, double2 alpha, const dou
 } // namespace fmm
 
 using namespace fmm;
+
+// lanes that share an element's far points: a power of two up to a warp
+static int point_group(int npts)
+{
+    int g = 1;
+    while (g < 32 && g < npts) g *= 2;
+    return g;
+}
 
 static std::vector<double> leaf_centres(const Plan *P)
 {
@@ -862,7 +836,7 @@ extern "C" int fmm_vjp(fmm_plan *plan, const cuDoubleComplex *x, const double *d
     size_t loc = (size_t)nbl * pl * pl, locd = (size_t)nbl * (pl + 1) * (pl + 1);
     double2 *xd = nullptr, *pb = nullptr, *rhs = nullptr, *mu = nullptr, *tmp = nullptr, *D = nullptr, *Dz = nullptr, *Dp = nullptr,
             *Dm = nullptr;
-    double *ptd = nullptr, *gd = nullptr, *ctr = nullptr;
+    double *ptd = nullptr, *gd = nullptr, *ctr = nullptr, *tgt = nullptr;
     std::vector<double> hctr = leaf_centres(P);
 #define VTRY(call)                                                                                              \
     do {                                                                                                        \
@@ -881,17 +855,21 @@ extern "C" int fmm_vjp(fmm_plan *plan, const cuDoubleComplex *x, const double *d
     VTRY(cudaMalloc(&ptd, sizeof(double) * 3 * npts));
     VTRY(cudaMalloc(&gd, sizeof(double) * 3 * nv));
     VTRY(cudaMalloc(&ctr, sizeof(double) * hctr.size()));
+    VTRY(cudaMalloc(&tgt, sizeof(double) * 6 * nf));
     VTRY(cudaMemcpyAsync(xd, x, sizeof(double2) * nf, cudaMemcpyDefault, st));
     VTRY(cudaMemcpyAsync(pb, pbar, sizeof(double2) * npts, cudaMemcpyDefault, st));
     VTRY(cudaMemcpyAsync(ptd, pts, sizeof(double) * 3 * npts, cudaMemcpyDefault, st));
     VTRY(cudaMemcpyAsync(ctr, hctr.data(), sizeof(double) * hctr.size(), cudaMemcpyHostToDevice, st));
     VTRY(cudaMemsetAsync(gd, 0, sizeof(double) * 3 * nv, st));
     VTRY(cudaMemsetAsync(mu, 0, sizeof(double2) * nf, st));
+    VTRY(cudaMemsetAsync(tgt, 0, sizeof(double) * 6 * nf, st));
     {
-        const int T = 128, B = std::min((nf + T - 1) / T, 152 * 8);
+        // elementwise kernels: small CTAs, so that a few thousand elements reach every SM
+        const int T = 32, B = (nf + T - 1) / T, grp = point_group(npts), PB = (int)(((long long)nf * grp + 127) / 128);
         // adjoint system A^T mu = F^T conj(pbar)
         double2 nb = make_double2(-P->opt.b_re, -P->opt.b_im), nc = make_double2(-P->opt.c_re, -P->opt.c_im);
-        vjp_adjoint_rhs_kernel<<<B, T, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, P->opt.rule, nb, nc, ptd, npts, pb, rhs);
+        vjp_adjoint_rhs_kernel<<<PB, 128, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, P->opt.rule, nb, nc, ptd, npts, pb,
+                                                  rhs, grp);
         VTRY(cudaGetLastError());
         int it = 0;
         double rr = 0.0;
@@ -905,7 +883,7 @@ extern "C" int fmm_vjp(fmm_plan *plan, const cuDoubleComplex *x, const double *d
         deriv_coef_kernel<<<(unsigned)std::min<size_t>((locd + 255) / 256, 152 * 8), 256, 0, st>>>(nbl, pl, P->opt.k,
                                                                                                  P->lev[lmax].Dl64, Dz, Dp, Dm);
         double2 bco = make_double2(P->opt.b_re, P->opt.b_im), cco = make_double2(P->opt.c_re, P->opt.c_im);
-        vjp_far_source_kernel<<<B, T, 0, st>>>(P->V_dev, P->F_dev, nf, pl, P->opt.k, P->opt.rule, bco, cco, P->elem_leaf,
+        vjp_far_source_kernel<<<(unsigned)(((long long)nf * 9 + 127) / 128), 128, 0, st>>>(P->V_dev, P->F_dev, nf, pl, P->opt.k, P->opt.rule, bco, cco, P->elem_leaf,
                                                ctr, P->lev[lmax].Dl64, Dz, Dp, Dm, xd, gd);
         vjp_far_target_kernel<<<B, T, 0, st>>>(P->V_dev, P->F_dev, nf, pl, P->opt.k, P->elem_leaf, ctr, D, mu, gd);
         const double2 alpha = make_double2(P->opt.alpha_re, P->opt.alpha_im);
@@ -917,14 +895,18 @@ extern "C" int fmm_vjp(fmm_plan *plan, const cuDoubleComplex *x, const double *d
                                                                                                      D, Dz, Dp, Dm);
             vjp_far_target_bm_kernel<<<B, T, 0, st>>>(P->V_dev, P->F_dev, nf, pl, P->opt.k, alpha, P->elem_leaf, ctr, Dz,
                                                       Dp, Dm, mu, gd);
-            vjp_near_bm_kernel<<<std::min((nf + 3) / 4, 152 * 16), 128, 0, st>>>(
-                P->V_dev, P->F_dev, nf, P->near_beg, P->near_col, P->opt.k, bco, cco, alpha, P->opt.rule, mu, xd, gd);
             if (dir)
                 vjp_rhs_bm_kernel<<<B, T, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, dir[0], dir[1], dir[2], alpha, mu, gd);
         }
-        vjp_near_kernel<<<std::min((nf + 7) / 8, 152 * 16), 256, 0, st>>>(P->V_dev, P->F_dev, nf, P->near_beg, P->near_col,
-                                                                        P->opt.k, bco, cco, P->opt.rule, mu, xd, gd);
-        vjp_farpts_kernel<<<B, T, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, P->opt.rule, nb, nc, ptd, npts, pb, xd, gd);
+        const unsigned NB = (unsigned)((P->num_near + 127) / 128);
+        if (bm)
+            vjp_near_kernel<true><<<NB, 128, 0, st>>>(P->V_dev, P->F_dev, nf, P->num_near, P->near_beg, P->near_col, P->opt.k,
+                                                      bco, cco, alpha, P->opt.rule, mu, xd, gd, tgt);
+        else
+            vjp_near_kernel<false><<<NB, 128, 0, st>>>(P->V_dev, P->F_dev, nf, P->num_near, P->near_beg, P->near_col, P->opt.k,
+                                                       bco, cco, alpha, P->opt.rule, mu, xd, gd, tgt);
+        vjp_near_self_kernel<<<(3 * nf + T - 1) / T, T, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, bco, cco, alpha, mu, xd, tgt, gd);
+        vjp_farpts_kernel<<<PB, 128, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, P->opt.rule, nb, nc, ptd, npts, pb, xd, gd, grp);
         if (dir)
             vjp_rhs_kernel<<<B, T, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, dir[0], dir[1], dir[2], mu, gd);
         VTRY(cudaGetLastError());
@@ -940,7 +922,7 @@ extern "C" int fmm_vjp(fmm_plan *plan, const cuDoubleComplex *x, const double *d
 done:
 #undef VTRY
     for (void *q : {(void *)xd, (void *)pb, (void *)rhs, (void *)mu, (void *)tmp, (void *)D, (void *)Dz, (void *)Dp, (void *)Dm,
-                    (void *)ptd, (void *)gd, (void *)ctr})
+                    (void *)ptd, (void *)gd, (void *)ctr, (void *)tgt})
         if (q) cudaFree(q);
     return rc;
 }
@@ -1021,8 +1003,9 @@ extern "C" int fmm_vjp_admittance(fmm_plan *plan, const cuDoubleComplex *x, cons
     {
         const int T = 128, B = std::min((nf + T - 1) / T, 152 * 8);
         // w = (dF/db)^T conj(pbar): the far-field operator -int G of unit b
-        vjp_adjoint_rhs_kernel<<<B, T, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, P->opt.rule, make_double2(-1.0, 0.0),
-                                                make_double2(0.0, 0.0), ptd, npts, pb, w);
+        const int grp = point_group(npts), PB = (int)(((long long)nf * grp + 127) / 128);
+        vjp_adjoint_rhs_kernel<<<PB, 128, 0, st>>>(P->V_dev, P->F_dev, nf, P->opt.k, P->opt.rule, make_double2(-1.0, 0.0),
+                                                  make_double2(0.0, 0.0), ptd, npts, pb, w, grp);
         vjp_admittance_kernel<<<B, T, 0, st>>>(nf, P->opt.k, make_double2(P->opt.alpha_re, P->opt.alpha_im), w, z, mu, xd, g);
         ATRY(cudaGetLastError());
         hg.resize(nf);
