@@ -1,348 +1,343 @@
-// Batched translations for the mixed-precision matvec: M2M, M2L and L2L as direction-grouped
-// tiles of register-blocked small matrix products.
+// Batched translations for the mixed-precision matvec: M2M, M2L and L2L as tiles of
+// register-blocked small matrix products.
 //
 // Every translation is rotation - coaxial - rotation (RCR) as in transMatsVecsMul_SR_rcr
-// (reference translation.cu:1864-1961).  All translations of one level that share a
-// direction (one of 316 M2L offsets, or one of 8 octants for M2M/L2L) use the same real
-// rotation block H, the same phases e^{i m phi} and the same coaxial blocks.  A CTA takes TC
-// of them as the columns of a matrix:
-//   stage 0  gather the TC source vectors into shared memory as X[nm][t] and apply
-//            e^{i m phi} (zero-padded to order p, zero columns beyond the item's count);
-//   stage 1  W_n = H_n X_n for every degree n (H_n is (2n+1) x (2n+1), real);
-//   stage 2  X_m = C_|m| W_m for every order m (C_|m| is the (p-|m|)^2 coaxial block, complex;
-//            +m and -m share it);
-//   stage 3  Y_n = H_n X_n for n < pout, times e^{-i m' phi}, added into the destinations.
-// A thread computes R rows x CG columns of one block per unit of work (CG = TC, or 16-column
-// groups when TC is 32 or 64): the CG-wide rows of X and W are read as shared-memory
-// broadcasts and every H or C entry loaded from L1/L2 feeds 2 CG (real H) or 4 CG (complex
-// C) FMAs.  Units are ordered by cost within each column group so the long blocks start
-// first.  Destinations are added with FP32 vector atomics where several items reach
-// the same box (M2M, M2L), and with a plain read-add-write where every box is reached once
-// (L2L).
+// (reference translation.cu:1864-1961).  Translations of one operator class -- the M2L directions
+// of equal (dz, dx^2 + dy^2), which have one polar angle and one length (61 classes of the 316
+// directions); the octants of M2M / L2L of equal z bit -- share the rotation and coaxial blocks
+// and differ by their azimuthal phases.  A CTA takes TC of them (times the right-hand sides) as the
+// columns of a matrix in shared memory:
+//   gather   x_m e^{i m phi}, as the sums x+_m = x_m + x_-m and differences x-_m = x_m - x_-m;
+//   rotate   W+_n = P_n X+_n, W-_n = Q_n X-_n for every degree n: the rotation block is centrally
+//            symmetric (H_{-m',-m} = H_{m',m}), so it splits into two blocks of half its size;
+//   coaxial  X+-_m = C_m W+-_m for every order m (complex, the same block for both signs);
+//   rotate   back, and write x_+-m = (W+ +- W-)/2 times e^{-+i m phi} into the destinations.
+// A lane owns 4 columns x R rows of one block (a unit): an operand row of 4 columns is two 16-byte
+// shared-memory loads and R table entries one load (the tables are padded for it), for 8 R
+// (rotation) or 32 (coaxial, two rows) multiply-adds, issued as packed pairs (re, im).  The stages work
+// in place: a round of units holds whole blocks, which depend on their own rows only, and writes
+// after a barrier.  That halves the shared memory, so that three CTAs share an SM and its L1 keeps
+// the class's tables.  Every output is summed in the same order whatever the tile.  Destinations
+// are added with FP32 vector atomics where several items reach the same box (M2M, M2L), and with a
+// plain read-add-write where every box is reached once (L2L).
+//
+// What bounds it: the shared-memory / L1 path (16 bytes of table and 32 of operands per lane for 32
+// multiply-adds: 65-80 % busy at p = 10-20) and, at p = 30-40, the latency of table rows from L2.
+// M2L of 16 columns on the 81,920-triangle sphere, against one tile per direction with the whole
+// rotation blocks in two buffers: p = 40 2.50 -> 1.31 ms, p = 30 4.55 -> 2.60, p = 20 6.65 -> 4.03;
+// the sphere's matvec 2.15 -> 1.59 ms, 64 columns on the head 145 -> 117 ms, 24 bodies as a scene
+// 2.74 -> 1.93 ms.  Tried: two CTAs of 128 registers (28 -> 32 ms for 16 columns), 8 columns per
+// lane (28 -> 31), table rows loaded 2 to 6 steps ahead (slower than one ahead).
 #include "plan.h"
+#include "f32x2.cuh"
 #include <algorithm>
 #include <cstdlib>
 #include <vector>
 
 namespace fmm {
 
-static __device__ __forceinline__ void nm_of(int i, int &n, int &m)
+// ---- table layouts
+__host__ __device__ __forceinline__ int up_to(int n, int q) { return (n + q - 1) / q * q; }
+// folded rotation tables: degree n holds P_n as [m = 0..n][rows 0..n, padded to 4], then Q_n as
+// [m = 1..n][rows 1..n, padded to 4]
+static int rot32_size(int p)
 {
-    int q = (int)sqrtf((float)i);
-    while (q * q > i) q--;
-    while ((q + 1) * (q + 1) <= i) q++;
-    n = q;
-    m = i - q * q - q;
+    int s = 0;
+    for (int n = 0; n < p; n++) s += (n + 1) * up_to(n + 1, 4) + n * up_to(n, 4);
+    return s;
+}
+// coaxial tables of order p: order m holds [n = m..p-1][rows m..p-1, padded to 2]
+__host__ __device__ __forceinline__ int coax2_sum(int n) { return n * (n + 1) * (2 * n + 1) / 6 + ((n + 1) / 2) * ((n + 1) / 2); }
+__host__ __device__ __forceinline__ int coax2_off(int p, int m) { return coax2_sum(p) - coax2_sum(p - m); }
+static int coax2_size(int p) { return coax2_sum(p); }
+
+// P and Q of the classes' representative rows rep[k] of H, degree blockIdx.x (see rot32_size)
+__global__ void rot32_table_kernel(int pmax, const int *__restrict__ rep, const int *__restrict__ off, int stride,
+                                   const double *__restrict__ H, float *__restrict__ out)
+{
+    const int n = blockIdx.x, k = blockIdx.y, w = 2 * n + 1, rp = up_to(n + 1, 4), rm = up_to(n, 4);
+    const double *Hn = H + (size_t)rep[k] * rot_size(pmax) + rot_off(n);
+    float *o = out + (size_t)k * stride + off[n];
+    for (int t = threadIdx.x; t < (n + 1) * rp + n * rm; t += blockDim.x) {
+        double v = 0.0;
+        if (t < (n + 1) * rp) {
+            const int m = t / rp, r = t % rp;
+            if (r <= n) {
+                const double a = Hn[(n + m) * w + n + r], b = Hn[(n - m) * w + n + r];
+                v = m ? (r ? a + b : 0.5 * (a + b)) : (r ? a + Hn[n * w + n - r] : a);
+            }
+        } else {
+            const int u = t - (n + 1) * rp, m = u / rm + 1, r = u % rm + 1;
+            if (r <= n) v = Hn[(n + m) * w + n + r] - Hn[(n - m) * w + n + r];
+        }
+        o[t] = (float)v;
+    }
 }
 
-// Tiles X and W hold p^2 rows of TC complex columns.  The 16-byte chunks of row q are
-// XOR-swizzled by q mod 8 (mod TC/2 for TC = 8) so that units reading rows of different
-// degrees in one warp hit different banks.
+// the coaxial tables of order p (layout of coax_off, blockIdx.y = table) in the padded layout
+__global__ void coax2_table_kernel(int p, const float2 *__restrict__ in, float2 *__restrict__ out)
+{
+    const int m = blockIdx.x, sz = p - m, ld = up_to(sz, 2);
+    const float2 *a = in + (size_t)blockIdx.y * coax_size(p) + coax_off(p, m);
+    float2 *o = out + (size_t)blockIdx.y * coax2_sum(p) + coax2_off(p, m);
+    for (int t = threadIdx.x; t < sz * ld; t += blockDim.x) {
+        const int n = t / ld, r = t % ld;
+        o[t] = r < sz ? a[n * sz + r] : make_float2(0.f, 0.f);
+    }
+}
+
+// element (row, column) of a tile: the 16-byte chunks (2 columns) of a row are XOR-swizzled by the
+// row, so that lanes on different rows spread over the banks
 template <int TC>
-static __device__ __forceinline__ float4 *chunk(float2 *base, int row, int ch)
+__device__ __forceinline__ int swz(int row)
 {
     constexpr int M = (TC / 2 < 8 ? TC / 2 : 8) - 1;
-    return reinterpret_cast<float4 *>(base + (size_t)row * TC) + (ch ^ (row & M));
+    return row & M;
 }
 
-// rows row0..row0+R-1 of W_n = H_n X_n (r = 2n+1 rows) for the CG columns starting at chunk
-// ch0; X row of step m is rb + m; Hn column-major (m', m).  The H entries of step m+1 are
-// loaded while step m computes.
-template <int TC, int CG, int R>
-static __device__ __forceinline__ void rot_rows(const float *__restrict__ Hn, int r, int row0, float2 *X, int rb,
-                                                int ch0, float2 (&acc)[R][CG])
+template <int R> struct Rows;
+template <> struct Rows<4> { typedef float4 t; };
+template <> struct Rows<2> { typedef float2 t; };
+constexpr int THREADS = 256, CG = 4;  // threads of a CTA, columns of a lane
+
+// One rotation stage, in place.  Round k gives thread t unit k UC + t / CL and the
+// column pairs cl, cl + CL (cl = t % CL): (n | sign << 8 | first row << 16, table offset), R rows of P_n or Q_n.  All
+// units of a block (n, sign) are in one round, which writes after everyone has read.
+template <int TC, int R>
+__device__ __forceinline__ void rot_stage(const float *__restrict__ rot, ulonglong2 *X, const int2 *__restrict__ units, int rounds)
 {
+    constexpr int CL = TC / CG, UC = THREADS / CL, NC = CG / 2;
+    const int cl = threadIdx.x % CL, ul = threadIdx.x / CL;
+    for (int k = 0; k < rounds; k++) {
+        const int2 info = __ldg(units + k * UC + ul);
+        const bool on = info.x >= 0;
+        const int n = on ? info.x & 255 : 0, minus = on ? (info.x >> 8) & 1 : 0, row0 = on ? info.x >> 16 : 0;
+        const int steps = on ? (minus ? n : n + 1) : 0, ld = up_to(minus ? n : n + 1, 4), c0 = n * n + n;
+        const float *h = rot + info.y;
+        f2 acc[R][CG];
 #pragma unroll
-    for (int k = 0; k < R; k++)
+        for (int r = 0; r < R; r++)
 #pragma unroll
-        for (int t = 0; t < CG; t++) acc[k][t] = make_float2(0.f, 0.f);
-    float hn[R];
+            for (int c = 0; c < CG; c++) acc[r][c] = 0ull;
+        int row = minus ? c0 - 1 : c0;
+        const int dr = minus ? -1 : 1;
+        typename Rows<R>::t hn = __ldg(reinterpret_cast<const typename Rows<R>::t *>(h));
+#pragma unroll 2
+        for (int m = 0; m < steps; m++) {
+            const typename Rows<R>::t hv = hn;
+            if (m + 1 < steps) h += ld;  // the last step loads its own entries again
+            hn = __ldg(reinterpret_cast<const typename Rows<R>::t *>(h));
+            ulonglong2 x[NC];
+            const ulonglong2 *xr = X + row * (TC / 2);
+            const int s = swz<TC>(row);
 #pragma unroll
-    for (int k = 0; k < R; k++) hn[k] = (row0 + k < r) ? Hn[row0 + k] : 0.f;
-    for (int m = 0; m < r; m++) {
-        float h[R];
+            for (int i = 0; i < NC; i++) x[i] = xr[(cl + i * CL) ^ s];
+            row += dr;
+            const float *hc = reinterpret_cast<const float *>(&hv);
 #pragma unroll
-        for (int k = 0; k < R; k++) {
-            h[k] = hn[k];
-            hn[k] = (m + 1 < r && row0 + k < r) ? Hn[(m + 1) * r + row0 + k] : 0.f;
-        }
+            for (int r = 0; r < R; r++) {
+                const f2 hh = f2_pack(hc[r], hc[r]);
 #pragma unroll
-        for (int c = 0; c < CG / 2; c++) {
-            float4 x = *chunk<TC>(X, rb + m, ch0 + c);
-#pragma unroll
-            for (int k = 0; k < R; k++) {
-                acc[k][2 * c].x = fmaf(h[k], x.x, acc[k][2 * c].x);
-                acc[k][2 * c].y = fmaf(h[k], x.y, acc[k][2 * c].y);
-                acc[k][2 * c + 1].x = fmaf(h[k], x.z, acc[k][2 * c + 1].x);
-                acc[k][2 * c + 1].y = fmaf(h[k], x.w, acc[k][2 * c + 1].y);
+                for (int i = 0; i < NC; i++) {
+                    acc[r][2 * i] = f2_fma(hh, x[i].x, acc[r][2 * i]);
+                    acc[r][2 * i + 1] = f2_fma(hh, x[i].y, acc[r][2 * i + 1]);
+                }
             }
         }
+        __syncthreads();
+        const int nrow = steps - row0;  // rows of the block from row0 on
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (r < nrow) {
+                const int q = minus ? c0 - 1 - row0 - r : c0 + row0 + r;
+#pragma unroll
+                for (int i = 0; i < NC; i++)
+                    X[q * (TC / 2) + ((cl + i * CL) ^ swz<TC>(q))] = make_ulonglong2(acc[r][2 * i], acc[r][2 * i + 1]);
+            }
     }
 }
 
-static __device__ __forceinline__ void cmac(float2 &acc, float2 c, float ar, float ai)
+// The coaxial stage, in place, in rounds as above.  Unit: |m| | sign << 8 | first row << 16, two of
+// the rows of order +-m.
+template <int TC>
+__device__ __forceinline__ void coax_stage(int p, int nin, int nq, const float2 *__restrict__ Cc, ulonglong2 *X,
+                                           const int *__restrict__ units, int rounds)
 {
-    acc.x = fmaf(c.x, ar, acc.x);
-    acc.x = fmaf(-c.y, ai, acc.x);
-    acc.y = fmaf(c.x, ai, acc.y);
-    acc.y = fmaf(c.y, ar, acc.y);
+    constexpr int CL = TC / CG, UC = THREADS / CL, NC = CG / 2;
+    const int cl = threadIdx.x % CL, ul = threadIdx.x / CL;
+    for (int k = 0; k < rounds; k++) {
+        const int info = __ldg(units + k * UC + ul);
+        const bool on = info >= 0;
+        const int am = on ? info & 255 : 0, minus = on ? (info >> 8) & 1 : 0, row0 = on ? info >> 16 : 0;
+        const int steps = on ? nin - am : 0, ld = up_to(p - am, 2);
+        const float4 *c = reinterpret_cast<const float4 *>(Cc + coax2_off(p, am) + row0);
+        f2 a0[2][CG], a1[2][CG];
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int j = 0; j < CG; j++) a0[r][j] = a1[r][j] = 0ull;
+        const int sm = minus ? -am : am;
+        int row = am * am + am + sm, dr = 2 * am + 2;
+        float4 cn = __ldg(c);
+#pragma unroll 2
+        for (int n = 0; n < steps; n++) {
+            const float4 cc = cn;
+            if (n + 1 < steps) c += ld / 2;
+            cn = __ldg(c);
+            ulonglong2 x[NC];
+            const ulonglong2 *xr = X + row * (TC / 2);
+            const int s = swz<TC>(row);
+#pragma unroll
+            for (int i = 0; i < NC; i++) x[i] = xr[(cl + i * CL) ^ s];
+            row += dr;
+            dr += 2;
+            const f2 re[2] = {f2_pack(cc.x, cc.x), f2_pack(cc.z, cc.z)}, im[2] = {f2_pack(cc.y, cc.y), f2_pack(cc.w, cc.w)};
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+#pragma unroll
+                for (int i = 0; i < NC; i++) {
+                    a0[r][2 * i] = f2_fma(re[r], x[i].x, a0[r][2 * i]);
+                    a0[r][2 * i + 1] = f2_fma(re[r], x[i].y, a0[r][2 * i + 1]);
+                    a1[r][2 * i] = f2_fma(im[r], x[i].x, a1[r][2 * i]);
+                    a1[r][2 * i + 1] = f2_fma(im[r], x[i].y, a1[r][2 * i + 1]);
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+            if (on && row0 + r < nq - am) {
+                const int nn = am + row0 + r, q = nn * nn + nn + sm;
+                f2 y[CG];
+#pragma unroll
+                for (int j = 0; j < CG; j++) {
+                    const float2 v = f2_parts(a0[r][j]), w = f2_parts(a1[r][j]);
+                    y[j] = f2_pack(v.x - w.y, v.y + w.x);
+                }
+#pragma unroll
+                for (int i = 0; i < NC; i++)
+                    X[q * (TC / 2) + ((cl + i * CL) ^ swz<TC>(q))] = make_ulonglong2(y[2 * i], y[2 * i + 1]);
+            }
+    }
 }
 
-// One tile: item it = (direction, first column, count, coaxial block) of pass ps, with the
-// CTA's dynamic shared memory smem4 and its column indices s_src / s_dst.  SHC also stages
-// the direction's rotation block and coaxial block in shared memory, after the two tiles.
-//
-// A stage lasts as long as its busiest thread.  The units of a stage are ordered by cost
-// (longest first); without BAL thread t takes units t, t + B, t + 2B, ... (B threads), which
-// leaves most threads idle while the few longest units finish when the units barely outnumber
-// the threads.  BAL takes them in boustrophedon order (t, 2B - 1 - t, 2B + t, ...), so a thread
-// that drew a long unit in one round draws a short one in the next, ranks the column groups
-// inside each cost class, and gives +m and -m of the coaxial stage units of their own; with
-// one- or two-row units the busiest thread does about 1.05-1.15 times the average work at
-// p = 20-40 (counting each unit's FMAs and loads), against about 1.8 times with the default
-// schedule.  Every output is still summed in the same order, so the results do not depend on
-// BAL, R1 or R2.
-template <int TC, int CG, int R1, int R2, bool SHC, bool BAL = false>
-static __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float4 *smem4, int *s_src, int *s_dst)
+// One tile: item it = (class, first column, count, coaxial table) of pass ps, with the
+// CTA's dynamic shared memory and its column indices.
+template <int TC, int R>
+__device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float4 *smem4, int *s_src, int *s_dst, int *s_dir)
 {
-    const int p = ps.p, pp = p * p;
-    float2 *X = reinterpret_cast<float2 *>(smem4);
-    float2 *W = X + (size_t)pp * TC;
-    float2 *sC = W + (size_t)pp * TC;
-    float *sH = reinterpret_cast<float *>(sC + coax_size(p));
-    const int cnt = it.z;
-    const float *Hg = ps.H + (size_t)(ps.hrep ? ps.hrep[it.x] : it.x) * ps.hstride;
-    const float2 *ph = ps.PH + (size_t)it.x * ps.phstride + ps.phoff;
-    const float2 *Cg = ps.Cc + (size_t)it.w * coax_size(p);
-    const float *H = SHC ? sH : Hg;
-    const float2 *Cc = SHC ? sC : Cg;
+    const int p = ps.p, nin = min(ps.pin, p), nq = min(ps.pout, p), cnt = it.z;
+    ulonglong2 *X = reinterpret_cast<ulonglong2 *>(smem4);
+    float2 *Xf = reinterpret_cast<float2 *>(X);
     if (threadIdx.x < TC) {
         // column e = translation t x nrhs + right-hand side r; the expansions hold the columns
-        // of a box next to each other ([box][rhs][p^2]), so a tile's sources are contiguous runs
-        bool v = (int)threadIdx.x < cnt;
-        int e = it.y + threadIdx.x, t = e / ps.nrhs, r = e - t * ps.nrhs;
-        s_src[threadIdx.x] = v ? ps.g_src[t] * ps.nrhs + r : -1;
-        s_dst[threadIdx.x] = v ? ps.g_dst[t] * ps.nrhs + r : -1;
-    }
-    if (SHC) {
-        const int rs = rot_size(p), cs = coax_size(p);
-        for (int i = threadIdx.x; i < rs; i += blockDim.x) sH[i] = __ldg(Hg + i);
-        for (int i = threadIdx.x; i < cs; i += blockDim.x) sC[i] = __ldg(Cg + i);
+        // of a box next to each other ([box][rhs][p^2])
+        const int e = it.y + min((int)threadIdx.x, cnt - 1), t = e / ps.nrhs, r = e - t * ps.nrhs;
+        s_src[threadIdx.x] = ps.g_src[t] * ps.nrhs + r;
+        s_dst[threadIdx.x] = ps.g_dst[t] * ps.nrhs + r;
+        s_dir[threadIdx.x] = ps.g_dir[t];
     }
     __syncthreads();
-
-    // stage 0: gather, phase, zero padding
-    const int pin = min(ps.pin, p), pin2 = pin * pin, sstride = ps.pin * ps.pin;
-    for (int i = threadIdx.x; i < pp * TC; i += blockDim.x) {
-        int nm = i / TC, t = i % TC;
-        float2 v = make_float2(0.f, 0.f);
-        int s = s_src[t];
-        if (s >= 0 && nm < pin2) {
-            int n, m;
-            nm_of(nm, n, m);
-            v = cmul(__ldg(ps.src + (size_t)s * sstride + nm), ph[m]);
-        }
-        reinterpret_cast<float2 *>(chunk<TC>(X, nm, t >> 1))[t & 1] = v;
-    }
-    __syncthreads();
-
-    // stage 1: W_n = H_n X_n, n < p; a unit is R1 rows x CG columns, longest blocks first
-    constexpr int G = TC / CG, HC = CG / 2;
-    const int B = blockDim.x, tid = threadIdx.x;
-    int U = 0;
-    for (int n = 0; n < p; n++) U += (2 * n + R1) / R1;
-    for (int k = 0;; k++) {
-        const int u = k * B + ((BAL && (k & 1)) ? B - 1 - tid : tid);
-        if (u >= U * G) break;
-        const int g = BAL ? u % G : u / U;
-        int n = p - 1, q = BAL ? u / G : u - g * U;
-        while (q >= (2 * n + R1) / R1) {
-            q -= (2 * n + R1) / R1;
-            n--;
-        }
-        const int r = 2 * n + 1, row0 = q * R1;
-        float2 acc[R1][CG];
-        rot_rows<TC, CG, R1>(H + rot_off(n), r, row0, X, n * n, g * HC, acc);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int gi = lane & 7, gc = lane >> 3;  // gather / scatter: 8 pairs (n, m >= 0) x 4 columns per warp
+    {
+        const int np = nin * (nin + 1) / 2, nb = (np + 7) / 8 * (TC / 4), sstride = ps.pin * ps.pin;
+        constexpr int GU = 4;  // blocks in flight per warp
+        for (int b0 = warp; b0 < nb; b0 += GU * nw) {
+            int nm[GU];
+            float2 vp[GU], vm[GU], e[GU];
 #pragma unroll
-        for (int k = 0; k < R1; k++)
-            if (row0 + k < r) {
-#pragma unroll
-                for (int c = 0; c < HC; c++)
-                    *chunk<TC>(W, n * n + row0 + k, g * HC + c) =
-                        make_float4(acc[k][2 * c].x, acc[k][2 * c].y, acc[k][2 * c + 1].x, acc[k][2 * c + 1].y);
+            for (int j = 0; j < GU; j++) {
+                const int b = b0 + j * nw, q = b / (TC / 4) * 8 + gi;
+                nm[j] = b < nb && q < np ? __ldg(ps.pairs + q) : -1;
             }
-    }
-    __syncthreads();
-
-    // stage 2: X_{+-m} = C_|m| W_{+-m} for the rows n' < nq (the ones stage 3 reads)
-    const int nq = min(ps.pout, p);
-    if constexpr (!BAL) {
-        U = 0;
-        for (int am = 0; am < nq; am++) U += (nq - am + R2 - 1) / R2;
-        for (int u = threadIdx.x; u < U * G; u += blockDim.x) {
-            const int g = u / U;
-            int am = 0, q = u - g * U;
-            while (q >= (nq - am + R2 - 1) / R2) {
-                q -= (nq - am + R2 - 1) / R2;
-                am++;
-            }
-            const int sz = p - am, nrow = nq - am, j0 = q * R2;
-            const float2 *Cb = Cc + coax_off(p, am);
-            float2 accP[R2][CG], accM[R2][CG];
 #pragma unroll
-            for (int k = 0; k < R2; k++)
-#pragma unroll
-                for (int t = 0; t < CG; t++) accP[k][t] = accM[k][t] = make_float2(0.f, 0.f);
-            float2 cn[R2];
-#pragma unroll
-            for (int k = 0; k < R2; k++) cn[k] = (j0 + k < nrow) ? Cb[j0 + k] : make_float2(0.f, 0.f);
-            for (int j = 0; j < sz; j++) {
-                float2 c[R2];
-#pragma unroll
-                for (int k = 0; k < R2; k++) {
-                    c[k] = cn[k];
-                    cn[k] = (j + 1 < sz && j0 + k < nrow) ? Cb[(j + 1) * sz + j0 + k] : make_float2(0.f, 0.f);
-                }
-                const int n = am + j, rp = n * n + n + am, rm = n * n + n - am;
-#pragma unroll
-                for (int cc = 0; cc < HC; cc++) {
-                    float4 a = *chunk<TC>(W, rp, g * HC + cc), b = *chunk<TC>(W, rm, g * HC + cc);
-#pragma unroll
-                    for (int k = 0; k < R2; k++) {
-                        cmac(accP[k][2 * cc], c[k], a.x, a.y);
-                        cmac(accP[k][2 * cc + 1], c[k], a.z, a.w);
-                        cmac(accM[k][2 * cc], c[k], b.x, b.y);
-                        cmac(accM[k][2 * cc + 1], c[k], b.z, b.w);
+            for (int j = 0; j < GU; j++) {
+                const int c = (b0 + j * nw) % (TC / 4) * 4 + gc, m = nm[j] >> 16, r0 = nm[j] & 0xffff;
+                vp[j] = vm[j] = make_float2(0.f, 0.f);
+                e[j] = make_float2(1.f, 0.f);
+                if (nm[j] >= 0 && c < cnt) {
+                    const float2 *in = ps.src + (size_t)s_src[c] * sstride + r0;
+                    vp[j] = __ldg(in + m);
+                    if (m > 0) {
+                        vm[j] = __ldg(in - m);
+                        e[j] = __ldg(ps.PHall + (size_t)s_dir[c] * ps.phstride + ps.phoff + m);
                     }
                 }
             }
 #pragma unroll
-            for (int k = 0; k < R2; k++)
-                if (j0 + k < nrow) {
-                    const int np = am + j0 + k;
-#pragma unroll
-                    for (int cc = 0; cc < HC; cc++) {
-                        *chunk<TC>(X, np * np + np + am, g * HC + cc) =
-                            make_float4(accP[k][2 * cc].x, accP[k][2 * cc].y, accP[k][2 * cc + 1].x, accP[k][2 * cc + 1].y);
-                        if (am > 0)
-                            *chunk<TC>(X, np * np + np - am, g * HC + cc) = make_float4(
-                                accM[k][2 * cc].x, accM[k][2 * cc].y, accM[k][2 * cc + 1].x, accM[k][2 * cc + 1].y);
-                    }
-                }
-        }
-    } else {
-        // units (|m|, row block, sign, column group), |m| ascending = cost descending
-        U = 0;
-        for (int am = 0; am < nq; am++) U += (am > 0 ? 2 : 1) * ((nq - am + R2 - 1) / R2);
-        for (int k = 0;; k++) {
-            const int u = k * B + ((k & 1) ? B - 1 - tid : tid);
-            if (u >= U * G) break;
-            const int g = u % G;
-            int am = 0, q = u / G;
-            while (q >= (am > 0 ? 2 : 1) * ((nq - am + R2 - 1) / R2)) {
-                q -= (am > 0 ? 2 : 1) * ((nq - am + R2 - 1) / R2);
-                am++;
+            for (int j = 0; j < GU; j++) {
+                if (nm[j] < 0) continue;
+                const int c = (b0 + j * nw) % (TC / 4) * 4 + gc, m = nm[j] >> 16, r0 = nm[j] & 0xffff, rp = r0 + m, rm = r0 - m;
+                // m = 0: x itself (vm = 0, e = 1)
+                const float2 a = make_float2(vp[j].x + vm[j].x, vp[j].y + vm[j].y);
+                const float2 d = make_float2(vp[j].x - vm[j].x, vp[j].y - vm[j].y);
+                Xf[rp * TC + (((c >> 1) ^ swz<TC>(rp)) << 1) + (c & 1)] =
+                    make_float2(e[j].x * a.x - e[j].y * d.y, e[j].x * a.y + e[j].y * d.x);
+                if (m > 0)
+                    Xf[rm * TC + (((c >> 1) ^ swz<TC>(rm)) << 1) + (c & 1)] =
+                        make_float2(e[j].x * d.x - e[j].y * a.y, e[j].x * d.y + e[j].y * a.x);
             }
-            const int sg = am > 0 ? (q & 1) : 0, m = sg ? -am : am;
-            const int sz = p - am, nrow = nq - am, j0 = (am > 0 ? q >> 1 : q) * R2;
-            const float2 *Cb = Cc + coax_off(p, am);
-            float2 acc[R2][CG];
-#pragma unroll
-            for (int r = 0; r < R2; r++)
-#pragma unroll
-                for (int t = 0; t < CG; t++) acc[r][t] = make_float2(0.f, 0.f);
-            float2 cn[R2];
-#pragma unroll
-            for (int r = 0; r < R2; r++) cn[r] = (j0 + r < nrow) ? Cb[j0 + r] : make_float2(0.f, 0.f);
-            for (int j = 0; j < sz; j++) {
-                float2 c[R2];
-#pragma unroll
-                for (int r = 0; r < R2; r++) {
-                    c[r] = cn[r];
-                    cn[r] = (j + 1 < sz && j0 + r < nrow) ? Cb[(j + 1) * sz + j0 + r] : make_float2(0.f, 0.f);
-                }
-                const int n = am + j, row = n * n + n + m;
-#pragma unroll
-                for (int cc = 0; cc < HC; cc++) {
-                    const float4 a = *chunk<TC>(W, row, g * HC + cc);
-#pragma unroll
-                    for (int r = 0; r < R2; r++) {
-                        cmac(acc[r][2 * cc], c[r], a.x, a.y);
-                        cmac(acc[r][2 * cc + 1], c[r], a.z, a.w);
-                    }
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < R2; r++)
-                if (j0 + r < nrow) {
-                    const int np = am + j0 + r;
-#pragma unroll
-                    for (int cc = 0; cc < HC; cc++)
-                        *chunk<TC>(X, np * np + np + m, g * HC + cc) =
-                            make_float4(acc[r][2 * cc].x, acc[r][2 * cc].y, acc[r][2 * cc + 1].x, acc[r][2 * cc + 1].y);
-                }
         }
     }
     __syncthreads();
-
-    // stage 3: Y_n = e^{-i m' phi} H_n X_n for n < nq, into the destinations
-    const int po2 = ps.pout * ps.pout;
-    U = 0;
-    for (int n = 0; n < nq; n++) U += (2 * n + R1) / R1;
-    for (int k = 0;; k++) {
-        const int u = k * B + ((BAL && (k & 1)) ? B - 1 - tid : tid);
-        if (u >= U * G) break;
-        const int g = BAL ? u % G : u / U;
-        int n = nq - 1, q = BAL ? u / G : u - g * U;
-        while (q >= (2 * n + R1) / R1) {
-            q -= (2 * n + R1) / R1;
-            n--;
-        }
-        const int r = 2 * n + 1, row0 = q * R1;
-        float2 acc[R1][CG];
-        rot_rows<TC, CG, R1>(H + rot_off(n), r, row0, X, n * n, g * HC, acc);
-#pragma unroll
-        for (int k = 0; k < R1; k++) {
-            if (row0 + k >= r) continue;
-            const float2 e = ph[row0 + k - n];
-            const int idx = n * n + row0 + k;
-#pragma unroll
-            for (int c = 0; c < CG; c++) {
-                const int t = g * CG + c;
-                if (t >= cnt) break;
-                float2 a = acc[k][c];
-                float2 v = make_float2(e.x * a.x + e.y * a.y, e.x * a.y - e.y * a.x);
-                float2 *d = ps.dst + (size_t)s_dst[t] * po2 + idx;
-                if (ps.atomic) {
-                    atomicAdd(d, v);
-                } else {
-                    float2 o = *d;
-                    *d = make_float2(o.x + v.x, o.y + v.y);
+    const float *rot = ps.rot + (size_t)it.x * ps.rot_stride;
+    rot_stage<TC, R>(rot, X, ps.u1, ps.n1);
+    __syncthreads();
+    coax_stage<TC>(p, nin, nq, ps.coax + (size_t)it.w * coax2_sum(p), X, ps.u2, ps.n2);
+    __syncthreads();
+    rot_stage<TC, R>(rot, X, ps.u3, ps.n3);
+    __syncthreads();
+    {
+        const int np = nq * (nq + 1) / 2, nb = (np + 7) / 8 * (TC / 4), dstride = ps.pout * ps.pout;
+        for (int b = warp; b < nb; b += nw) {
+            const int q = b / (TC / 4) * 8 + gi, c = b % (TC / 4) * 4 + gc;
+            if (q >= np || c >= cnt) continue;
+            const int nm = __ldg(ps.pairs + q), m = nm >> 16, r0 = nm & 0xffff, rp = r0 + m, rm = r0 - m;
+            float2 *out = ps.dst + (size_t)s_dst[c] * dstride + r0;
+            float2 yp = Xf[rp * TC + (((c >> 1) ^ swz<TC>(rp)) << 1) + (c & 1)], ym = yp;
+            if (m > 0) {
+                const float2 v = Xf[rm * TC + (((c >> 1) ^ swz<TC>(rm)) << 1) + (c & 1)];
+                const float2 e = __ldg(ps.PHall + (size_t)s_dir[c] * ps.phstride + ps.phoff + m);
+                const float2 a = make_float2(0.5f * (yp.x + v.x), 0.5f * (yp.y + v.y));
+                const float2 d = make_float2(0.5f * (yp.x - v.x), 0.5f * (yp.y - v.y));
+                yp = make_float2(e.x * a.x + e.y * a.y, e.x * a.y - e.y * a.x);
+                ym = make_float2(e.x * d.x - e.y * d.y, e.x * d.y + e.y * d.x);
+            }
+            if (ps.atomic) {
+                atomicAdd(out + m, yp);
+                if (m > 0) atomicAdd(out - m, ym);
+            } else {
+                const float2 o = out[m];
+                out[m] = make_float2(o.x + yp.x, o.y + yp.y);
+                if (m > 0) {
+                    const float2 v = out[-m];
+                    out[-m] = make_float2(v.x + ym.x, v.y + ym.y);
                 }
             }
         }
     }
 }
 
-template <int TC, int CG, int R1, int R2, bool SHC, bool BAL = false>
-__global__ void __launch_bounds__(256, 2) rcr_tile_kernel(RcrPass ps)
+template <int TC, int R>
+__global__ void __launch_bounds__(THREADS, 3) rcr_tile_kernel(RcrPass ps)
 {
     extern __shared__ float4 smem4[];
-    __shared__ int s_src[TC], s_dst[TC];
-    rcr_tile<TC, CG, R1, R2, SHC, BAL>(ps, ps.items[blockIdx.x], smem4, s_src, s_dst);
+    __shared__ int s_src[TC], s_dst[TC], s_dir[TC];
+    rcr_tile<TC, R>(ps, ps.items[blockIdx.x], smem4, s_src, s_dst, s_dir);
 }
 
 // Persistent form for many passes at once (the translation passes of many plans, one phase
 // of a lockstep matvec): a grid of resident CTAs takes work items (pass, tile) from a device
 // queue, in the order given (longest first), until it is empty.  The queue head is an
 // atomic counter, zeroed before the launch; no CTA waits on another.
-template <int TC, int CG, int R1, int R2, bool SHC, bool BAL = false>
-__global__ void __launch_bounds__(256, 2) rcr_queue_kernel(const RcrPass *__restrict__ passes, const int *__restrict__ work_pass,
+template <int TC, int R>
+__global__ void __launch_bounds__(THREADS, 3) rcr_queue_kernel(const RcrPass *__restrict__ passes, const int *__restrict__ work_pass,
                                                            const int4 *__restrict__ work_item, const int *__restrict__ nwork,
                                                            int *head)
 {
     extern __shared__ float4 smem4[];
-    __shared__ int s_src[TC], s_dst[TC];
+    __shared__ int s_src[TC], s_dst[TC], s_dir[TC];
     __shared__ int s_w;
     const int n = *nwork;
     for (;;) {
@@ -350,98 +345,39 @@ __global__ void __launch_bounds__(256, 2) rcr_queue_kernel(const RcrPass *__rest
         __syncthreads();
         const int w = s_w;
         if (w >= n) break;
-        rcr_tile<TC, CG, R1, R2, SHC, BAL>(passes[work_pass[w]], work_item[w], smem4, s_src, s_dst);
+        rcr_tile<TC, R>(passes[work_pass[w]], work_item[w], smem4, s_src, s_dst, s_dir);
         __syncthreads();
     }
 }
 
-size_t rcr_tile_smem(int p, int tc, int shc)
-{
-    size_t s = 2 * (size_t)p * p * tc * sizeof(float2);
-    if (shc) s += (size_t)coax_size(p) * sizeof(float2) + (size_t)rot_size(p) * sizeof(float);
-    return s;
-}
+// a tile of p^2 rows (p the larger of the orders a pass uses) of tc complex columns
+size_t rcr_tile_smem(int p, int tc) { return (size_t)p * p * tc * sizeof(float2); }
 
-template <int TC, int CG, int R1, int R2, bool SHC, bool BAL = false>
-static int launch_tile(const RcrPass &ps, int n_items, size_t sm, cudaStream_t st)
-{
-    static size_t attr = 0;
-    int e = raise_smem_limit((const void *)rcr_tile_kernel<TC, CG, R1, R2, SHC, BAL>, sm, &attr);
-    if (e) return e;
-    rcr_tile_kernel<TC, CG, R1, R2, SHC, BAL><<<n_items, 256, sm, st>>>(ps);
-    FMM_CUDA_TRY(cudaGetLastError());
-    return FMM_OK;
-}
-
-// The tile shapes, as template arguments: Tile<TC, CG, R1, R2, SHC, BAL>
-template <int TC_, int CG_, int R1_, int R2_, bool SHC_, bool BAL_>
-struct Tile {
-    static constexpr int TC = TC_, CG = CG_, R1 = R1_, R2 = R2_;
-    static constexpr bool SHC = SHC_, BAL = BAL_;
+template <int TC_, int R_> struct Tile {
+    static constexpr int TC = TC_, R = R_;
 };
 
-// Calls f(Tile<...>{}) for the shape that serves (columns tc, staged blocks shc, schedule bal):
-// bal 0 the default schedule, 1 the balanced one with narrow column groups where they pay, 2 the
-// balanced one with the default groups; a (tc, shc, bal) without a balanced shape runs bal 0.
+// Calls f(Tile<...>{}) for tc columns and units of four rows (bal = 0) or two (1)
 template <class F>
-static int with_tile(int tc, int shc, int bal, F &&f)
+static int with_tile(int tc, int bal, F &&f)
 {
-    if (bal == 2) {
-        if (shc) {
-            if (tc == 32) return f(Tile<32, 16, 1, 1, true, true>{});
-        } else {
-            switch (tc) {
-            case 32: return f(Tile<32, 16, 1, 1, false, true>{});
-            case 16: return f(Tile<16, 16, 1, 1, false, true>{});
-            case 8: return f(Tile<8, 8, 1, 1, false, true>{});
-            case 4: return f(Tile<4, 4, 1, 1, false, true>{});
-            default: break;
-            }
-        }
-    }
-    if (bal == 1) {
-        if (shc) {
-            switch (tc) {
-            case 64: return f(Tile<64, 16, 1, 1, true, true>{});
-            case 32: return f(Tile<32, 8, 1, 1, true, true>{});
-            default: break;
-            }
-        } else {
-            switch (tc) {
-            case 64: return f(Tile<64, 16, 1, 1, false, true>{});
-            case 32: return f(Tile<32, 8, 1, 1, false, true>{});
-            case 16: return f(Tile<16, 8, 1, 1, false, true>{});
-            case 8: return f(Tile<8, 8, 2, 1, false, true>{});
-            case 4: return f(Tile<4, 4, 2, 1, false, true>{});
-            default: break;
-            }
-        }
-    }
-    if (shc) {
-        switch (tc) {
-        case 64: return f(Tile<64, 16, 2, 1, true, false>{});
-        case 32: return f(Tile<32, 16, 2, 1, true, false>{});
-        case 16: return f(Tile<16, 16, 2, 1, true, false>{});
-        default: return f(Tile<8, 8, 4, 2, true, false>{});
-        }
-    }
     switch (tc) {
-    case 64: return f(Tile<64, 16, 2, 1, false, false>{});
-    case 32: return f(Tile<32, 16, 2, 1, false, false>{});
-    case 16: return f(Tile<16, 16, 2, 1, false, false>{});
-    case 4: return f(Tile<4, 4, 8, 4, false, false>{});
-    default: return f(Tile<8, 8, 4, 2, false, false>{});
+    case 64: return bal ? f(Tile<64, 2>{}) : f(Tile<64, 4>{});
+    case 32: return bal ? f(Tile<32, 2>{}) : f(Tile<32, 4>{});
+    case 16: return bal ? f(Tile<16, 2>{}) : f(Tile<16, 4>{});
+    case 8: return bal ? f(Tile<8, 2>{}) : f(Tile<8, 4>{});
+    default: return bal ? f(Tile<4, 2>{}) : f(Tile<4, 4>{});
     }
 }
 
 // Raise the queue kernel's shared-memory limit and size its grid: every CTA resident at once
 // (SMs x CTAs per SM at this shared memory), no more than the items.
-int rcr_queue_prepare(int tc, int shc, int bal, size_t sm, int nwork, int *grid)
+int rcr_queue_prepare(int tc, int bal, size_t sm, int nwork, int *grid)
 {
-    return with_tile(tc, shc, bal, [&](auto t) -> int {
+    return with_tile(tc, bal, [&](auto t) -> int {
         using T = decltype(t);
         static size_t attr = 0;
-        const void *fn = (const void *)rcr_queue_kernel<T::TC, T::CG, T::R1, T::R2, T::SHC, T::BAL>;
+        const void *fn = (const void *)rcr_queue_kernel<T::TC, T::R>;
         int e = raise_smem_limit(fn, sm, &attr);
         if (e) return e;
         int dev = 0, nsm = 0, per_sm = 0;
@@ -453,30 +389,27 @@ int rcr_queue_prepare(int tc, int shc, int bal, size_t sm, int nwork, int *grid)
     });
 }
 
-int launch_rcr_queue(int tc, int shc, int bal, const RcrPass *passes, const int *work_pass, const int4 *work_item,
+int launch_rcr_queue(int tc, int bal, const RcrPass *passes, const int *work_pass, const int4 *work_item,
                      const int *nwork, int *head, size_t sm, int grid, cudaStream_t st)
 {
-    return with_tile(tc, shc, bal, [&](auto t) -> int {
+    return with_tile(tc, bal, [&](auto t) -> int {
         using T = decltype(t);
-        rcr_queue_kernel<T::TC, T::CG, T::R1, T::R2, T::SHC, T::BAL><<<grid, 256, sm, st>>>(passes, work_pass, work_item,
-                                                                                         nwork, head);
+        rcr_queue_kernel<T::TC, T::R><<<grid, 256, sm, st>>>(passes, work_pass, work_item, nwork, head);
         FMM_CUDA_TRY(cudaGetLastError());
         return FMM_OK;
     });
 }
 
-void rcr_list_items(const RcrList &Lst, std::vector<int4> &items) { build_items(Lst, 1, Lst.tc, 0, true, items); }
-
 // Work items over the columns e = t nrhs + r of a list: tiles of at most `width` columns of
-// one direction (or octant), item .w = the direction's coaxial block when coax_w.  Where the
+// one key, item .w = the key's coaxial block when coax_w.  Where the
 // expansions a pass touches for nrhs columns (ws_bytes) are more than L2 keeps, the
 // destination boxes are cut into Morton ranges and the items ordered range by range, so that
-// the tiles in flight share their sources and destinations in L2.  Each direction's
+// the tiles in flight share their sources and destinations in L2.  Each key's
 // translations are sorted by the Morton rank of their destination, so a range is one
-// contiguous run of every direction.
+// contiguous run of every key.
 static const size_t L2_BUDGET = 48u << 20;
 
-void build_items(const RcrList &Lst, int nrhs, int width, size_t ws_bytes, bool coax_w, std::vector<int4> &items)
+void build_items(const KeyedList &Lst, int nrhs, int width, size_t ws_bytes, bool coax_w, std::vector<int4> &items)
 {
     items.clear();
     const int nkeys = (int)Lst.key_beg.size() - 1, nd = std::max(Lst.ndst_rank, 1);
@@ -497,15 +430,83 @@ void build_items(const RcrList &Lst, int nrhs, int width, size_t ws_bytes, bool 
     }
 }
 
+// translations in class order: source, destination, phase row of direction key0 + d
+__global__ void class_order_kernel(int n, const int *__restrict__ perm, const int *__restrict__ src, const int *__restrict__ dst,
+                                   const int *__restrict__ key_beg, int nkeys, int key0, int *__restrict__ csrc,
+                                   int *__restrict__ cdst, short *__restrict__ cdir)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int t = perm[i];
+        int lo = 0, hi = nkeys;  // the last direction whose run begins at or before t
+        while (hi - lo > 1) {
+            const int m = (lo + hi) >> 1;
+            if (key_beg[m] <= t) lo = m; else hi = m;
+        }
+        csrc[i] = src[t];
+        cdst[i] = dst[t];
+        cdir[i] = (short)(key0 + lo);
+    }
+}
+
+// The list by operator class, on first use of the SIMT tiles.
+static int ensure_classes(RcrList &Lst)
+{
+    if (Lst.csrc || Lst.key_beg.empty() || Lst.key_beg.back() == 0) return FMM_OK;
+    const int n = Lst.key_beg.back(), nkeys = (int)Lst.key_beg.size() - 1;
+    KeyedList &C = Lst.cls;
+    const int ncls = *std::max_element(Lst.cls_of_key.begin(), Lst.cls_of_key.end()) + 1, nd = Lst.ndst_rank;
+    // two stable counting sorts: by destination rank, then by class
+    std::vector<int> cls(n), byrank(n), perm(n), cnt(nd + 1, 0);
+    for (int d = 0; d < nkeys; d++)
+        for (int t = Lst.key_beg[d]; t < Lst.key_beg[d + 1]; t++) cls[t] = Lst.cls_of_key[d];
+    for (int t = 0; t < n; t++) cnt[Lst.dst_rank[t] + 1]++;
+    for (int r = 0; r < nd; r++) cnt[r + 1] += cnt[r];
+    for (int t = 0; t < n; t++) byrank[cnt[Lst.dst_rank[t]]++] = t;
+    C.key_beg.assign(ncls + 1, 0);
+    C.key_w.assign(ncls, 0);
+    C.ndst_rank = nd;
+    for (int d = 0; d < nkeys; d++) C.key_w[Lst.cls_of_key[d]] = Lst.key_w[d];
+    for (int t = 0; t < n; t++) C.key_beg[cls[t] + 1]++;
+    for (int c = 0; c < ncls; c++) C.key_beg[c + 1] += C.key_beg[c];
+    std::vector<int> fill(C.key_beg.begin(), C.key_beg.end());
+    C.dst_rank.resize(n);
+    for (int t : byrank) {
+        const int i = fill[cls[t]]++;
+        perm[i] = t;
+        C.dst_rank[i] = Lst.dst_rank[t];
+    }
+    int *tmp = nullptr, *cs = nullptr;
+    FMM_CUDA_TRY(cudaMalloc(&tmp, sizeof(int) * (n + nkeys + 1)));
+    cudaError_t ce = cudaMalloc(&cs, sizeof(int) * n);
+    if (ce == cudaSuccess) ce = cudaMalloc(&Lst.cdst, sizeof(int) * n);
+    if (ce == cudaSuccess) ce = cudaMalloc(&Lst.cdir, sizeof(short) * n);
+    if (ce == cudaSuccess) ce = cudaMemcpy(tmp, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(tmp + n, Lst.key_beg.data(), sizeof(int) * (nkeys + 1), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) {
+        class_order_kernel<<<std::min((n + 255) / 256, 152 * 16), 256>>>(n, tmp, Lst.src, Lst.dst, tmp + n, nkeys, Lst.key0, cs,
+                                                                        Lst.cdst, Lst.cdir);
+        ce = cudaGetLastError();
+    }
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);
+    cudaFree(tmp);
+    if (ce != cudaSuccess) cudaFree(cs);
+    FMM_CUDA_TRY(ce);
+    Lst.csrc = cs;
+    return FMM_OK;
+}
+
 // Device items of a SIMT pass for nrhs right-hand sides, rebuilt when nrhs changes.
 static int ensure_items(RcrList &Lst, int nrhs, size_t ws_bytes)
 {
     if (Lst.items_nrhs == nrhs) return FMM_OK;
+    int e = ensure_classes(Lst);
+    if (e) return e;
     std::vector<int4> items;
-    build_items(Lst, nrhs, Lst.tc, ws_bytes, true, items);
+    build_items(Lst.cls, nrhs, Lst.tc, ws_bytes, true, items);
     if (items.size() > Lst.items_cap) {
         if (Lst.items) cudaFree(Lst.items);
         Lst.items = nullptr;
+        Lst.items_cap = 0;
         FMM_CUDA_TRY(cudaMalloc(&Lst.items, sizeof(int4) * items.size()));
         Lst.items_cap = items.size();
     }
@@ -516,53 +517,216 @@ static int ensure_items(RcrList &Lst, int nrhs, size_t ws_bytes)
     return FMM_OK;
 }
 
-int launch_rcr_pass(RcrList &Lst, RcrPass ps, cudaStream_t st)
+int rcr_list_items(RcrList &Lst, std::vector<int4> &items)
+{
+    int e = ensure_classes(Lst);
+    if (e) return e;
+    build_items(Lst.cls, 1, Lst.tc, 0, true, items);
+    return FMM_OK;
+}
+
+static size_t tile_bytes(const RcrPass &ps, int tc)
+{
+    return rcr_tile_smem(std::max(std::min(ps.pin, ps.p), std::min(ps.pout, ps.p)), tc);
+}
+
+int launch_rcr_pass(const Plan *P, RcrList &Lst, RcrPass ps, cudaStream_t st)
 {
     if (Lst.key_beg.empty() || Lst.key_beg.back() == 0) return FMM_OK;
+    if (int e = set_tile_tables(P, Lst, ps)) return e;
     {
         size_t ws = ((size_t)ps.nsrc * ps.pin * ps.pin + (size_t)ps.ndst * ps.pout * ps.pout) * sizeof(float2) * ps.nrhs;
         int e = ensure_items(Lst, ps.nrhs, ws);
         if (e) return e;
     }
     ps.items = Lst.items;
-    ps.g_src = Lst.src;
-    ps.g_dst = Lst.dst;
-    const int p = ps.p;
-    size_t sm = rcr_tile_smem(p, Lst.tc, Lst.shc);
-    return with_tile(Lst.tc, Lst.shc, Lst.bal, [&](auto t) -> int {
+    const size_t sm = tile_bytes(ps, Lst.tc);
+    return with_tile(Lst.tc, Lst.bal, [&](auto t) -> int {
         using T = decltype(t);
-        return launch_tile<T::TC, T::CG, T::R1, T::R2, T::SHC, T::BAL>(ps, Lst.n_items, sm, st);
+        static size_t attr = 0;
+        int e = raise_smem_limit((const void *)rcr_tile_kernel<T::TC, T::R>, sm, &attr);
+        if (e) return e;
+        rcr_tile_kernel<T::TC, T::R><<<Lst.n_items, 256, sm, st>>>(ps);
+        FMM_CUDA_TRY(cudaGetLastError());
+        return FMM_OK;
     });
 }
 
 // Shared memory that keeps two CTAs on an SM: 228 KB per SM, 1 KB reserved and the static
 // arrays per CTA.
 static const size_t TWO_CTA_SMEM = (228 * 1024) / 2 - 1024 - 1024;
-// and the most one CTA may take (227 KB less the static column indices)
-const size_t MAX_TILE_SMEM = 227 * 1024 - 1024;
 
-// Columns per CTA: the largest of 64, 32, 16 whose tiles (and, where they also fit, the
-// staged rotation and coaxial blocks) keep two CTAs per SM, else 8 (one CTA per SM, p <= 42),
-// else 4 (p <= 60).  With 16-column groups that gives every thread of the CTA a unit of work
-// down to p = 10.
-static void pick_tile(int p, int &tc, int &shc)
+// Columns per CTA: the most that keep two CTAs on an SM, so that one computes while the other
+// gathers or waits at a barrier; at least 4 (p <= 60).
+static int pick_tile(int p)
 {
-    for (tc = 64; tc >= 16; tc /= 2) {
-        if (rcr_tile_smem(p, tc, 1) <= TWO_CTA_SMEM) { shc = 1; return; }
-        if (rcr_tile_smem(p, tc, 0) <= TWO_CTA_SMEM) { shc = 0; return; }
+    for (int tc = 64; tc > 4; tc /= 2)
+        if (rcr_tile_smem(p, tc) <= TWO_CTA_SMEM) return tc;
+    return 4;
+}
+
+// Classes of a pass's keys with one rotation and length: M2L directions of equal (dz, dx^2 + dy^2),
+// M2M / L2L octants of equal z bit.  cls[key] = class, rep[class] = its first key.
+void direction_classes(const Plan *P, int which, int nkeys, std::vector<int> &cls, std::vector<int> &rep)
+{
+    cls.assign(nkeys, -1);
+    rep.clear();
+    std::vector<int> off(nkeys, 0), seen;
+    if (which == PASS_M2L)
+        for (int q = 0; q < 343; q++)
+            if (P->dir_slot[q] >= 0 && P->dir_slot[q] < nkeys) off[P->dir_slot[q]] = q;
+    for (int d = 0; d < nkeys; d++) {
+        const int dx = off[d] / 49 - 3, dy = (off[d] / 7) % 7 - 3, dz = off[d] % 7 - 3;
+        const int key = which == PASS_M2L ? (dz + 8) * 1000 + dx * dx + dy * dy : d & 1;
+        const size_t c = std::find(seen.begin(), seen.end(), key) - seen.begin();
+        if (c == seen.size()) {
+            seen.push_back(key);
+            rep.push_back(d);
+        }
+        cls[d] = (int)c;
     }
-    tc = rcr_tile_smem(p, 8, 0) <= MAX_TILE_SMEM ? 8 : 4;
-    shc = 0;
+}
+
+// Folded rotation tables of the classes (M2L, then M2M and L2L), padded coaxial tables, and the
+// coefficient pairs (n, m >= 0).
+static int build_tile_tables(Plan *P)
+{
+    const int pmax = P->pmax;
+    std::vector<int> cls, rep, rows, off(pmax + 1, 0);
+    for (int which : {PASS_M2L, PASS_M2M, PASS_L2L}) {
+        direction_classes(P, which, which == PASS_M2L ? NDIR : 8, cls, rep);
+        if (which == PASS_M2L) P->rot32_m2l = (int)rep.size();
+        for (int r : rep) rows.push_back((which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8) + r);
+    }
+    for (int n = 0; n < pmax; n++) off[n + 1] = off[n] + (n + 1) * up_to(n + 1, 4) + n * up_to(n, 4);
+    P->rot32_stride = rot32_size(pmax);
+    FMM_CUDA_TRY(dev_alloc(P, (void **)&P->rot32, sizeof(float) * rows.size() * (size_t)P->rot32_stride));
+    int *tmp = nullptr;
+    FMM_CUDA_TRY(cudaMalloc(&tmp, sizeof(int) * (rows.size() + off.size())));
+    cudaError_t ce = cudaMemcpy(tmp, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaMemcpy(tmp + rows.size(), off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) {
+        rot32_table_kernel<<<dim3(pmax, (unsigned)rows.size()), 128, 0, P->stream>>>(pmax, tmp, tmp + rows.size(), P->rot32_stride,
+                                                                                    P->Hsr64, P->rot32);
+        ce = cudaStreamSynchronize(P->stream);
+    }
+    cudaFree(tmp);
+    FMM_CUDA_TRY(ce);
+    for (int l = P->lmin; l <= P->lmax; l++) {
+        LevelDev &L = P->lev[l];
+        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Csr32p, sizeof(float2) * NDIST * (size_t)coax2_size(L.p)));
+        coax2_table_kernel<<<dim3(L.p, NDIST), 128, 0, P->stream>>>(L.p, L.Csr32, L.Csr32p);
+        if (l > P->lmin) {
+            const int pp = P->lev[l - 1].p;
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Crr32p, sizeof(float2) * coax2_size(pp)));
+            coax2_table_kernel<<<dim3(pp, 1), 128, 0, P->stream>>>(pp, L.Crr32, L.Crr32p);
+            if (L.Crr32L) {
+                FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Crr32Lp, sizeof(float2) * coax2_size(pp)));
+                coax2_table_kernel<<<dim3(pp, 1), 128, 0, P->stream>>>(pp, L.Crr32L, L.Crr32Lp);
+            }
+        }
+    }
+    FMM_CUDA_TRY(cudaGetLastError());
+    std::vector<int> pairs;
+    P->rot32_off = off;
+    for (int n = 0; n < pmax; n++)
+        for (int m = 0; m <= n; m++) pairs.push_back((n * n + n) | m << 16);
+    FMM_CUDA_TRY(dev_alloc(P, (void **)&P->pairs, sizeof(int) * pairs.size()));
+    FMM_CUDA_TRY(cudaMemcpy(P->pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice));
+    return FMM_OK;
+}
+
+// Rounds of a stage's work units: blocks (all units of one degree or order and sign) in the given
+// order, longest first, as many as fit the UC units of a round; idle places elsewhere.
+template <class U>
+static int pack_rounds(const std::vector<std::vector<U>> &blocks, int UC, U idle, std::vector<U> &out)
+{
+    int rounds = 0, left = 0;
+    for (const std::vector<U> &b : blocks) {
+        if (b.empty()) continue;
+        if ((int)b.size() > left) {
+            out.resize(out.size() + left, idle);
+            left = UC;
+            rounds++;
+        }
+        out.insert(out.end(), b.begin(), b.end());
+        left -= (int)b.size();
+    }
+    out.resize(out.size() + left, idle);
+    return rounds;
+}
+
+// The work units of a list's tile shape, on the device (kept until the shape changes).
+static int ensure_units(const std::vector<int> &rot_off, RcrList &Lst, const RcrPass &ps)
+{
+    if (Lst.units_tc == Lst.tc && Lst.units_bal == Lst.bal) return FMM_OK;
+    const int UC = THREADS / (Lst.tc / CG), R = Lst.bal ? 2 : 4, nin = std::min(ps.pin, ps.p), nq = std::min(ps.pout, ps.p);
+    std::vector<int2> ur;
+    std::vector<int> uc;
+    auto rot = [&](int deg) {
+        std::vector<std::vector<int2>> blocks;
+        for (int n = deg - 1; n >= 0; n--)
+            for (int sg = 0; sg < 2; sg++) {
+                const int nr = sg ? n : n + 1, base = rot_off[n] + (sg ? (n + 1) * up_to(n + 1, 4) : 0);
+                std::vector<int2> b;
+                for (int r = 0; r < nr; r += R) b.push_back(make_int2(n | sg << 8 | r << 16, base + r));
+                blocks.push_back(b);
+            }
+        return pack_rounds(blocks, UC, make_int2(-1, 0), ur);
+    };
+    Lst.n1 = rot(nin);
+    Lst.at3 = ur.size();
+    Lst.n3 = rot(nq);
+    std::vector<std::vector<int>> blocks;
+    for (int am = 0; am < nq; am++)
+        for (int sg = 0; sg < (am ? 2 : 1); sg++) {
+            std::vector<int> b;
+            for (int r = 0; r < nq - am; r += 2) b.push_back(am | sg << 8 | r << 16);
+            blocks.push_back(b);
+        }
+    Lst.n2 = pack_rounds(blocks, UC, -1, uc);
+    cudaFree(Lst.urot);
+    cudaFree(Lst.ucoax);
+    Lst.urot = nullptr;
+    Lst.ucoax = nullptr;
+    Lst.units_tc = 0;
+    FMM_CUDA_TRY(cudaMalloc(&Lst.urot, sizeof(int2) * ur.size()));
+    FMM_CUDA_TRY(cudaMalloc(&Lst.ucoax, sizeof(int) * uc.size()));
+    FMM_CUDA_TRY(cudaMemcpy(Lst.urot, ur.data(), sizeof(int2) * ur.size(), cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(cudaMemcpy(Lst.ucoax, uc.data(), sizeof(int) * uc.size(), cudaMemcpyHostToDevice));
+    Lst.units_tc = Lst.tc;
+    Lst.units_bal = Lst.bal;
+    return FMM_OK;
+}
+
+// The tile kernels' tables, class order and units of a pass
+int set_tile_tables(const Plan *P, RcrList &Lst, RcrPass &ps)
+{
+    int e = ensure_classes(Lst);
+    if (!e) e = ensure_units(P->rot32_off, Lst, ps);
+    if (e) return e;
+    ps.rot = P->rot32 + (size_t)Lst.rot0 * P->rot32_stride;
+    ps.rot_stride = P->rot32_stride;
+    ps.PHall = P->PHsr32;
+    ps.u1 = Lst.urot;
+    ps.n1 = Lst.n1;
+    ps.u3 = Lst.urot + Lst.at3;
+    ps.n3 = Lst.n3;
+    ps.u2 = Lst.ucoax;
+    ps.n2 = Lst.n2;
+    ps.pairs = P->pairs;
+    ps.g_src = Lst.csrc;
+    ps.g_dst = Lst.cdst;
+    ps.g_dir = Lst.cdir;
+    return FMM_OK;
 }
 
 // drank: Morton rank of each destination box among the ndst boxes of its level.  The list is
 // sorted by key, and within a key by the destination's Morton rank (two stable counting sorts).
-static int upload_list(Plan *P, RcrList &Lst, const std::vector<int> &key, const std::vector<int> &src,
+static int upload_list(Plan *P, RcrList &Lst, int which, const std::vector<int> &key, const std::vector<int> &src,
                        const std::vector<int> &dst, int nkeys, const std::vector<int> &key_w, int p,
                        const std::vector<int> &drank, int ndst)
 {
-    int tc, shc;
-    pick_tile(p, tc, shc);
     size_t T = key.size();
     std::vector<int> byrank(std::max<size_t>(T, 1));
     {
@@ -586,12 +750,15 @@ static int upload_list(Plan *P, RcrList &Lst, const std::vector<int> &key, const
     Lst.ndst_rank = ndst;
     Lst.key_beg.assign(cnt.begin(), cnt.end());
     Lst.key_w = key_w;
-    Lst.tc = tc;
-    Lst.shc = shc;
+    Lst.tc = pick_tile(p);
     Lst.items_nrhs = 0;
+    Lst.rot0 = which == PASS_M2L ? 0 : which == PASS_M2M ? P->rot32_m2l : P->rot32_m2l + 2;
+    Lst.key0 = which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8;
+    {
+        std::vector<int> rep;
+        direction_classes(P, which, nkeys, Lst.cls_of_key, rep);
+    }
     if (T == 0) return FMM_OK;
-    int e = ensure_items(Lst, 1, 0);
-    if (e) return e;
     FMM_CUDA_TRY(dev_alloc(P, (void **)&Lst.src, sizeof(int) * T));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&Lst.dst, sizeof(int) * T));
     FMM_CUDA_TRY(cudaMemcpy(Lst.src, gs.data(), sizeof(int) * T, cudaMemcpyHostToDevice));
@@ -603,6 +770,8 @@ static int upload_list(Plan *P, RcrList &Lst, const std::vector<int> &key, const
 // the M2M pairs (box -> parent) and the L2L pairs (parent -> box) grouped by octant.
 int build_rcr_lists(Plan *P)
 {
+    int e = build_tile_tables(P);
+    if (e) return e;
     // Morton rank of every box of every level (the level sets hold the boxes' Morton numbers
     // in first-occurrence order)
     std::vector<std::vector<int>> rank(P->lmax + 1);
@@ -629,7 +798,7 @@ int build_rcr_lists(Plan *P)
                     key[t] = dir[t];
                 }
             std::vector<int> kw(P->dir_dist, P->dir_dist + NDIR);
-            int st = upload_list(P, L.m2l, key, src, dst, NDIR, kw, L.p, rank[l], L.nb);
+            int st = upload_list(P, L.m2l, PASS_M2L, key, src, dst, NDIR, kw, L.p, rank[l], L.nb);
             if (st) return st;
         }
         if (l > P->lmin) {
@@ -643,33 +812,30 @@ int build_rcr_lists(Plan *P)
                 self[b] = b;
             }
             std::vector<int> kw(8, 0);
-            int st = upload_list(P, L.m2m, key, self, par, 8, kw, PL.p, rank[l - 1], PL.nb);
+            int st = upload_list(P, L.m2m, PASS_M2M, key, self, par, 8, kw, PL.p, rank[l - 1], PL.nb);
             if (st) return st;
-            st = upload_list(P, L.l2l, key, par, self, 8, kw, PL.p, rank[l], L.nb);
+            st = upload_list(P, L.l2l, PASS_L2L, key, par, self, 8, kw, PL.p, rank[l], L.nb);
             if (st) return st;
         }
     }
     return FMM_OK;
 }
 
-} // namespace fmm
-
-namespace fmm {
-// Tile width and schedule per pass, chosen at plan creation by timing the candidates on this
-// plan's own lists and tables (one right-hand side): the default from pick_tile and a narrower
-// tile -- 4 columns where the default is 8 (large p, few items per direction: more CTAs, two
-// per SM), half the width where it is 16, 32 or 64 -- each with the default and the balanced
-// unit schedule (BAL).  The winner is kept; matvec results do not depend on the choice beyond the
-// order of the FP32 atomic additions.
+// Columns and rows per unit of each pass, chosen at plan creation by timing on this plan's own lists
+// and tables (one right-hand side): the columns of pick_tile, half and a quarter of them (passes of
+// few translations fill more SMs with narrower tiles), units of four rows, or of two (more units
+// for the threads of a narrow tile).  Matvec results do not depend on the choice beyond the order of
+// the FP32 atomic additions.  Passes that run in a tensor-core form are not timed.
 int tune_rcr_tiles(Plan *P)
 {
-    // FMMBEM_TILE_BAL=0/1/2 forces one schedule on every pass (default tile width; a shape
-    // without that schedule runs the default one), for tests
+    // FMMBEM_TILE_BAL=0/1/2 forces one shape on every pass, for tests: 0 the columns of pick_tile and
+    // units of four rows, 1 units of two rows, 2 half the columns and units of two rows
     if (const char *env = getenv("FMMBEM_TILE_BAL")) {
         const int bal = std::max(0, std::min(2, atoi(env)));
         for (int l = P->lmin; l <= P->lmax; l++)
             for (RcrList *R : {&P->lev[l].m2m, &P->lev[l].m2l, &P->lev[l].l2l}) {
-                R->bal = bal;
+                R->bal = bal ? 1 : 0;
+                if (bal == 2) R->tc = std::max(4, R->tc / 2);
                 R->items_nrhs = 0;
             }
         return FMM_OK;
@@ -683,24 +849,15 @@ int tune_rcr_tiles(Plan *P)
         for (int which = PASS_M2M; which <= PASS_L2L && rc == FMM_OK; which++) {
             if (which != PASS_M2L && l == P->lmin) continue;
             RcrList &Lst = which == PASS_M2M ? L.m2m : which == PASS_M2L ? L.m2l : L.l2l;
-            if (Lst.key_beg.empty() || Lst.key_beg.back() == 0) continue;
-            int p = which == PASS_M2L ? L.p : P->lev[l - 1].p;
-            std::vector<int3> cand = {{Lst.tc, Lst.shc, 0}};
-            if (Lst.tc == 8) cand.push_back({4, 0, 0});
-            if (Lst.tc == 16) cand.push_back({8, 0, 0});
-            if (Lst.tc >= 32) cand.push_back({Lst.tc / 2, rcr_tile_smem(p, Lst.tc / 2, 1) <= TWO_CTA_SMEM ? 1 : 0, 0});
-            // balanced variants (1: narrow column groups where they pay, 2: the default groups, one-row
-            // units) exist for every width without staged blocks, and for 32 (and 64: 1 only) with
-            for (size_t i = 0, n0 = cand.size(); i < n0; i++) {
-                if (cand[i].y == 0 || cand[i].x >= 32) cand.push_back({cand[i].x, cand[i].y, 1});
-                if (cand[i].x <= 32 && (cand[i].y == 0 || cand[i].x == 32)) cand.push_back({cand[i].x, cand[i].y, 2});
-            }
+            if (Lst.key_beg.empty() || Lst.key_beg.back() == 0 || Lst.td.on) continue;
+            std::vector<int2> cand;
+            for (int tc = Lst.tc; tc >= 4 && 4 * tc >= Lst.tc; tc /= 2)
+                for (int bal = 0; bal < 2; bal++) cand.push_back({tc, bal});
             float best = 1e30f;
-            int3 pick = cand[0];
+            int2 pick = cand[0];
             for (auto &c : cand) {
                 Lst.tc = c.x;
-                Lst.shc = c.y;
-                Lst.bal = c.z;
+                Lst.bal = c.y;
                 Lst.items_nrhs = 0;
                 float tot = 0.f;
                 for (int rep = 0; rep < 4 && rc == FMM_OK; rep++) {
@@ -719,8 +876,7 @@ int tune_rcr_tiles(Plan *P)
                 }
             }
             Lst.tc = pick.x;
-            Lst.shc = pick.y;
-            Lst.bal = pick.z;
+            Lst.bal = pick.y;
             Lst.items_nrhs = 0;
         }
     }

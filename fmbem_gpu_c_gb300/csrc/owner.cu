@@ -30,6 +30,7 @@
 // deterministic mixed on the 20,480-triangle sphere 2.36 -> 1.26 ms.
 #include "plan.h"
 #include "ff.cuh"
+#include "f32x2.cuh"
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -90,43 +91,9 @@ template <> struct Ops<double> {
 // FP32 instructions (two FP32 operations each, at the FP32 pipes' rate but half the issue slots)
 // work on re and im together.  Each operation rounds as its scalar form: ff_mac is ff_fma
 // (ff.cuh) on both parts.
-typedef unsigned long long f2;
 struct __align__(16) ffv {
     f2 hi, lo;
 };
-__device__ __forceinline__ f2 f2_pack(float a, float b)
-{
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 f2_parts(f2 a)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
-    return r;
-}
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
-{
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
-{
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
-{
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-// a - b
-__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) { return f2_fma(b, 0xbf800000bf800000ull, a); }
-
 // a table entry with both halves equal, so that a 16-byte load gives the operands of the packed
 // instructions
 struct __align__(16) ffs {

@@ -409,7 +409,7 @@ static RcrPass make_pass(int p, int pin, int pout, int atomic, const float *H, i
     ps.dst = dst;
     ps.items = nullptr;
     ps.g_src = ps.g_dst = nullptr;
-    ps.hrep = nullptr;
+    ps.g_dir = nullptr;
     return ps;
 }
 
@@ -421,7 +421,7 @@ RcrList *pass32_desc(Plan *P, int l, int which, int nrhs, RcrPass &ps)
     LevelDev &L = P->lev[l];
     if (which == PASS_M2L) {
         ps = make_pass(L.p, L.p, L.p, 1, P->Hsr32, rs, P->PHsr32, w, pmax - 1, L.Csr32, L.Cm32, L.Dl32, nrhs, L.nb, L.nb);
-        ps.hrep = P->hrep_dev;
+        ps.coax = L.Csr32p;
         return &L.m2l;
     }
     if (l <= P->lmin) return nullptr;
@@ -429,10 +429,12 @@ RcrList *pass32_desc(Plan *P, int l, int which, int nrhs, RcrPass &ps)
     if (which == PASS_M2M) {
         ps = make_pass(PL.p, L.p, PL.p, 1, P->Hss32, rs, P->PHss32, w, pmax - 1, L.Crr32, L.Cm32, PL.Cm32, nrhs, L.nb,
                        PL.nb);
+        ps.coax = L.Crr32p;
         return &L.m2m;
     }
     ps = make_pass(PL.p, PL.p, L.p, 0, P->Hrr32, rs, P->PHrr32, w, pmax - 1, L.Crr32L ? L.Crr32L : L.Crr32, PL.Dl32,
                    L.Dl32, nrhs, PL.nb, L.nb);
+    ps.coax = L.Crr32Lp ? L.Crr32Lp : L.Crr32p;
     return &L.l2l;
 }
 
@@ -442,7 +444,7 @@ int launch_pass32(Plan *P, int l, int which, int nrhs, cudaStream_t st)
     RcrList *Lst = pass32_desc(P, l, which, nrhs, ps);
     if (Lst && Lst->t3.on) return launch_tc3_pass(P, l, which, nrhs, st);
     if (Lst && Lst->td.on) return launch_tc_dense(P, l, which, nrhs, st);
-    return Lst ? launch_rcr_pass(*Lst, ps, st) : FMM_OK;
+    return Lst ? launch_rcr_pass(P, *Lst, ps, st) : FMM_OK;
 }
 
 // The mixed path's translation passes for nrhs columns: zero the expansions, M2M up, the

@@ -88,16 +88,17 @@ static void free_plan(Plan *P)
     for (int l = 0; l <= FMM_MAX_LEVEL + 1; l++) {
         LevelDev &L = P->lev[l];
         F(L.parent); F(L.octant); F(L.child_beg); F(L.child_list); F(L.sr_beg); F(L.sr_src); F(L.sr_dir);
-        F(L.Cm64); F(L.Dl64); F(L.Csr_ff); F(L.Crr_ff); F(L.CrrL_ff); F(L.Cm_ff); F(L.Dl_ff); F(L.Cm32); F(L.Dl32); F(L.Csr64); F(L.Csr32); F(L.Crr64); F(L.Crr32); F(L.Crr32L);
+        F(L.Cm64); F(L.Dl64); F(L.Csr_ff); F(L.Crr_ff); F(L.CrrL_ff); F(L.Cm_ff); F(L.Dl_ff); F(L.Cm32); F(L.Dl32); F(L.Csr64); F(L.Csr32); F(L.Crr64); F(L.Crr32); F(L.Crr32L); F(L.Csr32p); F(L.Crr32p); F(L.Crr32Lp);
         for (RcrList *R : {&L.m2l, &L.m2m, &L.l2l}) {
-            F(R->items); F(R->src); F(R->dst);
+            F(R->items); F(R->src); F(R->dst); F(R->csrc); F(R->cdst); F(R->cdir); F(R->urot); F(R->ucoax);
             Tc3 &t = R->t3;
             F(t.opsR); F(t.opsC); F(t.blkR); F(t.blkC); F(t.t_dir); F(t.itR1); F(t.itC); F(t.itR2);
             F(t.listR); F(t.listC); F(t.W); F(t.Z);
             F(R->td.B); F(R->td.items); F(R->td.src); F(R->td.dst); F(R->td.dir);
         }
     }
-    F(P->tc_err); F(P->tc_ones); F(P->hrep_dev); F(P->PHall_ff); F(P->dsc_leaf_dev);
+    F(P->rot32); F(P->pairs);
+    F(P->tc_err); F(P->tc_ones); F(P->PHall_ff); F(P->dsc_leaf_dev);
     F(P->Hsr64); F(P->PHsr64); F(P->Hsr32); F(P->PHsr32);
     F(P->V_dev); F(P->F_dev); F(P->elem_leaf); F(P->leaf_beg); F(P->leaf_elem);
     F(P->U64); F(P->Rv64); F(P->U32); F(P->Rv32); F(P->near_beg); F(P->near_col); F(P->near64); F(P->near32);
@@ -194,8 +195,8 @@ static int plan_create_impl(std::vector<double> &&V, std::vector<int> &&F, const
         P->pmax = std::max(P->pmax, p);
     }
     P->pleaf = P->lev[P->lmax].p;
-    if (P->opt.build_mixed && rcr_tile_smem(P->pmax, 4, 0) > MAX_TILE_SMEM) {
-        // the batched FP32 translations keep two p^2 x 4 complex tiles in shared memory at least
+    if (P->opt.build_mixed && P->pmax > MAX_MIXED_ORDER) {
+        // the batched FP32 translations keep a p^2 x 4 complex tile in shared memory at least
         P->opt.build_mixed = 0;
         snprintf(P->mixed_note, sizeof(P->mixed_note),
                  "mixed precision needs truncation orders <= 60 (this plan has %d); use FMM_FP64", P->pmax);
@@ -209,8 +210,6 @@ static int plan_create_impl(std::vector<double> &&V, std::vector<int> &&F, const
     CTRY(cudaMemcpy(P->elem_leaf, P->tree.elem_leaf.data(), sizeof(int) * nf, cudaMemcpyHostToDevice));
     TRY(gen_rotation_tables(P));
     TRY(set_dir_dist(P->dir_dist));
-    CTRY(dev_alloc(P, (void **)&P->hrep_dev, sizeof(int) * NDIR));
-    CTRY(cudaMemcpy(P->hrep_dev, P->dir_hrep, sizeof(int) * NDIR, cudaMemcpyHostToDevice));
     TRY(build_lists(P));
     TRY(gen_coax_tables(P));
     for (int l = P->lmin; l <= P->lmax; l++) {
@@ -240,8 +239,8 @@ static int plan_create_impl(std::vector<double> &&V, std::vector<int> &&F, const
     TRY(gen_near_field(P));
     if (P->opt.build_mixed) {
         TRY(build_rcr_lists(P));
-        TRY(tune_rcr_tiles(P));
         TRY(tune_tc_dense(P));
+        TRY(tune_rcr_tiles(P));
         TRY(tune_tc3(P));
     }
     CTRY(dev_alloc(P, (void **)&P->xbuf, sizeof(double2) * nf));

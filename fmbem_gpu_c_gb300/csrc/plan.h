@@ -56,20 +56,35 @@ struct TcDense {
     int n_items = 0, items_nrhs = 0;
 };
 
-// Work list of one batched translation pass: translations sorted by direction (src, dst,
-// key_beg per direction, key_w = coaxial block per direction) and the device items
-// (direction, first column, count, coaxial block) for items_nrhs right-hand sides, tc
-// columns per item at most.
-struct RcrList {
+// Translations sorted by key, and within a key by the Morton rank of their destination.
+struct KeyedList {
+    std::vector<int> key_beg, key_w;  // per key: first translation; coaxial block
+    std::vector<int> dst_rank;        // Morton rank of each translation's destination (list order)
+    int ndst_rank = 0;                // boxes of the destination level
+};
+
+// Work list of one batched translation pass: the translations by direction (src, dst), the same by
+// operator class (cls; csrc, cdst, cdir on the device, made on first use) and the device items
+// (class, first column, count, coaxial block) of the SIMT tiles for items_nrhs right-hand sides,
+// tc columns per item at most.
+struct RcrList : KeyedList {
+    int *src = nullptr, *dst = nullptr;
+    KeyedList cls;
+    std::vector<int> cls_of_key;
+    int rot0 = 0, key0 = 0;       // rotation table of class 0; phase row of direction 0
+    int *csrc = nullptr, *cdst = nullptr;
+    short *cdir = nullptr;        // phase row
     int4 *items = nullptr;
     size_t items_cap = 0;
-    int *src = nullptr, *dst = nullptr;
-    std::vector<int> key_beg, key_w;
-    std::vector<int> dst_rank;    // Morton rank of each translation's destination (list order)
-    int ndst_rank = 0;            // boxes of the destination level
     int n_items = 0, items_nrhs = 0;
-    int tc = 8, shc = 0;          // columns per item; rotation/coaxial blocks staged in shared memory
-    int bal = 0;                  // balanced unit schedule (1, 2: two tile shapes; one-row units, boustrophedon order)
+    int tc = 8;                   // columns per item
+    int bal = 0;                  // work units of two rows (0: of four)
+    // work units of the tile's stages for (units_tc, units_bal): rotations (the second from at3),
+    // coaxial; rounds of each stage
+    int2 *urot = nullptr;
+    int *ucoax = nullptr;
+    size_t at3 = 0;
+    int units_tc = 0, units_bal = 0, n1 = 0, n2 = 0, n3 = 0;
     Tc3 t3;                       // three-stage tensor-core form (used where t3.on)
     TcDense td;                   // dense tensor-core form (used where td.on)
 };
@@ -79,14 +94,22 @@ struct RcrPass {
     int p, pin, pout, atomic;        // RCR order, source order, destination order
     int nrhs, nsrc, ndst;            // right-hand sides; boxes per right-hand side in src and dst
     int hstride, phstride, phoff;    // per-direction strides of H and the phases; phase index m + phoff
-    const int *hrep;                 // M2L: direction -> the direction whose H table it reads (null: its own)
     const float *H;
     const float2 *PH;
     const float2 *Cc;                // coaxial blocks, item.w selects one (stride coax_size(p))
     const float2 *src;               // [boxes][rhs][pin^2]
     float2 *dst;                     // [boxes][rhs][pout^2]
-    const int4 *items;               // (direction, first, count, coaxial block) over columns e = t nrhs + r
+    const int4 *items;               // (class, first, count, coaxial block) over columns e = t nrhs + r
     const int *g_src, *g_dst;        // source and destination box of translation t
+    const short *g_dir;              // its phase row in PHall
+    // tables of the tile kernels: folded rotations per class, padded coaxial blocks, all phases,
+    // work units of the three stages, coefficient pairs (n, m >= 0)
+    const float *rot;
+    int rot_stride;
+    const float2 *coax, *PHall;
+    const int2 *u1, *u3;
+    const int *u2, *pairs;
+    int n1, n2, n3;
 };
 
 // One pass of the translations without atomics (owner.cu): translations ("slots", in destination
@@ -126,6 +149,7 @@ struct LevelDev {
     double2 *Crr64 = nullptr;     // coaxial (R|R) at order p_{l-1} for M2M into / L2L out of level l-1
     float2 *Crr32 = nullptr;      // FP32 (R|R) of the M2M (and of the L2L when not scaled)
     float2 *Crr32L = nullptr;     // FP32 (R|R) of the L2L in plans with scaled expansions
+    float2 *Csr32p = nullptr, *Crr32p = nullptr, *Crr32Lp = nullptr; // the same padded for the tile kernels
     // batched passes of the mixed path: M2L of this level, M2M (this level -> parents),
     // L2L (parents -> this level)
     RcrList m2l, m2m, l2l;
@@ -147,9 +171,6 @@ struct Plan {
     // direction tables
     int dir_slot[343];            // (dx+3)*49+(dy+3)*7+(dz+3) -> 0..315 or -1
     int dir_dist[NDIR];           // direction -> distance slot
-    int dir_hrep[NDIR];           // direction -> the first direction of equal polar angle, whose
-                                  // rotation table (bit-identical: the same acos(dz / |d|)) it reads
-    int *hrep_dev = nullptr;      // dir_hrep on the device
     double *Hsr64 = nullptr, *Hss64 = nullptr, *Hrr64 = nullptr; // real rotation coefficients at pmax
     float *Hsr32 = nullptr, *Hss32 = nullptr, *Hrr32 = nullptr;
     double2 *PHsr64 = nullptr, *PHss64 = nullptr, *PHrr64 = nullptr; // e^{i m phi}, m = -(pmax-1)..pmax-1
@@ -189,6 +210,11 @@ struct Plan {
     float4 *PHall_ff = nullptr;   // float-float phases
     int ff_ready = 0;             // 1 once the float-float tables exist, -1 where they cannot
     double *dsc_leaf_dev = nullptr; // degree scales d_n of the leaf level (plans with scaled expansions)
+    // tables of the tile kernels (batched.cu): folded rotations per class, coefficient pairs
+    float *rot32 = nullptr;
+    int rot32_stride = 0, rot32_m2l = 0;  // entries per class; M2L classes (M2M's and L2L's follow)
+    std::vector<int> rot32_off;   // per degree, inside a class
+    int *pairs = nullptr;         // coefficient pairs (n, m >= 0): n^2 + n | m << 16
     // translations without atomics (owner.cu), per type (OWN_*), level and pass
     OwnPass own[3][FMM_MAX_LEVEL + 2][3];
     int own_ready[3] = {0, 0, 0}, own_ncls = 0;
@@ -265,9 +291,6 @@ void launch_axpby(double a, const double2 *x, double b, double2 *y, size_t n, cu
 // Dense FP64 operators of a pass (passes.cu): T[c][i][j] (pout^2 x pin^2), the RCR translation
 // of key keys[c] applied to the unit source e_j; M2L without its azimuthal phases.
 int gen_dense_rcr(Plan *P, int l, int which, const int *keys, int nkeys, double2 *T);
-// Classes of a pass's keys with one rotation: M2L directions of equal (dz, dx^2 + dy^2), M2M /
-// L2L octants of equal z bit.  cls[key] = class, rep[class] = its first key.  (tc_rcr3.cu)
-void direction_classes(const Plan *P, int which, int nkeys, std::vector<int> &cls, std::vector<int> &rep);
 int tune_tc_dense(Plan *P);
 int launch_tc_dense(Plan *P, int l, int which, int nrhs, cudaStream_t st);
 int check_tc_error(Plan *P);
@@ -278,21 +301,25 @@ int launch_tc3_pass(Plan *P, int l, int which, int nrhs, cudaStream_t st);
 int tune_tc3(Plan *P);
 
 // batched.cu
+// Classes of a pass's keys with one rotation and length: M2L directions of equal (dz, dx^2 + dy^2),
+// M2M / L2L octants of equal z bit.  cls[key] = class, rep[class] = its first key.
+void direction_classes(const Plan *P, int which, int nkeys, std::vector<int> &cls, std::vector<int> &rep);
 int build_rcr_lists(Plan *P);
 int tune_rcr_tiles(Plan *P);
-size_t rcr_tile_smem(int p, int tc, int shc);
-extern const size_t MAX_TILE_SMEM;
-int launch_rcr_pass(RcrList &Lst, RcrPass ps, cudaStream_t st);
-// work items (direction, first column, count, coaxial block) of a list for one right-hand side
-void rcr_list_items(const RcrList &Lst, std::vector<int4> &out);
-// items for nrhs columns in tiles of `width`, ordered by destination Morton ranges where the
-// pass's expansions (ws_bytes) exceed L2
-void build_items(const RcrList &Lst, int nrhs, int width, size_t ws_bytes, bool coax_w, std::vector<int4> &items);
-// persistent work-queue launch over many passes of one tile shape (tc, shc, schedule bal as in
-// RcrList); smem for the largest order among them; grid from rcr_queue_prepare (resident CTAs)
-int rcr_queue_prepare(int tc, int shc, int bal, size_t smem, int nwork, int *grid);
+size_t rcr_tile_smem(int p, int tc);
+constexpr int MAX_MIXED_ORDER = 60;
+int set_tile_tables(const Plan *P, RcrList &Lst, RcrPass &ps);
+int launch_rcr_pass(const Plan *P, RcrList &Lst, RcrPass ps, cudaStream_t st);
+// work items of a list for one right-hand side, with its class order on the device
+int rcr_list_items(RcrList &Lst, std::vector<int4> &out);
+// items (key, first column, count, coaxial block) for nrhs columns in tiles of `width`, ordered
+// by destination Morton ranges where the pass's expansions (ws_bytes) exceed L2
+void build_items(const KeyedList &Lst, int nrhs, int width, size_t ws_bytes, bool coax_w, std::vector<int4> &items);
+// persistent work-queue launch over many passes of one tile shape (tc, bal); smem for the largest
+// order among them; grid from rcr_queue_prepare (resident CTAs)
+int rcr_queue_prepare(int tc, int bal, size_t smem, int nwork, int *grid);
 // (*nwork: the number of items, read on the device)
-int launch_rcr_queue(int tc, int shc, int bal, const RcrPass *passes, const int *work_pass, const int4 *work_item,
+int launch_rcr_queue(int tc, int bal, const RcrPass *passes, const int *work_pass, const int4 *work_item,
                      const int *nwork, int *head, size_t smem, int grid, cudaStream_t st);
 
 } // namespace fmm

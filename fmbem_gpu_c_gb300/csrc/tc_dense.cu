@@ -783,71 +783,43 @@ int check_tc_error(Plan *P)
     return FMM_OK;
 }
 
-static void td_free(Plan *P, TcDense &g)
-{
-    cudaFree(g.B);
-    P->device_bytes -= g.B_bytes;
-    cudaFree(g.items);
-    cudaFree(g.src);
-    cudaFree(g.dst);
-    cudaFree(g.dir);
-    g = TcDense();
-}
+// M2L levels that run dense (order p <= 16, T translations).  Large levels: the dense form is the
+// faster one (16 columns on the 81,920-triangle sphere: p = 10, 650,304 translations 5.1 ms against
+// 9.3 on the SIMT tiles; p = 14, 192,528 translations 4.8 against 6.0).  Small ones are even (6 to 8
+// thousand translations: 10 to 60 us either way); a plan keeps the form there that its timing used to
+// choose, so that its rounding (TF32 halves against FP32) stays the same: dense from 2,000
+// translations on at p = 6..14 and from 10,000 on at p = 15, 16 (tiles of 128 columns of one of 61
+// classes, which fewer translations do not fill).
+static bool dense_pays(int p, int T) { return p < 6 ? T >= 20000 : p <= 14 ? T >= 2000 : T >= 10000; }
 
-// For every pass whose source and destination orders are both <= 16 (M2L of a level, M2M
-// into and L2L out of its parent level): build the dense split operators and keep the
-// tensor-core pass where it beats the SIMT tiles on this plan (4 timed runs each), else free
-// its tables.  FMMBEM_TENSOR_M2L (M2L) and FMMBEM_TENSOR_M2M (M2M and L2L) = 0 keep the SIMT
-// tiles, = 1 take the tensor cores wherever they apply.  M2M and L2L stay on the SIMT tiles
-// unless FMMBEM_TENSOR_M2M is set: their dense form is twice as fast but about ten times
-// less accurate on the 81,920-triangle sphere (mixed against FP64 8.9e-7 against 7.7e-8),
-// which costs the refined solves more iterations than it saves.
+// Builds the dense split operators of the passes that run on the tensor cores: the M2L levels of
+// order <= 16 that dense_pays() names.  FMMBEM_TENSOR_M2L (M2L) and FMMBEM_TENSOR_M2M (M2M and
+// L2L, where both orders are <= 16) = 0 keep the SIMT tiles, = 1 take the tensor cores wherever
+// they apply.  M2M and L2L stay on the SIMT tiles unless FMMBEM_TENSOR_M2M is set: their dense
+// form is about ten times less accurate on the 81,920-triangle sphere (mixed against FP64
+// 8.9e-7 against 7.7e-8), which costs the refined solves more iterations than it saves.
 int tune_tc_dense(Plan *P)
 {
     const char *env_l = getenv("FMMBEM_TENSOR_M2L"), *env_m = getenv("FMMBEM_TENSOR_M2M");
     const int mode_l = env_l ? atoi(env_l) : -1, mode_m = env_m ? atoi(env_m) : 0;
     if (mode_l == 0 && mode_m == 0) return FMM_OK;
-    if (!P->tc_err) {
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&P->tc_err, sizeof(int)));
-        FMM_CUDA_TRY(cudaMemset(P->tc_err, 0, sizeof(int)));
-    }
-    cudaEvent_t a, b;
-    FMM_CUDA_TRY(cudaEventCreate(&a));
-    FMM_CUDA_TRY(cudaEventCreate(&b));
-    int rc = FMM_OK;
-    for (int l = P->lmin; l <= P->lmax && rc == FMM_OK; l++) {
-        for (int which = PASS_M2M; which <= PASS_L2L && rc == FMM_OK; which++) {
+    for (int l = P->lmin; l <= P->lmax; l++)
+        for (int which = PASS_M2M; which <= PASS_L2L; which++) {
             const int mode = which == PASS_M2L ? mode_l : mode_m;
             if (mode == 0) continue;
             int pin = 0, pout = 0;
             RcrList *Lst = dense_list(P, l, which, pin, pout);
             if (!Lst || Lst->key_beg.empty() || Lst->key_beg.back() == 0) continue;
-            rc = build_tc_dense(P, l, which);
-            if (rc) break;
-            if (!Lst->td.B) continue;  // orders beyond the dense form
-            float ms[2] = {0.f, 0.f};
-            for (int on = 0; on < 2 && rc == FMM_OK && mode != 1; on++) {
-                Lst->td.on = on;
-                for (int rep = 0; rep < 4 && rc == FMM_OK; rep++) {
-                    if (cudaEventRecord(a, P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    if (rc == FMM_OK) rc = launch_pass32(P, l, which, 1, P->stream);
-                    if (rc == FMM_OK && cudaEventRecord(b, P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    if (rc == FMM_OK && cudaEventSynchronize(b) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    float t = 0.f;
-                    cudaEventElapsedTime(&t, a, b);
-                    if (rep > 0) ms[on] += t;
-                }
+            if (mode != 1 && !dense_pays(pin, Lst->key_beg.back())) continue;
+            if (!P->tc_err) {
+                FMM_CUDA_TRY(dev_alloc(P, (void **)&P->tc_err, sizeof(int)));
+                FMM_CUDA_TRY(cudaMemset(P->tc_err, 0, sizeof(int)));
             }
-            if (rc == FMM_OK) rc = check_tc_error(P);
-            if (rc) break;
-            Lst->td.on = (mode == 1 || ms[1] < ms[0]) ? 1 : 0;
-            if (!Lst->td.on) td_free(P, Lst->td);
+            int rc = build_tc_dense(P, l, which);
+            if (rc) return rc;
+            Lst->td.on = Lst->td.B ? 1 : 0;  // (orders beyond the dense form have no operators)
         }
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    if (rc == FMM_ERR_CUDA && !fmm_last_error()[0]) fmm_set_error("tensor-core pass tuning: %s", cudaGetErrorString(cudaGetLastError()));
-    return rc;
+    return FMM_OK;
 }
 
 } // namespace fmm

@@ -548,34 +548,6 @@ static inline void t3_put(float *tab, long long base, int Npad, int o, int k, do
 }
 
 // polar-angle class of every key (direction or octant) of a pass
-void direction_classes(const Plan *P, int which, int nkeys, std::vector<int> &cls, std::vector<int> &rep)
-{
-    cls.assign(nkeys, -1);
-    rep.clear();
-    std::map<long long, int> seen;
-    for (int d = 0; d < nkeys; d++) {
-        long long key;
-        if (which == PASS_M2L) {
-            int s = -1;
-            for (int q = 0; q < 343; q++)
-                if (P->dir_slot[q] == d) s = q;
-            int dx = s / 49 - 3, dy = (s / 7) % 7 - 3, dz = s % 7 - 3;
-            key = (long long)(dz + 8) * 1000 + dx * dx + dy * dy;
-        } else {
-            key = d & 1; // octant: the z bit fixes the polar angle
-        }
-        auto itc = seen.find(key);
-        if (itc == seen.end()) {
-            int id = (int)rep.size();
-            seen[key] = id;
-            rep.push_back(d);
-            cls[d] = id;
-        } else {
-            cls[d] = itc->second;
-        }
-    }
-}
-
 int build_tc3(Plan *P, int l, int which)
 {
     RcrPass ps;
