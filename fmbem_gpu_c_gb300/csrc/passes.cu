@@ -84,7 +84,7 @@ __device__ void rcr_block(int p, int pmax, const double *__restrict__ H, const d
         sW2[i] = mk2(ar, ai);
     }
     __syncthreads();
-    const int po2 = pout * pout;
+    const int po2 = min(p, pout) * min(p, pout);  // no outputs beyond the translation's order
     for (int i = tid; i < po2; i += nt) {
         int n, mp;
         decode_nm(i, n, mp);
@@ -612,27 +612,24 @@ static int run_matvec_t(Plan *P, const double2 *x, double2 *y, int transpose, in
 }
 
 // Dense operators for the tensor-core passes: T[c][i][j] (pout^2 x pin^2, FP64), the RCR
-// translation of key keys[c] applied to the unit source e_j.  M2L (ph = null): direction
-// keys[c] with its azimuthal phases left out (rotation by the polar angle, coaxial
-// translation, rotation back); the translation of any direction d with the same polar angle
-// and distance is then diag(e^{-i m' phi_d}) T diag(e^{i m phi_d}).  M2M / L2L: octant keys[c]
-// with its phases.  One CTA per (operator, column).
+// translation of key keys[c] (M2L direction, M2M / L2L octant) applied to the unit source e_j, with
+// its azimuthal phases left out (rotation by the polar angle, coaxial translation, rotation back);
+// the translation of any key d with the same polar angle and distance is then
+// diag(e^{-i m' phi_d}) T diag(e^{i m phi_d}).  One CTA per (operator, column).
 __global__ void dense_rcr_kernel(int p, int pmax, int pin, int pout, const int *__restrict__ keys,
-                                 const double *__restrict__ H, const double2 *__restrict__ PH,
-                                 const double2 *__restrict__ Cc, int coax_per_dir, double2 *__restrict__ T)
+                                 const double *__restrict__ H, const double2 *__restrict__ Cc, int coax_per_dir,
+                                 double2 *__restrict__ T)
 {
     extern __shared__ unsigned char smraw[];
     const int P2 = p * p, c = blockIdx.x, d = keys[c], j = blockIdx.y, rs = rot_size(pmax), w = 2 * pmax - 1;
     const int pi2 = pin * pin, po2 = pout * pout;
-    double2 *sE = (double2 *)smraw, *sX = sE + P2, *sW1 = sX + P2, *sW2 = sW1 + P2, *sY = sW2 + P2, *sOne = sY + P2;
-    for (int i = threadIdx.x; i < P2; i += blockDim.x) {
-        sE[i] = make_double2(i == j ? 1.0 : 0.0, 0.0);
-        sY[i] = make_double2(0.0, 0.0);
-    }
+    double2 *sE = (double2 *)smraw, *sX = sE + P2, *sW1 = sX + P2, *sW2 = sW1 + P2, *sY = sW2 + P2, *sOne = sY + max(P2, po2);
+    for (int i = threadIdx.x; i < P2; i += blockDim.x) sE[i] = make_double2(i == j ? 1.0 : 0.0, 0.0);
+    for (int i = threadIdx.x; i < po2; i += blockDim.x) sY[i] = make_double2(0.0, 0.0);
     for (int i = threadIdx.x; i < w; i += blockDim.x) sOne[i] = make_double2(1.0, 0.0);
     __syncthreads();
     const double2 *cb = Cc + (coax_per_dir ? (size_t)c_dir_dist[d] * coax_size(p) : 0);
-    rcr_block(p, pmax, H + (size_t)d * rs, PH ? PH + (size_t)d * w : sOne, cb, sE, pin, sX, sW1, sW2, sY, pout);
+    rcr_block(p, pmax, H + (size_t)d * rs, sOne, cb, sE, pin, sX, sW1, sW2, sY, pout);
     for (int i = threadIdx.x; i < po2; i += blockDim.x) T[((size_t)c * po2 + i) * pi2 + j] = sY[i];
 }
 
@@ -641,11 +638,10 @@ int gen_dense_rcr(Plan *P, int l, int which, const int *keys, int nkeys, double2
     const LevelDev &L = P->lev[l];
     int p, pin, pout;
     const double *H;
-    const double2 *PH, *Cc;
+    const double2 *Cc;
     if (which == PASS_M2L) {
         p = pin = pout = L.p;
         H = P->Hsr64;
-        PH = nullptr;
         Cc = L.Csr64;
     } else {
         const int pp = P->lev[l - 1].p;  // the RCR order of M2M / L2L is the parent's
@@ -653,13 +649,12 @@ int gen_dense_rcr(Plan *P, int l, int which, const int *keys, int nkeys, double2
         pin = which == PASS_M2M ? L.p : pp;
         pout = which == PASS_M2M ? pp : L.p;
         H = which == PASS_M2M ? P->Hss64 : P->Hrr64;
-        PH = which == PASS_M2M ? P->PHss64 : P->PHrr64;
         Cc = L.Crr64;
     }
-    size_t sm = ((size_t)5 * p * p + 2 * P->pmax) * sizeof(double2);
+    size_t sm = ((size_t)4 * p * p + std::max(p, pout) * std::max(p, pout) + 2 * P->pmax) * sizeof(double2);
     if (sm > 48 * 1024) FMM_CUDA_TRY(cudaFuncSetAttribute(dense_rcr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    dense_rcr_kernel<<<dim3(nkeys, pin * pin), 128, sm, P->stream>>>(p, P->pmax, pin, pout, keys, H, PH, Cc,
-                                                                   which == PASS_M2L ? 1 : 0, T);
+    dense_rcr_kernel<<<dim3(nkeys, pin * pin), 128, sm, P->stream>>>(p, P->pmax, pin, pout, keys, H, Cc, which == PASS_M2L ? 1 : 0,
+                                                                   T);
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
@@ -690,9 +685,9 @@ static int ensure_rhs32(Plan *P, int nrhs)
         cudaFree(L.Dl32);
         L.Cm32 = nullptr;
         L.Dl32 = nullptr;
-        P->device_bytes -= 2 * sizeof(float2) * n * P->rhs_cap32;
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Cm32, sizeof(float2) * n * nrhs));
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Dl32, sizeof(float2) * n * nrhs));
+        P->device_bytes -= 2 * sizeof(float2) * (n * P->rhs_cap32 + 1);
+        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Cm32, sizeof(float2) * (n * nrhs + 1)));
+        FMM_CUDA_TRY(dev_alloc(P, (void **)&L.Dl32, sizeof(float2) * (n * nrhs + 1)));
     }
     P->rhs_cap32 = nrhs;
     P->buf_gen++;

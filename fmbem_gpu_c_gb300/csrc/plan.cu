@@ -98,7 +98,7 @@ static void free_plan(Plan *P)
         }
     }
     F(P->rot32); F(P->pairs);
-    F(P->tc_err); F(P->tc_ones); F(P->PHall_ff); F(P->dsc_leaf_dev);
+    F(P->tc_err); F(P->PHall_ff); F(P->dsc_leaf_dev);
     F(P->Hsr64); F(P->PHsr64); F(P->Hsr32); F(P->PHsr32);
     F(P->V_dev); F(P->F_dev); F(P->elem_leaf); F(P->leaf_beg); F(P->leaf_elem);
     F(P->U64); F(P->Rv64); F(P->U32); F(P->Rv32); F(P->near_beg); F(P->near_col); F(P->near64); F(P->near32);
@@ -218,8 +218,8 @@ static int plan_create_impl(std::vector<double> &&V, std::vector<int> &&F, const
         CTRY(dev_alloc(P, (void **)&L.Cm64, sizeof(double2) * n));
         CTRY(dev_alloc(P, (void **)&L.Dl64, sizeof(double2) * n));
         if (P->opt.build_mixed) {
-            CTRY(dev_alloc(P, (void **)&L.Cm32, sizeof(float2) * n));
-            CTRY(dev_alloc(P, (void **)&L.Dl32, sizeof(float2) * n));
+            CTRY(dev_alloc(P, (void **)&L.Cm32, sizeof(float2) * (n + 1)));
+            CTRY(dev_alloc(P, (void **)&L.Dl32, sizeof(float2) * (n + 1)));
         }
     }
     {

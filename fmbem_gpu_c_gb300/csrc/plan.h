@@ -3,6 +3,7 @@
 #include "fmm_common.cuh"
 #include "octree_host.h"
 #include "../../include/fmmbem.h"
+#include <stdint.h>
 #include <vector>
 
 namespace fmm {
@@ -40,15 +41,47 @@ struct Tc3 {
 // so the class's directions differ only by their azimuthal phases, which the kernel applies
 // to each row.  M2M / L2L: one operator per octant.  Real-embedded and split into TF32 hi/lo
 // parts in the layout the MMA reads.
+constexpr int TC_MAXCH = 40, TC_MAXPIECE = 10, TC_MAXSUB = 4;
+constexpr int TC_PAD = 256;
+
+// Output degrees [beg, end) of a dense pass: MMA widths of the sums' and differences' blocks, offset of
+// their operator in a class's (floats), groups of degrees of the epilogue and those of its second warp.
+struct TcSub {
+    int beg, end, nP, nQ, boff, ngrp;
+    unsigned second;
+    unsigned char grp[18];
+};
+
+// A run of source coefficients copied at a time (from c0 on) and its chunks [beg, end).
+struct TcPiece {
+    int c0, cnt, beg, end;
+};
+
+// An input of a dense pass: offsets of its coefficients (n, m) and (n, -m) in their piece and of the phase
+// of m, in bytes (m = TC_PAD: none).
+struct TcIn {
+    int pos, neg, m;
+};
+
+// Shape of a dense pass (tc_dense.cu).
+struct TcShape {
+    int nch, npiece, nsub;
+    int fold;                              // sums and differences of x_m, x_-m (else both as they are)
+    int sets, setw, nst;                   // sets of accumulators and their TMEM columns; stages
+    int bstage, row_stride, epi_stride;    // bytes of a stage's operator, of a source row's piece, of a staged row
+    int cls_floats;                        // operator of a class
+    TcPiece piece[TC_MAXPIECE];
+    TcSub sub[TC_MAXSUB];
+    TcIn tab[4 * TC_MAXCH];                // four per chunk
+};
+
 struct TcDense {
     int on = 0;                   // the pass runs on the tensor cores
     int pin = 0, pout = 0;        // source and destination orders
-    int phased = 0;               // M2L: operators per class, phases per row
-    int KC = 40, nch = 0, nhalf = 1, CH = 0, Nmma = 0;
-    int res = 0;                  // the whole operator of a class stays in shared memory (small p)
+    TcShape sh = {};
     int ncls = 0;                 // operators
     std::vector<int> cls_of_dir;  // key (direction or octant) -> operator
-    float *B = nullptr;           // [class][half][chunk][hi, lo][Nmma x KC core-matrix tile]
+    float *B = nullptr;           // the operators' blocks in the order of their copies
     size_t B_bytes = 0;
     int4 *items = nullptr;        // (class, first column, count, 0), 128 columns each
     size_t items_cap = 0;
@@ -206,7 +239,6 @@ struct Plan {
     cudaGraphExec_t graph_exec = nullptr; // captured mixed translation passes for graph_nrhs columns
     int graph_nrhs = 0, graph_seen = 0;
     int *tc_err = nullptr;        // set by a tensor-core pass when one of its waits gives up
-    float2 *tc_ones = nullptr;    // phases of the tensor-core passes without phases (all 1)
     float4 *PHall_ff = nullptr;   // float-float phases
     int ff_ready = 0;             // 1 once the float-float tables exist, -1 where they cannot
     double *dsc_leaf_dev = nullptr; // degree scales d_n of the leaf level (plans with scaled expansions)

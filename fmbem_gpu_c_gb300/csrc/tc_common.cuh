@@ -1,4 +1,4 @@
-// Helpers shared by the tcgen05 kernels (tc_m2l.cu, tc_rcr3.cu): the no-swizzle K-major
+// Helpers shared by the tcgen05 kernels (tc_dense.cu, tc_rcr3.cu): the no-swizzle K-major
 // core-matrix layout of shared-memory operands, shared-memory matrix descriptors, TF32 hi/lo
 // splitting, and mbarrier waits with a time limit.
 #pragma once
@@ -32,16 +32,22 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
 }
 
-// wait for the phase of the given parity of an mbarrier, at most `limit` SM clock cycles;
-// false when the wait gave up
+// one try of a wait for the phase of the given parity of an mbarrier
+__device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done;
+}
+
+// wait for that phase, at most `limit` SM clock cycles; false when the wait gave up
 __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, long long limit)
 {
+    if (mbar_try(bar, parity)) return true;
     long long t0 = clock64();
     for (int tries = 0;; tries++) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
+        if (mbar_try(bar, parity)) return true;
         if (clock64() - t0 > limit) return false;
         // a waiting warp leaves its issue slots to the warps that work
         if (tries >= 4) __nanosleep(64);
@@ -50,6 +56,27 @@ __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, l
 
 // the kernel's waits: at most ~1 s of SM clock
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_wait_limit(bar, parity, 2000000000LL); }
+
+// mbar_wait() by a whole warp, with one outcome for all its lanes: the warp stays converged, so that what
+// follows can keep its operands in uniform registers.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity)
+{
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+    const long long t0 = clock64();
+    for (int tries = 0;; tries++) {
+        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, clock64() - t0 > 2000000000LL)) return false;
+        if (tries >= 4) __nanosleep(64);
+    }
+}
+
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(one));
+    return one != 0;
+}
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 {

@@ -1,39 +1,52 @@
 // Batched translation passes of the mixed path on the 5th-generation tensor cores
 // (tcgen05.mma, kind::tf32) as dense operators: the M2L of the levels whose operators are small
 // enough to store densely (p <= 16, the levels that carry most translations) and, on request,
-// the M2M and L2L of those levels (one operator per octant).
+// the M2M and L2L of those levels.
 //
 // The translation of direction d is T_d = diag(e^{-i m' phi_d}) S_c diag(e^{i m phi_d}) (the RCR
 // product of translation.cu:1864-1961 with its azimuthal phases taken out), where S_c (p^2 x p^2
-// complex, formed once at plan time) depends only on the polar angle and the distance of d:
-// the 316 directions fall into about 60 classes c of equal (dz, dx^2 + dy^2).  With the rows of
-// a tile being 128 translations of one class (times right-hand sides), the pass is the real GEMM
-//     D[t][o] = sum_k A[t][k] B[o][k],   A[t] = source expansion of translation t times e^{i m phi},
-//                                         B    = S_c embedded as a real 2p^2 x 2p^2 matrix,
-// k and o running over interleaved (re, im) parts, and the epilogue multiplies row t's outputs
-// by e^{-i m' phi} of its own direction.  Split TF32 (3 products hi*hi + hi*lo + lo*hi of
-// rounded 11-bit halves) gives close to FP32 accuracy.
+// complex, formed once at plan time) depends only on the polar angle and the distance of d: the
+// 316 M2L directions fall into 61 classes c of equal (dz, dx^2 + dy^2), the 8 octants of M2M and
+// L2L into 2.  S_c moves along a vector of the x-z plane, so the reflection y -> -y (m -> -m)
+// commutes with it: in the sums and differences x_m + x_-m, x_m - x_-m (m >= 0) of the phased
+// source it falls into two blocks of p (p + 1) / 2 and p (p - 1) / 2 coefficients, half the
+// products of the whole operator.  A tile is 128 translations of one class (times right-hand
+// sides); the pass is the pair of real GEMMs
+//     D[t][o] = sum_k A[t][k] B[o][k],   A = sums (differences) of the phased source, re and im,
+//                                         B = the block, embedded as a real matrix,
+// and the epilogue turns sums and differences back into m and -m and applies e^{-i m' phi} of the
+// row's own direction.  (Levels with fewer translations keep x_m and x_-m as the two operands
+// and all four blocks, fold_pays().)  Split TF32 (3 products hi*hi + hi*lo + lo*hi of rounded 11-bit halves)
+// gives close to FP32 accuracy.
 //
-// A persistent, warp-specialised kernel (one CTA per SM, 18 warps) runs over the tiles
-// (128 translations x one output half):
-//   warp 0     issues the MMAs (one thread) into one of two TMEM accumulators (2 x 256 columns)
-//              and commits each K chunk to its stage's "empty" barrier, each tile to its
-//              accumulator's "full" barrier;
-//   warp 1     copies the operator's K chunks (hi and lo tiles, contiguous) with cp.async.bulk;
-//   warps 2-9  gather the source expansions, two threads per row (translation), each half of
-//              every 16-wide K chunk, apply the row's phases, split them into TF32 hi / lo and
-//              store them in the no-swizzle K-major core-matrix layout;
-//   warps 10-17 read a finished accumulator (tcgen05.ld; two warps per TMEM lane quarter, on
-//              alternate 32-column blocks), stage 32 columns at a time in shared memory, apply
-//              each row's phases and add them into the destination expansions with 16-byte FP32
-//              atomics, overlapping the next tile's MMAs.
-// Four shared-memory stages of KC = 16; every wait has a time limit, after which the thread sets
-// the plan's error flag and stops.  Where one output half's whole operator fits beside the A
-// stages (p <= 8), it stays resident instead: each CTA takes a contiguous range of tiles, warp 1
-// copies a class's operator once per run of its tiles (operator-full barrier), and the MMA
-// warp releases it after the run's last tile (a commit to the operator-empty barrier).
+// A persistent, warp-specialised kernel (one CTA per SM, 19 warps) runs over the tiles
+// (128 translations x one range of output degrees):
+//   warp 0     issues the MMAs (one thread) into one of two sets of TMEM accumulators and commits
+//              each K chunk to the "empty" barriers of its operands, each tile to its
+//              accumulators' "full" barrier;
+//   warp 1     copies the operator's K chunks (hi and lo tiles of both blocks) with cp.async.bulk;
+//   warp 2     copies the source expansions, row by row, in pieces of whole degrees;
+//   warps 3-10 (two per TMEM lane quarter, on alternate chunks; lane = row) read four coefficient
+//              pairs (n, m), (n, -m) of their row, apply its phases, form sums and differences,
+//              split them into TF32 hi / lo and write them to TMEM as the MMA's A operand;
+//   warps 11-18 (two per quarter, on alternate groups of degrees) read the finished accumulators,
+//              form the group's coefficients of their row in shared memory and add them into the
+//              destination expansions with 16-byte FP32 atomics, overlapping the next tile's MMAs.
+// Every wait has a time limit, after which the thread sets the plan's error flag and stops.
+//
+// What bounds it: 16 columns on the 81,920-triangle sphere, p = 14 (192,528 translations) 2.78 ms and
+// p = 10 (650,304) 3.21 ms.  At p = 10 a tile takes 10,000 cycles, of which the MMAs need 4,400 (52 cycles
+// each at N = 112 / 96, the full TF32 rate) and the reductions into L2 4,900 (20 bytes a cycle and SM is
+// what the L2 takes from all of them); the issue slots are 63 % busy, a third of them with A's phases
+// and splits.  At p = 14 (one set of accumulators) reading them out, 10,000 of 36,000 cycles, is not hidden.  An earlier
+// form, with the whole operator, A in shared memory and one atomic per 16 bytes of output, took 5.96
+// and 5.58 ms (its load/store unit 80 % busy with rows read 16 bytes a lane, A's stores and the atomics).
+// What made the difference: half the products; A through TMEM; source rows by cp.async, a row per
+// instruction; outputs by bulk reductions, a row's group per instruction; the MMA's issue by one
+// elected thread with operands in uniform registers (500 instead of 950 cycles per six MMAs).
 #include "plan.h"
 #include "tc_common.cuh"
+#include "f32x2.cuh"
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -42,426 +55,572 @@
 namespace fmm {
 
 constexpr int TC_M = 128;               // translations per tile (MMA M)
-constexpr int TC_KC = 16;               // K per stage (2 MMA K-steps of 8)
-constexpr int TC_STAGES = 4;
-constexpr int TC_AWARPS = 8;            // source-gather warps (2..9)
-constexpr int TC_EPI0 = 2 + TC_AWARPS;  // first epilogue warp
-constexpr int TC_EWARPS = 8;            // epilogue warps (10..17), two per TMEM lane quarter
-constexpr int TC_THREADS = 32 * (TC_EPI0 + TC_EWARPS);
-// orders up to 16: at p = 20 (K = 800) the dense form's rounding (FP32 accumulation of 300
-// split products per output) raised the iterations of the refined 64-column solve on the
-// 200,000-triangle head-like body from 48 to 56, which cost more than its faster M2L saved
+constexpr int TC_KC = 8;                // K per chunk and block: four complex inputs (n, m >= 0)
+constexpr int TC_RW = 2;                // warps that copy source rows
+constexpr int TC_A0 = 2 + TC_RW, TC_AW = 8;  // source warps
+constexpr int TC_E0 = TC_A0 + TC_AW, TC_EW = 8;  // epilogue warps
+constexpr int TC_THREADS = 32 * (TC_E0 + TC_EW);
+// orders up to 16: at p = 20 the dense form's rounding (FP32 accumulation of 300 split products
+// per output) raised the iterations of the refined 64-column solve on the 200,000-triangle
+// head-like body from 48 to 56, which cost more than its faster M2L saved
 constexpr int TC_MAXP = 16;
-constexpr int TC_MTAB = TC_MAXP * TC_MAXP + 8;  // order m of every coefficient (int8), zero padded
-constexpr int TC_EPI_LD = 33;           // staging row stride (floats) of the epilogue
+constexpr int TC_SLOTS = 2;             // pieces of 128 rows in shared memory
+constexpr int TC_STAGES = 6;            // stages of the operands, at most
+constexpr int TC_ACOL = 4 * TC_KC;      // TMEM columns of an A stage: hi and lo of both blocks
 constexpr size_t TC_SMEM_MAX = 232448;  // 227 KB of dynamic shared memory per CTA
 
 struct TcPass {
+    TcShape sh;
     const int4 *items;
     const int *g_src, *g_dst, *g_dir;    // per translation (class order): boxes and direction
     const float2 *PH;                    // phases e^{i m phi} of direction d at d phstride + phoff + m
     int phstride, phoff;
-    int phased;                          // M2L: phases per row (pin = pout); M2M / L2L: none (PH a
-                                         // table of ones, phstride 0)
-    int nrhs, nsrc, ndst;
-    int pin, P2o, K, nch, nhalf, CH, Nmma, ntiles;  // K = 2 pin^2 inputs, P2o = pout^2 outputs
-    int res;                      // operator resident: one output half, whole operator in shared memory
+    int nrhs, P2, P2o, ntiles;           // P2 = pin^2, P2o = pout^2
     const float *B;
     const float2 *src;
     float2 *dst;
     int *err;
 };
 
-static size_t tc_stage_bytes(int Nmma) { return (size_t)8 * TC_KC * (TC_M + Nmma); }
-// res = 0: stages of (A hi, A lo, B hi, B lo); res = 1: stages of (A hi, A lo) and the whole
-// operator of one direction (nch chunks of B hi, B lo) resident
-static size_t tc_smem_bytes(int Nmma, int res, int nch)
+static __host__ __device__ __forceinline__ int up16(int n) { return (n + 15) / 16 * 16; }
+
+// stride of a row of `coefs` coefficients in shared memory, one to spare: 16-byte steps, an odd number
+static int tc_stride(int coefs) { return 16 * (((8 * coefs + 8 + 15) / 16) | 1); }
+static size_t tc_smem_bytes(const TcShape &g)
 {
-    size_t main = res ? TC_STAGES * (size_t)8 * TC_KC * TC_M + (size_t)nch * 8 * TC_KC * Nmma : TC_STAGES * tc_stage_bytes(Nmma);
-    return main + TC_EWARPS * 32 * TC_EPI_LD * sizeof(float) + (2 * TC_STAGES + 6) * 8 + 16 + TC_MTAB;
+    return (size_t)g.nst * g.bstage + (size_t)TC_SLOTS * TC_M * g.row_stride + (size_t)TC_EW * 32 * g.epi_stride +
+           (2 * (TC_SLOTS + g.nst) + 4) * 8 + 16;
 }
 
-// Output halves and MMA width for source order pin and destination order pout: each half holds
-// CH coefficients (2 CH real outputs, Nmma = that rounded up to 16, <= 256); K = 2 pin^2 in
-// chunks of 16.
-static bool tc_geometry(int pin, int pout, TcDense &g)
+// The pass's shape for source order pin and destination order pout.
+// Inputs: the pairs (n, m >= 0), degree by degree, in pieces of whole degrees (a row's copy), each
+// piece in chunks of four; the cut with the fewest chunks.
+// Outputs: ranges of degrees, each two blocks of MMA columns (rounded up to 16, at most 256).  Where
+// all degrees take at most 208 columns (p <= 10), two sets of accumulators and three A stages fit
+// into the 512 of TMEM, and the epilogue overlaps the next tile's MMAs; beyond, one set of up to 416 columns
+// (the cut with the fewest): forming A once for all of a row's outputs saves more than the
+// overlap would (17.5 against 17.8 ms for 16 columns on the 81,920-triangle sphere, 1.13 against 1.17 ms for
+// one on a 27,380-triangle body with p = 16 and 12).  Without the fold a chunk's operator takes twice the
+// room, so there are always ranges of at most 208 columns and two sets.
+// Pieces and groups as large as shared memory allows.
+static bool tc_shape(int pin, int pout, int fold, TcShape &g)
 {
     if (pin < 4 || pin > TC_MAXP || pout < 4 || pout > TC_MAXP) return false;
-    const int P2 = pout * pout, K = 2 * pin * pin;
-    for (g.nhalf = 1;; g.nhalf++) {
-        g.CH = (P2 + g.nhalf - 1) / g.nhalf;
-        g.Nmma = (2 * g.CH + 15) / 16 * 16;
-        if (g.Nmma <= 256) break;
+    auto tri = [](int n) { return n * (n + 1) / 2; };
+    auto cut = [](int p, auto cost, std::vector<int> &at) {  // cost(a, b) < 0: degrees [a, b) do not fit
+        std::vector<int> best(p + 1, 1 << 30), from(p + 1, 0);
+        best[0] = 0;
+        for (int b = 1; b <= p; b++)
+            for (int a = 0; a < b; a++) {
+                const int c = cost(a, b);
+                if (c >= 0 && best[a] + c < best[b]) best[b] = best[a] + c, from[b] = a;
+            }
+        at.clear();
+        for (int b = p; b > 0; b = from[b]) at.push_back(from[b]);
+        std::reverse(at.begin(), at.end());
+        at.push_back(p);
+    };
+    std::vector<int> at;
+    auto sums = [&](int a, int b) { return up16(2 * (tri(b) - tri(a))); };
+    auto diffs = [&](int a, int b) { return up16(std::max(2 * (tri(b - 1) - tri(a - 1)), 16)); };
+    g.fold = fold;
+    g.sets = !fold || sums(0, pout) + diffs(0, pout) <= 208 ? 2 : 1;
+    const int most_columns = fold ? 416 : 208, parts = fold ? 1 : 2;
+    cut(pout, [&](int a, int b) {
+        const int w = sums(a, b) + diffs(a, b);
+        return w > most_columns || sums(a, b) > 256 ? -1 : w + 8;
+    }, at);
+    g.nsub = (int)at.size() - 1;
+    if (g.nsub > TC_MAXSUB) return false;
+    g.setw = 0;
+    for (int i = 0; i < g.nsub; i++) {
+        TcSub &s = g.sub[i];
+        s.beg = at[i];
+        s.end = at[i + 1];
+        s.nP = sums(s.beg, s.end);
+        s.nQ = diffs(s.beg, s.end);
+        g.setw = std::max(g.setw, s.nP + s.nQ);
     }
-    g.KC = TC_KC;
-    g.nch = (K + TC_KC - 1) / TC_KC;
-    if (tc_smem_bytes(g.Nmma, 0, g.nch) > TC_SMEM_MAX) return false;
-    // one output half whose whole operator fits beside the A stages (p <= 8): the operator
-    // stays in shared memory while a CTA's consecutive tiles keep its class
-    g.res = g.nhalf == 1 && tc_smem_bytes(g.Nmma, 1, g.nch) <= TC_SMEM_MAX ? 1 : 0;
-    return true;
+    g.bstage = parts * 2 * TC_KC * 4 * g.setw;
+    static const int sizes[][2] = {{53, 36}, {53, 32}, {36, 36}, {36, 32}, {31, 31}};  // a degree of p <= 16 has up to 31
+    for (auto &size : sizes) {
+        const int piece = size[0], group = size[1];
+        cut(pin, [&](int a, int b) { return b * b - a * a > piece ? -1 : 64 * ((tri(b) - tri(a) + 3) / 4) + 1; }, at);
+        g.npiece = (int)at.size() - 1;
+        if (g.npiece > TC_MAXPIECE) continue;
+        g.nch = g.row_stride = 0;
+        for (int i = 0; i < g.npiece; i++) {
+            const int a = at[i], b = at[i + 1], nc = (tri(b) - tri(a) + 3) / 4;
+            g.piece[i] = {a * a, b * b - a * a, g.nch, g.nch + nc};
+            g.row_stride = std::max(g.row_stride, tc_stride(b * b - a * a));
+            if (g.nch + nc > TC_MAXCH) return false;
+            int k = 4 * g.nch;
+            for (int n = a; n < b; n++)
+                for (int m = 0; m <= n; m++) g.tab[k++] = {8 * (n * n + n + m - a * a), 8 * (n * n + n - m - a * a), 8 * m};
+            g.nch += nc;
+            while (k < 4 * g.nch) g.tab[k++] = {0, 0, TC_PAD};  // coefficient 0 of the piece against a zero operator
+        }
+        g.epi_stride = tc_stride(group);
+        for (int i = 0; i < g.nsub; i++) {
+            // groups of degrees of the epilogue, few of them and few that start on an odd coefficient, and
+            // the warp of a quarter that takes each (the larger first, to the warp with less)
+            TcSub &s = g.sub[i];
+            const int most = std::min(group, std::max(2 * s.end - 1, (s.end * s.end - s.beg * s.beg) / 2 + 8));
+            cut(s.end - s.beg, [&](int a, int b) {
+                a += s.beg, b += s.beg;
+                return b * b - a * a > most ? -1 : 3 + 2 * (a & 1);
+            }, at);
+            s.ngrp = (int)at.size() - 1;
+            for (int k = 0; k <= s.ngrp; k++) s.grp[k] = (unsigned char)(s.beg + at[k]);
+            auto coefs = [&](int k) { return s.grp[k + 1] * s.grp[k + 1] - s.grp[k] * s.grp[k]; };
+            std::vector<int> order(s.ngrp);
+            for (int k = 0; k < s.ngrp; k++) order[k] = k;
+            std::sort(order.begin(), order.end(), [&](int a, int b) { return coefs(a) > coefs(b); });
+            int load[2] = {0, 0};
+            s.second = 0;
+            for (int k : order) {
+                const int w = load[1] < load[0];
+                load[w] += coefs(k);
+                s.second |= (unsigned)w << k;
+            }
+        }
+        const int room = (512 - g.sets * g.setw) / TC_ACOL;
+        for (g.nst = std::min(TC_STAGES, room); g.nst > 3 && tc_smem_bytes(g) > TC_SMEM_MAX; g.nst--) {}
+        if (g.nst >= 3 && tc_smem_bytes(g) <= TC_SMEM_MAX) {
+            g.cls_floats = 0;
+            for (int i = 0; i < g.nsub; i++) {
+                g.sub[i].boff = g.cls_floats;
+                g.cls_floats += parts * g.nch * 2 * TC_KC * (g.sub[i].nP + g.sub[i].nQ);
+            }
+            return true;
+        }
+    }
+    return false;
 }
 
-// degree n and order m of coefficient i = n^2 + n + m
-__device__ __forceinline__ void tc_nm(int i, int &n, int &m)
+__device__ __forceinline__ void tc_commit(uint32_t bar)
 {
-    int q = (int)sqrtf((float)i);
-    while (q * q > i) q--;
-    while ((q + 1) * (q + 1) <= i) q++;
-    n = q;
-    m = i - q * q - q;
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// destination / source expansion of row r of tile (it): column e = translation t x nrhs + r,
-// expansions stored [box][rhs][p^2]
-__device__ __forceinline__ int tile_box(const TcPass &ps, int4 it, int r, bool source)
+__device__ __forceinline__ void tc_bulk(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
 {
-    if (r >= it.z) return -1;
-    int e = it.y + r, t = e / ps.nrhs, rr = e - t * ps.nrhs;
-    return (source ? ps.g_src[t] : ps.g_dst[t]) * ps.nrhs + rr;
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
 }
 
-__global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(TcPass ps)
+__device__ __forceinline__ void tc_reduce(float2 *dst, uint32_t src, uint32_t bytes)
+{
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+                 : "memory");
+}
+
+__device__ __forceinline__ void tc_expect(uint32_t bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// one split product: A in TMEM, B in shared memory (low half of its descriptor; K-adjacent core
+// matrices 128 bytes apart, groups of 8 rows 256)
+constexpr uint32_t TC_DESC_LO = 128u >> 4 << 16, TC_DESC_HI = 256u >> 4 | 1u << 14;
+__device__ __forceinline__ void tc_mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t add)
+{
+    asm volatile("{\n\t.reg .pred q;\n\t.reg .b64 bd;\n\tmov.b64 bd, {%2, %5};\n\tsetp.ne.b32 q, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], bd, %3, q;\n\t}" ::"r"(d),
+                 "r"(a), "r"(b), "r"(idesc), "r"(add), "r"(TC_DESC_HI));
+}
+
+__device__ __forceinline__ void tc_ld16(uint32_t (&v)[16], uint32_t ta)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+                   "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(ta));
+}
+
+__device__ __forceinline__ void tc_st32(uint32_t ta, const uint32_t (&v)[32])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+                 "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(ta),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+                 "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
+                 "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
+                 "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+                 : "memory");
+}
+
+// a ring of stages: index and phase parity
+struct Ring {
+    int i = 0, par = 0;
+    __device__ __forceinline__ void next(int n)
+    {
+        if (++i == n) {
+            i = 0;
+            par ^= 1;
+        }
+    }
+};
+
+// a row of a tile: its expansion's index box nrhs + rhs (< 0: none) and its direction
+struct TileRow {
+    int row = -1, dir = 0;
+};
+
+__device__ __forceinline__ TileRow tile_row(const TcPass &ps, int4 it, int r, const int *box)
+{
+    TileRow o;
+    if (r < it.z) {
+        const int e = it.y + r, t = e / ps.nrhs;
+        o.row = box[t] * ps.nrhs + (e - t * ps.nrhs);
+        o.dir = ps.g_dir[t];
+    }
+    return o;
+}
+
+// Up to eight coefficient pairs (m = 0..last) of a degree from the columns of their sums (from p on) and
+// differences (from q on, none for m = 0 where `first`) to y[m], y[-m] of the lane's row; columns past the last
+// pair's are not used.
+__device__ __forceinline__ void unfold(uint32_t p, uint32_t q, int last, const float2 (&f)[8], float2 *y, bool first, int fold)
+{
+    uint32_t u[16], w[16];
+    tc_ld16(u, p);
+    tc_ld16(w, q);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        if (j > last) break;
+        const float sr = __uint_as_float(u[2 * j]), si = __uint_as_float(u[2 * j + 1]);
+        if (first && j == 0) {
+            y[0] = make_float2(sr, si);
+            continue;
+        }
+        const float dr = __uint_as_float(w[2 * j]), di = __uint_as_float(w[2 * j + 1]);
+        const float pr = fold ? sr + dr : sr, pi = fold ? si + di : si, mr = fold ? sr - dr : dr, mi = fold ? si - di : di;
+        const int m = first ? j : j + 8;
+        y[m] = make_float2(pr * f[j].x + pi * f[j].y, pi * f[j].x - pr * f[j].y);
+        y[-m] = make_float2(mr * f[j].x - mi * f[j].y, mr * f[j].y + mi * f[j].x);
+    }
+}
+
+__global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_constant__ TcPass ps)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int Nmma = ps.Nmma, K = ps.K, P2 = ps.pin * ps.pin, P2o = ps.P2o, nch = ps.nch, res = ps.res;
-    const uint32_t tA = (uint32_t)TC_M * TC_KC * 4, tB = (uint32_t)Nmma * TC_KC * 4, stage = 2 * tA + (res ? 0 : 2 * tB);
-    unsigned char *bres = smem + TC_STAGES * stage;  // resident operator (res)
-    float *epi = reinterpret_cast<float *>(bres + (res ? (size_t)nch * 2 * tB : 0));
-    uint64_t *bars = reinterpret_cast<uint64_t *>(epi + TC_EWARPS * 32 * TC_EPI_LD);
-    uint64_t *full = bars, *empty = bars + TC_STAGES, *accf = bars + 2 * TC_STAGES, *acce = accf + 2;
-    uint64_t *bfull = acce + 2, *bempty = bfull + 1;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bempty + 1);
-    signed char *s_m = reinterpret_cast<signed char *>(tslot + 4);  // m of coefficient i, 0 beyond p^2
-    for (int i = threadIdx.x; i < TC_MTAB; i += blockDim.x) {
-        int n, m;
-        tc_nm(i, n, m);
-        s_m[i] = i < P2 ? (signed char)m : (signed char)0;
-    }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // tiles of this CTA: strided over the grid, or (res) one contiguous range, so that
-    // consecutive tiles share their class and its resident operator
-    const int q_first = res ? (int)((long long)blockIdx.x * ps.ntiles / gridDim.x) : (int)blockIdx.x;
-    const int q_end = res ? (int)((long long)(blockIdx.x + 1) * ps.ntiles / gridDim.x) : ps.ntiles;
-    const int q_step = res ? 1 : (int)gridDim.x;
+    const TcShape &sh = ps.sh;
+    const int nst = sh.nst, nsub = sh.nsub;
+    unsigned char *rows = smem + (size_t)nst * sh.bstage;
+    unsigned char *epi = rows + (size_t)TC_SLOTS * TC_M * sh.row_stride;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(epi + (size_t)TC_EW * 32 * sh.epi_stride);
+    uint64_t *rfull = bars, *rempty = rfull + TC_SLOTS, *full = rempty + TC_SLOTS, *empty = full + nst, *accf = empty + nst,
+             *acce = accf + 2;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + 2);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 32) {
-        for (int s = 0; s < TC_STAGES; s++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(full + s)), "r"(TC_AWARPS + (res ? 0 : 1)));  // A warps (+ B copy)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(empty + s)));  // MMA commit
+        auto init = [](uint64_t *b, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n)); };
+        for (int i = 0; i < TC_SLOTS; i++) {
+            init(rfull + i, 32 * TC_RW);  // row copies
+            init(rempty + i, TC_AW);   // source warps
         }
-        for (int a = 0; a < 2; a++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(accf + a)));   // MMA commit
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(acce + a)), "r"(TC_EWARPS));  // epilogue warps
+        for (int i = 0; i < nst; i++) {
+            init(full + i, 5);         // source warps of the chunk, one per lane quarter; operator copy
+            init(empty + i, 1);        // MMA commit
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bfull)));   // operator copy (res)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bempty)));  // MMA commit (res)
+        for (int i = 0; i < 2; i++) {
+            init(accf + i, 1);         // MMA commit
+            init(acce + i, TC_EW);     // epilogue warps
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem = *tslot, tmem_a = tmem + (uint32_t)(sh.sets * sh.setw);
+    const int ntile = (ps.ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    // the CTA's i-th tile: its item and range of output degrees; where the grid is a multiple of the
+    // ranges (of uneven width), each round takes the next one, so that every CTA meets them all
+    const int spin = gridDim.x % nsub == 0 ? 1 : 0;
+    auto tile = [&](int i) { return ((int)blockIdx.x + i * (int)gridDim.x) / nsub; };
+    auto range = [&](int i) -> const TcSub & { return sh.sub[((int)blockIdx.x + i * ((int)gridDim.x + spin)) % nsub]; };
+    // its accumulators: set and phase parity
+    const int two = sh.sets == 2;
+    auto set_of = [&](int i) { return two ? i & 1 : 0; };
+    auto set_par = [&](int i) { return two ? (i >> 1) & 1 : i & 1; };
     bool ok = true;
 
     if (warp == 0) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc =
-                (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(Nmma >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
-            const uint32_t lbo = 128, sbo = 32 * TC_KC;
-            int g = 0, i = 0, loads = 0, cur = -1;
-            for (int q = q_first; q < q_end && ok; q += q_step, i++) {
-                const int a = i & 1;
-                ok = mbar_wait(smem_u32(acce + a), ((i >> 1) & 1) ^ 1);
-                if (ok && res && ps.items[q].x != cur) {
-                    // this tile's operator: the copy of the next class run
-                    ok = mbar_wait(smem_u32(bfull), loads & 1);
-                    loads++;
-                    cur = ps.items[q].x;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;");
-                const uint32_t d_tmem = tmem + (uint32_t)(a * 256);
-                for (int c = 0; c < nch && ok; c++, g++) {
-                    const int s = g % TC_STAGES;
-                    ok = mbar_wait(smem_u32(full + s), (g / TC_STAGES) & 1);
-                    if (!ok) break;
+        // An MMA's issue waits until the tensor core can take it, so what lies between two chunks' MMAs is
+        // time lost to it: one thread, and little arithmetic.
+        if (elect_one()) {
+            Ring rs;
+            const int fold = sh.fold;
+            const uint32_t b0 = (smem_u32(smem) >> 4) | TC_DESC_LO, bstep = (uint32_t)sh.bstage >> 4;
+            for (int i = 0; i < ntile && ok; i++) {
+                const TcSub &s = range(i);
+                const int a = set_of(i);
+                const uint32_t kind = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TC_M >> 4) << 24);
+                const uint32_t i1 = kind | (uint32_t)(s.nP >> 3) << 17, i2 = kind | (uint32_t)(s.nQ >> 3) << 17;
+                const uint32_t d1 = tmem + (uint32_t)(a * sh.setw), d2 = d1 + (uint32_t)s.nP;
+                const uint32_t l1 = (uint32_t)(s.nP * TC_KC) >> 2, l2 = (uint32_t)(s.nQ * TC_KC) >> 2;
+                ok = mbar_wait(smem_u32(acce + a), set_par(i) ^ 1);
+                uint32_t add = 0;
+                for (int c = 0; c < sh.nch && ok; c++, add = 1) {
+                    ok = mbar_wait(smem_u32(full + rs.i), rs.par);
                     asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t a_hi = smem_u32(smem + s * stage), a_lo = a_hi + tA;
-                    const uint32_t b_hi = res ? smem_u32(bres) + (uint32_t)c * 2 * tB : a_hi + 2 * tA, b_lo = b_hi + tB;
-#pragma unroll
-                    for (int ks = 0; ks < TC_KC / 8; ks++)
-#pragma unroll
-                        for (int pass = 0; pass < 3; pass++) {
-                            uint64_t ad = smem_desc((pass == 2 ? a_lo : a_hi) + ks * 256, lbo, sbo);
-                            uint64_t bd = smem_desc((pass == 1 ? b_lo : b_hi) + ks * 256, lbo, sbo);
-                            uint32_t acc = (c > 0 || ks > 0 || pass > 0) ? 1u : 0u;
-                            asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
-                                         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, q;\n\t}" ::"r"(d_tmem),
-                                         "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-                        }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     smem_u32(empty + s))
-                                 : "memory");
+                    const uint32_t at = tmem_a + (uint32_t)(rs.i * TC_ACOL), b1 = b0 + (uint32_t)rs.i * bstep, b2 = b1 + 2 * l1;
+                    const uint32_t a2 = at + 2 * TC_KC;
+                    tc_mma(d1, at, b1, i1, add);
+                    tc_mma(d1, at, b1 + l1, i1, 1);
+                    tc_mma(d1, at + TC_KC, b1, i1, 1);
+                    if (fold) {
+                        tc_mma(d2, a2, b2, i2, add);
+                        tc_mma(d2, a2, b2 + l2, i2, 1);
+                        tc_mma(d2, a2 + TC_KC, b2, i2, 1);
+                    } else {
+                        const uint32_t c1 = b2 + 2 * l2, c2 = c1 + 2 * l1;
+                        tc_mma(d2, at, b2, i2, add);
+                        tc_mma(d2, at, b2 + l2, i2, 1);
+                        tc_mma(d2, at + TC_KC, b2, i2, 1);
+                        tc_mma(d1, a2, c1, i1, 1);
+                        tc_mma(d1, a2, c1 + l1, i1, 1);
+                        tc_mma(d1, a2 + TC_KC, c1, i1, 1);
+                        tc_mma(d2, a2, c2, i2, 1);
+                        tc_mma(d2, a2, c2 + l2, i2, 1);
+                        tc_mma(d2, a2 + TC_KC, c2, i2, 1);
+                    }
+                    tc_commit(smem_u32(empty + rs.i));
+                    rs.next(nst);
                 }
-                if (ok)
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     smem_u32(accf + a))
-                                 : "memory");
-                // the last tile of a class run releases the resident operator once its MMAs are done
-                if (ok && res && (q + 1 >= q_end || ps.items[q + 1].x != cur))
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     smem_u32(bempty))
-                                 : "memory");
+                if (ok) tc_commit(smem_u32(accf + a));
             }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- operator copies
-        if (lane == 0 && res) {
-            // one copy of a class's whole operator per class run
-            const uint32_t bytes = (uint32_t)nch * 2 * tB;
-            int loads = 0, cur = -1;
-            for (int q = q_first; q < q_end && ok; q += q_step) {
-                const int4 it = ps.items[q];
-                if (it.x == cur) continue;
-                if (loads > 0) {
-                    ok = mbar_wait(smem_u32(bempty), (loads - 1) & 1);
+        if (lane == 0) {
+            Ring rs;
+            for (int i = 0; i < ntile && ok; i++) {
+                const TcSub &s = range(i);
+                const uint32_t fl = (uint32_t)((sh.fold ? 2 : 4) * TC_KC * (s.nP + s.nQ));
+                const float *B = ps.B + (size_t)ps.items[tile(i)].x * sh.cls_floats + s.boff;
+                for (int c = 0; c < sh.nch; c++, B += fl) {
+                    ok = mbar_wait(smem_u32(empty + rs.i), rs.par ^ 1);
                     if (!ok) break;
-                }
-                const uint32_t bar = smem_u32(bfull), dst = smem_u32(bres);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                             "l"(ps.B + (size_t)it.x * nch * 2 * Nmma * TC_KC), "r"(bytes), "r"(bar)
-                             : "memory");
-                loads++;
-                cur = it.x;
-            }
-        } else if (lane == 0) {
-            const uint32_t bytes = 2 * tB;
-            int g = 0;
-            for (int q = q_first; q < q_end && ok; q += q_step) {
-                const int item = q / ps.nhalf, h = q - item * ps.nhalf;
-                const int4 it = ps.items[item];
-                const float *Bd = ps.B + (size_t)(it.x * ps.nhalf + h) * nch * 2 * Nmma * TC_KC;
-                for (int c = 0; c < nch && ok; c++, g++) {
-                    const int s = g % TC_STAGES;
-                    ok = mbar_wait(smem_u32(empty + s), ((g / TC_STAGES) & 1) ^ 1);
-                    if (!ok) break;
-                    const uint32_t bar = smem_u32(full + s), dst = smem_u32(smem + s * stage + 2 * tA);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                                 "l"(Bd + (size_t)c * 2 * Nmma * TC_KC), "r"(bytes), "r"(bar)
-                                 : "memory");
+                    const uint32_t bar = smem_u32(full + rs.i);
+                    tc_expect(bar, 4 * fl);
+                    tc_bulk(smem_u32(smem + (size_t)rs.i * sh.bstage), B, 4 * fl, bar);
+                    rs.next(nst);
                 }
             }
         }
-    } else if (warp < TC_EPI0) {
-        // ---------------------------------------------------------------- source gather
-        // two threads per row (translation), each 8 of every 16-wide K chunk; the loads of the
-        // next two chunks are in flight while a chunk waits for its stage and is stored
-        constexpr int KH = TC_KC / 2;
-        static_assert(KH == 8, "four complex coefficients per thread and chunk half");
-        const int at = tid - 64, r = at & (TC_M - 1), kh = (at >> 7) * KH;
-        const float *srcf = reinterpret_cast<const float *>(ps.src);
-        const bool vec4 = (K & 3) == 0;
-        // The CTA's tiles as one stream of chunks u = (tile, chunk); the loads run two chunks
-        // ahead of the stores, also across tile boundaries.  The row of the tile after the one
-        // being loaded is looked up in two steps while the loads cross the current tile: its
-        // work item when they enter it, its translation's source box and direction half way
-        // through, so that neither lookup stalls the stream.
-        const int ntile = q_first < q_end ? (q_end - q_first + q_step - 1) / q_step : 0;
-        const int U = ntile * nch, cmid = nch / 2;
-        struct RowSrc {
-            const float *row;
-            const float2 *ph;
-            bool v;
-        };
-        auto tile_item = [&](int i) -> int4 {
-            return i < ntile ? ps.items[(q_first + i * q_step) / ps.nhalf] : make_int4(0, 0, 0, 0);
-        };
-        // row r of a tile from its translation's raw source box / direction (box < 0: empty row)
-        auto row_src = [&](int box, int rr, int dir) -> RowSrc {
-            RowSrc o{srcf, ps.PH + ps.phoff, false};
-            if (box < 0) return o;
-            o.row = srcf + (size_t)(box * ps.nrhs + rr) * K;
-            o.ph = ps.PH + (size_t)dir * ps.phstride + ps.phoff;
-            o.v = true;
-            return o;
-        };
-        int lt = 0, lc = 0;          // tile and chunk of the next load
-        int nbox = -1, nrr = 0, ndir = 0;
-        auto lookup = [&](int4 it) {  // the translation of row r of item it
-            nbox = -1;
-            if (r < it.z) {
-                const int e = it.y + r, t = e / ps.nrhs;
-                nrr = e - t * ps.nrhs;
-                nbox = ps.g_src[t];
-                ndir = ps.g_dir[t];
-            }
-        };
-        lookup(tile_item(0));
-        RowSrc cur = row_src(nbox, nrr, ndir);
-        int4 itn = tile_item(1);
-        // the row's source coefficients of chunk u and their phases e^{i m phi}: KH / 2 = 4
-        // complex coefficients from i0 = k0 / 2 on (i0 a multiple of 4, so their four orders
-        // are one 32-bit word of the m table)
-        auto load = [&](float(&x)[KH], float2(&f)[KH / 2]) {
-            if (lc == nch) {
-                lc = 0;
-                lt++;
-                cur = row_src(nbox, nrr, ndir);
-                itn = tile_item(lt + 1);
-            }
-            if (lc == cmid) lookup(itn);
-            const int k0 = lc * TC_KC + kh;
-            lc++;
-            {
-                const uint32_t mm = *reinterpret_cast<const uint32_t *>(s_m + (k0 >> 1));
+    } else if (warp < TC_A0) {
+        // ---------------------------------------------------------------- source rows
+        // A warp's rows one after another, a lane per 16 bytes (a bulk copy per row, issued by each row's
+        // lane, took 80 cycles a row).  A row that starts on an odd coefficient is copied from
+        // the one before on, one of odd length to the one after (the expansions are allocated
+        // with one coefficient to spare).
+        constexpr int NR = TC_M / TC_RW / 32;  // rows per lane
+        const int r0 = (warp - 2) * 32 * NR;
+        Ring rr;
+        for (int i = 0; i < ntile && ok; i++) {
+            const int4 it = ps.items[tile(i)];
+            long long at[NR];
 #pragma unroll
-                for (int j = 0; j < KH / 2; j++) f[j] = __ldg(cur.ph + (int)(signed char)(mm >> (8 * j)));
-            }
+            for (int j = 0; j < NR; j++) at[j] = (long long)tile_row(ps, it, r0 + lane + 32 * j, ps.g_src).row * ps.P2;
+            for (int pc = 0; pc < sh.npiece; pc++) {
+                const int c0 = sh.piece[pc].c0, cnt = sh.piece[pc].cnt;
+                ok = mbar_wait_warp(smem_u32(rempty + rr.i), rr.par ^ 1);
+                if (!ok) break;
+                uint32_t slot = smem_u32(rows + (size_t)(rr.i * TC_M + r0) * sh.row_stride) + 16 * lane;
+                const char *src = reinterpret_cast<const char *>(ps.src) + 16 * lane;
 #pragma unroll
-            for (int j = 0; j < KH; j += 4) {
-                const int k = k0 + j;
-                if (cur.v && vec4 && k + 3 < K) {
-                    float4 v = __ldg(reinterpret_cast<const float4 *>(cur.row + k));
-                    x[j] = v.x; x[j + 1] = v.y; x[j + 2] = v.z; x[j + 3] = v.w;
-                } else {
-                    float2 v0 = make_float2(0.f, 0.f), v1 = make_float2(0.f, 0.f);
-                    if (cur.v && k + 1 < K) v0 = __ldg(reinterpret_cast<const float2 *>(cur.row + k));
-                    if (cur.v && k + 3 < K) v1 = __ldg(reinterpret_cast<const float2 *>(cur.row + k + 2));
-                    x[j] = v0.x; x[j + 1] = v0.y; x[j + 2] = v1.x; x[j + 3] = v1.y;
+                for (int j = 0; j < NR; j++) {
+                    // the lane's own row: its first 16 bytes, counted in 16 bytes, and their number
+                    const int odd = (int)((at[j] + c0) & 1);
+                    const uint32_t first = (uint32_t)((at[j] + c0) >> 1);
+                    const int num = at[j] >= 0 ? (cnt + odd + 1) >> 1 : 0;
+                    for (int k0 = 0; k0 < 32; k0 += 8) {
+                        uint32_t from[8];
+                        int n[8];
+#pragma unroll
+                        for (int k = 0; k < 8; k++) {
+                            from[k] = __shfl_sync(0xffffffffu, first, k0 + k);
+                            n[k] = __shfl_sync(0xffffffffu, num, k0 + k);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 8; k++, slot += sh.row_stride)
+                            asm volatile("{\n\t.reg .pred q;\n\tsetp.lt.s32 q, %2, %3;\n\t@q cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(slot),
+                                         "l"(src + 16ull * from[k]), "r"(lane), "r"(n[k]));
+                    }
                 }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(rfull + rr.i)) : "memory");
+                rr.next(TC_SLOTS);
             }
-        };
-        auto store = [&](float(&x)[KH], const float2(&f)[KH / 2], int u) -> bool {
-            const int s = u % TC_STAGES;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp < TC_E0) {
+        // ---------------------------------------------------------------- A operand
+        const int quarter = warp & 3, grp = (warp - TC_A0) >> 2, r = 32 * quarter + lane, fold = sh.fold;
+        const uint32_t ta0 = tmem_a + ((uint32_t)(quarter * 32) << 16);
+        Ring rr, rs;
+        int turn = 0;
+        TileRow next;
+        if (ntile > 0) next = tile_row(ps, ps.items[tile(0)], r, ps.g_src);
+        for (int i = 0; i < ntile && ok; i++) {
+            const TileRow cur = next;
+            // the next tile's row: its item now, its box and direction after the first piece, so
+            // that neither lookup stalls the chunks
+            const int4 itn = i + 1 < ntile ? ps.items[tile(i + 1)] : make_int4(0, 0, 0, 0);
+            const unsigned char *ph = reinterpret_cast<const unsigned char *>(ps.PH + (size_t)cur.dir * ps.phstride + ps.phoff);
+            const int base = cur.row >= 0 ? (int)(((long long)cur.row * ps.P2) & 1) : 0;
+            for (int pc = 0; pc < sh.npiece && ok; pc++) {
+                const int c0 = sh.piece[pc].c0, ce = sh.piece[pc].end;
+                ok = mbar_wait_warp(smem_u32(rfull + rr.i), rr.par);
+                if (!ok) break;
+                const unsigned char *x = rows + (size_t)(rr.i * TC_M + r) * sh.row_stride + 8 * ((base + c0) & 1);
+                // the coefficients and phases of a chunk are read before the one before it is stored
+                float2 f[4], xp[4], xm[4];
+                auto load = [&](int c) {
 #pragma unroll
-            for (int j = 0; j < KH / 2; j++) {
-                const float xr = x[2 * j], xi = x[2 * j + 1];
-                x[2 * j] = xr * f[j].x - xi * f[j].y;
-                x[2 * j + 1] = xr * f[j].y + xi * f[j].x;
-            }
-            if (!mbar_wait(smem_u32(empty + s), ((u / TC_STAGES) & 1) ^ 1)) return false;
-            unsigned char *Ahi = smem + s * stage, *Alo = Ahi + tA;
+                    for (int j = 0; j < 4; j++) {
+                        const TcIn &w = sh.tab[4 * c + j];
+                        f[j] = __ldg(reinterpret_cast<const float2 *>(ph + (w.m & 0xff)));
+                        xp[j] = *reinterpret_cast<const float2 *>(x + w.pos);
+                        xm[j] = *reinterpret_cast<const float2 *>(x + w.neg);
+                    }
+                };
+                int c = sh.piece[pc].beg + (turn ^ grp);
+                if (c < ce) load(c);
+                if (turn != grp) rs.next(nst);
+                for (; c < ce; c += 2) {
+                    uint32_t v[32];
 #pragma unroll
-            for (int j = 0; j < KH; j += 4) {
-                float4 hi, lo;
-                hi.x = tf32_round(x[j]); lo.x = tf32_round(x[j] - hi.x);
-                hi.y = tf32_round(x[j + 1]); lo.y = tf32_round(x[j + 1] - hi.y);
-                hi.z = tf32_round(x[j + 2]); lo.z = tf32_round(x[j + 2] - hi.z);
-                hi.w = tf32_round(x[j + 3]); lo.w = tf32_round(x[j + 3] - hi.w);
-                const uint32_t o = core_off(r, kh + j, TC_KC);
-                *reinterpret_cast<float4 *>(Ahi + o) = hi;
-                *reinterpret_cast<float4 *>(Alo + o) = lo;
+                    for (int j = 0; j < 4; j++) {
+                        float s[4];
+                        if (fold) {  // x_m e + x_-m e*, x_m e - x_-m e*
+                            const float sr = xp[j].x + xm[j].x, si = xp[j].y + xm[j].y, dr = xp[j].x - xm[j].x, di = xp[j].y - xm[j].y;
+                            s[0] = sr * f[j].x - di * f[j].y, s[1] = si * f[j].x + dr * f[j].y;
+                            s[2] = dr * f[j].x - si * f[j].y, s[3] = di * f[j].x + sr * f[j].y;
+                        } else {  // x_m e, x_-m e*
+                            s[0] = xp[j].x * f[j].x - xp[j].y * f[j].y, s[1] = xp[j].x * f[j].y + xp[j].y * f[j].x;
+                            s[2] = xm[j].x * f[j].x + xm[j].y * f[j].y, s[3] = xm[j].y * f[j].x - xm[j].x * f[j].y;
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; k += 2) {
+                            const float h0 = tf32_round(s[k]), h1 = tf32_round(s[k + 1]);
+                            const float2 lo = f2_parts(f2_sub(f2_pack(s[k], s[k + 1]), f2_pack(h0, h1)));
+                            const int o = k * TC_KC + 2 * j;
+                            v[o] = __float_as_uint(h0);
+                            v[o + 1] = __float_as_uint(h1);
+                            v[o + TC_KC] = __float_as_uint(tf32_round(lo.x));
+                            v[o + TC_KC + 1] = __float_as_uint(tf32_round(lo.y));
+                        }
+                    }
+                    if (c + 2 < ce) load(c + 2);
+                    ok = mbar_wait_warp(smem_u32(empty + rs.i), rs.par ^ 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;");
+                    tc_st32(ta0 + (uint32_t)(rs.i * TC_ACOL), v);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(full + rs.i));
+                    rs.next(nst);
+                    if (c + 1 < ce) rs.next(nst);
+                }
+                turn ^= (ce - sh.piece[pc].beg) & 1;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(rempty + rr.i));
+                rr.next(TC_SLOTS);
+                if (pc == 0) next = tile_row(ps, itn, r, ps.g_src);
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(full + s));
-            return true;
-        };
-        float xa[KH], xb[KH], xc[KH];
-        float2 fa[KH / 2], fb[KH / 2], fc[KH / 2];
-        if (U > 0) load(xa, fa);
-        if (U > 1) load(xb, fb);
-        for (int u = 0; u < U && ok; u += 3) {
-            if (u + 2 < U) load(xc, fc);
-            ok = store(xa, fa, u);
-            if (!ok || u + 1 >= U) break;
-            if (u + 3 < U) load(xa, fa);
-            ok = store(xb, fb, u + 1);
-            if (!ok || u + 2 >= U) break;
-            if (u + 4 < U) load(xb, fb);
-            ok = store(xc, fc, u + 2);
         }
     } else {
         // ---------------------------------------------------------------- epilogue
-        // warp w reads TMEM lane quarter w % 4; the two warps of a quarter take alternate
-        // 32-column blocks
-        const int wq = warp & 3, eh = (warp - TC_EPI0) >> 2;
-        float *st = epi + (warp - TC_EPI0) * 32 * TC_EPI_LD;
-        // destinations of coefficient pairs 16-byte aligned: p^2 and the half width even
-        const bool pairs = (P2o % 2 == 0) && (ps.CH % 2 == 0);
-        int i = 0;
-        for (int q = q_first; q < q_end && ok; q += q_step, i++) {
-            const int a = i & 1, item = q / ps.nhalf, h = q - item * ps.nhalf;
-            const int4 it = ps.items[item];
-            const int row = wq * 32 + lane;
-            const int dbox = tile_box(ps, it, row, false);
-            const int drow = row < it.z ? ps.g_dir[(it.y + row) / ps.nrhs] : 0;
-            // rows of one class run hold each direction's translations contiguously, so a tile
-            // whose first and last rows share a direction has one direction (one set of phases);
-            // passes without phases read a table of ones (phstride 0)
-            const int d0 = ps.g_dir[it.y / ps.nrhs];
-            const bool uni = !ps.phased || d0 == ps.g_dir[(it.y + it.z - 1) / ps.nrhs];
-            const float2 *ph0 = ps.PH + (size_t)d0 * ps.phstride + ps.phoff;
-            const int co0 = h * ps.CH, nco = min(ps.CH, P2o - co0);
-            ok = mbar_wait(smem_u32(accf + a), (i >> 1) & 1);
+        const int quarter = warp & 3, eh = (warp - TC_E0) >> 2;
+        const int es = sh.epi_stride;
+        float2 *st = reinterpret_cast<float2 *>(epi + ((warp - TC_E0) * 32 + lane) * es);
+        const uint32_t st0 = smem_u32(epi + (warp - TC_E0) * 32 * es);
+        for (int i = 0; i < ntile && ok; i++) {
+            const int a = set_of(i);
+            const TcSub &s = range(i);
+            const TileRow tr = tile_row(ps, ps.items[tile(i)], quarter * 32 + lane, ps.g_dst);
+            // the row's phases, m = 0..7 and 8..15 (the tables hold 2 pmax - 1 >= 2 p - 1 of a direction)
+            const float2 *ph = ps.PH + (size_t)tr.dir * ps.phstride + ps.phoff;
+            float2 f0[8], f1[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                f0[j] = j < s.end ? __ldg(ph + j) : make_float2(0.f, 0.f);
+                f1[j] = j + 8 < s.end ? __ldg(ph + j + 8) : make_float2(0.f, 0.f);
+            }
+            const uint32_t tp = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(a * sh.setw), tq = tp + (uint32_t)s.nP;
+            const int p0 = s.beg * (s.beg + 1) / 2, q0 = s.beg * (s.beg - 1) / 2;
+            ok = mbar_wait_warp(smem_u32(accf + a), set_par(i));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
-            for (int cb = 32 * eh; cb < Nmma; cb += 64) {
-                uint32_t v[32];
-                const uint32_t ta = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(a * 256 + cb);
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                             "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                               "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                               "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-                               "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                               "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                             : "r"(ta));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int j = 0; j < 32; j++) st[lane * TC_EPI_LD + j] = __uint_as_float(v[j]);
+            unsigned left = (eh ? s.second : ~s.second) & ((1u << s.ngrp) - 1);
+            while (left) {
+                const int g = __ffs(left) - 1, na = s.grp[g], nb = s.grp[g + 1], c0 = na * na, cnt = nb * nb - c0;
+                const long long e0 = (long long)tr.row * ps.P2o + c0;
+                const int odd = (int)(e0 & 1);
+                left &= left - 1;
+                // the warp's last group is out of its staging
+                if (elect_one()) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 __syncwarp();
-                if (pairs) {
-                    // four rows per step, 8 pairs of coefficients per row, each pair added with one
-                    // 16-byte atomic; coefficient co of row rr times e^{-i m' phi} of its direction
-                    const int jq = lane & 7, co = co0 + cb / 2 + 2 * jq;
-                    const bool cv = cb + 4 * jq < 2 * nco;
-                    const int m0 = s_m[cv ? co : 0], m1 = s_m[cv ? co + 1 : 0];
-                    const float2 u0 = __ldg(ph0 + m0), u1 = __ldg(ph0 + m1);
-#pragma unroll 4
-                    for (int rq = 0; rq < 8; rq++) {
-                        const int rr = 4 * rq + (lane >> 3);
-                        const int d = __shfl_sync(0xffffffffu, dbox, rr);
-                        const int dr = __shfl_sync(0xffffffffu, drow, rr);
-                        if (d >= 0 && cv) {
-                            const float2 *pr = ps.PH + (size_t)dr * ps.phstride + ps.phoff;
-                            const float2 e0 = uni ? u0 : __ldg(pr + m0), e1 = uni ? u1 : __ldg(pr + m1);
-                            const float *y = st + rr * TC_EPI_LD + 4 * jq;
-                            const float4 w = make_float4(y[0] * e0.x + y[1] * e0.y, y[1] * e0.x - y[0] * e0.y,
-                                                         y[2] * e1.x + y[3] * e1.y, y[3] * e1.x - y[2] * e1.y);
-                            atomicAdd(reinterpret_cast<float4 *>(ps.dst + (size_t)d * P2o + co), w);
+                for (int n = na; n < nb; n++) {
+                    float2 *y = st + odd + (n * n + n - c0);
+                    const uint32_t pn = tp + (uint32_t)(2 * (n * (n + 1) / 2 - p0)), qn = tq + (uint32_t)(2 * (n * (n - 1) / 2 - q0)) - 2;
+                    unfold(pn, qn, n, f0, y, true, sh.fold);
+                    if (n >= 8) unfold(pn + 16, qn + 16, n - 8, f1, y, false, sh.fold);
+                }
+                if (!left) {  // the warp's last columns are read
+                    asm volatile("tcgen05.fence::before_thread_sync;");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(acce + a));
+                }
+                // a row's group is added by a bulk reduction of what lies on 16 bytes, single coefficients at
+                // the ends by its lane
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                float2 *o = ps.dst + e0;
+                const int whole = (cnt - odd) & ~1;
+                const uint32_t size = tr.row >= 0 ? 8u * (uint32_t)whole : 0u;
+                const unsigned alike = __match_any_sync(0xffffffffu, size << 1 | (uint32_t)odd);
+                if (alike == 0xffffffffu && size) {
+                    const uint32_t from = st0 + 16 * odd;
+                    for (int k0 = 0; k0 < 32; k0 += 8) {
+                        int row[8];
+#pragma unroll
+                        for (int k = 0; k < 8; k++) row[k] = __shfl_sync(0xffffffffu, tr.row, k0 + k);
+                        if (elect_one()) {
+#pragma unroll
+                            for (int k = 0; k < 8; k++)
+                                tc_reduce(ps.dst + (long long)row[k] * ps.P2o + (c0 + odd), from + (uint32_t)((k0 + k) * es), size);
                         }
                     }
                 } else {
-                    // two rows per step, 16 coefficients (32 columns) per row
-                    const int jc = lane & 15, c2 = cb + 2 * jc, co = co0 + c2 / 2;
-                    const bool cv = c2 < 2 * nco;
-                    const int mo = s_m[cv ? co : 0];
-                    const float2 fu = __ldg(ph0 + mo);
-#pragma unroll 4
-                    for (int rp = 0; rp < 16; rp++) {
-                        const int rr = 2 * rp + (lane >> 4);
-                        const int d = __shfl_sync(0xffffffffu, dbox, rr);
-                        const int dr = __shfl_sync(0xffffffffu, drow, rr);
-                        if (d >= 0 && cv) {
-                            const float2 e = uni ? fu : __ldg(ps.PH + (size_t)dr * ps.phstride + ps.phoff + mo);
-                            const float yr = st[rr * TC_EPI_LD + 2 * jc], yi = st[rr * TC_EPI_LD + 2 * jc + 1];
-                            atomicAdd(ps.dst + (size_t)d * P2o + co, make_float2(yr * e.x + yi * e.y, yi * e.x - yr * e.y));
-                        }
+                    for (int k = 0; k < 32; k++) {
+                        const unsigned long long to = __shfl_sync(0xffffffffu, (unsigned long long)(o + odd), k);
+                        const uint32_t sk = __shfl_sync(0xffffffffu, size, k), ok_ = __shfl_sync(0xffffffffu, odd, k);
+                        if (sk && elect_one()) tc_reduce(reinterpret_cast<float2 *>(to), st0 + (uint32_t)(k * es) + 16 * ok_, sk);
                     }
                 }
-                __syncwarp();
+                if (elect_one()) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                if (tr.row >= 0) {
+                    if (odd) atomicAdd(o, st[1]);
+                    if (odd + whole < cnt) atomicAdd(o + cnt - 1, st[odd + cnt - 1]);
+                }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(acce + a));
+            if (((eh ? s.second : ~s.second) & ((1u << s.ngrp) - 1)) == 0) {  // no group of this range is the warp's
+                asm volatile("tcgen05.fence::before_thread_sync;");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(acce + a));
+            }
         }
+        if (elect_one()) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     if (!ok) atomicExch(ps.err, 1);
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -469,38 +628,51 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(TcPass ps)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
-// The real-embedded operators of a pass, split into TF32 hi/lo, in the tile layout: element
-// (o, k) of half h, chunk c holds  Re T (o, k even-even / odd-odd), -Im T (o even, k odd) or
-// Im T (o odd, k even) of coefficient (h CH + o/2, (c KC + k)/2).
+// The blocks of a class's operator T, embedded as real matrices and split into TF32 hi / lo, in
+// the order of the copies: class, output range, chunk, (sums hi, lo, differences hi, lo; without the
+// fold outputs m hi, lo, outputs -m hi, lo of the inputs m, then of the inputs -m) in the core-matrix layout.  With P = x_m + x_-m, Q = x_m - x_-m of the inputs and y_+-m = S +- D of the
+// outputs:  S = sum (T_m'm + T_m'-m) / 2 P (half of that for m = 0, where P = 2 x_0),
+// D = sum (T_m'm - T_m'-m) / 2 Q.
 // fout / fin (plans with scaled FP32 expansions, else null): per-degree factors of the
 // destination and source coefficients, so that the operator maps the scaled expansions
 // (multipoles d_n M_n, locals L_n / d_n of their own levels).
-__global__ void tc_split_kernel(const double2 *__restrict__ T, int pin, int pout, int KC, int nch, int nhalf, int CH,
-                                int Nmma, const double *__restrict__ fout, const double *__restrict__ fin,
-                                float *__restrict__ B, size_t total)
+// Grid: (chunks, classes * output ranges).
+__global__ void tc_split_kernel(const double2 *__restrict__ T, int pin, int pout, const __grid_constant__ TcShape sh,
+                                const double *__restrict__ fout, const double *__restrict__ fin, float *__restrict__ B)
 {
-    const int P2i = pin * pin, P2o = pout * pout, K = 2 * P2i;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
-        size_t z = q;
-        int kcol = (int)(z % KC); z /= KC;
-        int nr = (int)(z % Nmma); z /= Nmma;
-        int part = (int)(z % 2); z /= 2;
-        int c = (int)(z % nch); z /= nch;
-        int h = (int)(z % nhalf);
-        int d = (int)(z / nhalf);
-        int k = c * KC + kcol, nco = min(CH, P2o - h * CH);
+    const int c = blockIdx.x, cls = blockIdx.y / sh.nsub, P2i = pin * pin, P2o = pout * pout;
+    const TcSub &s = sh.sub[blockIdx.y % sh.nsub];
+    int c0 = 0;
+    for (int i = 0; i < sh.npiece; i++)
+        if (c >= sh.piece[i].beg && c < sh.piece[i].end) c0 = sh.piece[i].c0;
+    const int parts = sh.fold ? 1 : 2, wide = s.nP + s.nQ;
+    float *out = B + (size_t)cls * sh.cls_floats + s.boff + (size_t)c * parts * 2 * TC_KC * wide;
+    for (int q = threadIdx.x; q < parts * wide * TC_KC; q += blockDim.x) {
+        const int k = q % TC_KC, part = q / TC_KC / wide, row = q / TC_KC - part * wide, second = row >= s.nP;
+        const int o = row - (second ? s.nP : 0);
+        const TcIn w = sh.tab[4 * c + k / 2];
+        // output o / 2 of the block: (n, m >= second), degree by degree
+        int n = s.beg, j = o / 2;
+        while (n < s.end && j > n - second) j -= n + 1 - second, n++;
         double v = 0.0;
-        if (nr < 2 * nco && k < K) {
-            const int io = h * CH + nr / 2, ii = k / 2;
-            double2 t = T[((size_t)d * P2o + io) * P2i + ii];
-            int po = nr & 1, pi = k & 1;
-            v = po == 0 ? (pi == 0 ? t.x : -t.y) : (pi == 0 ? t.y : t.x);
-            if (fout) v *= fout[(int)sqrtf((float)io + 0.5f)] * fin[(int)sqrtf((float)ii + 0.5f)];
+        if (n < s.end && w.m != TC_PAD) {
+            const int m = j + second, ip = c0 + w.pos / 8, im = c0 + w.neg / 8;
+            const double2 *row_m = T + ((size_t)cls * P2o + n * n + n + m) * P2i, *row_n = T + ((size_t)cls * P2o + n * n + n - m) * P2i;
+            double2 t;
+            if (sh.fold) {
+                const double h = ip == im ? 0.25 : 0.5;
+                t = second ? make_double2(h * (row_m[ip].x - row_m[im].x), h * (row_m[ip].y - row_m[im].y))
+                           : make_double2(h * (row_m[ip].x + row_m[im].x), h * (row_m[ip].y + row_m[im].y));
+            } else {
+                t = part && ip == im ? make_double2(0.0, 0.0) : (second ? row_n : row_m)[part ? im : ip];
+            }
+            v = (o & 1) == 0 ? ((k & 1) == 0 ? t.x : -t.y) : ((k & 1) == 0 ? t.y : t.x);
+            if (fout) v *= fout[n] * fin[(int)sqrtf((float)ip + 0.5f)];
         }
-        float hi = tf32_round((float)v);
-        float lo = tf32_round((float)(v - (double)hi));
-        size_t base = ((((size_t)d * nhalf + h) * nch + c) * 2 + part) * (size_t)Nmma * KC;
-        B[base + core_off(nr, kcol, KC) / 4] = part ? lo : hi;
+        const float hi = tf32_round((float)v), lo = tf32_round((float)(v - (double)hi));
+        float *blk = out + part * 2 * TC_KC * wide + (second ? 2 * TC_KC * s.nP : 0);
+        blk[core_off(o, k, TC_KC) / 4] = hi;
+        blk[(second ? s.nQ : s.nP) * TC_KC + core_off(o, k, TC_KC) / 4] = lo;
     }
 }
 
@@ -520,28 +692,31 @@ static RcrList *dense_list(Plan *P, int l, int which, int &pin, int &pout)
     return which == PASS_M2M ? &L.m2m : &L.l2l;
 }
 
+// Levels that run on sums and differences (T translations).  The fold halves the products and their rounding
+// errors; at 100,000 translations and more it takes 0.45 against 0.51 ms (p = 14, 192,528 translations, one
+// column) and less with more columns (17.5 against 19.5 ms for 16).  On smaller levels the
+// gain is 10 to 20 us a pass (p = 12, 29,590 translations: 57 against 78 us with the level before it), and refined
+// solves, which run on bodies of that size, would stop at other steps: their stopping test sees the
+// operator's error, and solutions would move by more than they differ from run to run (adjoint of a 5,120-triangle body
+// at tol = 1e-8: 4e-9 against 1e-9).
+static bool fold_pays(int T) { return T >= 100000; }
+
 static int build_tc_dense(Plan *P, int l, int which)
 {
     int pin = 0, pout = 0;
     RcrList *Lst = dense_list(P, l, which, pin, pout);
     if (!Lst || Lst->key_beg.empty() || Lst->key_beg.back() == 0) return FMM_OK;
     TcDense &g = Lst->td;
-    if (!tc_geometry(pin, pout, g)) return FMM_OK;
+    const char *env = getenv("FMMBEM_TENSOR_FOLD");
+    const int fold = env ? atoi(env) != 0 : fold_pays(Lst->key_beg.back());
+    if (!tc_shape(pin, pout, fold, g.sh)) return FMM_OK;
     g.pin = pin;
     g.pout = pout;
     const int nkeys = (int)Lst->key_beg.size() - 1, P2i = pin * pin, P2o = pout * pout;
     std::vector<int> rep;
-    if (which == PASS_M2L) {
-        g.phased = 1;
-        direction_classes(P, PASS_M2L, nkeys, g.cls_of_dir, rep);
-    } else {
-        g.phased = 0;  // eight octant operators, phases included
-        g.cls_of_dir.resize(nkeys);
-        for (int d = 0; d < nkeys; d++) g.cls_of_dir[d] = d;
-        rep = g.cls_of_dir;
-    }
+    direction_classes(P, which, nkeys, g.cls_of_dir, rep);
     g.ncls = (int)rep.size();
-    size_t total = (size_t)g.ncls * g.nhalf * g.nch * 2 * g.Nmma * g.KC;
+    const size_t total = (size_t)g.ncls * g.sh.cls_floats;
     double2 *T = nullptr;
     int *rep_dev = nullptr;
     double *fdev = nullptr;
@@ -582,7 +757,7 @@ static int build_tc_dense(Plan *P, int l, int which)
     e = dev_alloc(P, (void **)&g.B, sizeof(float) * total);
     if (e != cudaSuccess) return fail(e);
     g.B_bytes = sizeof(float) * total;
-    tc_split_kernel<<<152 * 16, 256, 0, P->stream>>>(T, pin, pout, g.KC, g.nch, g.nhalf, g.CH, g.Nmma, fo, fi, g.B, total);
+    tc_split_kernel<<<dim3(g.sh.nch, g.ncls * g.sh.nsub), 256, 0, P->stream>>>(T, pin, pout, g.sh, fo, fi, g.B);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
     cudaFree(T);
@@ -689,37 +864,24 @@ int launch_tc_dense(Plan *P, int l, int which, int nrhs, cudaStream_t st)
     const size_t ws = ((size_t)rp.nsrc * pin * pin + (size_t)rp.ndst * pout * pout) * sizeof(float2) * nrhs;
     int e = ensure_td_items(*Lst, ws, nrhs, st);
     if (e) return e;
-    if (!P->tc_ones) {
-        std::vector<float2> ones(2 * TC_MAXP + 1, make_float2(1.f, 0.f));
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&P->tc_ones, sizeof(float2) * ones.size()));
-        FMM_CUDA_TRY(cudaMemcpy(P->tc_ones, ones.data(), sizeof(float2) * ones.size(), cudaMemcpyHostToDevice));
-    }
     TcPass ps;
+    ps.sh = g.sh;
     ps.items = g.items;
     ps.g_src = g.src;
     ps.g_dst = g.dst;
     ps.g_dir = g.dir;
-    ps.phased = g.phased;
-    ps.PH = g.phased ? P->PHsr32 : P->tc_ones;
-    ps.phstride = g.phased ? 2 * P->pmax - 1 : 0;
-    ps.phoff = g.phased ? P->pmax - 1 : TC_MAXP;
+    ps.PH = rp.PH;
+    ps.phstride = rp.phstride;
+    ps.phoff = rp.phoff;
     ps.nrhs = nrhs;
-    ps.nsrc = rp.nsrc;
-    ps.ndst = rp.ndst;
-    ps.pin = pin;
+    ps.P2 = pin * pin;
     ps.P2o = pout * pout;
-    ps.K = 2 * pin * pin;
-    ps.nch = g.nch;
-    ps.nhalf = g.nhalf;
-    ps.CH = g.CH;
-    ps.Nmma = g.Nmma;
-    ps.ntiles = g.n_items * g.nhalf;
-    ps.res = g.res;
+    ps.ntiles = g.n_items * g.sh.nsub;
     ps.B = g.B;
     ps.src = rp.src;
     ps.dst = rp.dst;
     ps.err = P->tc_err;
-    size_t sm = tc_smem_bytes(g.Nmma, g.res, g.nch);
+    const size_t sm = tc_smem_bytes(g.sh);
     static size_t attr = 0;
     e = raise_smem_limit((const void *)tc_dense_kernel, sm, &attr);
     if (e) return e;
@@ -784,8 +946,8 @@ int check_tc_error(Plan *P)
 }
 
 // M2L levels that run dense (order p <= 16, T translations).  Large levels: the dense form is the
-// faster one (16 columns on the 81,920-triangle sphere: p = 10, 650,304 translations 5.1 ms against
-// 9.3 on the SIMT tiles; p = 14, 192,528 translations 4.8 against 6.0).  Small ones are even (6 to 8
+// faster one (16 columns on the 81,920-triangle sphere: p = 10, 650,304 translations 3.2 ms against
+// 9.3 on the SIMT tiles; p = 14, 192,528 translations 2.8 against 6.0).  Small ones are even (6 to 8
 // thousand translations: 10 to 60 us either way); a plan keeps the form there that its timing used to
 // choose, so that its rounding (TF32 halves against FP32) stays the same: dense from 2,000
 // translations on at p = 6..14 and from 10,000 on at p = 15, 16 (tiles of 128 columns of one of 61
@@ -795,7 +957,7 @@ static bool dense_pays(int p, int T) { return p < 6 ? T >= 20000 : p <= 14 ? T >
 // Builds the dense split operators of the passes that run on the tensor cores: the M2L levels of
 // order <= 16 that dense_pays() names.  FMMBEM_TENSOR_M2L (M2L) and FMMBEM_TENSOR_M2M (M2M and
 // L2L, where both orders are <= 16) = 0 keep the SIMT tiles, = 1 take the tensor cores wherever
-// they apply.  M2M and L2L stay on the SIMT tiles unless FMMBEM_TENSOR_M2M is set: their dense
+// they apply; FMMBEM_TENSOR_FOLD = 0 or 1 overrides fold_pays().  M2M and L2L stay on the SIMT tiles unless FMMBEM_TENSOR_M2M is set: their dense
 // form is about ten times less accurate on the 81,920-triangle sphere (mixed against FP64
 // 8.9e-7 against 7.7e-8), which costs the refined solves more iterations than it saves.
 int tune_tc_dense(Plan *P)
