@@ -290,6 +290,7 @@ int gen_element_tables(Plan *P);
 int gen_near_field(Plan *P);
 int gen_operator_part(Plan *P, double2 bco, double2 cco, double2 *U, double2 *Rv_tmp, double2 *nearv);
 int launch_far_field(Plan *P, const double2 *p, const double *pts, int npts, double2 *out);
+int far_slices(int nf, int npts);
 int launch_plane_wave(Plan *P, const double *dir, double2 *rhs);
 int gen_rotation_matrices_f32(const double *alpha, const double *beta, const double *gamma, int n, int p, float2 *host_out);
 int gen_coax_matrices_f32(double k, const double *t, int n, int p, int sr, float2 *host_out);
