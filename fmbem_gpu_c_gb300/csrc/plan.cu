@@ -98,7 +98,8 @@ static void free_plan(Plan *P)
         }
     }
     F(P->rot32); F(P->pairs);
-    F(P->tc_err); F(P->PHall_ff); F(P->dsc_leaf_dev);
+    cudaFreeHost(P->tc_err_host);
+    F(P->PHall_ff); F(P->dsc_leaf_dev);
     F(P->Hsr64); F(P->PHsr64); F(P->Hsr32); F(P->PHsr32);
     F(P->V_dev); F(P->F_dev); F(P->elem_leaf); F(P->leaf_beg); F(P->leaf_elem);
     F(P->U64); F(P->Rv64); F(P->U32); F(P->Rv32); F(P->near_beg); F(P->near_col); F(P->near64); F(P->near32);

@@ -238,7 +238,7 @@ struct Plan {
     int nside = 2;                // side streams in use (FMMBEM_M2L_STREAMS, 1..NSIDE)
     cudaGraphExec_t graph_exec = nullptr; // captured mixed translation passes for graph_nrhs columns
     int graph_nrhs = 0, graph_seen = 0;
-    int *tc_err = nullptr;        // set by a tensor-core pass when one of its waits gives up
+    int *tc_err = nullptr, *tc_err_host = nullptr;  // set by a tensor-core pass when one of its waits gives up
     float4 *PHall_ff = nullptr;   // float-float phases
     int ff_ready = 0;             // 1 once the float-float tables exist, -1 where they cannot
     double *dsc_leaf_dev = nullptr; // degree scales d_n of the leaf level (plans with scaled expansions)
@@ -326,6 +326,7 @@ void launch_axpby(double a, const double2 *x, double b, double2 *y, size_t n, cu
 int gen_dense_rcr(Plan *P, int l, int which, const int *keys, int nkeys, double2 *T);
 int tune_tc_dense(Plan *P);
 int launch_tc_dense(Plan *P, int l, int which, int nrhs, cudaStream_t st);
+int ensure_tc_err(Plan *P);
 int check_tc_error(Plan *P);
 
 // tc_rcr3.cu

@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1) rcr3_kernel(T3Args a)
                 const int s = (g + j) % T3_SA;
                 if (!mbar_wait(smem_u32(emptya + s), (((g + j) / T3_SA) & 1) ^ 1)) {
                     ok = false;
-                    atomicExch(a.err, 1);
+                    *(volatile int *)a.err = 1;
                     break;
                 }
                 unsigned char *Ahi = aring + (size_t)s * 2 * T3_TA, *Alo = Ahi + T3_TA;
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1) rcr3_kernel(T3Args a)
             __syncwarp();
         }
     }
-    if (!ok) atomicExch(a.err, 1);
+    if (!ok) *(volatile int *)a.err = 1;
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -862,10 +862,7 @@ int tune_tc3(Plan *P)
     const char *env = getenv("FMMBEM_TC3");
     const int mode = env ? atoi(env) : -1;
     if (mode == 0) return FMM_OK;
-    if (!P->tc_err) {
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&P->tc_err, sizeof(int)));
-        FMM_CUDA_TRY(cudaMemset(P->tc_err, 0, sizeof(int)));
-    }
+    if (int rc = ensure_tc_err(P)) return rc;
     cudaEvent_t a, b;
     FMM_CUDA_TRY(cudaEventCreate(&a));
     FMM_CUDA_TRY(cudaEventCreate(&b));
@@ -890,6 +887,7 @@ int tune_tc3(Plan *P)
                     if (rep > 0) ms[on] += t;
                 }
             }
+            if (rc == FMM_OK && cudaStreamSynchronize(P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
             if (rc == FMM_OK) rc = check_tc_error(P);
             if (rc) break;
             Lst->t3.on = (mode == 1 || ms[1] < ms[0]) ? 1 : 0;
