@@ -16,6 +16,9 @@
 //   int copy(double2 *dst, const double2 *src), zero(double2 *dst)       whole vectors
 //   double2 *tmp_alloc(), void tmp_free(double2 *)                       a whole vector
 //   int sync()
+//   bool step_fits(); int step(int nvec, double2 *W, double2 *next, h1, h2, hn)   where there: for one column, the
+//                                                                        two rounds of dots and sub_dots, the norm and
+//                                                                        next = W / norm at once
 //   void active(const std::vector<int> &on)                              columns whose matvec results
 //                                                                        are used (the others may be skipped)
 #pragma once
@@ -23,9 +26,14 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 namespace fmm {
+
+template <class Ops, class = void> struct HasStep : std::false_type {};
+template <class Ops> struct HasStep<Ops, decltype((void)std::declval<Ops &>().step_fits())> : std::true_type {};
 
 // Every Krylov step applies the operator to all R columns at once; classical Gram-Schmidt
 // applied twice (CGS2), FP64 vectors on the device, Hessenberg least squares by Givens
@@ -82,11 +90,18 @@ int gmres_core(Ops &o, const double2 *B, double2 *X, int R, const std::vector<do
             double2 *W = o.w();
             o.active(running);
             if ((st = o.matvec(o.V(j), W, precision))) return st;
-            if ((st = o.dots(j + 1, W, h1))) return st;
-            o.sub_dots(j + 1, W);
-            if ((st = o.dots(j + 1, W, h2))) return st;
-            o.sub_dots(j + 1, W);
-            if ((st = o.norms(W, hn))) return st;
+            bool at_once = false;
+            if constexpr (HasStep<Ops>::value) {
+                at_once = R == 1 && o.step_fits();
+                if (at_once && (st = o.step(j + 1, W, o.V(j + 1), h1, h2, hn))) return st;
+            }
+            if (!at_once) {
+                if ((st = o.dots(j + 1, W, h1))) return st;
+                o.sub_dots(j + 1, W);
+                if ((st = o.dots(j + 1, W, h2))) return st;
+                o.sub_dots(j + 1, W);
+                if ((st = o.norms(W, hn))) return st;
+            }
             total++;
             any = 0;
             for (int r = 0; r < R; r++) {
@@ -128,7 +143,7 @@ int gmres_core(Ops &o, const double2 *B, double2 *X, int R, const std::vector<do
                 alpha[r] = 1.0 / h;
                 any = 1;
             }
-            if (j + 1 < m) {
+            if (j + 1 < m && !at_once) {
                 if ((st = o.scale(alpha, W, o.V(j + 1)))) return st;
             }
             if (!any) { j++; break; }
