@@ -129,17 +129,12 @@ __global__ void p2m_kernel(int pl, const int *__restrict__ leaf_beg, const int *
     __shared__ C s_x[MAXE][G];
     const int b = blockIdx.x, ppl = pl * pl, r0 = blockIdx.y * G, ng = min(G, nrhs - r0);
     const int s0 = leaf_beg[b], ne = leaf_beg[b + 1] - s0;
-    for (int j = threadIdx.x; j < ne; j += blockDim.x) {
-        const int e = leaf_elem[s0 + j];
-        if (j < MAXE) s_e[j] = e;
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            if (g >= ng) break;
-            const size_t k_e = (size_t)(r0 + g) * nf + e;
-            const double2 xe = x[k_e];
-            if (j < MAXE) s_x[j][g] = mk2((T)(-k * xe.y), (T)(k * xe.x));  // i k x_e
-            if (x32) x32[k_e] = make_float2((float)xe.x, (float)xe.y);
-        }
+    for (int q = threadIdx.x; q < ne * G; q += blockDim.x) {
+        const int j = q / G, g = q % G, e = leaf_elem[s0 + j];
+        if (g == 0 && j < MAXE) s_e[j] = e;
+        const double2 xe = g < ng ? x[(size_t)(r0 + g) * nf + e] : make_double2(0.0, 0.0);
+        if (j < MAXE) s_x[j][g] = mk2((T)(-k * xe.y), (T)(k * xe.x));  // i k x_e
+        if (x32 && g < ng) x32[(size_t)e * nrhs + r0 + g] = make_float2((float)xe.x, (float)xe.y);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < ppl; i += blockDim.x) {
@@ -157,7 +152,6 @@ __global__ void p2m_kernel(int pl, const int *__restrict__ leaf_beg, const int *
             const C u = U[(size_t)s_e[j] * ppl + q];
 #pragma unroll
             for (int g = 0; g < G; g++) {
-                if (g >= ng) break;
                 const C xe = s_x[j][g];
                 ar[g] += xe.x * u.x - xe.y * u.y;
                 ai[g] += xe.x * u.y + xe.y * u.x;
@@ -194,32 +188,57 @@ __global__ void to_float_kernel2(const double *in, float *out, size_t n)
 // (blockIdx.y): the near row and the element's basis are loaded once for the group, the x
 // gathers and the local expansions per right-hand side.  Each column's sums run in the same
 // order whatever the group, so a column's result does not depend on nrhs.  T = float gathers
-// the near field's x from x32, the FP32 copy P2M wrote (the same values as converting x here).
+// the near field's x from x32, the FP32 copy P2M wrote (the same values as converting x here), a
+// column group of an element together (with a column's entries together a 32-byte sector was read for
+// each 8 bytes).
+// The identity's FP64 arithmetic runs once for a block's 8 elements and all their columns, a lane each: an FP64
+// instruction takes the pipe 16 cycles whatever lanes are on, and one lane per element and column was
+// half of the kernel.  64 columns on the 200,000-triangle head 6.8 -> 3.4 ms, 16 on the 81,920-triangle
+// sphere 0.85 -> 0.47 ms; what is left is the latency of the gathers (22 % of the issue slots used).
+constexpr int L2P_WARPS = 8;
 template <typename T, int G>
-__global__ void l2p_near_kernel(int nf, int pl, const int *__restrict__ elem_leaf, const typename Cx<T>::t *__restrict__ Dl,
+__global__ void __launch_bounds__(32 * L2P_WARPS) l2p_near_kernel(int nf, int pl, const int *__restrict__ elem_leaf, const typename Cx<T>::t *__restrict__ Dl,
                                 const typename Cx<T>::t *__restrict__ Rv, const int *__restrict__ near_beg,
                                 const int *__restrict__ near_col, const typename Cx<T>::t *__restrict__ nearv,
                                 const double2 *__restrict__ x, const float2 *__restrict__ x32, double2 a,
                                 double2 *__restrict__ y, int flip, int nb, int nrhs)
 {
     typedef typename Cx<T>::t C;
-    int lane = threadIdx.x & 31;
-    int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (e >= nf) return;
+    __shared__ C s_sum[L2P_WARPS][G];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int e0 = blockIdx.x * L2P_WARPS, e = min(e0 + warp, nf - 1);
     const int r0 = blockIdx.y * G, ng = min(G, nrhs - r0);
     int ppl = pl * pl;
+    const bool whole = ng == G && nrhs % 2 == 0;  // a group's columns of an element lie on 16 bytes
     T ar[G], ai[G];
 #pragma unroll
     for (int g = 0; g < G; g++) ar[g] = ai[g] = 0;
     for (int s = near_beg[e] + lane; s < near_beg[e + 1]; s += 32) {
         const C v = nearv[s];
         const int col = near_col[s];
+        if constexpr (sizeof(T) == 4 && G % 2 == 0) {
+            if (whole) {
+                const float4 *xc = reinterpret_cast<const float4 *>(x32 + (size_t)col * nrhs + r0);
+                float4 xg[G / 2];
+#pragma unroll
+                for (int g = 0; g < G / 2; g++) xg[g] = xc[g];
+#pragma unroll
+                for (int g = 0; g < G; g += 2) {
+                    const float4 xf = xg[g / 2];
+                    ar[g] += v.x * xf.x - v.y * xf.y;
+                    ai[g] += v.x * xf.y + v.y * xf.x;
+                    ar[g + 1] += v.x * xf.z - v.y * xf.w;
+                    ai[g + 1] += v.x * xf.w + v.y * xf.z;
+                }
+                continue;
+            }
+        }
 #pragma unroll
         for (int g = 0; g < G; g++) {
             if (g >= ng) break;
             T xr, xi;
             if constexpr (sizeof(T) == 4) {
-                const float2 xf = x32[(size_t)(r0 + g) * nf + col];
+                const float2 xf = x32[(size_t)col * nrhs + r0 + g];
                 xr = xf.x;
                 xi = xf.y;
             } else {
@@ -241,12 +260,14 @@ __global__ void l2p_near_kernel(int nf, int pl, const int *__restrict__ elem_lea
             q = n * n + n - m;
         }
         const C r = R[q];
+        // (columns past the last read the last one's: loads without a branch between them are in flight together)
+        C d[G];
+#pragma unroll
+        for (int g = 0; g < G; g++) d[g] = Dl[(db + r0 + min(g, ng - 1)) * ppl + i];
 #pragma unroll
         for (int g = 0; g < G; g++) {
-            if (g >= ng) break;
-            const C d = Dl[(db + r0 + g) * ppl + i];
-            ar[g] += d.x * r.x - d.y * r.y;
-            ai[g] += d.x * r.y + d.y * r.x;
+            ar[g] += d[g].x * r.x - d[g].y * r.y;
+            ai[g] += d[g].x * r.y + d[g].y * r.x;
         }
     }
 #pragma unroll
@@ -257,11 +278,16 @@ __global__ void l2p_near_kernel(int nf, int pl, const int *__restrict__ elem_lea
             sr += __shfl_xor_sync(0xffffffffu, sr, o);
             si += __shfl_xor_sync(0xffffffffu, si, o);
         }
-        if (lane == 0) {
-            const size_t k = (size_t)(r0 + g) * nf + e;
-            const double2 xe = x[k];
-            y[k] = make_double2(a.x * xe.x - a.y * xe.y + (double)sr, a.x * xe.y + a.y * xe.x + (double)si);
-        }
+        if (lane == g) s_sum[warp][g] = mk2(sr, si);
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < L2P_WARPS * ng; q += 32 * L2P_WARPS) {
+        const int w = q % L2P_WARPS, g = q / L2P_WARPS;
+        if (e0 + w >= nf) continue;
+        const size_t k = (size_t)(r0 + g) * nf + e0 + w;
+        const double2 xe = x[k];
+        const C s = s_sum[w][g];
+        y[k] = make_double2(a.x * xe.x - a.y * xe.y + (double)s.x, a.x * xe.y + a.y * xe.x + (double)s.y);
     }
 }
 
@@ -594,7 +620,7 @@ static int run_matvec_t(Plan *P, const double2 *x, double2 *y, int transpose, in
     {
         const int *nb_ = transpose ? P->nearT_beg : P->near_beg, *nc_ = transpose ? P->nearT_col : P->near_col;
         const C *nv_ = transpose ? nearT : nearv, *rv_ = transpose ? U : Rv;
-        const unsigned gx = (unsigned)((P->nf * 32 + 255) / 256);
+        const unsigned gx = (unsigned)((P->nf + L2P_WARPS - 1) / L2P_WARPS);
         if (nrhs == 1)
             l2p_near_kernel<T, 1><<<dim3(gx, 1), 256, 0, st>>>(P->nf, LL.p, P->elem_leaf, Dl(lmax), rv_, nb_, nc_, nv_, x, x32,
                                                             a, y, transpose, LL.nb, 1);
