@@ -117,13 +117,33 @@ __device__ void rcr_block(int p, int pmax, const double *__restrict__ H, const d
 // With x32 given, the CTA also writes its elements' x in FP32 there (every element lies in one
 // leaf), for the gathers of the L2P + near-field pass: GB300 converts FP64 to FP32 at its FP64
 // rate, and the near field would otherwise convert each x once per near pair.
+// The blocks behind the leaf boxes zero the expansions that the translations add to (a memset per
+// level and kind, one after another, was 5 us of a 50 us matvec on 320 triangles).
+struct ZeroList {
+    float4 *ptr[2 * (FMM_MAX_LEVEL + 2)];
+    unsigned end[2 * (FMM_MAX_LEVEL + 2)];          // blocks up to and with this entry
+    unsigned long long n[2 * (FMM_MAX_LEVEL + 2)];  // 16-byte words
+    unsigned words;                                 // per block: 16 KB, more where that takes over 64 blocks per SM
+    int count;
+};
+
 template <typename T, int G>
 __global__ void p2m_kernel(int pl, const int *__restrict__ leaf_beg, const int *__restrict__ leaf_elem,
                            const typename Cx<T>::t *__restrict__ U, const double2 *__restrict__ x, double k,
                            typename Cx<T>::t *__restrict__ Cm, int flip, int nf, int nb, int nrhs,
-                           float2 *__restrict__ x32)
+                           float2 *__restrict__ x32, const __grid_constant__ ZeroList zero)
 {
     typedef typename Cx<T>::t C;
+    if ((int)blockIdx.x >= nb) {
+        if (blockIdx.y) return;
+        unsigned z = blockIdx.x - nb, first = 0;
+        int i = 0;
+        while (z >= zero.end[i]) first = zero.end[i++];
+        const unsigned long long w0 = (unsigned long long)(z - first) * zero.words;
+        for (unsigned long long w = w0 + threadIdx.x; w < min(w0 + zero.words, zero.n[i]); w += blockDim.x)
+            zero.ptr[i][w] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
     constexpr int MAXE = 64;
     __shared__ int s_e[MAXE];
     __shared__ C s_x[MAXE][G];
@@ -473,7 +493,27 @@ int launch_pass32(Plan *P, int l, int which, int nrhs, cudaStream_t st)
     return Lst ? launch_rcr_pass(P, *Lst, ps, st) : FMM_OK;
 }
 
-// The mixed path's translation passes for nrhs columns: zero the expansions, M2M up, the
+// The expansions that the mixed path's translations add to, for nrhs columns: all multipoles above the
+// leaves and all locals (each buffer has one coefficient to spare, so whole 16-byte words).
+static ZeroList zero_list(const Plan *P, int nrhs)
+{
+    ZeroList z = {};
+    unsigned end = 0;
+    unsigned long long all = 0;
+    for (int l = P->lmin; l <= P->lmax; l++) all += (unsigned long long)P->lev[l].nb * P->lev[l].p * P->lev[l].p * nrhs;
+    z.words = (unsigned)std::max<unsigned long long>(1024, all / (152 * 64));
+    for (int l = P->lmin; l <= P->lmax; l++)
+        for (int c = l < P->lmax ? 0 : 1; c < 2; c++) {
+            const LevelDev &L = P->lev[l];
+            z.ptr[z.count] = reinterpret_cast<float4 *>(c ? L.Dl32 : L.Cm32);
+            z.n[z.count] = ((unsigned long long)L.nb * L.p * L.p * nrhs + 1) / 2;
+            end += (unsigned)((z.n[z.count] + z.words - 1) / z.words);
+            z.end[z.count++] = end;
+        }
+    return z;
+}
+
+// The mixed path's translation passes for nrhs columns (into expansions that P2M zeroed): M2M up, the
 // M2L of every level forked onto the side streams (one level's tail overlaps the next
 // level's work), join, L2L down.  M2M and M2L add into zeroed expansions with atomics; L2L
 // then adds the parents' locals top-down.
@@ -484,11 +524,6 @@ static int translate32_direct(Plan *P, int nrhs)
     if (P->profiling == 1) {
         cudaEventRecord(P->phase.beg, st);
         P->have_phase = 1;
-    }
-    for (int l = lmin; l <= lmax; l++) {
-        size_t n = (size_t)P->lev[l].nb * P->lev[l].p * P->lev[l].p * sizeof(float2) * nrhs;
-        if (l < lmax) FMM_CUDA_TRY(cudaMemsetAsync(P->lev[l].Cm32, 0, n, st));
-        FMM_CUDA_TRY(cudaMemsetAsync(P->lev[l].Dl32, 0, n, st));
     }
     for (int l = lmax; l > lmin; l--) {
         timer_begin(P, pass_names[PASS_M2M][l]);
@@ -603,12 +638,15 @@ static int run_matvec_t(Plan *P, const double2 *x, double2 *y, int transpose, in
     timer_begin(P, "p2m");
     // the transposed operator swaps the roles of the element moments and the centroid basis
     // (index-flipped), keeps every translation, and uses the transposed near-field matrix
+    const ZeroList zero = owner ? ZeroList{} : zero_list(P, nrhs);
+    const unsigned blocks = LL.nb + (zero.count ? zero.end[zero.count - 1] : 0);
     if (nrhs == 1)
-        p2m_kernel<T, 1><<<dim3(LL.nb, 1), 128, 0, st>>>(LL.p, P->leaf_beg, P->leaf_elem, transpose ? Rv : U, x, P->opt.k,
-                                                      Cm(lmax), transpose, P->nf, LL.nb, 1, x32);
+        p2m_kernel<T, 1><<<dim3(blocks, 1), 128, 0, st>>>(LL.p, P->leaf_beg, P->leaf_elem, transpose ? Rv : U, x, P->opt.k,
+                                                      Cm(lmax), transpose, P->nf, LL.nb, 1, x32, zero);
     else
-        p2m_kernel<T, 8><<<dim3(LL.nb, (nrhs + 7) / 8), 128, 0, st>>>(LL.p, P->leaf_beg, P->leaf_elem, transpose ? Rv : U, x,
-                                                                   P->opt.k, Cm(lmax), transpose, P->nf, LL.nb, nrhs, x32);
+        p2m_kernel<T, 8><<<dim3(blocks, (nrhs + 7) / 8), 128, 0, st>>>(LL.p, P->leaf_beg, P->leaf_elem, transpose ? Rv : U, x,
+                                                                   P->opt.k, Cm(lmax), transpose, P->nf, LL.nb, nrhs, x32,
+                                                                   zero);
     timer_end(P);
     {
         int e = owner ? translate_owner(P, ffm2l ? OWN_FF : f64 ? OWN_FP64 : OWN_FP32, pass_begin, pass_end) : translate32(P, nrhs);
