@@ -76,6 +76,8 @@ struct TcPass {
     const float2 *PH;                    // phases e^{i m phi} of direction d at d phstride + phoff + m
     int phstride, phoff;
     int nrhs, P2, P2o, ntiles;           // P2 = pin^2, P2o = pout^2
+    unsigned long long per;              // e / nrhs = e per >> shift for columns e < 2^31: per = 2^shift / nrhs, rounded
+    int shift;                           // up, 2^(shift - 31) >= nrhs
     const float *B;
     const float2 *src;
     float2 *dst;
@@ -271,7 +273,7 @@ __device__ __forceinline__ TileRow tile_row(const TcPass &ps, int4 it, int r, co
 {
     TileRow o;
     if (r < it.z) {
-        const int e = it.y + r, t = e / ps.nrhs;
+        const int e = it.y + r, t = (int)(((unsigned long long)e * ps.per) >> ps.shift);
         o.row = box[t] * ps.nrhs + (e - t * ps.nrhs);
         o.dir = ps.g_dir[t];
     }
@@ -281,7 +283,8 @@ __device__ __forceinline__ TileRow tile_row(const TcPass &ps, int4 it, int r, co
 // Up to eight coefficient pairs (m = 0..last) of a degree from the columns of their sums (from p on) and
 // differences (from q on, none for m = 0 where `first`) to y[m], y[-m] of the lane's row; columns past the last
 // pair's are not used.
-__device__ __forceinline__ void unfold(uint32_t p, uint32_t q, int last, const float2 (&f)[8], float2 *y, bool first, int fold)
+template <bool FOLD>
+__device__ __forceinline__ void unfold(uint32_t p, uint32_t q, int last, const float2 (&f)[8], float2 *y, bool first)
 {
     uint32_t u[16], w[16];
     tc_ld16(u, p);
@@ -296,13 +299,14 @@ __device__ __forceinline__ void unfold(uint32_t p, uint32_t q, int last, const f
             continue;
         }
         const float dr = __uint_as_float(w[2 * j]), di = __uint_as_float(w[2 * j + 1]);
-        const float pr = fold ? sr + dr : sr, pi = fold ? si + di : si, mr = fold ? sr - dr : dr, mi = fold ? si - di : di;
+        const float pr = FOLD ? sr + dr : sr, pi = FOLD ? si + di : si, mr = FOLD ? sr - dr : dr, mi = FOLD ? si - di : di;
         const int m = first ? j : j + 8;
         y[m] = make_float2(pr * f[j].x + pi * f[j].y, pi * f[j].x - pr * f[j].y);
         y[-m] = make_float2(mr * f[j].x - mi * f[j].y, mr * f[j].y + mi * f[j].x);
     }
 }
 
+template <bool FOLD>
 __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_constant__ TcPass ps)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -357,7 +361,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
         // time lost to it: one thread, and little arithmetic.
         if (elect_one()) {
             Ring rs;
-            const int fold = sh.fold;
             const uint32_t b0 = (smem_u32(smem) >> 4) | TC_DESC_LO, bstep = (uint32_t)sh.bstage >> 4;
             for (int i = 0; i < ntile && ok; i++) {
                 const TcSub &s = range(i);
@@ -376,7 +379,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
                     tc_mma(d1, at, b1, i1, add);
                     tc_mma(d1, at, b1 + l1, i1, 1);
                     tc_mma(d1, at + TC_KC, b1, i1, 1);
-                    if (fold) {
+                    if constexpr (FOLD) {
                         tc_mma(d2, a2, b2, i2, add);
                         tc_mma(d2, a2, b2 + l2, i2, 1);
                         tc_mma(d2, a2 + TC_KC, b2, i2, 1);
@@ -404,7 +407,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
             Ring rs;
             for (int i = 0; i < ntile && ok; i++) {
                 const TcSub &s = range(i);
-                const uint32_t fl = (uint32_t)((sh.fold ? 2 : 4) * TC_KC * (s.nP + s.nQ));
+                const uint32_t fl = (uint32_t)((FOLD ? 2 : 4) * TC_KC * (s.nP + s.nQ));
                 const float *B = ps.B + (size_t)ps.items[tile(i)].x * sh.cls_floats + s.boff;
                 for (int c = 0; c < sh.nch; c++, B += fl) {
                     ok = mbar_wait(smem_u32(empty + rs.i), rs.par ^ 1);
@@ -463,7 +466,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp < TC_E0) {
         // ---------------------------------------------------------------- A operand
-        const int quarter = warp & 3, grp = (warp - TC_A0) >> 2, r = 32 * quarter + lane, fold = sh.fold;
+        const int quarter = warp & 3, grp = (warp - TC_A0) >> 2, r = 32 * quarter + lane;
         const uint32_t ta0 = tmem_a + ((uint32_t)(quarter * 32) << 16);
         Ring rr, rs;
         int turn = 0;
@@ -500,7 +503,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         float s[4];
-                        if (fold) {  // x_m e + x_-m e*, x_m e - x_-m e*
+                        if constexpr (FOLD) {  // x_m e + x_-m e*, x_m e - x_-m e*
                             const float sr = xp[j].x + xm[j].x, si = xp[j].y + xm[j].y, dr = xp[j].x - xm[j].x, di = xp[j].y - xm[j].y;
                             s[0] = sr * f[j].x - di * f[j].y, s[1] = si * f[j].x + dr * f[j].y;
                             s[2] = dr * f[j].x - si * f[j].y, s[3] = di * f[j].x + sr * f[j].y;
@@ -573,8 +576,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
                 for (int n = na; n < nb; n++) {
                     float2 *y = st + odd + (n * n + n - c0);
                     const uint32_t pn = tp + (uint32_t)(2 * (n * (n + 1) / 2 - p0)), qn = tq + (uint32_t)(2 * (n * (n - 1) / 2 - q0)) - 2;
-                    unfold(pn, qn, n, f0, y, true, sh.fold);
-                    if (n >= 8) unfold(pn + 16, qn + 16, n - 8, f1, y, false, sh.fold);
+                    unfold<FOLD>(pn, qn, n, f0, y, true);
+                    if (n >= 8) unfold<FOLD>(pn + 16, qn + 16, n - 8, f1, y, false);
                 }
                 if (!left) {  // the warp's last columns are read
                     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -874,6 +877,9 @@ int launch_tc_dense(Plan *P, int l, int which, int nrhs, cudaStream_t st)
     ps.phstride = rp.phstride;
     ps.phoff = rp.phoff;
     ps.nrhs = nrhs;
+    ps.shift = 31;
+    while (1ll << (ps.shift - 31) < nrhs) ps.shift++;
+    ps.per = ((1ull << ps.shift) + nrhs - 1) / nrhs;
     ps.P2 = pin * pin;
     ps.P2o = pout * pout;
     ps.ntiles = g.n_items * g.sh.nsub;
@@ -882,8 +888,9 @@ int launch_tc_dense(Plan *P, int l, int which, int nrhs, cudaStream_t st)
     ps.dst = rp.dst;
     ps.err = P->tc_err;
     const size_t sm = tc_smem_bytes(g.sh);
-    static size_t attr = 0;
-    e = raise_smem_limit((const void *)tc_dense_kernel, sm, &attr);
+    const auto kernel = g.sh.fold ? tc_dense_kernel<true> : tc_dense_kernel<false>;
+    static size_t attr[2] = {0, 0};
+    e = raise_smem_limit((const void *)kernel, sm, &attr[g.sh.fold ? 1 : 0]);
     if (e) return e;
     // persistent: one CTA per SM (its shared memory and 512 TMEM columns take the SM)
     static int nsm = 0;
@@ -893,7 +900,7 @@ int launch_tc_dense(Plan *P, int l, int which, int nrhs, cudaStream_t st)
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         if (nsm <= 0) nsm = 152;
     }
-    tc_dense_kernel<<<std::min(ps.ntiles, nsm), TC_THREADS, sm, st>>>(ps);
+    kernel<<<std::min(ps.ntiles, nsm), TC_THREADS, sm, st>>>(ps);
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
