@@ -100,10 +100,17 @@ template <> struct Rows<4> { typedef float4 t; };
 template <> struct Rows<2> { typedef float2 t; };
 constexpr int THREADS = 256, CG = 4;  // threads of a CTA, columns of a lane
 
+// A table entry, from global memory or (S) from the tile's copy in shared memory
+template <bool S, class T> __device__ __forceinline__ T entry(const T *p)
+{
+    if constexpr (S) return *p;
+    else return __ldg(p);
+}
+
 // One rotation stage, in place.  Round k gives thread t unit k UC + t / CL and the
 // column pairs cl, cl + CL (cl = t % CL): (n | sign << 8 | first row << 16, table offset), R rows of P_n or Q_n.  All
 // units of a block (n, sign) are in one round, which writes after everyone has read.
-template <int TC, int R>
+template <int TC, int R, bool S>
 __device__ __forceinline__ void rot_stage(const float *__restrict__ rot, ulonglong2 *X, const int2 *__restrict__ units, int rounds)
 {
     constexpr int CL = TC / CG, UC = THREADS / CL, NC = CG / 2;
@@ -121,12 +128,12 @@ __device__ __forceinline__ void rot_stage(const float *__restrict__ rot, ulonglo
             for (int c = 0; c < CG; c++) acc[r][c] = 0ull;
         int row = minus ? c0 - 1 : c0;
         const int dr = minus ? -1 : 1;
-        typename Rows<R>::t hn = __ldg(reinterpret_cast<const typename Rows<R>::t *>(h));
+        typename Rows<R>::t hn = entry<S>(reinterpret_cast<const typename Rows<R>::t *>(h));
 #pragma unroll 2
         for (int m = 0; m < steps; m++) {
             const typename Rows<R>::t hv = hn;
             if (m + 1 < steps) h += ld;  // the last step loads its own entries again
-            hn = __ldg(reinterpret_cast<const typename Rows<R>::t *>(h));
+            hn = entry<S>(reinterpret_cast<const typename Rows<R>::t *>(h));
             ulonglong2 x[NC];
             const ulonglong2 *xr = X + row * (TC / 2);
             const int s = swz<TC>(row);
@@ -159,7 +166,7 @@ __device__ __forceinline__ void rot_stage(const float *__restrict__ rot, ulonglo
 
 // The coaxial stage, in place, in rounds as above.  Unit: |m| | sign << 8 | first row << 16, two of
 // the rows of order +-m.
-template <int TC>
+template <int TC, bool S>
 __device__ __forceinline__ void coax_stage(int p, int nin, int nq, const float2 *__restrict__ Cc, ulonglong2 *X,
                                            const int *__restrict__ units, int rounds)
 {
@@ -178,12 +185,12 @@ __device__ __forceinline__ void coax_stage(int p, int nin, int nq, const float2 
             for (int j = 0; j < CG; j++) a0[r][j] = a1[r][j] = 0ull;
         const int sm = minus ? -am : am;
         int row = am * am + am + sm, dr = 2 * am + 2;
-        float4 cn = __ldg(c);
+        float4 cn = entry<S>(c);
 #pragma unroll 2
         for (int n = 0; n < steps; n++) {
             const float4 cc = cn;
             if (n + 1 < steps) c += ld / 2;
-            cn = __ldg(c);
+            cn = entry<S>(c);
             ulonglong2 x[NC];
             const ulonglong2 *xr = X + row * (TC / 2);
             const int s = swz<TC>(row);
@@ -222,13 +229,28 @@ __device__ __forceinline__ void coax_stage(int p, int nin, int nq, const float2 
 }
 
 // One tile: item it = (class, first column, count, coaxial table) of pass ps, with the
-// CTA's dynamic shared memory and its column indices.
-template <int TC, int R>
+// CTA's dynamic shared memory and its column indices.  S: the class's rotation table and the
+// coaxial table are copied to shared memory behind the tile (ps.tile_words 16-byte words) while the
+// columns are gathered.  Each step of a stage waits for its table entries; in a pass of so few tiles that each SM
+// has one or two, nothing hides their way from the L2.
+template <int TC, int R, bool S>
 __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float4 *smem4, int *s_src, int *s_dst, int *s_dir)
 {
     const int p = ps.p, nin = min(ps.pin, p), nq = min(ps.pout, p), cnt = it.z;
     ulonglong2 *X = reinterpret_cast<ulonglong2 *>(smem4);
     float2 *Xf = reinterpret_cast<float2 *>(X);
+    const float *rot = ps.rot + (size_t)it.x * ps.rot_stride;
+    const float2 *coax = ps.coax + (size_t)it.w * coax2_sum(p);
+    if constexpr (S) {
+        const float4 *r4 = reinterpret_cast<const float4 *>(rot), *c4 = reinterpret_cast<const float4 *>(coax);
+        float4 *to = smem4 + ps.tile_words;
+        const int nr = ps.rot_words, nc = coax2_sum(p) / 2;
+        for (int i = threadIdx.x; i < nr + nc; i += THREADS)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + i)),
+                         "l"(i < nr ? r4 + i : c4 + (i - nr)) : "memory");
+        rot = reinterpret_cast<const float *>(to);
+        coax = reinterpret_cast<const float2 *>(to + nr);
+    }
     if (threadIdx.x < TC) {
         // column e = translation t x nrhs + right-hand side r; the expansions hold the columns
         // of a box next to each other ([box][rhs][p^2])
@@ -280,13 +302,13 @@ __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float
             }
         }
     }
+    if constexpr (S) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const float *rot = ps.rot + (size_t)it.x * ps.rot_stride;
-    rot_stage<TC, R>(rot, X, ps.u1, ps.n1);
+    rot_stage<TC, R, S>(rot, X, ps.u1, ps.n1);
     __syncthreads();
-    coax_stage<TC>(p, nin, nq, ps.coax + (size_t)it.w * coax2_sum(p), X, ps.u2, ps.n2);
+    coax_stage<TC, S>(p, nin, nq, coax, X, ps.u2, ps.n2);
     __syncthreads();
-    rot_stage<TC, R>(rot, X, ps.u3, ps.n3);
+    rot_stage<TC, R, S>(rot, X, ps.u3, ps.n3);
     __syncthreads();
     {
         const int np = nq * (nq + 1) / 2, nb = (np + 7) / 8 * (TC / 4), dstride = ps.pout * ps.pout;
@@ -319,12 +341,12 @@ __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float
     }
 }
 
-template <int TC, int R>
+template <int TC, int R, bool S>
 __global__ void __launch_bounds__(THREADS, 3) rcr_tile_kernel(RcrPass ps)
 {
     extern __shared__ float4 smem4[];
     __shared__ int s_src[TC], s_dst[TC], s_dir[TC];
-    rcr_tile<TC, R>(ps, ps.items[blockIdx.x], smem4, s_src, s_dst, s_dir);
+    rcr_tile<TC, R, S>(ps, ps.items[blockIdx.x], smem4, s_src, s_dst, s_dir);
 }
 
 // Persistent form for many passes at once (the translation passes of many plans, one phase
@@ -345,7 +367,7 @@ __global__ void __launch_bounds__(THREADS, 3) rcr_queue_kernel(const RcrPass *__
         __syncthreads();
         const int w = s_w;
         if (w >= n) break;
-        rcr_tile<TC, R>(passes[work_pass[w]], work_item[w], smem4, s_src, s_dst, s_dir);
+        rcr_tile<TC, R, false>(passes[work_pass[w]], work_item[w], smem4, s_src, s_dst, s_dir);
         __syncthreads();
     }
 }
@@ -541,12 +563,26 @@ int launch_rcr_pass(const Plan *P, RcrList &Lst, RcrPass ps, cudaStream_t st)
     }
     ps.items = Lst.items;
     const size_t sm = tile_bytes(ps, Lst.tc);
+    ps.tile_words = (int)(sm / 16);
+    ps.rot_words = rot32_size(ps.p) / 4;
+    const size_t sm_tab = sm + (size_t)ps.rot_words * 16 + (size_t)coax2_size(ps.p) * sizeof(float2);
+    static int nsm = 0;
+    if (!nsm) {
+        int dev = 0;
+        FMM_CUDA_TRY(cudaGetDevice(&dev));
+        FMM_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    }
+    // tables in shared memory where every tile is resident at once all the same, three CTAs of up to 74 KB on an
+    // SM (a matvec on 5,120 triangles, orders 16, 14, 12: 198 us without, 179 with; larger tables, 81,920
+    // triangles with orders up to 40: no gain)
+    const bool staged = sm_tab <= 74 * 1024 && Lst.n_items <= 3 * nsm;
     return with_tile(Lst.tc, Lst.bal, [&](auto t) -> int {
         using T = decltype(t);
-        static size_t attr = 0;
-        int e = raise_smem_limit((const void *)rcr_tile_kernel<T::TC, T::R>, sm, &attr);
+        static size_t attr[2] = {0, 0};
+        const auto kernel = staged ? rcr_tile_kernel<T::TC, T::R, true> : rcr_tile_kernel<T::TC, T::R, false>;
+        int e = raise_smem_limit((const void *)kernel, staged ? sm_tab : sm, &attr[staged]);
         if (e) return e;
-        rcr_tile_kernel<T::TC, T::R><<<Lst.n_items, 256, sm, st>>>(ps);
+        kernel<<<Lst.n_items, 256, staged ? sm_tab : sm, st>>>(ps);
         FMM_CUDA_TRY(cudaGetLastError());
         return FMM_OK;
     });

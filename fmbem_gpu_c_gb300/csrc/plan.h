@@ -143,6 +143,7 @@ struct RcrPass {
     const int2 *u1, *u3;
     const int *u2, *pairs;
     int n1, n2, n3;
+    int tile_words, rot_words;       // 16-byte words of a tile and of a class's rotation table (tables in shared memory)
 };
 
 // One pass of the translations without atomics (owner.cu): translations ("slots", in destination
