@@ -328,23 +328,17 @@ def gpu_arm(args, world, rank, local):
     rcr_ms = float(np.mean(kernel_ms["translations"]))  # the M2M/M2L/L2L phase as a whole
     bf16_peak, hbm_peak, peak_kind = peaks()
     achieved_tflops = rcr_flops / (rcr_ms / 1e3) / 1e12
-    # the M2L levels on the tensor cores (tc_dense_kernel): split-TF32 GEMMs over dense operators,
-    # 3 MMAs of 128 x Nmma x 8 per 8 of K for every 128 translations and output half
+    # the M2L levels on the tensor cores (tc_dense_kernel): split-TF32 GEMMs over dense operators, three
+    # products per input and output, re and im.  From 100,000 translations on two blocks, sums and
+    # differences of m and -m; below, the whole operator in four.  (Padding left out.)
     tc_levels = [l for l in range(info.lmin, info.lmax + 1) if info.m2l_tensor[l]]
     tc = None
     if tc_levels:
         ex = 0.0
         for l in tc_levels:
-            p = info.p_level[l]
-            nhalf = 1
-            while True:
-                ch = -(-p * p // nhalf)
-                nmma = (2 * ch + 15) // 16 * 16
-                if nmma <= 256:
-                    break
-                nhalf += 1
-            nch = -(-2 * p * p // 16)
-            ex += info.num_m2l[l] * nhalf * nch * 16 * 6 * nmma
+            p, t = info.p_level[l], info.num_m2l[l]
+            sums, diffs = p * (p + 1), p * (p - 1)  # real inputs and outputs of the two blocks
+            ex += 6.0 * t * (sums ** 2 + diffs ** 2 if t >= 100000 else (sums + diffs) ** 2)
         tc_ms = sum(float(np.mean(kernel_ms["m2l_l%d" % l])) for l in tc_levels)
         tc_alg = sum(info.num_m2l[l] * f_rcr(info.p_level[l]) for l in tc_levels)
         tc = {"kernel": "tc_dense_kernel (tcgen05.mma kind::tf32, split TF32, TMEM accumulators)", "levels": tc_levels,

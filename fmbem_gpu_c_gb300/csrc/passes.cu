@@ -571,7 +571,7 @@ void drop_graph(Plan *P)
 
 // Translation passes as a CUDA graph: the second call with the same number of columns
 // captures them (the first has built the work items and set the kernels' attributes), later
-// calls replay the graph, which saves the ~25 launches and memsets per matvec.  Per-pass
+// calls replay the graph, which saves the ~15 launches per matvec.  Per-pass
 // profiling (mode 1) runs the passes directly so that each pass gets its own timer.
 static int translate32(Plan *P, int nrhs)
 {
@@ -615,7 +615,7 @@ static int run_matvec_t(Plan *P, const double2 *x, double2 *y, int transpose, in
 {
     typedef typename Cx<T>::t C;
     const bool f64 = sizeof(T) == 8;
-    // owner-computes translations: the FP64 path, and the mixed path of deterministic plans
+    // translations without atomics (owner.cu): the FP64 path, and the mixed path of deterministic plans
     const bool owner = f64 || P->opt.deterministic;
     const int lmax = P->lmax;
     cudaStream_t st = P->stream;
@@ -772,7 +772,7 @@ int run_matvec(Plan *P, const double2 *x, double2 *y, int precision, int transpo
         int st = ensure_rhs32(P, nrhs);
         if (st) return st;
         if (!P->opt.deterministic) return run_matvec_t<float>(P, x, y, transpose, nrhs);
-        // the owner-computes kernels take one right-hand side
+        // the translations without atomics take one right-hand side
         for (int r = 0; r < nrhs; r++) {
             st = run_matvec_t<float>(P, x + (size_t)r * P->nf, y + (size_t)r * P->nf, transpose, 1);
             if (st) return st;

@@ -19,19 +19,20 @@
 // and all four blocks, fold_pays().)  Split TF32 (3 products hi*hi + hi*lo + lo*hi of rounded 11-bit halves)
 // gives close to FP32 accuracy.
 //
-// A persistent, warp-specialised kernel (one CTA per SM, 19 warps) runs over the tiles
+// A persistent, warp-specialised kernel (one CTA per SM, 20 warps) runs over the tiles
 // (128 translations x one range of output degrees):
-//   warp 0     issues the MMAs (one thread) into one of two sets of TMEM accumulators and commits
-//              each K chunk to the "empty" barriers of its operands, each tile to its
+//   warp 0     issues the MMAs (one thread) into a set of TMEM accumulators (of two, or the one) and
+//              commits each K chunk to its stage's "empty" barrier, each tile to its
 //              accumulators' "full" barrier;
 //   warp 1     copies the operator's K chunks (hi and lo tiles of both blocks) with cp.async.bulk;
-//   warp 2     copies the source expansions, row by row, in pieces of whole degrees;
-//   warps 3-10 (two per TMEM lane quarter, on alternate chunks; lane = row) read four coefficient
+//   warps 2, 3 copy the source expansions, row by row, in pieces of whole degrees;
+//   warps 4-11 (two per TMEM lane quarter, on alternate chunks; lane = row) read four coefficient
 //              pairs (n, m), (n, -m) of their row, apply its phases, form sums and differences,
 //              split them into TF32 hi / lo and write them to TMEM as the MMA's A operand;
-//   warps 11-18 (two per quarter, on alternate groups of degrees) read the finished accumulators,
-//              form the group's coefficients of their row in shared memory and add them into the
-//              destination expansions with 16-byte FP32 atomics, overlapping the next tile's MMAs.
+//   warps 12-19 (two per quarter, each its groups of degrees) read the finished accumulators, form the
+//              group's coefficients of their row in shared memory and add them into the destination
+//              expansions, a row's group with one bulk reduction (single coefficients with atomics where it does
+//              not lie on 16 bytes), overlapping the next tile's MMAs where there are two sets.
 // Every wait has a time limit, after which the thread sets the plan's error flag and stops.
 //
 // What bounds it: 16 columns on the 81,920-triangle sphere, p = 14 (192,528 translations) 2.78 ms and

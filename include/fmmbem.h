@@ -72,10 +72,10 @@ typedef struct {
                                  degree-scaled coaxial entries exceed the FP32 range) */
     int device;               /* CUDA device ordinal */
     double alpha_re, alpha_im;/* Burton-Miller coupling alpha (0: the conventional operator) */
-    int deterministic;        /* FMM_MIXED without atomics: each destination box accumulates its
-                                 FP32 translations in one CTA (owner-computes, as the FP64 path),
-                                 one right-hand side after another, so that mixed results are
-                                 reproducible bit for bit; slower than the batched tiles */
+    int deterministic;        /* FMM_MIXED without atomics: each FP32 translation writes a slot of its
+                                 own and a destination box adds its slots in a fixed order (as the
+                                 FP64 path), one right-hand side after another, so that mixed results
+                                 are reproducible bit for bit; slower than the batched tiles */
 } fmm_options;
 
 typedef struct {
@@ -91,7 +91,9 @@ typedef struct {
     int m2l_tensor[FMM_MAX_LEVEL + 1];   /* mixed path: 1 where the level's M2L runs on the tensor cores
                                             (tcgen05, split TF32, dense operators per class of directions; levels with
                                             p <= 16 and enough translations, or all of them
-                                            with FMMBEM_TENSOR_M2L=1; none with FMMBEM_TENSOR_M2L=0) */
+                                            with FMMBEM_TENSOR_M2L=1; none with FMMBEM_TENSOR_M2L=0; from 100,000
+                                            translations on in blocks of sums and differences of +-m,
+                                            FMMBEM_TENSOR_FOLD=0/1: nowhere / everywhere) */
     int expansions_scaled;               /* mixed path: 1 where the FP32 expansions are kept scaled by degree
                                             (low k t, where the plain coaxial entries would leave the FP32
                                             range): multipoles d_n M_n, locals L_n / d_n per level */
