@@ -43,6 +43,13 @@ namespace {
 // x+ row m' = j, row j > n the x- row m' = j - n (its m = 0 entry is zero)
 __host__ __device__ __forceinline__ int fold_off(int n) { return n * (4 * n * n + 3 * n - 1) / 6; }
 __host__ __device__ __forceinline__ int fold_size(int p) { return fold_off(p); }
+// whole rotation tables of the FP32 tiles: degree n holds 2n + 1 columns of 2n + 1 rows, padded to 4, so that a
+// lane's four rows are one load
+__host__ __device__ __forceinline__ int pad4(int n) { return (n + 3) & ~3; }
+__host__ __device__ __forceinline__ int pad_off(int n)
+{
+    return 2 * n * (n - 1) * (2 * n - 1) / 3 + 4 * n * (n - 1) + 3 * n + (n & 1 ? n : -n);
+}
 
 // ---- arithmetic of one type: V a complex number (one 8- or 16-byte value in memory), X the same
 // prepared for multiply-adds, S a real table entry, K a complex one, E a phase; V accumulates
@@ -269,25 +276,32 @@ __device__ __forceinline__ void rot_stage(const typename Ops<T>::S *__restrict__
         const int first = minus ? 1 + (g - np) * R : g * R;         // m' (FP32: row) of the first row
         const int last = O::FOLD ? n : w - 1;
         const int steps = O::FOLD ? n + 1 : w;
-        const typename O::S *h = rot + (O::FOLD ? fold_off(n) : rot_off(n)) + (minus ? n : 0) + first;
+        const typename O::S *h = rot + (O::FOLD ? fold_off(n) : pad_off(n)) + (minus ? n : 0) + first;
+        const int ld = O::FOLD ? w : pad4(w);
+        auto rows = [](typename O::S(&v)[R], const typename O::S *p) {
+            if constexpr (O::FOLD) {
+#pragma unroll
+                for (int k = 0; k < R; k++) v[k] = O::table(p + k);  // rows past the last read the next entry; their sums are dropped
+            } else {
+                static_assert(R == 4, "four rows a load");
+                const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
+                v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+            }
+        };
         const typename O::V *x = X + (O::FOLD ? r0 : n * n) * TC + c;
         const int dx = minus ? -TC : TC;
         typename O::V acc[R];
         typename O::S hn[R];
 #pragma unroll
-        for (int k = 0; k < R; k++) {
-            acc[k] = O::zero();
-            hn[k] = O::table(h + k);  // rows past the last read the next entry; their sums are dropped
-        }
+        for (int k = 0; k < R; k++) acc[k] = O::zero();
+        rows(hn, h);
 #pragma unroll 4
         for (int m = 0; m < steps; m++) {
             typename O::S hc[R];
-            if (m + 1 < steps) h += w;  // the last step loads its own entries again
+            if (m + 1 < steps) h += ld;  // the last step loads its own entries again
 #pragma unroll
-            for (int k = 0; k < R; k++) {
-                hc[k] = hn[k];
-                hn[k] = O::table(h + k);
-            }
+            for (int k = 0; k < R; k++) hc[k] = hn[k];
+            rows(hn, h);
             const typename O::X xv = O::prep(O::load(x));
             x += dx;
 #pragma unroll
@@ -533,6 +547,15 @@ __global__ void own_unfold_ff_kernel(const ffv *__restrict__ in, double2 *__rest
     }
 }
 
+// whole rotation tables of the classes' representative rows rep[k] of H (see pad_off)
+__global__ void own_pad_table_kernel(int pmax, const int *__restrict__ rep, const float *__restrict__ H, float *__restrict__ out)
+{
+    const int n = blockIdx.x, k = blockIdx.y, w = 2 * n + 1, ld = pad4(w);
+    const float *Hn = H + (size_t)rep[k] * rot_size(pmax) + rot_off(n);
+    float *o = out + (size_t)k * pad_off(pmax) + pad_off(n);
+    for (int t = threadIdx.x; t < w * ld; t += blockDim.x) o[t] = t % ld < w ? Hn[t / ld * w + t % ld] : 0.f;
+}
+
 // folded rotation tables of the classes' representative rows rep[k] of H (see fold_off)
 __global__ void own_fold_table_kernel(int pmax, const int *__restrict__ rep, const double *__restrict__ H,
                                       double *__restrict__ o64, ffs *__restrict__ off2)
@@ -592,13 +615,15 @@ unsigned ew_grid(size_t n) { return (unsigned)std::max<size_t>(1, std::min<size_
 // multiply-adds (M2L of the head in float-float, 8 / 16 / 32 columns: p = 8 8.2 / 6.8 / 5.9 ms,
 // p = 10 4.0 / 3.3 / 3.1); where only 8 columns leave room for two CTAs (p = 20) 16 columns in one
 // CTA measured the same (FP64 5.08 against 5.02 ms), and 4 columns in one of two CTAs as 8 in one
-// (p = 30: 3.86 against 3.91).
-constexpr size_t TWO_CTA = 112 * 1024 + 512, ONE_CTA = 226 * 1024;
+// (p = 30: 3.86 against 3.91).  FP32 tiles stop at 76 KB: their tables, four rows a load, then keep room in
+// L1 (a deterministic matvec on 20,480 triangles 1.20 -> 1.15 ms; 40 KB: 1.25; float-float 15.05 with
+// TWO_CTA, 15.38 with 76 KB).
+constexpr size_t TWO_CTA = 112 * 1024 + 512, ONE_CTA = 226 * 1024, F32_TILE = 76 * 1024;
 
-int pick_cols(int rows, size_t elem)
+int pick_cols(int rows, size_t elem, size_t most)
 {
     for (int tc : {32, 16, 8})
-        if (2 * elem * rows * tc <= TWO_CTA) return tc;
+        if (2 * elem * rows * tc <= most) return tc;
     for (int tc : {8, 4, 2})
         if (2 * elem * rows * tc <= ONE_CTA) return tc;
     return 0;
@@ -632,7 +657,7 @@ int build_pass(Plan *P, int l, int which, OwnPass &O)
     O.pout = which == PASS_L2L ? L.p : pp;
     const int nin = std::min(O.pin, pp), nq = std::min(O.pout, pp), ndst = which == PASS_M2M ? P->lev[l - 1].nb : L.nb;
     O.rows = std::max(nin, nq) * std::max(nin, nq);
-    O.tc = pick_cols(O.rows, sizeof(C));
+    O.tc = pick_cols(O.rows, sizeof(C), std::is_same<T, float>::value ? F32_TILE : TWO_CTA);
     if (!O.tc) {
         fmm_set_error("translation order %d above 60", pp);
         return FMM_ERR_CUDA;
@@ -713,7 +738,7 @@ int build_pass(Plan *P, int l, int which, OwnPass &O)
             for (int k = 0; k < ncls; k++) {
                 const int cnt = bins[(size_t)c * ncls + k];
                 bins[(size_t)c * ncls + k] = pos;
-                const int rrow = std::is_same<T, float>::value ? key0 + rep[k] : cls0 + k;
+                const int rrow = cls0 + k;
                 for (int a = 0; a < cnt; a += O.tc)
                     items.push_back(make_int4(rrow, pos + a, std::min(O.tc, cnt - a), which == PASS_M2L ? P->dir_dist[rep[k]] : 0));
                 pos += cnt;
@@ -771,8 +796,8 @@ template <> int tables_of<ff>(Plan *P, OwnArgs<ff> &a)
 }
 template <> int tables_of<float>(Plan *P, OwnArgs<float> &a)
 {
-    a.rot = P->Hsr32;
-    a.rot_stride = rot_size(P->pmax);
+    a.rot = P->own_rot32;
+    a.rot_stride = pad_off(P->pmax);
     a.ph = P->PHsr32;
     return FMM_OK;
 }
@@ -865,24 +890,30 @@ int ensure_own(Plan *P)
         direction_classes(P, PASS_M2L, NDIR, cls, rep);
         P->own_ncls = (int)rep.size();
     }
-    if (Ops<T>::FOLD) {
-        const bool f64 = std::is_same<T, double>::value;
+    {
+        const bool f64 = std::is_same<T, double>::value, f32 = std::is_same<T, float>::value;
         std::vector<int> reps, cls, rep;
         for (int which : {PASS_M2L, PASS_M2M, PASS_L2L}) {
             const int key0 = which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8;
             direction_classes(P, which, which == PASS_M2L ? NDIR : 8, cls, rep);
             for (int r : rep) reps.push_back(key0 + r);
         }
-        const size_t n = reps.size() * (size_t)fold_size(P->pmax) + TABLE_PAD;
-        if (f64)
+        const size_t n = reps.size() * (size_t)(f32 ? pad_off(P->pmax) : fold_size(P->pmax)) + TABLE_PAD;
+        if (f32)
+            FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot32, sizeof(float) * n));
+        else if (f64)
             FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot64, sizeof(double) * n));
         else
             FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot_ff, sizeof(ffs) * n));
         int *d_rep = nullptr;
         FMM_CUDA_TRY(cudaMalloc(&d_rep, sizeof(int) * reps.size()));
         cudaError_t ce = cudaMemcpyAsync(d_rep, reps.data(), sizeof(int) * reps.size(), cudaMemcpyHostToDevice, P->stream);
-        own_fold_table_kernel<<<dim3(P->pmax, (unsigned)reps.size()), 128, 0, P->stream>>>(
-            P->pmax, d_rep, P->Hsr64, f64 ? P->own_rot64 : nullptr, f64 ? nullptr : reinterpret_cast<ffs *>(P->own_rot_ff));
+        const dim3 grid(P->pmax, (unsigned)reps.size());
+        if (f32)
+            own_pad_table_kernel<<<grid, 128, 0, P->stream>>>(P->pmax, d_rep, P->Hsr32, P->own_rot32);
+        else
+            own_fold_table_kernel<<<grid, 128, 0, P->stream>>>(P->pmax, d_rep, P->Hsr64, f64 ? P->own_rot64 : nullptr,
+                                                               f64 ? nullptr : reinterpret_cast<ffs *>(P->own_rot_ff));
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(P->stream);
         cudaFree(d_rep);
         FMM_CUDA_TRY(ce);
@@ -962,6 +993,7 @@ void free_owner(Plan *P)
     cudaFree(P->own_part);
     cudaFree(P->own_rot64);
     cudaFree(P->own_rot_ff);
+    cudaFree(P->own_rot32);
 }
 
 } // namespace fmm

@@ -253,6 +253,7 @@ struct Plan {
     int own_ready[3] = {0, 0, 0}, own_ncls = 0;
     double *own_rot64 = nullptr;  // folded rotation tables per class, FP64 and float-float
     float4 *own_rot_ff = nullptr; // (hi, hi, lo, lo) per entry
+    float *own_rot32 = nullptr;   // whole rotation tables per class, FP32 (deterministic plans)
     void *own_part = nullptr;     // translated expansions of one chunk, before their sums
     size_t own_part_bytes = 0;
     size_t device_bytes = 0;
