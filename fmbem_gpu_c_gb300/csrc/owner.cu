@@ -21,13 +21,13 @@
 // plain basis and the order of operations of the mixed tiles' predecessor, so that deterministic
 // results stay what they were bit for bit.
 //
-// What bounds it: the FP64 pipe (2 multiply-adds per clock and SM; the fine levels run at 75-80 %
-// of it), in float-float the FP32 pipes (15 instructions per multiply-add): 16 p^3 / 3
+// What bounds it: the FP64 pipe (2 multiply-adds per clock and SM; the tiles keep it 95-97 %
+// busy), in float-float the FP32 pipes (15 instructions per multiply-add): 16 p^3 / 3
 // multiply-adds per translation against 8 p^3 with the whole rotation block.  Measured against one
 // CTA per destination box, which took its translations one after another with a lane per
 // output: FP64 matvec on the 81,920-triangle sphere (p = 40 .. 10) 69.7 -> 27.3 ms (level-6 M2L
 // 23.5 -> 8.4), float-float on the 200,000-triangle head (p = 40 .. 8) 30.1 -> 15.1 ms,
-// deterministic mixed on the 20,480-triangle sphere 2.36 -> 1.26 ms.
+// deterministic mixed on the 20,480-triangle sphere 2.36 -> 1.14 ms.
 #include "plan.h"
 #include "ff.cuh"
 #include "f32x2.cuh"

@@ -41,7 +41,7 @@ struct Tc3 {
 // so the class's directions differ only by their azimuthal phases, which the kernel applies
 // to each row.  M2M / L2L: one operator per octant.  Real-embedded and split into TF32 hi/lo
 // parts in the layout the MMA reads.
-constexpr int TC_MAXCH = 40, TC_MAXPIECE = 10, TC_MAXSUB = 4;
+constexpr int TC_MAXCH = 40, TC_MAXPIECE = 12, TC_MAXSUB = 4;
 constexpr int TC_PAD = 256;
 
 // Output degrees [beg, end) of a dense pass: MMA widths of the sums' and differences' blocks, offset of
@@ -57,16 +57,16 @@ struct TcPiece {
     int c0, cnt, beg, end;
 };
 
-// An input of a dense pass: offsets of its coefficients (n, m) and (n, -m) in their piece and of the phase
-// of m, in bytes (m = TC_PAD: none).
-struct TcIn {
-    int pos, neg, m;
+// A pair of inputs of a dense pass, offsets in bytes.  Folded: its coefficients (n, m) and (n, -m) in their piece
+// and the phase of m (mn = TC_PAD: none).  Not folded: two coefficients and their phases.
+struct alignas(16) TcIn {
+    int pos, neg, m, mn;
 };
 
 // Shape of a dense pass (tc_dense.cu).
 struct TcShape {
     int nch, npiece, nsub;
-    int fold;                              // sums and differences of x_m, x_-m (else both as they are)
+    int fold;                              // sums and differences of x_m, x_-m (else the coefficients as they are)
     int sets, setw, nst;                   // sets of accumulators and their TMEM columns; stages
     int bstage, row_stride, epi_stride;    // bytes of a stage's operator, of a source row's piece, of a staged row
     int cls_floats;                        // operator of a class

@@ -15,8 +15,8 @@
 //     D[t][o] = sum_k A[t][k] B[o][k],   A = sums (differences) of the phased source, re and im,
 //                                         B = the block, embedded as a real matrix,
 // and the epilogue turns sums and differences back into m and -m and applies e^{-i m' phi} of the
-// row's own direction.  (Levels with fewer translations keep x_m and x_-m as the two operands
-// and all four blocks, fold_pays().)  Split TF32 (3 products hi*hi + hi*lo + lo*hi of rounded 11-bit halves)
+// row's own direction.  (Levels with fewer translations keep the whole operator, a chunk's first and last four
+// coefficients as the two operands, fold_pays().)  Split TF32 (3 products hi*hi + hi*lo + lo*hi of rounded 11-bit halves)
 // gives close to FP32 accuracy.
 //
 // A persistent, warp-specialised kernel (one CTA per SM, 20 warps) runs over the tiles
@@ -96,8 +96,9 @@ static size_t tc_smem_bytes(const TcShape &g)
 }
 
 // The pass's shape for source order pin and destination order pout.
-// Inputs: the pairs (n, m >= 0), degree by degree, in pieces of whole degrees (a row's copy), each
-// piece in chunks of four; the cut with the fewest chunks.
+// Inputs, folded: the pairs (n, m >= 0), degree by degree, in pieces of whole degrees (a row's copy), each
+// piece in chunks of four; the cut with the fewest chunks.  Not folded: the coefficients in their order,
+// eight a chunk (two steps of the MMA's K one after another).
 // Outputs: ranges of degrees, each two blocks of MMA columns (rounded up to 16, at most 256).  Where
 // all degrees take at most 208 columns (p <= 10), two sets of accumulators and three A stages fit
 // into the 512 of TMEM, and the epilogue overlaps the next tile's MMAs; beyond, one set of up to 416 columns
@@ -148,20 +149,35 @@ static bool tc_shape(int pin, int pout, int fold, TcShape &g)
     static const int sizes[][2] = {{53, 36}, {53, 32}, {36, 36}, {36, 32}, {31, 31}};  // a degree of p <= 16 has up to 31
     for (auto &size : sizes) {
         const int piece = size[0], group = size[1];
-        cut(pin, [&](int a, int b) { return b * b - a * a > piece ? -1 : 64 * ((tri(b) - tri(a) + 3) / 4) + 1; }, at);
+        g.nch = g.row_stride = 0;
+        if (fold) {
+            cut(pin, [&](int a, int b) { return b * b - a * a > piece ? -1 : 64 * ((tri(b) - tri(a) + 3) / 4) + 1; }, at);
+        } else {  // runs of whole chunks
+            at.clear();
+            for (int c = 0; c < pin * pin; c += piece / 8 * 8) at.push_back(c);
+            at.push_back(pin * pin);
+        }
         g.npiece = (int)at.size() - 1;
         if (g.npiece > TC_MAXPIECE) continue;
-        g.nch = g.row_stride = 0;
         for (int i = 0; i < g.npiece; i++) {
-            const int a = at[i], b = at[i + 1], nc = (tri(b) - tri(a) + 3) / 4;
-            g.piece[i] = {a * a, b * b - a * a, g.nch, g.nch + nc};
-            g.row_stride = std::max(g.row_stride, tc_stride(b * b - a * a));
+            const int a = at[i], b = at[i + 1], c0 = fold ? a * a : a, cnt = fold ? b * b - c0 : b - a;
+            const int nc = fold ? (tri(b) - tri(a) + 3) / 4 : (cnt + 7) / 8;
+            g.piece[i] = {c0, cnt, g.nch, g.nch + nc};
+            g.row_stride = std::max(g.row_stride, tc_stride(cnt));
             if (g.nch + nc > TC_MAXCH) return false;
             int k = 4 * g.nch;
-            for (int n = a; n < b; n++)
-                for (int m = 0; m <= n; m++) g.tab[k++] = {8 * (n * n + n + m - a * a), 8 * (n * n + n - m - a * a), 8 * m};
+            if (fold) {
+                for (int n = a; n < b; n++)
+                    for (int m = 0; m <= n; m++) g.tab[k++] = {8 * (n * n + n + m - c0), 8 * (n * n + n - m - c0), 8 * m, 0};
+                while (k < 4 * (g.nch + nc)) g.tab[k++] = {0, 0, 0, TC_PAD};  // coefficient 0 of the piece against a zero operator
+            } else {
+                for (; k < 4 * (g.nch + nc); k++) {
+                    const int lo = 8 * (k / 4) + k % 4, hi = lo + 4;
+                    auto order = [](int i) { int n = 0; while ((n + 1) * (n + 1) <= i) n++; return i - n * n - n; };
+                    g.tab[k] = {lo < b ? 8 * (lo - c0) : 0, hi < b ? 8 * (hi - c0) : 0, lo < b ? 8 * order(lo) : 0, hi < b ? 8 * order(hi) : 0};
+                }
+            }
             g.nch += nc;
-            while (k < 4 * g.nch) g.tab[k++] = {0, 0, TC_PAD};  // coefficient 0 of the piece against a zero operator
         }
         g.epi_stride = tc_stride(group);
         for (int i = 0; i < g.nsub; i++) {
@@ -486,12 +502,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
                 if (!ok) break;
                 const unsigned char *x = rows + (size_t)(rr.i * TC_M + r) * sh.row_stride + 8 * ((base + c0) & 1);
                 // the coefficients and phases of a chunk are read before the one before it is stored
-                float2 f[4], xp[4], xm[4];
+                float2 f[4], xp[4], xm[4], fm[FOLD ? 1 : 4];
                 auto load = [&](int c) {
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         const TcIn &w = sh.tab[4 * c + j];
-                        f[j] = __ldg(reinterpret_cast<const float2 *>(ph + (w.m & 0xff)));
+                        f[j] = __ldg(reinterpret_cast<const float2 *>(ph + w.m));
+                        if constexpr (!FOLD) fm[j] = __ldg(reinterpret_cast<const float2 *>(ph + w.mn));
                         xp[j] = *reinterpret_cast<const float2 *>(x + w.pos);
                         xm[j] = *reinterpret_cast<const float2 *>(x + w.neg);
                     }
@@ -508,9 +525,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
                             const float sr = xp[j].x + xm[j].x, si = xp[j].y + xm[j].y, dr = xp[j].x - xm[j].x, di = xp[j].y - xm[j].y;
                             s[0] = sr * f[j].x - di * f[j].y, s[1] = si * f[j].x + dr * f[j].y;
                             s[2] = dr * f[j].x - si * f[j].y, s[3] = di * f[j].x + sr * f[j].y;
-                        } else {  // x_m e, x_-m e*
+                        } else {
                             s[0] = xp[j].x * f[j].x - xp[j].y * f[j].y, s[1] = xp[j].x * f[j].y + xp[j].y * f[j].x;
-                            s[2] = xm[j].x * f[j].x + xm[j].y * f[j].y, s[3] = xm[j].y * f[j].x - xm[j].x * f[j].y;
+                            s[2] = xm[j].x * fm[j].x - xm[j].y * fm[j].y, s[3] = xm[j].x * fm[j].y + xm[j].y * fm[j].x;
                         }
 #pragma unroll
                         for (int k = 0; k < 4; k += 2) {
@@ -634,7 +651,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
 
 // The blocks of a class's operator T, embedded as real matrices and split into TF32 hi / lo, in
 // the order of the copies: class, output range, chunk, (sums hi, lo, differences hi, lo; without the
-// fold outputs m hi, lo, outputs -m hi, lo of the inputs m, then of the inputs -m) in the core-matrix layout.  With P = x_m + x_-m, Q = x_m - x_-m of the inputs and y_+-m = S +- D of the
+// fold outputs m hi, lo, outputs -m hi, lo of a chunk's first four inputs, then of its other four) in the core-matrix layout.  With P = x_m + x_-m, Q = x_m - x_-m of the inputs and y_+-m = S +- D of the
 // outputs:  S = sum (T_m'm + T_m'-m) / 2 P (half of that for m = 0, where P = 2 x_0),
 // D = sum (T_m'm - T_m'-m) / 2 Q.
 // fout / fin (plans with scaled FP32 expansions, else null): per-degree factors of the
@@ -659,8 +676,9 @@ __global__ void tc_split_kernel(const double2 *__restrict__ T, int pin, int pout
         int n = s.beg, j = o / 2;
         while (n < s.end && j > n - second) j -= n + 1 - second, n++;
         double v = 0.0;
-        if (n < s.end && w.m != TC_PAD) {
-            const int m = j + second, ip = c0 + w.pos / 8, im = c0 + w.neg / 8;
+        const int in = 8 * c + 4 * part + k / 2;  // (not folded) the coefficient
+        if (n < s.end && (sh.fold ? w.mn != TC_PAD : in < P2i)) {
+            const int m = j + second, ip = sh.fold ? c0 + w.pos / 8 : in, im = c0 + w.neg / 8;
             const double2 *row_m = T + ((size_t)cls * P2o + n * n + n + m) * P2i, *row_n = T + ((size_t)cls * P2o + n * n + n - m) * P2i;
             double2 t;
             if (sh.fold) {
@@ -668,7 +686,7 @@ __global__ void tc_split_kernel(const double2 *__restrict__ T, int pin, int pout
                 t = second ? make_double2(h * (row_m[ip].x - row_m[im].x), h * (row_m[ip].y - row_m[im].y))
                            : make_double2(h * (row_m[ip].x + row_m[im].x), h * (row_m[ip].y + row_m[im].y));
             } else {
-                t = part && ip == im ? make_double2(0.0, 0.0) : (second ? row_n : row_m)[part ? im : ip];
+                t = (second ? row_n : row_m)[in];
             }
             v = (o & 1) == 0 ? ((k & 1) == 0 ? t.x : -t.y) : ((k & 1) == 0 ? t.y : t.x);
             if (fout) v *= fout[n] * fin[(int)sqrtf((float)ip + 0.5f)];
@@ -699,10 +717,11 @@ static RcrList *dense_list(Plan *P, int l, int which, int &pin, int &pout)
 // Levels that run on sums and differences (T translations).  The fold halves the products and their rounding
 // errors; at 100,000 translations and more it takes 0.45 against 0.51 ms (p = 14, 192,528 translations, one
 // column) and less with more columns (17.5 against 19.5 ms for 16).  On smaller levels the
-// gain is 10 to 20 us a pass (p = 12, 29,590 translations: 57 against 78 us with the level before it), and refined
+// gain is 10 to 20 us a pass, and refined
 // solves, which run on bodies of that size, would stop at other steps: their stopping test sees the
 // operator's error, and solutions would move by more than they differ from run to run (adjoint of a 5,120-triangle body
-// at tol = 1e-8: 4e-9 against 1e-9).
+// at tol = 1e-8: 4e-9 against 1e-9).  The whole operator sums its products in the coefficients' order, eight at a
+// time, hi hi, hi lo, lo hi, as it always has.
 static bool fold_pays(int T) { return T >= 100000; }
 
 static int build_tc_dense(Plan *P, int l, int which)
