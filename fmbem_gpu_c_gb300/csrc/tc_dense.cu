@@ -982,14 +982,22 @@ int check_tc_error(Plan *P)
     return FMM_OK;
 }
 
-// M2L levels that run dense (order p <= 16, T translations).  Large levels: the dense form is the
-// faster one (16 columns on the 81,920-triangle sphere: p = 10, 650,304 translations 3.2 ms against
-// 9.3 on the SIMT tiles; p = 14, 192,528 translations 2.8 against 6.0).  Small ones are even (6 to 8
-// thousand translations: 10 to 60 us either way); a plan keeps the form there that its timing used to
-// choose, so that its rounding (TF32 halves against FP32) stays the same: dense from 2,000
-// translations on at p = 6..14 and from 10,000 on at p = 15, 16 (tiles of 128 columns of one of 61
-// classes, which fewer translations do not fill).
-static bool dense_pays(int p, int T) { return p < 6 ? T >= 20000 : p <= 14 ? T >= 2000 : T >= 10000; }
+// M2L levels that run dense (order p <= 16, T translations, nb boxes).  Large levels: the dense form is the faster
+// one (16 columns on the 81,920-triangle sphere: p = 10, 650,304 translations 3.2 ms against 9.3 on the SIMT
+// tiles; p = 14, 192,528 translations 2.8 against 6.0).  Small ones: the SIMT tiles are, by little (one column, tiles
+// against dense: T = 2,504 p = 9 12 against 18 us, p = 14 18 against 24; T = 10,592 p = 9 18 against 20, p = 14 37
+// against 41, p = 16 45 against 59).  The line lies where slower tiles used to lose: a level keeps
+// its form and with it its rounding (TF32 halves against FP32), since a body's results
+// would move by up to eleven times what two runs differ by (44 columns on a 3,380-triangle sphere, orders 18, 16).
+// Dense from 2,000 translations on at p = 6..14 (at p = 11, 13, 14 from 4,000 on where they spread over more than
+// the 64 boxes of level 2: thin bodies, few directions with many translations each), from 10,000 on at p = 15 and
+// 9,500 at p = 16.
+static bool dense_pays(int p, int T, int nb)
+{
+    if (p < 6) return T >= 20000;
+    if (p == 11 || p == 13 || p == 14) return T >= (nb > 64 ? 4000 : 2000);
+    return T >= (p <= 14 ? 2000 : p == 15 ? 10000 : 9500);
+}
 
 // Builds the dense split operators of the passes that run on the tensor cores: the M2L levels of
 // order <= 16 that dense_pays() names.  FMMBEM_TENSOR_M2L (M2L) and FMMBEM_TENSOR_M2M (M2M and
@@ -1009,7 +1017,7 @@ int tune_tc_dense(Plan *P)
             int pin = 0, pout = 0;
             RcrList *Lst = dense_list(P, l, which, pin, pout);
             if (!Lst || Lst->key_beg.empty() || Lst->key_beg.back() == 0) continue;
-            if (mode != 1 && !dense_pays(pin, Lst->key_beg.back())) continue;
+            if (mode != 1 && !dense_pays(pin, Lst->key_beg.back(), P->lev[l].nb)) continue;
             int rc = ensure_tc_err(P);
             if (rc == FMM_OK) rc = build_tc_dense(P, l, which);
             if (rc) return rc;
