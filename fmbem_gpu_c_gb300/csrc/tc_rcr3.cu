@@ -547,7 +547,6 @@ static inline void t3_put(float *tab, long long base, int Npad, int o, int k, do
     tab[t + (long long)Npad * T3_KC + core_off(o, kc, T3_KC) / 4] = lo;
 }
 
-// polar-angle class of every key (direction or octant) of a pass
 int build_tc3(Plan *P, int l, int which)
 {
     RcrPass ps;
@@ -853,51 +852,38 @@ static void t3_free(Plan *P, Tc3 &t)
     t = Tc3();
 }
 
-// Plan-time choice per batched pass: the three-stage tensor-core form where it beats the
-// pass's current form (SIMT tiles, or the dense tensor-core M2L) on this plan, timed with one
-// right-hand side.  FMMBEM_TC3=0 keeps the current forms, FMMBEM_TC3=1 takes the three-stage
-// form wherever it applies.
+// Passes that run in three tensor-core stages, by order (p of the parents, pc of the boxes) and number of boxes:
+// the M2M of high orders on levels of few boxes, which fill few SIMT tiles, and the L2L of the highest.  The
+// line lies where slower tiles used to lose: at p = 40 with 272 boxes the stages take 54 us, the tiles 36 now (at
+// p = 44 and beyond the stages are the faster ones), but their TF32 halves are the largest part of a large body's
+// rounding, and its results would move by up to 4.5 times what two runs differ by (57 columns on a
+// 35,280-triangle body, orders 40, 30, 20, 14).
+static bool tc3_pays(int which, int p, int pc, int nb)
+{
+    if (which == PASS_M2M) return p >= (nb <= 250 ? 33 : nb <= 350 ? 36 : 43);
+    if (which == PASS_L2L) return nb <= 250 ? p >= 38 && pc >= 32 : p >= 48;
+    return false;
+}
+
+// Builds the three-stage form of the passes that tc3_pays() names.  FMMBEM_TC3=0: of none, 1: of all whose orders
+// allow it.
 int tune_tc3(Plan *P)
 {
     const char *env = getenv("FMMBEM_TC3");
     const int mode = env ? atoi(env) : -1;
     if (mode == 0) return FMM_OK;
-    if (int rc = ensure_tc_err(P)) return rc;
-    cudaEvent_t a, b;
-    FMM_CUDA_TRY(cudaEventCreate(&a));
-    FMM_CUDA_TRY(cudaEventCreate(&b));
-    int rc = FMM_OK;
-    for (int l = P->lmin; l <= P->lmax && rc == FMM_OK; l++) {
-        for (int which = PASS_M2M; which <= PASS_L2L && rc == FMM_OK; which++) {
+    for (int l = P->lmin; l <= P->lmax; l++)
+        for (int which = PASS_M2M; which <= PASS_L2L; which++) {
             RcrPass ps;
             RcrList *Lst = pass32_desc(P, l, which, 1, ps);
             if (!Lst || Lst->key_beg.empty() || Lst->key_beg.back() == 0) continue;
-            rc = build_tc3(P, l, which);
-            if (rc || !Lst->t3.built) break;
-            float ms[2] = {0.f, 0.f};
-            for (int on = 0; on < 2 && rc == FMM_OK && mode != 1; on++) {
-                Lst->t3.on = on;
-                for (int rep = 0; rep < 4 && rc == FMM_OK; rep++) {
-                    if (cudaEventRecord(a, P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    if (rc == FMM_OK) rc = launch_pass32(P, l, which, 1, P->stream);
-                    if (rc == FMM_OK && cudaEventRecord(b, P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    if (rc == FMM_OK && cudaEventSynchronize(b) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    float t = 0.f;
-                    cudaEventElapsedTime(&t, a, b);
-                    if (rep > 0) ms[on] += t;
-                }
-            }
-            if (rc == FMM_OK && cudaStreamSynchronize(P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
-            if (rc == FMM_OK) rc = check_tc_error(P);
-            if (rc) break;
-            Lst->t3.on = (mode == 1 || ms[1] < ms[0]) ? 1 : 0;
-            if (!Lst->t3.on) t3_free(P, Lst->t3);
+            if (mode != 1 && !tc3_pays(which, ps.p, P->lev[l].p, P->lev[l].nb)) continue;
+            int rc = ensure_tc_err(P);
+            if (rc == FMM_OK) rc = build_tc3(P, l, which);
+            if (rc) return rc;
+            Lst->t3.on = Lst->t3.built;
         }
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    if (rc == FMM_ERR_CUDA && !fmm_last_error()[0]) fmm_set_error("three-stage tensor-core tuning: %s", cudaGetErrorString(cudaGetLastError()));
-    return rc;
+    return FMM_OK;
 }
 
 } // namespace fmm

@@ -101,8 +101,8 @@ typedef struct {
                                             (tcgen05, split TF32: rotation, coaxial, rotation GEMMs over the
                                             translations that share each operator) -- bit 0 the M2M from
                                             level l into l-1, bit 1 the M2L of level l, bit 2 the L2L from
-                                            l-1 into l; chosen at plan creation by timing against the other
-                                            forms (FMMBEM_TC3=0: never, 1: wherever the order allows) */
+                                            l-1 into l; by order and number of boxes
+                                            (FMMBEM_TC3=0: never, 1: wherever the order allows) */
     int pass_dense[FMM_MAX_LEVEL + 1];   /* mixed path: passes of level l run as one dense tensor-core GEMM
                                             per operator (tcgen05, split TF32; source and destination
                                             orders <= 16), same bits as pass_tc3 (bit 1 = m2l_tensor);

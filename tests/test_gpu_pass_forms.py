@@ -23,3 +23,16 @@ def test_dense_levels(fm):
     assert 2000 < plan_info(fm, thin, 3, {2: 14, 3: 14}).num_m2l[3] < 4000
     for p, on in ((11, 0), (12, 1), (13, 0), (14, 0)):
         assert plan_info(fm, thin, 3, {2: p, 3: p}).m2l_tensor[3] == on, p
+
+
+@pytest.mark.parametrize("p2,p3,bits", [(32, 24, 0), (33, 25, 1), (34, 31, 1), (40, 30, 1), (38, 34, 5), (44, 33, 5)])
+def test_three_stage_levels(fm, p2, p3, bits):
+    info = plan_info(fm, fm.geodesic_sphere(8, 0.1), 3, {2: p2, 3: p3})
+    assert info.num_box[3] == 248
+    assert [info.pass_tc3[l] for l in (2, 3)] == [0, bits]
+
+
+def test_three_stage_larger_levels(fm):
+    info = plan_info(fm, fm.geodesic_sphere(16, 0.1), 4, {2: 40, 3: 30, 4: 22})
+    assert info.num_box[3] == 272
+    assert [info.pass_tc3[l] for l in (2, 3, 4)] == [0, 1, 0]
