@@ -20,6 +20,8 @@
 // the class's tables.  Every output is summed in the same order whatever the tile.  Destinations
 // are added with FP32 vector atomics where several items reach the same box (M2M, M2L), and with a
 // plain read-add-write where every box is reached once (L2L).
+// Small bodies with many columns take another form of the tiles (FORM_WHOLE, tile_form()): one direction each, the
+// rotations whole, every product and sum rounded as by one thread per row of the plain basis.
 //
 // What bounds it: the shared-memory / L1 path (16 bytes of table and 32 of operands per lane for 32
 // multiply-adds: 65-80 % busy at p = 10-20) and, at p = 30-40, the latency of table rows from L2.
@@ -108,9 +110,10 @@ template <bool S, class T> __device__ __forceinline__ T entry(const T *p)
 }
 
 // One rotation stage, in place.  Round k gives thread t unit k UC + t / CL and the
-// column pairs cl, cl + CL (cl = t % CL): (n | sign << 8 | first row << 16, table offset), R rows of P_n or Q_n.  All
-// units of a block (n, sign) are in one round, which writes after everyone has read.
-template <int TC, int R, bool S>
+// column pairs cl, cl + CL (cl = t % CL): (n | sign << 8 | first row << 16, table offset), R rows of P_n or Q_n
+// (whole rotations: of H_n, no sign).  All units of a block (n, sign) are in one round, which writes after everyone
+// has read.
+template <int TC, int R, bool S, bool FOLD>
 __device__ __forceinline__ void rot_stage(const float *__restrict__ rot, ulonglong2 *X, const int2 *__restrict__ units, int rounds)
 {
     constexpr int CL = TC / CG, UC = THREADS / CL, NC = CG / 2;
@@ -119,7 +122,7 @@ __device__ __forceinline__ void rot_stage(const float *__restrict__ rot, ulonglo
         const int2 info = __ldg(units + k * UC + ul);
         const bool on = info.x >= 0;
         const int n = on ? info.x & 255 : 0, minus = on ? (info.x >> 8) & 1 : 0, row0 = on ? info.x >> 16 : 0;
-        const int steps = on ? (minus ? n : n + 1) : 0, ld = up_to(minus ? n : n + 1, 4), c0 = n * n + n;
+        const int len = FOLD ? (minus ? n : n + 1) : 2 * n + 1, steps = on ? len : 0, ld = up_to(len, 4), c0 = FOLD ? n * n + n : n * n;
         const float *h = rot + info.y;
         f2 acc[R][CG];
 #pragma unroll
@@ -165,8 +168,8 @@ __device__ __forceinline__ void rot_stage(const float *__restrict__ rot, ulonglo
 }
 
 // The coaxial stage, in place, in rounds as above.  Unit: |m| | sign << 8 | first row << 16, two of
-// the rows of order +-m.
-template <int TC, bool S>
+// the rows of order +-m.  Folded: the products with re(c) and im(c) in sums of their own; else one sum.
+template <int TC, bool S, bool FOLD>
 __device__ __forceinline__ void coax_stage(int p, int nin, int nq, const float2 *__restrict__ Cc, ulonglong2 *X,
                                            const int *__restrict__ units, int rounds)
 {
@@ -198,15 +201,20 @@ __device__ __forceinline__ void coax_stage(int p, int nin, int nq, const float2 
             for (int i = 0; i < NC; i++) x[i] = xr[(cl + i * CL) ^ s];
             row += dr;
             dr += 2;
-            const f2 re[2] = {f2_pack(cc.x, cc.x), f2_pack(cc.z, cc.z)}, im[2] = {f2_pack(cc.y, cc.y), f2_pack(cc.w, cc.w)};
+            const f2 re[2] = {f2_pack(cc.x, cc.x), f2_pack(cc.z, cc.z)}, im[2] = {f2_pack(FOLD ? cc.y : -cc.y, cc.y), f2_pack(FOLD ? cc.w : -cc.w, cc.w)};
 #pragma unroll
             for (int r = 0; r < 2; r++) {
 #pragma unroll
                 for (int i = 0; i < NC; i++) {
                     a0[r][2 * i] = f2_fma(re[r], x[i].x, a0[r][2 * i]);
                     a0[r][2 * i + 1] = f2_fma(re[r], x[i].y, a0[r][2 * i + 1]);
-                    a1[r][2 * i] = f2_fma(im[r], x[i].x, a1[r][2 * i]);
-                    a1[r][2 * i + 1] = f2_fma(im[r], x[i].y, a1[r][2 * i + 1]);
+                    if constexpr (FOLD) {
+                        a1[r][2 * i] = f2_fma(im[r], x[i].x, a1[r][2 * i]);
+                        a1[r][2 * i + 1] = f2_fma(im[r], x[i].y, a1[r][2 * i + 1]);
+                    } else {
+                        a0[r][2 * i] = f2_fma(im[r], f2_swap(x[i].x), a0[r][2 * i]);
+                        a0[r][2 * i + 1] = f2_fma(im[r], f2_swap(x[i].y), a0[r][2 * i + 1]);
+                    }
                 }
             }
         }
@@ -218,8 +226,11 @@ __device__ __forceinline__ void coax_stage(int p, int nin, int nq, const float2 
                 f2 y[CG];
 #pragma unroll
                 for (int j = 0; j < CG; j++) {
-                    const float2 v = f2_parts(a0[r][j]), w = f2_parts(a1[r][j]);
-                    y[j] = f2_pack(v.x - w.y, v.y + w.x);
+                    y[j] = a0[r][j];
+                    if constexpr (FOLD) {
+                        const float2 v = f2_parts(a0[r][j]), w = f2_parts(a1[r][j]);
+                        y[j] = f2_pack(v.x - w.y, v.y + w.x);
+                    }
                 }
 #pragma unroll
                 for (int i = 0; i < NC; i++)
@@ -228,18 +239,29 @@ __device__ __forceinline__ void coax_stage(int p, int nin, int nq, const float2 
     }
 }
 
+// v e and conj(e) v, each product and sum rounded in one fixed way
+__device__ __forceinline__ float2 phase_mul(float2 v, float2 e)
+{
+    return make_float2(__fmaf_rn(v.x, e.x, -__fmul_rn(v.y, e.y)), __fmaf_rn(v.y, e.x, __fmul_rn(v.x, e.y)));
+}
+__device__ __forceinline__ float2 conj_phase_mul(float2 e, float2 v)
+{
+    return make_float2(__fmaf_rn(e.x, v.x, __fmul_rn(e.y, v.y)), __fmaf_rn(e.x, v.y, -__fmul_rn(e.y, v.x)));
+}
+
 // One tile: item it = (class, first column, count, coaxial table) of pass ps, with the
 // CTA's dynamic shared memory and its column indices.  S: the class's rotation table and the
 // coaxial table are copied to shared memory behind the tile (ps.tile_words 16-byte words) while the
 // columns are gathered.  Each step of a stage waits for its table entries; in a pass of so few tiles that each SM
 // has one or two, nothing hides their way from the L2.
-template <int TC, int R, bool S>
+// FOLD = false: the rotations whole, in the plain basis, and each product and sum rounded in one fixed way.
+template <int TC, int R, bool S, bool FOLD>
 __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float4 *smem4, int *s_src, int *s_dst, int *s_dir)
 {
     const int p = ps.p, nin = min(ps.pin, p), nq = min(ps.pout, p), cnt = it.z;
     ulonglong2 *X = reinterpret_cast<ulonglong2 *>(smem4);
     float2 *Xf = reinterpret_cast<float2 *>(X);
-    const float *rot = ps.rot + (size_t)it.x * ps.rot_stride;
+    const float *rot = ps.rot + (size_t)(FOLD ? it.x : it.x & 255) * ps.rot_stride;
     const float2 *coax = ps.coax + (size_t)it.w * coax2_sum(p);
     if constexpr (S) {
         const float4 *r4 = reinterpret_cast<const float4 *>(rot), *c4 = reinterpret_cast<const float4 *>(coax);
@@ -257,7 +279,7 @@ __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float
         const int e = it.y + min((int)threadIdx.x, cnt - 1), t = e / ps.nrhs, r = e - t * ps.nrhs;
         s_src[threadIdx.x] = ps.g_src[t] * ps.nrhs + r;
         s_dst[threadIdx.x] = ps.g_dst[t] * ps.nrhs + r;
-        s_dir[threadIdx.x] = ps.g_dir[t];
+        s_dir[threadIdx.x] = FOLD ? ps.g_dir[t] : ps.key0 + (it.x >> 8);
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -292,6 +314,11 @@ __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float
                 if (nm[j] < 0) continue;
                 const int c = (b0 + j * nw) % (TC / 4) * 4 + gc, m = nm[j] >> 16, r0 = nm[j] & 0xffff, rp = r0 + m, rm = r0 - m;
                 // m = 0: x itself (vm = 0, e = 1)
+                if constexpr (!FOLD) {
+                    Xf[rp * TC + (((c >> 1) ^ swz<TC>(rp)) << 1) + (c & 1)] = phase_mul(vp[j], e[j]);
+                    if (m > 0) Xf[rm * TC + (((c >> 1) ^ swz<TC>(rm)) << 1) + (c & 1)] = phase_mul(vm[j], make_float2(e[j].x, -e[j].y));
+                    continue;
+                }
                 const float2 a = make_float2(vp[j].x + vm[j].x, vp[j].y + vm[j].y);
                 const float2 d = make_float2(vp[j].x - vm[j].x, vp[j].y - vm[j].y);
                 Xf[rp * TC + (((c >> 1) ^ swz<TC>(rp)) << 1) + (c & 1)] =
@@ -304,11 +331,11 @@ __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float
     }
     if constexpr (S) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    rot_stage<TC, R, S>(rot, X, ps.u1, ps.n1);
+    rot_stage<TC, R, S, FOLD>(rot, X, ps.u1, ps.n1);
     __syncthreads();
-    coax_stage<TC, S>(p, nin, nq, coax, X, ps.u2, ps.n2);
+    coax_stage<TC, S, FOLD>(p, nin, nq, coax, X, ps.u2, ps.n2);
     __syncthreads();
-    rot_stage<TC, R, S>(rot, X, ps.u3, ps.n3);
+    rot_stage<TC, R, S, FOLD>(rot, X, ps.u3, ps.n3);
     __syncthreads();
     {
         const int np = nq * (nq + 1) / 2, nb = (np + 7) / 8 * (TC / 4), dstride = ps.pout * ps.pout;
@@ -321,10 +348,15 @@ __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float
             if (m > 0) {
                 const float2 v = Xf[rm * TC + (((c >> 1) ^ swz<TC>(rm)) << 1) + (c & 1)];
                 const float2 e = __ldg(ps.PHall + (size_t)s_dir[c] * ps.phstride + ps.phoff + m);
-                const float2 a = make_float2(0.5f * (yp.x + v.x), 0.5f * (yp.y + v.y));
-                const float2 d = make_float2(0.5f * (yp.x - v.x), 0.5f * (yp.y - v.y));
-                yp = make_float2(e.x * a.x + e.y * a.y, e.x * a.y - e.y * a.x);
-                ym = make_float2(e.x * d.x - e.y * d.y, e.x * d.y + e.y * d.x);
+                if constexpr (FOLD) {
+                    const float2 a = make_float2(0.5f * (yp.x + v.x), 0.5f * (yp.y + v.y));
+                    const float2 d = make_float2(0.5f * (yp.x - v.x), 0.5f * (yp.y - v.y));
+                    yp = make_float2(e.x * a.x + e.y * a.y, e.x * a.y - e.y * a.x);
+                    ym = make_float2(e.x * d.x - e.y * d.y, e.x * d.y + e.y * d.x);
+                } else {
+                    yp = conj_phase_mul(e, yp);
+                    ym = conj_phase_mul(make_float2(e.x, -e.y), v);
+                }
             }
             if (ps.atomic) {
                 atomicAdd(out + m, yp);
@@ -341,12 +373,12 @@ __device__ __forceinline__ void rcr_tile(const RcrPass &ps, const int4 it, float
     }
 }
 
-template <int TC, int R, bool S>
+template <int TC, int R, bool S, bool FOLD>
 __global__ void __launch_bounds__(THREADS, 3) rcr_tile_kernel(RcrPass ps)
 {
     extern __shared__ float4 smem4[];
     __shared__ int s_src[TC], s_dst[TC], s_dir[TC];
-    rcr_tile<TC, R, S>(ps, ps.items[blockIdx.x], smem4, s_src, s_dst, s_dir);
+    rcr_tile<TC, R, S, FOLD>(ps, ps.items[blockIdx.x], smem4, s_src, s_dst, s_dir);
 }
 
 // Persistent form for many passes at once (the translation passes of many plans, one phase
@@ -367,7 +399,7 @@ __global__ void __launch_bounds__(THREADS, 3) rcr_queue_kernel(const RcrPass *__
         __syncthreads();
         const int w = s_w;
         if (w >= n) break;
-        rcr_tile<TC, R, false>(passes[work_pass[w]], work_item[w], smem4, s_src, s_dst, s_dir);
+        rcr_tile<TC, R, false, true>(passes[work_pass[w]], work_item[w], smem4, s_src, s_dst, s_dir);
         __syncthreads();
     }
 }
@@ -517,25 +549,29 @@ static int ensure_classes(RcrList &Lst)
     return FMM_OK;
 }
 
-// Device items of a SIMT pass for nrhs right-hand sides, rebuilt when nrhs changes.
-static int ensure_items(RcrList &Lst, int nrhs, size_t ws_bytes)
+// Device items of a form of a SIMT pass for nrhs right-hand sides, rebuilt when nrhs changes.
+static int ensure_items(RcrList &Lst, int form, int nrhs, size_t ws_bytes)
 {
-    if (Lst.items_nrhs == nrhs) return FMM_OK;
-    int e = ensure_classes(Lst);
-    if (e) return e;
+    TileForm &f = Lst.form[form];
+    if (f.items_nrhs == nrhs) return FMM_OK;
     std::vector<int4> items;
-    build_items(Lst.cls, nrhs, Lst.tc, ws_bytes, true, items);
-    if (items.size() > Lst.items_cap) {
-        if (Lst.items) cudaFree(Lst.items);
-        Lst.items = nullptr;
-        Lst.items_cap = 0;
-        FMM_CUDA_TRY(cudaMalloc(&Lst.items, sizeof(int4) * items.size()));
-        Lst.items_cap = items.size();
+    if (form == FORM_FOLDED) {
+        if (int e = ensure_classes(Lst)) return e;
+        build_items(Lst.cls, nrhs, f.tc, ws_bytes, true, items);
+    } else {
+        build_items(Lst, nrhs, f.tc, ws_bytes, true, items);
+        for (int4 &it : items) it.x = Lst.cls_of_key[it.x] | it.x << 8;
     }
-    if (!items.empty())
-        FMM_CUDA_TRY(cudaMemcpy(Lst.items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice));
-    Lst.n_items = (int)items.size();
-    Lst.items_nrhs = nrhs;
+    if (items.size() > f.items_cap) {
+        if (f.items) cudaFree(f.items);
+        f.items = nullptr;
+        f.items_cap = 0;
+        FMM_CUDA_TRY(cudaMalloc(&f.items, sizeof(int4) * items.size()));
+        f.items_cap = items.size();
+    }
+    if (!items.empty()) FMM_CUDA_TRY(cudaMemcpy(f.items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice));
+    f.n_items = (int)items.size();
+    f.items_nrhs = nrhs;
     return FMM_OK;
 }
 
@@ -543,7 +579,7 @@ int rcr_list_items(RcrList &Lst, std::vector<int4> &items)
 {
     int e = ensure_classes(Lst);
     if (e) return e;
-    build_items(Lst.cls, 1, Lst.tc, 0, true, items);
+    build_items(Lst.cls, 1, Lst.form[FORM_FOLDED].tc, 0, true, items);
     return FMM_OK;
 }
 
@@ -552,17 +588,36 @@ static size_t tile_bytes(const RcrPass &ps, int tc)
     return rcr_tile_smem(std::max(std::min(ps.pin, ps.p), std::min(ps.pout, ps.p)), tc);
 }
 
-int launch_rcr_pass(const Plan *P, RcrList &Lst, RcrPass ps, cudaStream_t st)
+// The form of the SIMT tiles for nrhs columns.  Folded rotations by class are the faster ones (27 columns on an
+// 8,820-triangle sphere 4.7 ms against 5.2, 49 on a 4,500-triangle ellipsoid 4.7 against 6.2; one tile per
+// direction with two buffers and units over the whole block took 6.4 and 7.3), but add a box's translations in
+// an order of their own: two runs of many columns on a small body differ by 2e-8 where directions one after
+// another, with several tiles each, differ by 5e-9, and the results move by four to ten times that.  So from
+// 16 columns on, bodies of fewer than 100,000 translations keep whole rotations
+// and the order of directions; with fewer columns, and on larger bodies, whose orders are no more
+// reproducible one way than the other, the results differ by what two runs differ by.
+static int tile_form(const Plan *P, int nrhs)
+{
+    long long T = 0;
+    for (int l = P->lmin; l <= P->lmax; l++) T += P->lev[l].num_sr;
+    return nrhs >= 16 && T < 100000 ? FORM_WHOLE : FORM_FOLDED;
+}
+
+int launch_rcr_pass(Plan *P, RcrList &Lst, RcrPass ps, cudaStream_t st)
 {
     if (Lst.key_beg.empty() || Lst.key_beg.back() == 0) return FMM_OK;
-    if (int e = set_tile_tables(P, Lst, ps)) return e;
+    const int form = tile_form(P, ps.nrhs);
+    if (form == FORM_WHOLE)
+        if (int e = ensure_whole_tables(P)) return e;
+    TileForm &f = Lst.form[form];
+    if (int e = set_tile_tables(P, Lst, form, ps)) return e;
     {
         size_t ws = ((size_t)ps.nsrc * ps.pin * ps.pin + (size_t)ps.ndst * ps.pout * ps.pout) * sizeof(float2) * ps.nrhs;
-        int e = ensure_items(Lst, ps.nrhs, ws);
+        int e = ensure_items(Lst, form, ps.nrhs, ws);
         if (e) return e;
     }
-    ps.items = Lst.items;
-    const size_t sm = tile_bytes(ps, Lst.tc);
+    ps.items = f.items;
+    const size_t sm = tile_bytes(ps, f.tc);
     ps.tile_words = (int)(sm / 16);
     ps.rot_words = rot32_size(ps.p) / 4;
     const size_t sm_tab = sm + (size_t)ps.rot_words * 16 + (size_t)coax2_size(ps.p) * sizeof(float2);
@@ -575,14 +630,15 @@ int launch_rcr_pass(const Plan *P, RcrList &Lst, RcrPass ps, cudaStream_t st)
     // tables in shared memory where every tile is resident at once all the same, three CTAs of up to 74 KB on an
     // SM (a matvec on 5,120 triangles, orders 16, 14, 12: 198 us without, 179 with; larger tables, 81,920
     // triangles with orders up to 40: no gain)
-    const bool staged = sm_tab <= 74 * 1024 && Lst.n_items <= 3 * nsm;
-    return with_tile(Lst.tc, Lst.bal, [&](auto t) -> int {
+    const bool staged = form == FORM_FOLDED && sm_tab <= 74 * 1024 && f.n_items <= 3 * nsm;
+    return with_tile(f.tc, f.bal, [&](auto t) -> int {
         using T = decltype(t);
-        static size_t attr[2] = {0, 0};
-        const auto kernel = staged ? rcr_tile_kernel<T::TC, T::R, true> : rcr_tile_kernel<T::TC, T::R, false>;
-        int e = raise_smem_limit((const void *)kernel, staged ? sm_tab : sm, &attr[staged]);
+        static size_t attr[3] = {0, 0, 0};
+        const auto kernel = form == FORM_WHOLE ? rcr_tile_kernel<T::TC, T::R, false, false>
+                            : staged ? rcr_tile_kernel<T::TC, T::R, true, true> : rcr_tile_kernel<T::TC, T::R, false, true>;
+        int e = raise_smem_limit((const void *)kernel, staged ? sm_tab : sm, &attr[form == FORM_WHOLE ? 2 : staged]);
         if (e) return e;
-        kernel<<<Lst.n_items, 256, staged ? sm_tab : sm, st>>>(ps);
+        kernel<<<f.n_items, 256, staged ? sm_tab : sm, st>>>(ps);
         FMM_CUDA_TRY(cudaGetLastError());
         return FMM_OK;
     });
@@ -672,6 +728,38 @@ static int build_tile_tables(Plan *P)
     return FMM_OK;
 }
 
+// whole rotation tables of the classes' representative rows rep[k] of H (see whole_off)
+__global__ void whole_table_kernel(int pmax, const int *__restrict__ rep, const float *__restrict__ H, float *__restrict__ out)
+{
+    const int n = blockIdx.x, k = blockIdx.y, w = 2 * n + 1, ld = pad4(w);
+    const float *Hn = H + (size_t)rep[k] * rot_size(pmax) + rot_off(n);
+    float *o = out + (size_t)k * whole_off(pmax) + whole_off(n);
+    for (int t = threadIdx.x; t < w * ld; t += blockDim.x) o[t] = t % ld < w ? Hn[t / ld * w + t % ld] : 0.f;
+}
+
+int ensure_whole_tables(Plan *P)
+{
+    if (P->rot32_whole) return FMM_OK;
+    std::vector<int> rows, cls, rep;
+    for (int which : {PASS_M2L, PASS_M2M, PASS_L2L}) {
+        direction_classes(P, which, which == PASS_M2L ? NDIR : 8, cls, rep);
+        for (int r : rep) rows.push_back((which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8) + r);
+    }
+    int *tmp = nullptr;
+    float *tab = nullptr;
+    FMM_CUDA_TRY(cudaMalloc(&tmp, sizeof(int) * rows.size()));
+    cudaError_t ce = dev_alloc(P, (void **)&tab, sizeof(float) * (rows.size() * (size_t)whole_off(P->pmax) + TABLE_PAD));
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(tmp, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice, P->stream);
+    if (ce == cudaSuccess) {
+        whole_table_kernel<<<dim3(P->pmax, (unsigned)rows.size()), 128, 0, P->stream>>>(P->pmax, tmp, P->Hsr32, tab);
+        ce = cudaStreamSynchronize(P->stream);
+    }
+    cudaFree(tmp);
+    FMM_CUDA_TRY(ce);
+    P->rot32_whole = tab;
+    return FMM_OK;
+}
+
 // Rounds of a stage's work units: blocks (all units of one degree or order and sign) in the given
 // order, longest first, as many as fit the UC units of a round; idle places elsewhere.
 template <class U>
@@ -692,27 +780,28 @@ static int pack_rounds(const std::vector<std::vector<U>> &blocks, int UC, U idle
     return rounds;
 }
 
-// The work units of a list's tile shape, on the device (kept until the shape changes).
-static int ensure_units(const std::vector<int> &rot_off, RcrList &Lst, const RcrPass &ps)
+// The work units of a form's tile shape, on the device (kept until the shape changes).
+static int ensure_units(const std::vector<int> &rot_off, TileForm &f, bool fold, const RcrPass &ps)
 {
-    if (Lst.units_tc == Lst.tc && Lst.units_bal == Lst.bal) return FMM_OK;
-    const int UC = THREADS / (Lst.tc / CG), R = Lst.bal ? 2 : 4, nin = std::min(ps.pin, ps.p), nq = std::min(ps.pout, ps.p);
+    if (f.units_tc == f.tc && f.units_bal == f.bal) return FMM_OK;
+    const int UC = THREADS / (f.tc / CG), R = f.bal ? 2 : 4, nin = std::min(ps.pin, ps.p), nq = std::min(ps.pout, ps.p);
     std::vector<int2> ur;
     std::vector<int> uc;
     auto rot = [&](int deg) {
         std::vector<std::vector<int2>> blocks;
         for (int n = deg - 1; n >= 0; n--)
-            for (int sg = 0; sg < 2; sg++) {
-                const int nr = sg ? n : n + 1, base = rot_off[n] + (sg ? (n + 1) * up_to(n + 1, 4) : 0);
+            for (int sg = 0; sg < (fold ? 2 : 1); sg++) {
+                const int nr = !fold ? 2 * n + 1 : sg ? n : n + 1;
+                const int base = fold ? rot_off[n] + (sg ? (n + 1) * up_to(n + 1, 4) : 0) : whole_off(n);
                 std::vector<int2> b;
                 for (int r = 0; r < nr; r += R) b.push_back(make_int2(n | sg << 8 | r << 16, base + r));
                 blocks.push_back(b);
             }
         return pack_rounds(blocks, UC, make_int2(-1, 0), ur);
     };
-    Lst.n1 = rot(nin);
-    Lst.at3 = ur.size();
-    Lst.n3 = rot(nq);
+    f.n1 = rot(nin);
+    f.at3 = ur.size();
+    f.n3 = rot(nq);
     std::vector<std::vector<int>> blocks;
     for (int am = 0; am < nq; am++)
         for (int sg = 0; sg < (am ? 2 : 1); sg++) {
@@ -720,40 +809,43 @@ static int ensure_units(const std::vector<int> &rot_off, RcrList &Lst, const Rcr
             for (int r = 0; r < nq - am; r += 2) b.push_back(am | sg << 8 | r << 16);
             blocks.push_back(b);
         }
-    Lst.n2 = pack_rounds(blocks, UC, -1, uc);
-    cudaFree(Lst.urot);
-    cudaFree(Lst.ucoax);
-    Lst.urot = nullptr;
-    Lst.ucoax = nullptr;
-    Lst.units_tc = 0;
-    FMM_CUDA_TRY(cudaMalloc(&Lst.urot, sizeof(int2) * ur.size()));
-    FMM_CUDA_TRY(cudaMalloc(&Lst.ucoax, sizeof(int) * uc.size()));
-    FMM_CUDA_TRY(cudaMemcpy(Lst.urot, ur.data(), sizeof(int2) * ur.size(), cudaMemcpyHostToDevice));
-    FMM_CUDA_TRY(cudaMemcpy(Lst.ucoax, uc.data(), sizeof(int) * uc.size(), cudaMemcpyHostToDevice));
-    Lst.units_tc = Lst.tc;
-    Lst.units_bal = Lst.bal;
+    f.n2 = pack_rounds(blocks, UC, -1, uc);
+    cudaFree(f.urot);
+    cudaFree(f.ucoax);
+    f.urot = nullptr;
+    f.ucoax = nullptr;
+    f.units_tc = 0;
+    FMM_CUDA_TRY(cudaMalloc(&f.urot, sizeof(int2) * ur.size()));
+    FMM_CUDA_TRY(cudaMalloc(&f.ucoax, sizeof(int) * uc.size()));
+    FMM_CUDA_TRY(cudaMemcpy(f.urot, ur.data(), sizeof(int2) * ur.size(), cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(cudaMemcpy(f.ucoax, uc.data(), sizeof(int) * uc.size(), cudaMemcpyHostToDevice));
+    f.units_tc = f.tc;
+    f.units_bal = f.bal;
     return FMM_OK;
 }
 
-// The tile kernels' tables, class order and units of a pass
-int set_tile_tables(const Plan *P, RcrList &Lst, RcrPass &ps)
+// The tile kernels' tables, order of the translations and units of a pass
+int set_tile_tables(const Plan *P, RcrList &Lst, int form, RcrPass &ps)
 {
-    int e = ensure_classes(Lst);
-    if (!e) e = ensure_units(P->rot32_off, Lst, ps);
+    TileForm &f = Lst.form[form];
+    const bool fold = form == FORM_FOLDED;
+    int e = fold ? ensure_classes(Lst) : FMM_OK;
+    if (!e) e = ensure_units(P->rot32_off, f, fold, ps);
     if (e) return e;
-    ps.rot = P->rot32 + (size_t)Lst.rot0 * P->rot32_stride;
-    ps.rot_stride = P->rot32_stride;
+    ps.rot_stride = fold ? P->rot32_stride : whole_off(P->pmax);
+    ps.rot = (fold ? P->rot32 : P->rot32_whole) + (size_t)Lst.rot0 * ps.rot_stride;
     ps.PHall = P->PHsr32;
-    ps.u1 = Lst.urot;
-    ps.n1 = Lst.n1;
-    ps.u3 = Lst.urot + Lst.at3;
-    ps.n3 = Lst.n3;
-    ps.u2 = Lst.ucoax;
-    ps.n2 = Lst.n2;
+    ps.u1 = f.urot;
+    ps.n1 = f.n1;
+    ps.u3 = f.urot + f.at3;
+    ps.n3 = f.n3;
+    ps.u2 = f.ucoax;
+    ps.n2 = f.n2;
     ps.pairs = P->pairs;
-    ps.g_src = Lst.csrc;
-    ps.g_dst = Lst.cdst;
-    ps.g_dir = Lst.cdir;
+    ps.g_src = fold ? Lst.csrc : Lst.src;
+    ps.g_dst = fold ? Lst.cdst : Lst.dst;
+    ps.g_dir = fold ? Lst.cdir : nullptr;
+    ps.key0 = Lst.key0;
     return FMM_OK;
 }
 
@@ -786,8 +878,9 @@ static int upload_list(Plan *P, RcrList &Lst, int which, const std::vector<int> 
     Lst.ndst_rank = ndst;
     Lst.key_beg.assign(cnt.begin(), cnt.end());
     Lst.key_w = key_w;
-    Lst.tc = pick_tile(p);
-    Lst.items_nrhs = 0;
+    Lst.form[FORM_FOLDED].tc = pick_tile(p);
+    // half as many: fewer directions in flight at a time, and four CTAs on an SM
+    Lst.form[FORM_WHOLE].tc = std::max(4, pick_tile(p) / 2);
     Lst.rot0 = which == PASS_M2L ? 0 : which == PASS_M2M ? P->rot32_m2l : P->rot32_m2l + 2;
     Lst.key0 = which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8;
     {
@@ -869,11 +962,12 @@ int tune_rcr_tiles(Plan *P)
     if (const char *env = getenv("FMMBEM_TILE_BAL")) {
         const int bal = std::max(0, std::min(2, atoi(env)));
         for (int l = P->lmin; l <= P->lmax; l++)
-            for (RcrList *R : {&P->lev[l].m2m, &P->lev[l].m2l, &P->lev[l].l2l}) {
-                R->bal = bal ? 1 : 0;
-                if (bal == 2) R->tc = std::max(4, R->tc / 2);
-                R->items_nrhs = 0;
-            }
+            for (RcrList *R : {&P->lev[l].m2m, &P->lev[l].m2l, &P->lev[l].l2l})
+                for (TileForm &f : R->form) {
+                    f.bal = bal ? 1 : 0;
+                    if (bal == 2) f.tc = std::max(4, f.tc / 2);
+                    f.items_nrhs = 0;
+                }
         return FMM_OK;
     }
     cudaEvent_t a, b;
@@ -886,15 +980,16 @@ int tune_rcr_tiles(Plan *P)
             if (which != PASS_M2L && l == P->lmin) continue;
             RcrList &Lst = which == PASS_M2M ? L.m2m : which == PASS_M2L ? L.m2l : L.l2l;
             if (Lst.key_beg.empty() || Lst.key_beg.back() == 0 || Lst.td.on) continue;
+            TileForm &f = Lst.form[FORM_FOLDED];
             std::vector<int2> cand;
-            for (int tc = Lst.tc; tc >= 4 && 4 * tc >= Lst.tc; tc /= 2)
+            for (int tc = f.tc; tc >= 4 && 4 * tc >= f.tc; tc /= 2)
                 for (int bal = 0; bal < 2; bal++) cand.push_back({tc, bal});
             float best = 1e30f;
             int2 pick = cand[0];
             for (auto &c : cand) {
-                Lst.tc = c.x;
-                Lst.bal = c.y;
-                Lst.items_nrhs = 0;
+                f.tc = c.x;
+                f.bal = c.y;
+                f.items_nrhs = 0;
                 float tot = 0.f;
                 for (int rep = 0; rep < 4 && rc == FMM_OK; rep++) {
                     if (cudaEventRecord(a, P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
@@ -911,9 +1006,9 @@ int tune_rcr_tiles(Plan *P)
                     pick = c;
                 }
             }
-            Lst.tc = pick.x;
-            Lst.bal = pick.y;
-            Lst.items_nrhs = 0;
+            f.tc = pick.x;
+            f.bal = pick.y;
+            f.items_nrhs = 0;
         }
     }
     cudaEventDestroy(a);

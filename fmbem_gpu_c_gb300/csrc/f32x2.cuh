@@ -18,6 +18,11 @@ __device__ __forceinline__ float2 f2_parts(f2 a)
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
     return r;
 }
+__device__ __forceinline__ f2 f2_swap(f2 a)
+{
+    const float2 v = f2_parts(a);
+    return f2_pack(v.y, v.x);
+}
 __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
 {
     f2 r;

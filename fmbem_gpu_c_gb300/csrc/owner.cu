@@ -43,14 +43,6 @@ namespace {
 // x+ row m' = j, row j > n the x- row m' = j - n (its m = 0 entry is zero)
 __host__ __device__ __forceinline__ int fold_off(int n) { return n * (4 * n * n + 3 * n - 1) / 6; }
 __host__ __device__ __forceinline__ int fold_size(int p) { return fold_off(p); }
-// whole rotation tables of the FP32 tiles: degree n holds 2n + 1 columns of 2n + 1 rows, padded to 4, so that a
-// lane's four rows are one load
-__host__ __device__ __forceinline__ int pad4(int n) { return (n + 3) & ~3; }
-__host__ __device__ __forceinline__ int pad_off(int n)
-{
-    return 2 * n * (n - 1) * (2 * n - 1) / 3 + 4 * n * (n - 1) + 3 * n + (n & 1 ? n : -n);
-}
-
 // ---- arithmetic of one type: V a complex number (one 8- or 16-byte value in memory), X the same
 // prepared for multiply-adds, S a real table entry, K a complex one, E a phase; V accumulates
 // real and CA complex products, value() is the finished sum.
@@ -276,7 +268,7 @@ __device__ __forceinline__ void rot_stage(const typename Ops<T>::S *__restrict__
         const int first = minus ? 1 + (g - np) * R : g * R;         // m' (FP32: row) of the first row
         const int last = O::FOLD ? n : w - 1;
         const int steps = O::FOLD ? n + 1 : w;
-        const typename O::S *h = rot + (O::FOLD ? fold_off(n) : pad_off(n)) + (minus ? n : 0) + first;
+        const typename O::S *h = rot + (O::FOLD ? fold_off(n) : whole_off(n)) + (minus ? n : 0) + first;
         const int ld = O::FOLD ? w : pad4(w);
         auto rows = [](typename O::S(&v)[R], const typename O::S *p) {
             if constexpr (O::FOLD) {
@@ -547,15 +539,6 @@ __global__ void own_unfold_ff_kernel(const ffv *__restrict__ in, double2 *__rest
     }
 }
 
-// whole rotation tables of the classes' representative rows rep[k] of H (see pad_off)
-__global__ void own_pad_table_kernel(int pmax, const int *__restrict__ rep, const float *__restrict__ H, float *__restrict__ out)
-{
-    const int n = blockIdx.x, k = blockIdx.y, w = 2 * n + 1, ld = pad4(w);
-    const float *Hn = H + (size_t)rep[k] * rot_size(pmax) + rot_off(n);
-    float *o = out + (size_t)k * pad_off(pmax) + pad_off(n);
-    for (int t = threadIdx.x; t < w * ld; t += blockDim.x) o[t] = t % ld < w ? Hn[t / ld * w + t % ld] : 0.f;
-}
-
 // folded rotation tables of the classes' representative rows rep[k] of H (see fold_off)
 __global__ void own_fold_table_kernel(int pmax, const int *__restrict__ rep, const double *__restrict__ H,
                                       double *__restrict__ o64, ffs *__restrict__ off2)
@@ -796,8 +779,8 @@ template <> int tables_of<ff>(Plan *P, OwnArgs<ff> &a)
 }
 template <> int tables_of<float>(Plan *P, OwnArgs<float> &a)
 {
-    a.rot = P->own_rot32;
-    a.rot_stride = pad_off(P->pmax);
+    a.rot = P->rot32_whole;
+    a.rot_stride = whole_off(P->pmax);
     a.ph = P->PHsr32;
     return FMM_OK;
 }
@@ -890,18 +873,19 @@ int ensure_own(Plan *P)
         direction_classes(P, PASS_M2L, NDIR, cls, rep);
         P->own_ncls = (int)rep.size();
     }
-    {
-        const bool f64 = std::is_same<T, double>::value, f32 = std::is_same<T, float>::value;
+    if (std::is_same<T, float>::value) {
+        int e = ensure_whole_tables(P);
+        if (e) return e;
+    } else {
+        const bool f64 = std::is_same<T, double>::value;
         std::vector<int> reps, cls, rep;
         for (int which : {PASS_M2L, PASS_M2M, PASS_L2L}) {
             const int key0 = which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8;
             direction_classes(P, which, which == PASS_M2L ? NDIR : 8, cls, rep);
             for (int r : rep) reps.push_back(key0 + r);
         }
-        const size_t n = reps.size() * (size_t)(f32 ? pad_off(P->pmax) : fold_size(P->pmax)) + TABLE_PAD;
-        if (f32)
-            FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot32, sizeof(float) * n));
-        else if (f64)
+        const size_t n = reps.size() * (size_t)fold_size(P->pmax) + TABLE_PAD;
+        if (f64)
             FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot64, sizeof(double) * n));
         else
             FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot_ff, sizeof(ffs) * n));
@@ -909,11 +893,8 @@ int ensure_own(Plan *P)
         FMM_CUDA_TRY(cudaMalloc(&d_rep, sizeof(int) * reps.size()));
         cudaError_t ce = cudaMemcpyAsync(d_rep, reps.data(), sizeof(int) * reps.size(), cudaMemcpyHostToDevice, P->stream);
         const dim3 grid(P->pmax, (unsigned)reps.size());
-        if (f32)
-            own_pad_table_kernel<<<grid, 128, 0, P->stream>>>(P->pmax, d_rep, P->Hsr32, P->own_rot32);
-        else
-            own_fold_table_kernel<<<grid, 128, 0, P->stream>>>(P->pmax, d_rep, P->Hsr64, f64 ? P->own_rot64 : nullptr,
-                                                               f64 ? nullptr : reinterpret_cast<ffs *>(P->own_rot_ff));
+        own_fold_table_kernel<<<grid, 128, 0, P->stream>>>(P->pmax, d_rep, P->Hsr64, f64 ? P->own_rot64 : nullptr,
+                                                           f64 ? nullptr : reinterpret_cast<ffs *>(P->own_rot_ff));
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(P->stream);
         cudaFree(d_rep);
         FMM_CUDA_TRY(ce);
@@ -993,7 +974,6 @@ void free_owner(Plan *P)
     cudaFree(P->own_part);
     cudaFree(P->own_rot64);
     cudaFree(P->own_rot_ff);
-    cudaFree(P->own_rot32);
 }
 
 } // namespace fmm

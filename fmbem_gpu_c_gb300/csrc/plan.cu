@@ -91,14 +91,15 @@ static void free_plan(Plan *P)
         F(L.parent); F(L.octant); F(L.child_beg); F(L.child_list); F(L.sr_beg); F(L.sr_src); F(L.sr_dir);
         F(L.Cm64); F(L.Dl64); F(L.Csr_ff); F(L.Crr_ff); F(L.CrrL_ff); F(L.Cm_ff); F(L.Dl_ff); F(L.Cm32); F(L.Dl32); F(L.Csr64); F(L.Csr32); F(L.Crr64); F(L.Crr32); F(L.Crr32L); F(L.Csr32p); F(L.Crr32p); F(L.Crr32Lp);
         for (RcrList *R : {&L.m2l, &L.m2m, &L.l2l}) {
-            F(R->items); F(R->src); F(R->dst); F(R->csrc); F(R->cdst); F(R->cdir); F(R->urot); F(R->ucoax);
+            F(R->src); F(R->dst); F(R->csrc); F(R->cdst); F(R->cdir);
+            for (TileForm &f : R->form) { F(f.items); F(f.urot); F(f.ucoax); }
             Tc3 &t = R->t3;
             F(t.opsR); F(t.opsC); F(t.blkR); F(t.blkC); F(t.t_dir); F(t.itR1); F(t.itC); F(t.itR2);
             F(t.listR); F(t.listC); F(t.W); F(t.Z);
             F(R->td.B); F(R->td.items); F(R->td.src); F(R->td.dst); F(R->td.dir);
         }
     }
-    F(P->rot32); F(P->pairs);
+    F(P->rot32); F(P->rot32_whole); F(P->pairs);
     cudaFreeHost(P->tc_err_host);
     F(P->PHall_ff); F(P->dsc_leaf_dev);
     F(P->Hsr64); F(P->PHsr64); F(P->Hsr32); F(P->PHsr32);
@@ -319,14 +320,14 @@ extern "C" int fmm_plan_info(const fmm_plan *plan, fmm_info *info)
         // the form a pass runs in: three-stage, else dense tensor-core, else SIMT tiles
         auto dense = [](const RcrList &R) { return R.td.on && !R.t3.on; };
         const LevelDev &L = P->lev[l];
-        info->m2l_columns[l] = P->opt.build_mixed ? (dense(L.m2l) ? 128 : L.m2l.tc) : 0;
+        info->m2l_columns[l] = P->opt.build_mixed ? (dense(L.m2l) ? 128 : L.m2l.form[FORM_FOLDED].tc) : 0;
         info->m2l_tensor[l] = P->opt.build_mixed && dense(L.m2l) ? 1 : 0;
         info->pass_dense[l] =
             P->opt.build_mixed ? (dense(L.m2m) ? 1 : 0) | (dense(L.m2l) ? 2 : 0) | (dense(L.l2l) ? 4 : 0) : 0;
         if (P->opt.build_mixed) {
             info->pass_tc3[l] = (P->lev[l].m2m.t3.on ? 1 : 0) | (P->lev[l].m2l.t3.on ? 2 : 0) | (P->lev[l].l2l.t3.on ? 4 : 0);
             // SIMT tiles in short work units: neither tensor-core form, and bal set
-            auto bal = [&](const RcrList &R) { return !R.t3.on && !dense(R) && R.bal; };
+            auto bal = [&](const RcrList &R) { return !R.t3.on && !dense(R) && R.form[FORM_FOLDED].bal; };
             info->pass_balanced[l] = (bal(L.m2m) ? 1 : 0) | (bal(L.m2l) ? 2 : 0) | (bal(L.l2l) ? 4 : 0);
         }
     }

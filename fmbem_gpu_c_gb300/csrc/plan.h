@@ -96,10 +96,23 @@ struct KeyedList {
     int ndst_rank = 0;                // boxes of the destination level
 };
 
-// Work list of one batched translation pass: the translations by direction (src, dst), the same by
-// operator class (cls; csrc, cdst, cdir on the device, made on first use) and the device items
-// (class, first column, count, coaxial block) of the SIMT tiles for items_nrhs right-hand sides,
-// tc columns per item at most.
+// A form of a pass's SIMT tiles: tc columns, work units of two rows (bal = 1) or four; the device items (class,
+// first column, count, coaxial block) for items_nrhs right-hand sides; the work units of the tile's stages
+// for (units_tc, units_bal): rotations (the second from at3), coaxial; rounds of each stage.
+struct TileForm {
+    int tc = 8, bal = 0;
+    int4 *items = nullptr;
+    size_t items_cap = 0;
+    int n_items = 0, items_nrhs = 0;
+    int2 *urot = nullptr;
+    int *ucoax = nullptr;
+    size_t at3 = 0;
+    int units_tc = 0, units_bal = 0, n1 = 0, n2 = 0, n3 = 0;
+};
+
+// Work list of one batched translation pass: the translations by direction (src, dst), and the same by
+// operator class (cls; csrc, cdst, cdir on the device, made on first use).
+enum { FORM_FOLDED = 0, FORM_WHOLE = 1 };
 struct RcrList : KeyedList {
     int *src = nullptr, *dst = nullptr;
     KeyedList cls;
@@ -107,17 +120,7 @@ struct RcrList : KeyedList {
     int rot0 = 0, key0 = 0;       // rotation table of class 0; phase row of direction 0
     int *csrc = nullptr, *cdst = nullptr;
     short *cdir = nullptr;        // phase row
-    int4 *items = nullptr;
-    size_t items_cap = 0;
-    int n_items = 0, items_nrhs = 0;
-    int tc = 8;                   // columns per item
-    int bal = 0;                  // work units of two rows (0: of four)
-    // work units of the tile's stages for (units_tc, units_bal): rotations (the second from at3),
-    // coaxial; rounds of each stage
-    int2 *urot = nullptr;
-    int *ucoax = nullptr;
-    size_t at3 = 0;
-    int units_tc = 0, units_bal = 0, n1 = 0, n2 = 0, n3 = 0;
+    TileForm form[2];             // folded rotations, by class; whole rotations, by direction (items' class: class | direction << 8)
     Tc3 t3;                       // three-stage tensor-core form (used where t3.on)
     TcDense td;                   // dense tensor-core form (used where td.on)
 };
@@ -134,8 +137,9 @@ struct RcrPass {
     float2 *dst;                     // [boxes][rhs][pout^2]
     const int4 *items;               // (class, first, count, coaxial block) over columns e = t nrhs + r
     const int *g_src, *g_dst;        // source and destination box of translation t
-    const short *g_dir;              // its phase row in PHall
-    // tables of the tile kernels: folded rotations per class, padded coaxial blocks, all phases,
+    const short *g_dir;              // its phase row in PHall (whole rotations: key0 + the item's direction)
+    int key0;
+    // tables of the tile kernels: folded or whole rotations per class, padded coaxial blocks, all phases,
     // work units of the three stages, coefficient pairs (n, m >= 0)
     const float *rot;
     int rot_stride;
@@ -248,12 +252,12 @@ struct Plan {
     int rot32_stride = 0, rot32_m2l = 0;  // entries per class; M2L classes (M2M's and L2L's follow)
     std::vector<int> rot32_off;   // per degree, inside a class
     int *pairs = nullptr;         // coefficient pairs (n, m >= 0): n^2 + n | m << 16
+    float *rot32_whole = nullptr; // whole rotation tables per class (whole_off), made on first use
     // translations without atomics (owner.cu), per type (OWN_*), level and pass
     OwnPass own[3][FMM_MAX_LEVEL + 2][3];
     int own_ready[3] = {0, 0, 0}, own_ncls = 0;
     double *own_rot64 = nullptr;  // folded rotation tables per class, FP64 and float-float
     float4 *own_rot_ff = nullptr; // (hi, hi, lo, lo) per entry
-    float *own_rot32 = nullptr;   // whole rotation tables per class, FP32 (deterministic plans)
     void *own_part = nullptr;     // translated expansions of one chunk, before their sums
     size_t own_part_bytes = 0;
     size_t device_bytes = 0;
@@ -344,8 +348,16 @@ int build_rcr_lists(Plan *P);
 int tune_rcr_tiles(Plan *P);
 size_t rcr_tile_smem(int p, int tc);
 constexpr int MAX_MIXED_ORDER = 60;
-int set_tile_tables(const Plan *P, RcrList &Lst, RcrPass &ps);
-int launch_rcr_pass(const Plan *P, RcrList &Lst, RcrPass ps, cudaStream_t st);
+int set_tile_tables(const Plan *P, RcrList &Lst, int form, RcrPass &ps);
+int launch_rcr_pass(Plan *P, RcrList &Lst, RcrPass ps, cudaStream_t st);
+// whole FP32 rotation tables of the operator classes (M2L, then M2M and L2L): degree n holds 2n + 1 columns of
+// 2n + 1 rows, padded to 4, from whole_off(n) on
+__host__ __device__ __forceinline__ int pad4(int n) { return (n + 3) & ~3; }
+__host__ __device__ __forceinline__ int whole_off(int n)
+{
+    return 2 * n * (n - 1) * (2 * n - 1) / 3 + 4 * n * (n - 1) + 3 * n + (n & 1 ? n : -n);
+}
+int ensure_whole_tables(Plan *P);
 // work items of a list for one right-hand side, with its class order on the device
 int rcr_list_items(RcrList &Lst, std::vector<int4> &out);
 // items (key, first column, count, coaxial block) for nrhs columns in tiles of `width`, ordered

@@ -437,12 +437,13 @@ static int build_scene(Scene *S)
                 RcrList *Lst = pass32_desc(P, l, which, 1, ps);
                 if (!Lst || Lst->key_beg.empty() || Lst->key_beg.back() == 0) continue;
                 int e = rcr_list_items(*Lst, items);
-                if (!e) e = set_tile_tables(P, *Lst, ps);
+                if (!e) e = set_tile_tables(P, *Lst, FORM_FOLDED, ps);
                 if (e) return e;
+                const TileForm &form = Lst->form[FORM_FOLDED];
                 int phase = which == PASS_M2M ? Lmax - l : which == PASS_M2L ? ph_m2l : ph_m2l + (l - 2);
-                size_t sm = rcr_tile_smem(std::max(std::min(ps.pin, ps.p), std::min(ps.pout, ps.p)), Lst->tc);
+                size_t sm = rcr_tile_smem(std::max(std::min(ps.pin, ps.p), std::min(ps.pout, ps.p)), form.tc);
                 int cls = sm <= 76 * 1024 ? 3 : sm <= 113 * 1024 ? 2 : 1;
-                int g = group_of(phase, Lst->tc, Lst->bal, cls);
+                int g = group_of(phase, form.tc, form.bal, cls);
                 smem[g] = std::max(smem[g], sm);
                 int pi = (int)passes.size();
                 passes.push_back(ps);
