@@ -543,7 +543,13 @@ static int ensure_classes(RcrList &Lst)
     }
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);
     cudaFree(tmp);
-    if (ce != cudaSuccess) cudaFree(cs);
+    if (ce != cudaSuccess) {
+        cudaFree(cs);
+        cudaFree(Lst.cdst);
+        cudaFree(Lst.cdir);
+        Lst.cdst = nullptr;
+        Lst.cdir = nullptr;
+    }
     FMM_CUDA_TRY(ce);
     Lst.csrc = cs;
     return FMM_OK;

@@ -627,11 +627,19 @@ int launch_tc(const OwnArgs<T> &a, int n_items, cudaStream_t st)
     return FMM_OK;
 }
 
+void free_pass(OwnPass &O)
+{
+    for (void *q : {(void *)O.items, (void *)O.slot, (void *)O.units, (void *)O.src_own, (void *)O.key_own}) cudaFree(q);
+    O = OwnPass();
+}
+
 // the lists and units of one pass (built on first use, on the plan's stream)
 template <typename T>
 int build_pass(Plan *P, int l, int which, OwnPass &O)
 {
     typedef typename Ops<T>::V C;
+    if (O.built) return FMM_OK;
+    free_pass(O);  // (what an attempt that failed left)
     LevelDev &L = P->lev[l];
     cudaStream_t st = P->stream;
     const int pp = which == PASS_M2L ? L.p : P->lev[l - 1].p;
@@ -885,6 +893,9 @@ int ensure_own(Plan *P)
             for (int r : rep) reps.push_back(key0 + r);
         }
         const size_t n = reps.size() * (size_t)fold_size(P->pmax) + TABLE_PAD;
+        // (an attempt that failed may have left the table)
+        cudaFree(f64 ? (void *)P->own_rot64 : (void *)P->own_rot_ff);
+        (f64 ? *(void **)&P->own_rot64 : *(void **)&P->own_rot_ff) = nullptr;
         if (f64)
             FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot64, sizeof(double) * n));
         else
@@ -964,13 +975,7 @@ void free_owner(Plan *P)
 {
     for (auto &ty : P->own)
         for (auto &lev : ty)
-            for (OwnPass &O : lev) {
-                cudaFree(O.items);
-                cudaFree(O.slot);
-                cudaFree(O.units);
-                cudaFree(O.src_own);
-                cudaFree(O.key_own);
-            }
+            for (OwnPass &O : lev) free_pass(O);
     cudaFree(P->own_part);
     cudaFree(P->own_rot64);
     cudaFree(P->own_rot_ff);
