@@ -627,146 +627,260 @@ int launch_tc(const OwnArgs<T> &a, int n_items, cudaStream_t st)
     return FMM_OK;
 }
 
-void free_pass(OwnPass &O)
+// device memory that is freed unless keep() takes it
+struct DevMem {
+    void *ptr = nullptr;
+    ~DevMem() { cudaFree(ptr); }
+    template <class Q> Q *keep()
+    {
+        Q *q = (Q *)ptr;
+        ptr = nullptr;
+        return q;
+    }
+};
+
+const int WHICH[3] = {PASS_M2M, PASS_M2L, PASS_L2L};
+int key_base(int which) { return which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8; }
+int slot_bytes(int wide) { return wide ? 16 : 8; }
+
+// The lists of every pass for coefficients of 16 bytes (wide) or 8, on the plan's stream: one allocation, one
+// count of all passes' (chunk, class) bins with one read-back (pass by pass, with four synchronizations each, the
+// first FP64 matvec on 320 triangles took 0.57 ms where later ones take 0.17).
+int build_lists(Plan *P, int wide)
 {
-    for (void *q : {(void *)O.items, (void *)O.slot, (void *)O.units, (void *)O.src_own, (void *)O.key_own}) cudaFree(q);
-    O = OwnPass();
+    OwnLists &lists = P->own_lists[wide ? 0 : 1];
+    if (lists.ready) return FMM_OK;
+    cudaStream_t st = P->stream;
+    OwnLists L;
+    std::vector<OwnPass *> passes;
+    std::vector<int> where;  // level * 3 + which
+    for (int l = P->lmin; l <= P->lmax; l++)
+        for (int which : WHICH) {
+            if (which != PASS_M2L && l == P->lmin) continue;
+            const LevelDev &D = P->lev[l];
+            OwnPass &O = L.pass[l][which];
+            O.p = which == PASS_M2L ? D.p : P->lev[l - 1].p;
+            O.pin = which == PASS_M2M ? D.p : O.p;
+            O.pout = which == PASS_L2L ? D.p : O.p;
+            O.rows = std::max(std::min(O.pin, O.p), std::min(O.pout, O.p));
+            O.rows *= O.rows;
+            O.n = which == PASS_M2L ? (int)D.num_sr : D.nb;
+            O.ndst = which == PASS_M2M ? P->lev[l - 1].nb : D.nb;
+            O.beg = which == PASS_M2L ? D.sr_beg : which == PASS_M2M ? P->lev[l - 1].child_beg : nullptr;
+            passes.push_back(&O);
+            where.push_back(3 * l + which);
+        }
+    // chunks of destinations whose results fit the scratch
+    const int np = (int)passes.size();
+    std::vector<std::vector<int>> beg(np);
+    bool wait = false;
+    for (int k = 0; k < np; k++) {
+        OwnPass &O = *passes[k];
+        const size_t cap = std::max<size_t>(1, PART_CAP / ((size_t)slot_bytes(wide) * O.pout * O.pout));
+        if (!O.beg || (size_t)O.n <= cap) continue;
+        beg[k].resize(O.ndst + 1);
+        FMM_CUDA_TRY(cudaMemcpyAsync(beg[k].data(), O.beg, sizeof(int) * (O.ndst + 1), cudaMemcpyDeviceToHost, st));
+        wait = true;
+    }
+    if (wait) FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    size_t ints = 0;
+    std::vector<int> host(NDIR + 16, 0);  // class of each key, then the passes' chunk beginnings, then their bins
+    std::vector<size_t> at_slot(np), at_src(np), at_key(np), at_chunk(np), at_bin(np);
+    auto take = [&](size_t n) {
+        const size_t at = ints;
+        ints += (n + 3) & ~(size_t)3;
+        return at;
+    };
+    size_t nbin = 0;
+    for (int k = 0; k < np; k++) {
+        OwnPass &O = *passes[k];
+        const int which = where[k] % 3, cap = (int)std::max<size_t>(1, std::min<size_t>(1u << 30, PART_CAP / ((size_t)slot_bytes(wide) * O.pout * O.pout)));
+        O.chunk_box.assign(1, 0);
+        O.chunk_slot.assign(1, 0);
+        if (beg[k].empty()) {
+            O.chunk_box.push_back(O.ndst);
+            O.chunk_slot.push_back(O.n);
+        } else {
+            for (int b = 0; b < O.ndst;) {
+                int e = b + 1;
+                while (e < O.ndst && beg[k][e + 1] - beg[k][b] <= cap) e++;
+                O.chunk_box.push_back(e);
+                O.chunk_slot.push_back(beg[k][e]);
+                b = e;
+            }
+        }
+        std::vector<int> cls;
+        direction_classes(P, which, which == PASS_M2L ? NDIR : 8, cls, O.rep);
+        for (size_t d = 0; d < cls.size(); d++) host[key_base(which) + d] = cls[d];
+        O.bins.assign((O.chunk_slot.size() - 1) * O.rep.size(), 0);
+        nbin += O.bins.size();
+        at_slot[k] = take(O.n);
+        if (which == PASS_M2M) at_src[k] = take(O.n);
+        if (which != PASS_M2L) at_key[k] = take((O.n + 1) / 2);
+    }
+    for (int k = 0; k < np; k++) {
+        at_chunk[k] = host.size();
+        host.insert(host.end(), passes[k]->chunk_slot.begin(), passes[k]->chunk_slot.end());
+    }
+    const size_t bins0 = host.size();
+    host.resize(bins0 + nbin, 0);
+    DevMem mem, tmp;
+    FMM_CUDA_TRY(cudaMalloc(&mem.ptr, sizeof(int) * std::max<size_t>(1, ints)));
+    FMM_CUDA_TRY(cudaMalloc(&tmp.ptr, sizeof(int) * host.size()));
+    int *m = (int *)mem.ptr, *t = (int *)tmp.ptr;
+    FMM_CUDA_TRY(cudaMemcpyAsync(t, host.data(), sizeof(int) * host.size(), cudaMemcpyHostToDevice, st));
+    size_t bin = bins0;
+    for (int k = 0; k < np; k++) {
+        OwnPass &O = *passes[k];
+        const int which = where[k] % 3, l = where[k] / 3;
+        const LevelDev &D = P->lev[l];
+        O.slot = m + at_slot[k];
+        if (which == PASS_M2L) {
+            O.src = D.sr_src;
+            O.key = D.sr_dir;
+        } else {
+            O.key = O.key_own = (short *)(m + at_key[k]);
+            if (which == PASS_M2M) {
+                O.src = O.src_own = m + at_src[k];
+                own_m2m_slots_kernel<<<ew_grid(D.nb), 256, 0, st>>>(D.nb, P->lev[l - 1].child_list, D.octant, O.src_own, O.key_own);
+            } else {
+                O.src = D.parent;
+                own_l2l_slots_kernel<<<ew_grid(D.nb), 256, 0, st>>>(D.nb, D.octant, O.key_own);
+            }
+        }
+        at_bin[k] = bin;
+        bin += O.bins.size();
+        own_bin_kernel<<<ew_grid(O.n), 256, 0, st>>>(O.n, O.key, t, t + at_chunk[k], (int)O.chunk_slot.size() - 1, (int)O.rep.size(),
+                                                     t + at_bin[k], nullptr);
+    }
+    FMM_CUDA_TRY(cudaGetLastError());
+    FMM_CUDA_TRY(cudaMemcpyAsync(host.data() + bins0, t + bins0, sizeof(int) * nbin, cudaMemcpyDeviceToHost, st));
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    for (int k = 0; k < np; k++) {
+        OwnPass &O = *passes[k];
+        int pos = 0;
+        for (size_t q = 0; q < O.bins.size(); q++) {
+            O.bins[q] = host[at_bin[k] + q];
+            host[at_bin[k] + q] = pos;
+            pos += O.bins[q];
+        }
+    }
+    FMM_CUDA_TRY(cudaMemcpyAsync(t + bins0, host.data() + bins0, sizeof(int) * nbin, cudaMemcpyHostToDevice, st));
+    for (int k = 0; k < np; k++) {
+        OwnPass &O = *passes[k];
+        own_bin_kernel<<<ew_grid(O.n), 256, 0, st>>>(O.n, O.key, t, t + at_chunk[k], (int)O.chunk_slot.size() - 1, (int)O.rep.size(),
+                                                     t + at_bin[k], O.slot);
+    }
+    FMM_CUDA_TRY(cudaGetLastError());
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    L.mem = mem.keep<int>();
+    L.ready = 1;
+    P->device_bytes += sizeof(int) * ints;
+    lists = L;
+    return FMM_OK;
 }
 
-// the lists and units of one pass (built on first use, on the plan's stream)
+// Tile shapes, items and work units of every pass of one type, in one allocation.
 template <typename T>
-int build_pass(Plan *P, int l, int which, OwnPass &O)
+int build_form(Plan *P, OwnForm &form)
 {
+    if (form.ready) return FMM_OK;
     typedef typename Ops<T>::V C;
-    if (O.built) return FMM_OK;
-    free_pass(O);  // (what an attempt that failed left)
-    LevelDev &L = P->lev[l];
-    cudaStream_t st = P->stream;
-    const int pp = which == PASS_M2L ? L.p : P->lev[l - 1].p;
-    O.p = pp;
-    O.pin = which == PASS_M2M ? L.p : pp;
-    O.pout = which == PASS_L2L ? L.p : pp;
-    const int nin = std::min(O.pin, pp), nq = std::min(O.pout, pp), ndst = which == PASS_M2M ? P->lev[l - 1].nb : L.nb;
-    O.rows = std::max(nin, nq) * std::max(nin, nq);
-    O.tc = pick_cols(O.rows, sizeof(C), std::is_same<T, float>::value ? F32_TILE : TWO_CTA);
-    if (!O.tc) {
-        fmm_set_error("translation order %d above 60", pp);
-        return FMM_ERR_CUDA;
-    }
-    // slots: the destination's translations in list order
-    std::vector<int> beg;
-    const int *beg_dev = which == PASS_M2L ? L.sr_beg : which == PASS_M2M ? P->lev[l - 1].child_beg : nullptr;
-    const int n = which == PASS_M2L ? (int)L.num_sr : L.nb;
-    O.beg = beg_dev;
-    if (beg_dev) {
-        beg.resize(ndst + 1);
-        FMM_CUDA_TRY(cudaMemcpyAsync(beg.data(), beg_dev, sizeof(int) * (ndst + 1), cudaMemcpyDeviceToHost, st));
-    }
-    if (which == PASS_M2L) {
-        O.src = L.sr_src;
-        O.key = L.sr_dir;
-    } else {
-        FMM_CUDA_TRY(dev_alloc(P, (void **)&O.key_own, sizeof(short) * std::max(1, L.nb)));
-        O.key = O.key_own;
-        if (which == PASS_M2M) {
-            FMM_CUDA_TRY(dev_alloc(P, (void **)&O.src_own, sizeof(int) * std::max(1, L.nb)));
-            O.src = O.src_own;
-            own_m2m_slots_kernel<<<ew_grid(L.nb), 256, 0, st>>>(L.nb, P->lev[l - 1].child_list, L.octant, O.src_own, O.key_own);
-        } else {
-            O.src = L.parent;
-            own_l2l_slots_kernel<<<ew_grid(L.nb), 256, 0, st>>>(L.nb, L.octant, O.key_own);
-        }
-    }
-    FMM_CUDA_TRY(cudaStreamSynchronize(st));
-    // chunks of destinations whose results fit the scratch
-    const size_t slot_bytes = sizeof(C) * O.pout * O.pout;
-    O.chunk_box.assign(1, 0);
-    std::vector<int> chunk_slot(1, 0);
-    size_t most = 0;
-    if (beg_dev) {
-        const int cap = (int)std::max<size_t>(1, PART_CAP / slot_bytes);
-        for (int b = 0; b < ndst;) {
-            int e = b + 1;
-            while (e < ndst && beg[e + 1] - beg[b] <= cap) e++;
-            most = std::max(most, (size_t)(beg[e] - beg[b]) * slot_bytes);
-            O.chunk_box.push_back(e);
-            chunk_slot.push_back(beg[e]);
-            b = e;
-        }
-    } else {
-        O.chunk_box.push_back(ndst);
-        chunk_slot.push_back(n);
-    }
-    O.part_bytes = most;
-    O.chunk_slot = chunk_slot;
-    const int nchunk = (int)chunk_slot.size() - 1;
-    // classes
-    std::vector<int> cls, rep;
-    const int nkeys = which == PASS_M2L ? NDIR : 8, key0 = which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8;
-    direction_classes(P, which, nkeys, cls, rep);
-    const int ncls = (int)rep.size(), cls0 = which == PASS_M2L ? 0 : which == PASS_M2M ? P->own_ncls : P->own_ncls + 2;
-    std::vector<int> cls_of_key(NDIR + 16, 0);
-    for (int d = 0; d < nkeys; d++) cls_of_key[key0 + d] = cls[d];
-    FMM_CUDA_TRY(dev_alloc(P, (void **)&O.slot, sizeof(int) * std::max(1, n)));
-    int *tmp = nullptr;  // class of key, chunk beginnings, bins
-    const size_t nbin = (size_t)nchunk * ncls;
-    FMM_CUDA_TRY(cudaMalloc(&tmp, sizeof(int) * (NDIR + 16 + chunk_slot.size() + nbin)));
-    int *d_cls = tmp, *d_chunk = tmp + NDIR + 16, *d_bins = d_chunk + chunk_slot.size();
-    std::vector<int> bins(nbin);
+    const bool wide = sizeof(C) == 16;
+    const OwnLists &lists = P->own_lists[wide ? 0 : 1];
+    OwnForm F;
     std::vector<int4> items;
-    cudaError_t ce = cudaMemcpyAsync(d_cls, cls_of_key.data(), sizeof(int) * cls_of_key.size(), cudaMemcpyHostToDevice, st);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_chunk, chunk_slot.data(), sizeof(int) * chunk_slot.size(), cudaMemcpyHostToDevice, st);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(d_bins, 0, sizeof(int) * nbin, st);
-    if (ce == cudaSuccess) {
-        own_bin_kernel<<<ew_grid(n), 256, 0, st>>>(n, O.key, d_cls, d_chunk, nchunk, ncls, d_bins, nullptr);
-        ce = cudaMemcpyAsync(bins.data(), d_bins, sizeof(int) * nbin, cudaMemcpyDeviceToHost, st);
-    }
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-    if (ce == cudaSuccess) {
-        O.chunk_item.assign(1, 0);
-        int pos = 0;
-        for (int c = 0; c < nchunk; c++) {
-            for (int k = 0; k < ncls; k++) {
-                const int cnt = bins[(size_t)c * ncls + k];
-                bins[(size_t)c * ncls + k] = pos;
-                const int rrow = cls0 + k;
-                for (int a = 0; a < cnt; a += O.tc)
-                    items.push_back(make_int4(rrow, pos + a, std::min(O.tc, cnt - a), which == PASS_M2L ? P->dir_dist[rep[k]] : 0));
-                pos += cnt;
-            }
-            O.chunk_item.push_back((int)items.size());
-        }
-        ce = cudaMemcpyAsync(d_bins, bins.data(), sizeof(int) * nbin, cudaMemcpyHostToDevice, st);
-        own_bin_kernel<<<ew_grid(n), 256, 0, st>>>(n, O.key, d_cls, d_chunk, nchunk, ncls, d_bins, O.slot);
-    }
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-    cudaFree(tmp);
-    FMM_CUDA_TRY(ce);
-    // work units, longest first: groups of R rows of one sign, 32 / tc groups each
-    const int rl = 32 / O.tc, R = Ops<T>::R;
     std::vector<int> un;
-    auto rot_units = [&](int deg) {
-        int k = 0;
-        for (int d = deg - 1; d >= 0; d--) {
-            const int ng = Ops<T>::FOLD ? (d + R) / R + (d + R - 1) / R : (2 * d + R) / R;
-            for (int g = 0; g < ng; g += rl, k++) un.push_back(d | g << 8);
+    std::vector<std::pair<size_t, size_t>> at;  // the passes' first item and unit
+    const int rows_m2l = (int)lists.pass[P->lmin][PASS_M2L].rep.size();
+    for (int l = P->lmin; l <= P->lmax; l++)
+        for (int which : WHICH) {
+            if (which != PASS_M2L && l == P->lmin) continue;
+            const OwnPass &O = lists.pass[l][which];
+            OwnTiles &W = F.pass[l][which];
+            W.tc = pick_cols(O.rows, sizeof(C), std::is_same<T, float>::value ? F32_TILE : TWO_CTA);
+            if (!W.tc) {
+                fmm_set_error("translation order %d above 60", O.p);
+                return FMM_ERR_CUDA;
+            }
+            at.push_back({items.size(), un.size()});
+            const size_t item0 = items.size(), ncls = O.rep.size();
+            const int row0 = which == PASS_M2L ? 0 : rows_m2l + (which == PASS_M2M ? 0 : 2);
+            W.chunk_item.assign(1, 0);
+            int pos = 0;
+            for (size_t q = 0; q < O.bins.size(); q++) {
+                const int k = (int)(q % ncls), cnt = O.bins[q];
+                for (int a = 0; a < cnt; a += W.tc)
+                    items.push_back(make_int4(row0 + k, pos + a, std::min(W.tc, cnt - a), which == PASS_M2L ? P->dir_dist[O.rep[k]] : 0));
+                pos += cnt;
+                if (k + 1 == (int)ncls) W.chunk_item.push_back((int)(items.size() - item0));
+            }
+            if (which != PASS_L2L)
+                for (size_t c = 0; c + 1 < O.chunk_slot.size(); c++)
+                    F.part_bytes = std::max(F.part_bytes, sizeof(C) * (size_t)(O.chunk_slot[c + 1] - O.chunk_slot[c]) * O.pout * O.pout);
+            // work units, longest first: groups of R rows of one sign, 32 / tc groups each
+            const int nin = std::min(O.pin, O.p), nq = std::min(O.pout, O.p), rl = 32 / W.tc, R = Ops<T>::R;
+            auto rot_units = [&](int deg) {
+                int k = 0;
+                for (int d = deg - 1; d >= 0; d--) {
+                    const int ng = Ops<T>::FOLD ? (d + R) / R + (d + R - 1) / R : (2 * d + R) / R;
+                    for (int g = 0; g < ng; g += rl, k++) un.push_back(d | g << 8);
+                }
+                return k;
+            };
+            W.n1 = rot_units(nin);
+            // orders m that the source does not reach (nq > nin) give rows of zeros
+            for (int am = 0; am < nq; am++) {
+                const int ng = (am ? 2 : 1) * ((nq - am + R - 1) / R);
+                for (int g = 0; g < ng; g += rl, W.n2++) un.push_back(am | g << 8);
+            }
+            W.n3 = rot_units(nq);
         }
-        return k;
-    };
-    O.n1 = rot_units(nin);
-    O.n2 = 0;
-    // orders m that the source does not reach (nq > nin) give rows of zeros
-    for (int am = 0; am < nq; am++) {
-        const int ng = (am ? 2 : 1) * ((nq - am + R - 1) / R);
-        for (int g = 0; g < ng; g += rl, O.n2++) un.push_back(am | g << 8);
+    DevMem mem;
+    const size_t bytes = sizeof(int4) * items.size() + sizeof(int) * un.size();
+    FMM_CUDA_TRY(cudaMalloc(&mem.ptr, std::max<size_t>(1, bytes)));
+    int4 *it = (int4 *)mem.ptr;
+    int *u = (int *)(it + items.size());
+    FMM_CUDA_TRY(cudaMemcpyAsync(it, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, P->stream));
+    FMM_CUDA_TRY(cudaMemcpyAsync(u, un.data(), sizeof(int) * un.size(), cudaMemcpyHostToDevice, P->stream));
+    FMM_CUDA_TRY(cudaStreamSynchronize(P->stream));
+    size_t k = 0;
+    for (int l = P->lmin; l <= P->lmax; l++)
+        for (int which : WHICH) {
+            if (which != PASS_M2L && l == P->lmin) continue;
+            F.pass[l][which].items = it + at[k].first;
+            F.pass[l][which].units = u + at[k++].second;
+        }
+    F.mem = mem.keep<int4>();
+    F.ready = 1;
+    P->device_bytes += bytes;
+    form = F;
+    return FMM_OK;
+}
+
+// folded rotation tables of the classes (M2L, then M2M and L2L)
+int build_folded(Plan *P, bool ff)
+{
+    if (ff ? (void *)P->own_rot_ff : (void *)P->own_rot64) return FMM_OK;
+    std::vector<int> reps, cls, rep;
+    for (int which : {PASS_M2L, PASS_M2M, PASS_L2L}) {
+        direction_classes(P, which, which == PASS_M2L ? NDIR : 8, cls, rep);
+        for (int r : rep) reps.push_back(key_base(which) + r);
     }
-    O.n3 = rot_units(nq);
-    FMM_CUDA_TRY(dev_alloc(P, (void **)&O.items, sizeof(int4) * std::max<size_t>(1, items.size())));
-    FMM_CUDA_TRY(dev_alloc(P, (void **)&O.units, sizeof(int) * un.size()));
-    FMM_CUDA_TRY(cudaMemcpyAsync(O.items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, st));
-    FMM_CUDA_TRY(cudaMemcpyAsync(O.units, un.data(), sizeof(int) * un.size(), cudaMemcpyHostToDevice, st));
-    FMM_CUDA_TRY(cudaStreamSynchronize(st));
-    O.built = 1;
+    const size_t bytes = (ff ? sizeof(ffs) : sizeof(double)) * (reps.size() * (size_t)fold_size(P->pmax) + TABLE_PAD);
+    DevMem tab, d_rep;
+    FMM_CUDA_TRY(cudaMalloc(&tab.ptr, bytes));
+    FMM_CUDA_TRY(cudaMalloc(&d_rep.ptr, sizeof(int) * reps.size()));
+    FMM_CUDA_TRY(cudaMemcpyAsync(d_rep.ptr, reps.data(), sizeof(int) * reps.size(), cudaMemcpyHostToDevice, P->stream));
+    own_fold_table_kernel<<<dim3(P->pmax, (unsigned)reps.size()), 128, 0, P->stream>>>(
+        P->pmax, (const int *)d_rep.ptr, P->Hsr64, ff ? nullptr : (double *)tab.ptr, ff ? (ffs *)tab.ptr : nullptr);
+    FMM_CUDA_TRY(cudaGetLastError());
+    FMM_CUDA_TRY(cudaStreamSynchronize(P->stream));
+    if (ff)
+        P->own_rot_ff = tab.keep<float4>();
+    else
+        P->own_rot64 = tab.keep<double>();
+    P->device_bytes += bytes;
     return FMM_OK;
 }
 
@@ -810,7 +924,7 @@ template <> LevelArrays<ff> arrays_of<ff>(LevelDev &L)
 }
 
 template <typename T>
-int run_pass(Plan *P, int l, int which, OwnPass &O)
+int run_pass(Plan *P, int l, int which, const OwnPass &O, const OwnTiles &W, void *part)
 {
     typedef typename Ops<T>::V C;
     cudaStream_t st = P->stream;
@@ -831,24 +945,24 @@ int run_pass(Plan *P, int l, int which, OwnPass &O)
     a.key = O.key;
     a.Cc = which == PASS_M2L ? A.Csr : which == PASS_M2M ? A.Cup : A.Cdown;
     a.in = which == PASS_L2L ? U.Dl : A.Cm;
-    a.u1 = O.units;
-    a.u2 = O.units + O.n1;
-    a.u3 = O.units + O.n1 + O.n2;
-    a.n1 = O.n1;
-    a.n2 = O.n2;
-    a.n3 = O.n3;
+    a.u1 = W.units;
+    a.u2 = W.units + W.n1;
+    a.u3 = W.units + W.n1 + W.n2;
+    a.n1 = W.n1;
+    a.n2 = W.n2;
+    a.n3 = W.n3;
     C *dst = which == PASS_M2M ? U.Cm : A.Dl;
     const int n2 = O.pout * O.pout;
     // a parent of lower order than the child reaches the child's first degrees only
     if (which == PASS_L2L && a.nq < O.pout)
         FMM_CUDA_TRY(cudaMemsetAsync(dst, 0, sizeof(C) * (size_t)L.nb * n2, st));
     for (size_t c = 0; c + 1 < O.chunk_box.size(); c++) {
-        const int n = O.chunk_item[c + 1] - O.chunk_item[c];
-        a.items = O.items + O.chunk_item[c];
+        const int n = W.chunk_item[c + 1] - W.chunk_item[c];
+        a.items = W.items + W.chunk_item[c];
         a.slot0 = O.chunk_slot[c];
-        a.out = which == PASS_L2L ? dst : (C *)P->own_part;
+        a.out = which == PASS_L2L ? dst : (C *)part;
         if (n > 0) {
-            switch (O.tc) {
+            switch (W.tc) {
             case 32: e = launch_tc<T, 32>(a, n, st); break;
             case 16: e = launch_tc<T, 16>(a, n, st); break;
             case 8: e = launch_tc<T, 8>(a, n, st); break;
@@ -861,100 +975,62 @@ int run_pass(Plan *P, int l, int which, OwnPass &O)
             const int b0 = O.chunk_box[c], b1 = O.chunk_box[c + 1];
             const int S = which == PASS_M2L ? std::max(1, L.m2l_split) : 1;
             own_reduce_kernel<T><<<ew_grid((size_t)(b1 - b0) * n2), 256, 0, st>>>(
-                b0, b1, n2, S, which == PASS_M2L && l > P->lmin, a.slot0, O.beg, (const C *)P->own_part, dst);
+                b0, b1, n2, S, which == PASS_M2L && l > P->lmin, a.slot0, O.beg, (const C *)part, dst);
             FMM_CUDA_TRY(cudaGetLastError());
         }
     }
     return FMM_OK;
 }
 
-template <typename T> int slot_of_type() { return std::is_same<T, double>::value ? 0 : std::is_same<T, ff>::value ? 1 : 2; }
+template <typename T> int type_of() { return std::is_same<T, double>::value ? OWN_FP64 : std::is_same<T, ff>::value ? OWN_FF : OWN_FP32; }
 
-// lists of every pass, folded tables and the scratch, on first use
+// lists, tiles and tables of a type
 template <typename T>
 int ensure_own(Plan *P)
 {
-    const int ty = slot_of_type<T>();
-    if (P->own_ready[ty]) return FMM_OK;
-    if (!P->own_ncls) {
-        std::vector<int> cls, rep;
-        direction_classes(P, PASS_M2L, NDIR, cls, rep);
-        P->own_ncls = (int)rep.size();
-    }
-    if (std::is_same<T, float>::value) {
-        int e = ensure_whole_tables(P);
-        if (e) return e;
-    } else {
-        const bool f64 = std::is_same<T, double>::value;
-        std::vector<int> reps, cls, rep;
-        for (int which : {PASS_M2L, PASS_M2M, PASS_L2L}) {
-            const int key0 = which == PASS_M2L ? 0 : which == PASS_M2M ? NDIR : NDIR + 8;
-            direction_classes(P, which, which == PASS_M2L ? NDIR : 8, cls, rep);
-            for (int r : rep) reps.push_back(key0 + r);
-        }
-        const size_t n = reps.size() * (size_t)fold_size(P->pmax) + TABLE_PAD;
-        // (an attempt that failed may have left the table)
-        cudaFree(f64 ? (void *)P->own_rot64 : (void *)P->own_rot_ff);
-        (f64 ? *(void **)&P->own_rot64 : *(void **)&P->own_rot_ff) = nullptr;
-        if (f64)
-            FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot64, sizeof(double) * n));
-        else
-            FMM_CUDA_TRY(dev_alloc(P, (void **)&P->own_rot_ff, sizeof(ffs) * n));
-        int *d_rep = nullptr;
-        FMM_CUDA_TRY(cudaMalloc(&d_rep, sizeof(int) * reps.size()));
-        cudaError_t ce = cudaMemcpyAsync(d_rep, reps.data(), sizeof(int) * reps.size(), cudaMemcpyHostToDevice, P->stream);
-        const dim3 grid(P->pmax, (unsigned)reps.size());
-        own_fold_table_kernel<<<grid, 128, 0, P->stream>>>(P->pmax, d_rep, P->Hsr64, f64 ? P->own_rot64 : nullptr,
-                                                           f64 ? nullptr : reinterpret_cast<ffs *>(P->own_rot_ff));
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(P->stream);
-        cudaFree(d_rep);
-        FMM_CUDA_TRY(ce);
-    }
-    size_t part = 0;
-    for (int l = P->lmin; l <= P->lmax; l++)
-        for (int which : {PASS_M2M, PASS_M2L, PASS_L2L}) {
-            if (which != PASS_M2L && l == P->lmin) continue;
-            OwnPass &O = P->own[ty][l][which];
-            int e = build_pass<T>(P, l, which, O);
-            if (e) return e;
-            part = std::max(part, O.part_bytes);
-        }
-    if (part > P->own_part_bytes) {
-        cudaFree(P->own_part);
-        P->own_part = nullptr;
-        P->device_bytes -= P->own_part_bytes;
-        P->own_part_bytes = 0;
-        FMM_CUDA_TRY(dev_alloc(P, &P->own_part, part));
-        P->own_part_bytes = part;
-    }
-    P->own_ready[ty] = 1;
-    return FMM_OK;
+    OwnForm &form = P->own_form[type_of<T>()];
+    int e = build_lists(P, sizeof(typename Ops<T>::V) == 16);
+    if (!e) e = std::is_same<T, float>::value ? ensure_whole_tables(P) : build_folded(P, std::is_same<T, ff>::value);
+    if (!e) e = build_form<T>(P, form);
+    return e;
 }
 
 template <typename T>
 int translate(Plan *P, void (*beg)(Plan *, int, int), void (*end)(Plan *))
 {
-    const int ty = slot_of_type<T>();
     int e = ensure_own<T>(P);
     if (e) return e;
+    const OwnLists &lists = P->own_lists[sizeof(typename Ops<T>::V) == 16 ? 0 : 1];
+    const OwnForm &form = P->own_form[type_of<T>()];
     LevelDev &LL = P->lev[P->lmax];
     cudaStream_t st = P->stream;
+    if (form.part_bytes > P->own_part_bytes) {
+        cudaFree(P->own_part);
+        P->own_part = nullptr;
+        P->device_bytes -= P->own_part_bytes;
+        P->own_part_bytes = 0;
+        FMM_CUDA_TRY(dev_alloc(P, &P->own_part, form.part_bytes));
+        P->own_part_bytes = form.part_bytes;
+    }
+    void *part = P->own_part;
+    auto pass = [&](int l, int which) { return run_pass<T>(P, l, which, lists.pass[l][which], form.pass[l][which], part); };
     const size_t np = (size_t)LL.nb * LL.p * (LL.p + 1) / 2;
     if (std::is_same<T, double>::value)
         own_fold_kernel<<<ew_grid(np), 256, 0, st>>>(LL.Cm64, LL.nb, LL.p, 1);
     else if (std::is_same<T, ff>::value)
         own_fold_ff_kernel<<<ew_grid(np), 256, 0, st>>>(LL.Cm64, reinterpret_cast<ffv *>(LL.Cm_ff), LL.nb, LL.p, P->dsc_leaf_dev);
-    for (int l = P->lmax; l > P->lmin; l--) {
+    for (int l = P->lmax; l > P->lmin && !e; l--) {
         beg(P, PASS_M2M, l);
-        if ((e = run_pass<T>(P, l, PASS_M2M, P->own[ty][l][PASS_M2M]))) return e;
+        e = pass(l, PASS_M2M);
         end(P);
     }
-    for (int l = P->lmin; l <= P->lmax; l++) {
+    for (int l = P->lmin; l <= P->lmax && !e; l++) {
         beg(P, PASS_M2L, l);
-        if (l > P->lmin && (e = run_pass<T>(P, l, PASS_L2L, P->own[ty][l][PASS_L2L]))) return e;
-        if ((e = run_pass<T>(P, l, PASS_M2L, P->own[ty][l][PASS_M2L]))) return e;
+        if (l > P->lmin) e = pass(l, PASS_L2L);
+        if (!e) e = pass(l, PASS_M2L);
         end(P);
     }
+    if (e) return e;
     if (std::is_same<T, double>::value)
         own_fold_kernel<<<ew_grid(np), 256, 0, st>>>(LL.Dl64, LL.nb, LL.p, 0);
     else if (std::is_same<T, ff>::value)
@@ -971,14 +1047,18 @@ int translate_owner(Plan *P, int type, void (*beg)(Plan *, int, int), void (*end
                             : type == OWN_FF ? translate<ff>(P, beg, end) : translate<float>(P, beg, end);
 }
 
+int prepare_owner(Plan *P, int type)
+{
+    return type == OWN_FP64 ? ensure_own<double>(P) : type == OWN_FF ? ensure_own<ff>(P) : ensure_own<float>(P);
+}
+
 void free_owner(Plan *P)
 {
-    for (auto &ty : P->own)
-        for (auto &lev : ty)
-            for (OwnPass &O : lev) free_pass(O);
-    cudaFree(P->own_part);
+    for (OwnLists &l : P->own_lists) cudaFree(l.mem);
+    for (OwnForm &f : P->own_form) cudaFree(f.mem);
     cudaFree(P->own_rot64);
     cudaFree(P->own_rot_ff);
+    cudaFree(P->own_part);
 }
 
 } // namespace fmm

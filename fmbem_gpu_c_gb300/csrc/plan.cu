@@ -254,6 +254,11 @@ static int plan_create_impl(std::vector<double> &&V, std::vector<int> &&F, const
             TRY(check_tc_error(P));
         }
     }
+    // the lists of the translations without atomics; where that fails (no memory), the first matvec that needs
+    // them says so
+    if (P->pmax <= MAX_MIXED_ORDER &&
+        (prepare_owner(P, OWN_FP64) || (P->opt.build_mixed && P->opt.deterministic && prepare_owner(P, OWN_FP32))))
+        cudaGetLastError();
     CTRY(dev_alloc(P, (void **)&P->xbuf, sizeof(double2) * nf));
     CTRY(dev_alloc(P, (void **)&P->ybuf, sizeof(double2) * nf));
     P->nrhs_cap = 1;

@@ -150,20 +150,35 @@ struct RcrPass {
     int tile_words, rot_words;       // 16-byte words of a tile and of a class's rotation table (tables in shared memory)
 };
 
-// One pass of the translations without atomics (owner.cu): translations ("slots", in destination
-// order) sorted by operator class inside chunks of consecutive destination boxes.
+// Translations without atomics (owner.cu).  The translations of one pass ("slots", in destination order) sorted by
+// operator class inside chunks of consecutive destination boxes; on the device in OwnLists::mem.
 struct OwnPass {
-    int built = 0, p = 0, pin = 0, pout = 0, rows = 0, tc = 0;
-    int4 *items = nullptr;        // (rotation table row, first, count, coaxial block)
-    int *slot = nullptr;          // slots in class order
-    const int *src = nullptr, *beg = nullptr;   // per slot: source box; per destination: its slots
-    const short *key = nullptr;   // per slot: phase row
-    int *src_own = nullptr;
+    int p = 0, pin = 0, pout = 0, rows = 0, n = 0, ndst = 0;
+    int *slot = nullptr, *src_own = nullptr;
     short *key_own = nullptr;
-    int *units = nullptr;         // work units of the three stages
-    int n1 = 0, n2 = 0, n3 = 0;
-    std::vector<int> chunk_box, chunk_slot, chunk_item;
-    size_t part_bytes = 0;
+    const int *src = nullptr, *beg = nullptr;   // per slot: source box; per destination: its slots
+    const short *key = nullptr;                 // per slot: phase row
+    std::vector<int> chunk_box, chunk_slot;
+    std::vector<int> rep, bins;                 // first key of each class; translations per (chunk, class)
+};
+struct OwnLists {                 // for expansions of 16 bytes per coefficient (FP64, float-float) or 8
+    int ready = 0;
+    int *mem = nullptr;
+    OwnPass pass[FMM_MAX_LEVEL + 2][3];
+};
+// Tiles of one type (OWN_*): per level and pass columns, items (rotation table row, first, count, coaxial block) by
+// chunk and the work units of the three stages, on the device in mem.
+struct OwnTiles {
+    int tc = 0, n1 = 0, n2 = 0, n3 = 0;
+    const int4 *items = nullptr;
+    const int *units = nullptr;
+    std::vector<int> chunk_item;
+};
+struct OwnForm {
+    int ready = 0;
+    int4 *mem = nullptr;
+    size_t part_bytes = 0;        // scratch: translated expansions of the largest chunk, before their sums
+    OwnTiles pass[FMM_MAX_LEVEL + 2][3];
 };
 
 struct LevelDev {
@@ -253,9 +268,9 @@ struct Plan {
     std::vector<int> rot32_off;   // per degree, inside a class
     int *pairs = nullptr;         // coefficient pairs (n, m >= 0): n^2 + n | m << 16
     float *rot32_whole = nullptr; // whole rotation tables per class (whole_off), made on first use
-    // translations without atomics (owner.cu), per type (OWN_*), level and pass
-    OwnPass own[3][FMM_MAX_LEVEL + 2][3];
-    int own_ready[3] = {0, 0, 0}, own_ncls = 0;
+    // translations without atomics (owner.cu)
+    OwnLists own_lists[2];
+    OwnForm own_form[3];          // per type (OWN_*)
     double *own_rot64 = nullptr;  // folded rotation tables per class, FP64 and float-float
     float4 *own_rot_ff = nullptr; // (hi, hi, lo, lo) per entry
     void *own_part = nullptr;     // translated expansions of one chunk, before their sums
@@ -321,6 +336,7 @@ RcrList *pass32_desc(Plan *P, int l, int which, int nrhs, RcrPass &ps);
 // (OWN_FF: from Cm64 to Dl64 through the float-float expansions); beg / end time a pass of a level
 enum { OWN_FP64 = 0, OWN_FF = 1, OWN_FP32 = 2 };
 int translate_owner(Plan *P, int type, void (*beg)(Plan *, int, int), void (*end)(Plan *));
+int prepare_owner(Plan *P, int type);  // lists and tables, otherwise made on first use
 void free_owner(Plan *P);
 
 // plan.cu: y = a x + b y over n entries

@@ -30,3 +30,13 @@ def test_mixed(fm):
     """Lists and work items of some 260,000 translations take 2 ms to build; a later matvec takes 0.6 ms."""
     first, later = first_and_later(fm, fm.FMM_MIXED, fm.icosphere(5, 0.2), k=73.0, depth=5, p_levels={2: 24, 3: 18, 4: 14, 5: 10})
     assert first < later + 0.7e-3
+
+
+@pytest.mark.parametrize("name", ["FMM_FP64", "FMM_FLOAT2", "deterministic"])
+def test_without_atomics(fm, name):
+    """The lists of some ten passes: with several allocations and synchronizations each, half a millisecond on a
+    small body whose later matvecs take 0.1 to 0.2 ms.  FMM_FLOAT2 makes its tables on first use: 0.3 ms."""
+    det = name == "deterministic"
+    first, later = first_and_later(fm, fm.FMM_MIXED if det else getattr(fm, name), fm.icosphere(3, 0.1), k=30.0, depth=4,
+                                   p_levels={2: 12, 3: 10, 4: 8}, deterministic=det)
+    assert first < later + (0.45e-3 if name == "FMM_FLOAT2" else 0.2e-3)
