@@ -32,6 +32,9 @@
 #include "ff.cuh"
 #include "f32x2.cuh"
 #include <algorithm>
+#include <condition_variable>
+#include <map>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -615,6 +618,122 @@ int pick_cols(int rows, size_t elem, size_t most)
 // bytes of the scratch that holds one chunk of translated expansions
 constexpr size_t PART_CAP = 128u << 20;
 
+// ---- scratch, shared by the plans of a device.  A plan takes a buffer while it enqueues its translations and gives it
+// back with an event behind them: the next one to take it waits for that event on its own stream (or finds it
+// passed).  Buffers are added while they stay under POOL_CAP in all, so that plans on several streams run side by
+// side; the last plan of the device to go frees them.  (128 MB in each plan for its life: 256 bodies of a scene
+// would have held 32 GB.)
+constexpr size_t POOL_CAP = 512u << 20, SMALL_PART = 16u << 20;
+struct Scratch {
+    void *ptr = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t done = nullptr;
+    bool busy = false;
+};
+struct Pool {
+    std::vector<Scratch> buf;
+    int users = 0;
+};
+std::mutex pool_mutex;
+std::condition_variable pool_free;
+std::map<int, Pool> pools;  // per device
+
+int pool_take(Plan *P, size_t bytes, void **ptr)
+{
+    std::unique_lock<std::mutex> lock(pool_mutex);
+    Pool &pool = pools[P->opt.device];
+    if (P->own_scratch == Plan::NO_POOL) {
+        pool.users++;
+        P->own_scratch = Plan::NO_SCRATCH;
+    }
+    for (;;) {
+        int mine = -1, idle = -1, behind = -1, small = -1, room = -1;
+        size_t all = 0;
+        for (int i = 0; i < (int)pool.buf.size(); i++) {
+            Scratch &s = pool.buf[i];
+            all += s.bytes;
+            if (!s.ptr) room = i;
+            if (s.busy) continue;
+            if (s.bytes < bytes) {
+                if (s.ptr) small = i;
+                continue;
+            }
+            if (i == P->own_scratch) {
+                mine = i;
+            } else if (cudaEventQuery(s.done) == cudaSuccess) {
+                idle = i;
+            } else {
+                cudaGetLastError();
+                behind = i;
+            }
+        }
+        int take = mine >= 0 ? mine : idle;
+        if (take < 0 && all > 0 && all + bytes > POOL_CAP) {
+            take = behind;
+            if (take < 0 && small >= 0) {  // none is large enough: a free one gives way
+                Scratch &s = pool.buf[small];
+                FMM_CUDA_TRY(cudaEventSynchronize(s.done));
+                cudaFree(s.ptr);
+                s.ptr = nullptr;
+                s.bytes = 0;
+                continue;
+            }
+            if (take < 0) {  // all are being handed out by other threads
+                pool_free.wait(lock);
+                continue;
+            }
+        }
+        if (take < 0) {
+            if (room < 0) {
+                pool.buf.emplace_back();
+                room = (int)pool.buf.size() - 1;
+            }
+            Scratch &s = pool.buf[room];
+            if (!s.done) FMM_CUDA_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
+            const cudaError_t ce = cudaMalloc(&s.ptr, bytes);
+            if (ce != cudaSuccess && behind < 0) FMM_CUDA_TRY(ce);
+            if (ce == cudaSuccess) {
+                s.bytes = bytes;
+                take = room;
+            } else {  // no memory for another one
+                cudaGetLastError();
+                s.ptr = nullptr;
+                take = behind;
+            }
+        }
+        Scratch &s = pool.buf[take];
+        FMM_CUDA_TRY(cudaStreamWaitEvent(P->stream, s.done, 0));
+        s.busy = true;
+        P->own_scratch = take;
+        *ptr = s.ptr;
+        return FMM_OK;
+    }
+}
+
+int pool_give(Plan *P)
+{
+    std::lock_guard<std::mutex> lock(pool_mutex);
+    Scratch &s = pools[P->opt.device].buf[P->own_scratch];
+    s.busy = false;
+    pool_free.notify_all();
+    FMM_CUDA_TRY(cudaEventRecord(s.done, P->stream));
+    return FMM_OK;
+}
+
+void pool_leave(Plan *P)
+{
+    if (P->own_scratch == Plan::NO_POOL) return;
+    std::lock_guard<std::mutex> lock(pool_mutex);
+    Pool &pool = pools[P->opt.device];
+    P->own_scratch = Plan::NO_POOL;
+    if (--pool.users > 0) return;
+    for (Scratch &s : pool.buf) {
+        cudaFree(s.ptr);
+        if (s.done) cudaEventDestroy(s.done);
+    }
+    pool.buf.clear();
+}
+
 template <typename T, int TC>
 int launch_tc(const OwnArgs<T> &a, int n_items, cudaStream_t st)
 {
@@ -1004,15 +1123,8 @@ int translate(Plan *P, void (*beg)(Plan *, int, int), void (*end)(Plan *))
     const OwnForm &form = P->own_form[type_of<T>()];
     LevelDev &LL = P->lev[P->lmax];
     cudaStream_t st = P->stream;
-    if (form.part_bytes > P->own_part_bytes) {
-        cudaFree(P->own_part);
-        P->own_part = nullptr;
-        P->device_bytes -= P->own_part_bytes;
-        P->own_part_bytes = 0;
-        FMM_CUDA_TRY(dev_alloc(P, &P->own_part, form.part_bytes));
-        P->own_part_bytes = form.part_bytes;
-    }
-    void *part = P->own_part;
+    void *part = nullptr;
+    if (form.part_bytes && (e = pool_take(P, form.part_bytes, &part))) return e;
     auto pass = [&](int l, int which) { return run_pass<T>(P, l, which, lists.pass[l][which], form.pass[l][which], part); };
     const size_t np = (size_t)LL.nb * LL.p * (LL.p + 1) / 2;
     if (std::is_same<T, double>::value)
@@ -1029,6 +1141,10 @@ int translate(Plan *P, void (*beg)(Plan *, int, int), void (*end)(Plan *))
         if (l > P->lmin) e = pass(l, PASS_L2L);
         if (!e) e = pass(l, PASS_M2L);
         end(P);
+    }
+    if (form.part_bytes) {
+        const int g = pool_give(P);
+        if (!e) e = g;
     }
     if (e) return e;
     if (std::is_same<T, double>::value)
@@ -1049,7 +1165,12 @@ int translate_owner(Plan *P, int type, void (*beg)(Plan *, int, int), void (*end
 
 int prepare_owner(Plan *P, int type)
 {
-    return type == OWN_FP64 ? ensure_own<double>(P) : type == OWN_FF ? ensure_own<ff>(P) : ensure_own<float>(P);
+    int e = type == OWN_FP64 ? ensure_own<double>(P) : type == OWN_FF ? ensure_own<ff>(P) : ensure_own<float>(P);
+    // a small scratch too (0.1 ms of a first matvec)
+    void *part = nullptr;
+    const size_t bytes = P->own_form[type].part_bytes;
+    if (!e && bytes && bytes <= SMALL_PART && !(e = pool_take(P, bytes, &part))) e = pool_give(P);
+    return e;
 }
 
 void free_owner(Plan *P)
@@ -1058,7 +1179,7 @@ void free_owner(Plan *P)
     for (OwnForm &f : P->own_form) cudaFree(f.mem);
     cudaFree(P->own_rot64);
     cudaFree(P->own_rot_ff);
-    cudaFree(P->own_part);
+    pool_leave(P);
 }
 
 } // namespace fmm

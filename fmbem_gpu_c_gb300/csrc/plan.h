@@ -273,8 +273,8 @@ struct Plan {
     OwnForm own_form[3];          // per type (OWN_*)
     double *own_rot64 = nullptr;  // folded rotation tables per class, FP64 and float-float
     float4 *own_rot_ff = nullptr; // (hi, hi, lo, lo) per entry
-    void *own_part = nullptr;     // translated expansions of one chunk, before their sums
-    size_t own_part_bytes = 0;
+    enum { NO_SCRATCH = -1, NO_POOL = -2 };
+    int own_scratch = NO_POOL;    // scratch buffer of the last translations; NO_POOL: the plan has not used the pool
     size_t device_bytes = 0;
     char mixed_note[160] = "plan was created without build_mixed";
     // FP32 expansions scaled by degree (low k t): multipole d_n M_n, local L_n / d_n per level

@@ -40,3 +40,22 @@ def test_without_atomics(fm, name):
     first, later = first_and_later(fm, fm.FMM_MIXED if det else getattr(fm, name), fm.icosphere(3, 0.1), k=30.0, depth=4,
                                    p_levels={2: 12, 3: 10, 4: 8}, deterministic=det)
     assert first < later + (0.45e-3 if name == "FMM_FLOAT2" else 0.2e-3)
+
+
+def test_plans_share_scratch(fm):
+    """Plans on one device share the scratch of the translations without atomics (up to 128 MB): each more that has
+    run an FP64 matvec holds little beyond what it held before."""
+    import torch
+
+    V, F = fm.icosphere(5, 0.2)
+    plans, held = [], []
+    for _ in range(4):
+        plan = fm.Plan(V, F, k=73.0, depth=5, p_levels={2: 24, 3: 18, 4: 14, 5: 10}, rule=1, a=0.5, b=0.0, c=-1.0)
+        before = torch.cuda.mem_get_info()[0]
+        y = plan.matvec(np.ones(plan.nf, np.complex128), fm.FMM_FP64)
+        held.append(before - torch.cuda.mem_get_info()[0])
+        plans.append((plan, y))
+    for plan, y in plans:
+        assert np.array_equal(y, plan.matvec(np.ones(plan.nf, np.complex128), fm.FMM_FP64))
+        plan.close()
+    assert max(held[1:]) < 16 << 20
