@@ -956,16 +956,69 @@ int build_rcr_lists(Plan *P)
     return FMM_OK;
 }
 
-// Columns and rows per unit of each pass, chosen at plan creation by timing on this plan's own lists
-// and tables (one right-hand side): the columns of pick_tile, half and a quarter of them (passes of
-// few translations fill more SMs with narrower tiles), units of four rows, or of two (more units
-// for the threads of a narrow tile).  Matvec results do not depend on the choice beyond the order of
-// the FP32 atomic additions.  Passes that run in a tensor-core form are not timed.
-int tune_rcr_tiles(Plan *P)
+// Columns and rows per unit of a pass, by timing on this plan's own list and tables (one right-hand side): the
+// columns of pick_tile, half and a quarter of them (passes of few translations fill more SMs with narrower
+// tiles), units of four rows, or of two (more units for the threads of a narrow tile).  Matvec results do not
+// depend on the choice beyond the order of the FP32 atomic additions.
+static int tune_list(Plan *P, int l, int which, RcrList &Lst)
+{
+    TileForm &f = Lst.form[FORM_FOLDED];
+    if (f.tuned || Lst.key_beg.empty() || Lst.key_beg.back() == 0) return FMM_OK;
+    std::vector<int2> cand;
+    for (int tc = f.tc; tc >= 4 && 4 * tc >= f.tc; tc /= 2)
+        for (int bal = 0; bal < 2; bal++) cand.push_back({tc, bal});
+    cudaEvent_t a = nullptr, b = nullptr;
+    float best = 1e30f;
+    int2 pick = cand[0];
+    int rc = FMM_OK;
+    auto timed = [&](float *ms) -> int {
+        FMM_CUDA_TRY(cudaEventRecord(a, P->stream));
+        if (int e = launch_pass32(P, l, which, 1, P->stream)) return e;
+        FMM_CUDA_TRY(cudaEventRecord(b, P->stream));
+        FMM_CUDA_TRY(cudaEventSynchronize(b));
+        FMM_CUDA_TRY(cudaEventElapsedTime(ms, a, b));
+        return FMM_OK;
+    };
+    if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) {
+        fmm_set_error("tile tuning: %s", cudaGetErrorString(cudaGetLastError()));
+        rc = FMM_ERR_CUDA;
+    }
+    const int dense = Lst.td.on;
+    Lst.td.on = 0;
+    for (auto &c : cand) {
+        f.tc = c.x;
+        f.bal = c.y;
+        f.items_nrhs = 0;
+        float tot = 0.f;
+        for (int rep = 0; rep < 4 && rc == FMM_OK; rep++) {
+            float ms = 0.f;
+            rc = timed(&ms);
+            if (rep > 0) tot += ms;
+        }
+        if (rc != FMM_OK) break;
+        if (tot < best) {
+            best = tot;
+            pick = c;
+        }
+    }
+    Lst.td.on = dense;
+    if (a) cudaEventDestroy(a);
+    if (b) cudaEventDestroy(b);
+    f.tc = pick.x;
+    f.bal = pick.y;
+    f.items_nrhs = 0;
+    f.tuned = rc == FMM_OK;
+    return rc;
+}
+
+// The tile shapes of a plan's passes, at plan creation.  Passes that run in the dense tensor-core form are left to
+// scenes (dense_too), which run all passes on the tiles: with the widest tile and units of four rows instead of what
+// timing picks there, 16 spheres of 2,420 triangles took 560 us for 482.
+int tune_rcr_tiles(Plan *P, bool dense_too)
 {
     // FMMBEM_TILE_BAL=0/1/2 forces one shape on every pass, for tests: 0 the columns of pick_tile and
     // units of four rows, 1 units of two rows, 2 half the columns and units of two rows
-    if (const char *env = getenv("FMMBEM_TILE_BAL")) {
+    if (const char *env = dense_too ? nullptr : getenv("FMMBEM_TILE_BAL")) {
         const int bal = std::max(0, std::min(2, atoi(env)));
         for (int l = P->lmin; l <= P->lmax; l++)
             for (RcrList *R : {&P->lev[l].m2m, &P->lev[l].m2l, &P->lev[l].l2l})
@@ -973,53 +1026,19 @@ int tune_rcr_tiles(Plan *P)
                     f.bal = bal ? 1 : 0;
                     if (bal == 2) f.tc = std::max(4, f.tc / 2);
                     f.items_nrhs = 0;
+                    f.tuned = true;
                 }
         return FMM_OK;
     }
-    cudaEvent_t a, b;
-    FMM_CUDA_TRY(cudaEventCreate(&a));
-    FMM_CUDA_TRY(cudaEventCreate(&b));
-    int rc = FMM_OK;
-    for (int l = P->lmin; l <= P->lmax && rc == FMM_OK; l++) {
+    for (int l = P->lmin; l <= P->lmax; l++) {
         LevelDev &L = P->lev[l];
-        for (int which = PASS_M2M; which <= PASS_L2L && rc == FMM_OK; which++) {
+        for (int which = PASS_M2M; which <= PASS_L2L; which++) {
             if (which != PASS_M2L && l == P->lmin) continue;
             RcrList &Lst = which == PASS_M2M ? L.m2m : which == PASS_M2L ? L.m2l : L.l2l;
-            if (Lst.key_beg.empty() || Lst.key_beg.back() == 0 || Lst.td.on) continue;
-            TileForm &f = Lst.form[FORM_FOLDED];
-            std::vector<int2> cand;
-            for (int tc = f.tc; tc >= 4 && 4 * tc >= f.tc; tc /= 2)
-                for (int bal = 0; bal < 2; bal++) cand.push_back({tc, bal});
-            float best = 1e30f;
-            int2 pick = cand[0];
-            for (auto &c : cand) {
-                f.tc = c.x;
-                f.bal = c.y;
-                f.items_nrhs = 0;
-                float tot = 0.f;
-                for (int rep = 0; rep < 4 && rc == FMM_OK; rep++) {
-                    if (cudaEventRecord(a, P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    if (rc == FMM_OK) rc = launch_pass32(P, l, which, 1, P->stream);
-                    if (rc == FMM_OK && cudaEventRecord(b, P->stream) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    if (rc == FMM_OK && cudaEventSynchronize(b) != cudaSuccess) rc = FMM_ERR_CUDA;
-                    float ms = 0.f;
-                    cudaEventElapsedTime(&ms, a, b);
-                    if (rep > 0) tot += ms;
-                }
-                if (rc != FMM_OK) break;
-                if (tot < best) {
-                    best = tot;
-                    pick = c;
-                }
-            }
-            f.tc = pick.x;
-            f.bal = pick.y;
-            f.items_nrhs = 0;
+            if (Lst.td.on && !dense_too) continue;
+            if (int e = tune_list(P, l, which, Lst)) return e;
         }
     }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    if (rc == FMM_ERR_CUDA) fmm_set_error("tile tuning: %s", cudaGetErrorString(cudaGetLastError()));
-    return rc;
+    return FMM_OK;
 }
 } // namespace fmm

@@ -243,7 +243,7 @@ static int plan_create_impl(std::vector<double> &&V, std::vector<int> &&F, const
     if (P->opt.build_mixed) {
         TRY(build_rcr_lists(P));
         TRY(tune_tc_dense(P));
-        TRY(tune_rcr_tiles(P));
+        TRY(tune_rcr_tiles(P, false));
         TRY(tune_tc3(P));
         // each pass once for one column, so that the first matvec finds its lists and work items (on 81,920
         // triangles they take 3 ms; it took 4.4 ms where later ones take 1.3)

@@ -101,6 +101,7 @@ struct KeyedList {
 // for (units_tc, units_bal): rotations (the second from at3), coaxial; rounds of each stage.
 struct TileForm {
     int tc = 8, bal = 0;
+    bool tuned = false;           // tc and bal are final (scenes hold the units' addresses from then on)
     int4 *items = nullptr;
     size_t items_cap = 0;
     int n_items = 0, items_nrhs = 0;
@@ -361,7 +362,7 @@ int tune_tc3(Plan *P);
 // M2M / L2L octants of equal z bit.  cls[key] = class, rep[class] = its first key.
 void direction_classes(const Plan *P, int which, int nkeys, std::vector<int> &cls, std::vector<int> &rep);
 int build_rcr_lists(Plan *P);
-int tune_rcr_tiles(Plan *P);
+int tune_rcr_tiles(Plan *P, bool dense_too);
 size_t rcr_tile_smem(int p, int tc);
 constexpr int MAX_MIXED_ORDER = 60;
 int set_tile_tables(const Plan *P, RcrList &Lst, int form, RcrPass &ps);

@@ -431,6 +431,7 @@ static int build_scene(Scene *S)
     std::vector<int4> items;
     for (int i = 0; i < n; i++) {
         Plan *P = S->plans[i];
+        if (int e = tune_rcr_tiles(P, true)) return e;
         for (int l = P->lmin; l <= P->lmax; l++)
             for (int which = PASS_M2M; which <= PASS_L2L; which++) {
                 RcrPass ps;
