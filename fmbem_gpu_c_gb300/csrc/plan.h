@@ -78,6 +78,7 @@ struct TcShape {
 struct TcDense {
     int on = 0;                   // the pass runs on the tensor cores
     int pin = 0, pout = 0;        // source and destination orders
+    int wide = 0;                 // the kernel for expansions of 64 GB and more, whatever their size
     TcShape sh = {};
     int ncls = 0;                 // operators
     std::vector<int> cls_of_dir;  // key (direction or octant) -> operator

@@ -51,6 +51,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace fmm {
@@ -297,6 +298,18 @@ __device__ __forceinline__ TileRow tile_row(const TcPass &ps, int4 it, int r, co
     return o;
 }
 
+// What is copied of the cnt coefficients from c0 on of expansion `row` (P2 coefficients each; none where it is
+// negative): n words of 16 bytes from the from-th on; with an odd first coefficient the one before it too.
+struct RowCopy {
+    unsigned long long from;
+    int n;
+};
+__host__ __device__ __forceinline__ RowCopy row_copy(int row, int P2, int c0, int cnt)
+{
+    const unsigned long long e = (unsigned long long)(unsigned)row * (unsigned)P2 + (unsigned)c0;
+    return RowCopy{e >> 1, row < 0 ? 0 : (cnt + (int)(e & 1) + 1) >> 1};
+}
+
 // Up to eight coefficient pairs (m = 0..last) of a degree from the columns of their sums (from p on) and
 // differences (from q on, none for m = 0 where `first`) to y[m], y[-m] of the lane's row; columns past the last
 // pair's are not used.
@@ -323,7 +336,9 @@ __device__ __forceinline__ void unfold(uint32_t p, uint32_t q, int last, const f
     }
 }
 
-template <bool FOLD>
+// WIDE: source expansions of 64 GB and more, whose 16-byte words take more than 32 bits to count (a third
+// exchange per row; in all passes it would cost 0.5 to 2 %).
+template <bool FOLD, bool WIDE>
 __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_constant__ TcPass ps)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -447,9 +462,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
         Ring rr;
         for (int i = 0; i < ntile && ok; i++) {
             const int4 it = ps.items[tile(i)];
-            long long at[NR];
+            int at[NR];
 #pragma unroll
-            for (int j = 0; j < NR; j++) at[j] = (long long)tile_row(ps, it, r0 + lane + 32 * j, ps.g_src).row * ps.P2;
+            for (int j = 0; j < NR; j++) at[j] = tile_row(ps, it, r0 + lane + 32 * j, ps.g_src).row;
             for (int pc = 0; pc < sh.npiece; pc++) {
                 const int c0 = sh.piece[pc].c0, cnt = sh.piece[pc].cnt;
                 ok = mbar_wait_warp(smem_u32(rempty + rr.i), rr.par ^ 1);
@@ -458,17 +473,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
                 const char *src = reinterpret_cast<const char *>(ps.src) + 16 * lane;
 #pragma unroll
                 for (int j = 0; j < NR; j++) {
-                    // the lane's own row: its first 16 bytes, counted in 16 bytes, and their number
-                    const int odd = (int)((at[j] + c0) & 1);
-                    const uint32_t first = (uint32_t)((at[j] + c0) >> 1);
-                    const int num = at[j] >= 0 ? (cnt + odd + 1) >> 1 : 0;
+                    const RowCopy own = row_copy(at[j], ps.P2, c0, cnt);  // of the lane's own row
+                    const uint32_t low = (uint32_t)own.from, high = (uint32_t)(own.from >> 32);
                     for (int k0 = 0; k0 < 32; k0 += 8) {
-                        uint32_t from[8];
+                        typename std::conditional<WIDE, unsigned long long, uint32_t>::type from[8];
                         int n[8];
 #pragma unroll
                         for (int k = 0; k < 8; k++) {
-                            from[k] = __shfl_sync(0xffffffffu, first, k0 + k);
-                            n[k] = __shfl_sync(0xffffffffu, num, k0 + k);
+                            from[k] = __shfl_sync(0xffffffffu, low, k0 + k);
+                            if constexpr (WIDE) from[k] |= (unsigned long long)__shfl_sync(0xffffffffu, high, k0 + k) << 32;
+                            n[k] = __shfl_sync(0xffffffffu, own.n, k0 + k);
                         }
 #pragma unroll
                         for (int k = 0; k < 8; k++, slot += sh.row_stride)
@@ -733,6 +747,8 @@ static int build_tc_dense(Plan *P, int l, int which)
     const char *env = getenv("FMMBEM_TENSOR_FOLD");
     const int fold = env ? atoi(env) != 0 : fold_pays(Lst->key_beg.back());
     if (!tc_shape(pin, pout, fold, g.sh)) return FMM_OK;
+    const char *wide = getenv("FMMBEM_TENSOR_WIDE");  // 1: the kernel for 64 GB and more, for tests
+    g.wide = wide && atoi(wide) != 0;
     g.pin = pin;
     g.pout = pout;
     const int nkeys = (int)Lst->key_beg.size() - 1, P2i = pin * pin, P2o = pout * pout;
@@ -908,9 +924,11 @@ int launch_tc_dense(Plan *P, int l, int which, int nrhs, cudaStream_t st)
     ps.dst = rp.dst;
     ps.err = P->tc_err;
     const size_t sm = tc_smem_bytes(g.sh);
-    const auto kernel = g.sh.fold ? tc_dense_kernel<true> : tc_dense_kernel<false>;
-    static size_t attr[2] = {0, 0};
-    e = raise_smem_limit((const void *)kernel, sm, &attr[g.sh.fold ? 1 : 0]);
+    const bool wide = g.wide || (size_t)rp.nsrc * nrhs * ps.P2 >= (size_t)1 << 33;
+    const auto kernel = g.sh.fold ? (wide ? tc_dense_kernel<true, true> : tc_dense_kernel<true, false>)
+                                  : (wide ? tc_dense_kernel<false, true> : tc_dense_kernel<false, false>);
+    static size_t attr[4] = {0, 0, 0, 0};
+    e = raise_smem_limit((const void *)kernel, sm, &attr[(g.sh.fold ? 1 : 0) + (wide ? 2 : 0)]);
     if (e) return e;
     // persistent: one CTA per SM (its shared memory and 512 TMEM columns take the SM)
     static int nsm = 0;
