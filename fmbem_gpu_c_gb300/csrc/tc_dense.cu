@@ -42,6 +42,10 @@
 // and splits.  At p = 14 (one set of accumulators) reading them out, 10,000 of 36,000 cycles, is not hidden.  An earlier
 // form, with the whole operator, A in shared memory and one atomic per 16 bytes of output, took 5.96
 // and 5.58 ms (its load/store unit 80 % busy with rows read 16 bytes a lane, A's stores and the atomics).
+// Orders up to 5 are bound by the epilogue's work per row: one group of all degrees, a tile each for the two warps of
+// a quarter in turn, and rows on odd coefficients (odd p^2) as many at a time as the others (649,008 translations, one
+// column: p = 4 115 -> 95 us, p = 5 216 -> 138, p = 9 414 -> 309, p = 10 274 -> 256; the
+// times above are from before).
 // What made the difference: half the products; A through TMEM; source rows by cp.async, a row per
 // instruction; outputs by bulk reductions, a row's group per instruction; the MMA's issue by one
 // elected thread with operands in uniform registers (500 instead of 950 cycles per six MMAs).
@@ -182,10 +186,12 @@ static bool tc_shape(int pin, int pout, int fold, TcShape &g)
         }
         g.epi_stride = tc_stride(group);
         for (int i = 0; i < g.nsub; i++) {
-            // groups of degrees of the epilogue, few of them and few that start on an odd coefficient, and
-            // the warp of a quarter that takes each (the larger first, to the warp with less)
+            // groups of degrees of the epilogue, few of them and few that start on an odd coefficient (all degrees in
+            // one where it holds them), and the warp of a quarter that takes each (the larger first, to the warp
+            // with less; with two sets of accumulators the warps change roles from tile to tile)
             TcSub &s = g.sub[i];
-            const int most = std::min(group, std::max(2 * s.end - 1, (s.end * s.end - s.beg * s.beg) / 2 + 8));
+            const int all = s.end * s.end - s.beg * s.beg;
+            const int most = all <= group ? group : std::min(group, std::max(2 * s.end - 1, all / 2 + 8));
             cut(s.end - s.beg, [&](int a, int b) {
                 a += s.beg, b += s.beg;
                 return b * b - a * a > most ? -1 : 3 + 2 * (a & 1);
@@ -286,6 +292,31 @@ struct Ring {
 struct TileRow {
     int row = -1, dir = 0;
 };
+
+// the same looked up ahead: what the row is made of, as loaded
+struct RowAhead {
+    int box = 0, rhs = -1, dir = 0;
+};
+__device__ __forceinline__ RowAhead row_ahead(const TcPass &ps, int4 it, int r, const int *box)
+{
+    RowAhead o;
+    if (r < it.z) {
+        const int e = it.y + r, t = (int)(((unsigned long long)e * ps.per) >> ps.shift);
+        o.box = __ldg(box + t);
+        o.rhs = e - t * ps.nrhs;
+        o.dir = __ldg(ps.g_dir + t);
+    }
+    return o;
+}
+__device__ __forceinline__ TileRow row_now(const TcPass &ps, const RowAhead &a)
+{
+    TileRow o;
+    if (a.rhs >= 0) {
+        o.row = a.box * ps.nrhs + a.rhs;
+        o.dir = a.dir;
+    }
+    return o;
+}
 
 __device__ __forceinline__ TileRow tile_row(const TcPass &ps, int4 it, int r, const int *box)
 {
@@ -460,11 +491,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
         constexpr int NR = TC_M / TC_RW / 32;  // rows per lane
         const int r0 = (warp - 2) * 32 * NR;
         Ring rr;
+        // rows are looked up a tile ahead, items two
+        auto item = [&](int i) { return i < ntile ? ps.items[tile(i)] : make_int4(0, 0, 0, 0); };
+        RowAhead next[NR];
+        int4 it = item(0);
+#pragma unroll
+        for (int j = 0; j < NR; j++) next[j] = row_ahead(ps, it, r0 + lane + 32 * j, ps.g_src);
+        it = item(1);
         for (int i = 0; i < ntile && ok; i++) {
-            const int4 it = ps.items[tile(i)];
             int at[NR];
 #pragma unroll
-            for (int j = 0; j < NR; j++) at[j] = tile_row(ps, it, r0 + lane + 32 * j, ps.g_src).row;
+            for (int j = 0; j < NR; j++) {
+                at[j] = row_now(ps, next[j]).row;
+                next[j] = row_ahead(ps, it, r0 + lane + 32 * j, ps.g_src);
+            }
+            it = item(i + 2);
             for (int pc = 0; pc < sh.npiece; pc++) {
                 const int c0 = sh.piece[pc].c0, cnt = sh.piece[pc].cnt;
                 ok = mbar_wait_warp(smem_u32(rempty + rr.i), rr.par ^ 1);
@@ -596,7 +637,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
             ok = mbar_wait_warp(smem_u32(accf + a), set_par(i));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
-            unsigned left = (eh ? s.second : ~s.second) & ((1u << s.ngrp) - 1);
+            const unsigned mine = ((two ? eh ^ (i & 1) : eh) ? s.second : ~s.second) & ((1u << s.ngrp) - 1);
+            unsigned left = mine;
             while (left) {
                 const int g = __ffs(left) - 1, na = s.grp[g], nb = s.grp[g + 1], c0 = na * na, cnt = nb * nb - c0;
                 const long long e0 = (long long)tr.row * ps.P2o + c0;
@@ -636,11 +678,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
                                 tc_reduce(ps.dst + (long long)row[k] * ps.P2o + (c0 + odd), from + (uint32_t)((k0 + k) * es), size);
                         }
                     }
-                } else {
-                    for (int k = 0; k < 32; k++) {
-                        const unsigned long long to = __shfl_sync(0xffffffffu, (unsigned long long)(o + odd), k);
-                        const uint32_t sk = __shfl_sync(0xffffffffu, size, k), ok_ = __shfl_sync(0xffffffffu, odd, k);
-                        if (sk && elect_one()) tc_reduce(reinterpret_cast<float2 *>(to), st0 + (uint32_t)(k * es) + 16 * ok_, sk);
+                } else {  // (an odd p^2: every second row of destinations begins on an odd coefficient)
+                    for (int k0 = 0; k0 < 32; k0 += 8) {
+                        int row[8];
+#pragma unroll
+                        for (int k = 0; k < 8; k++) row[k] = __shfl_sync(0xffffffffu, tr.row, k0 + k);
+                        if (elect_one()) {
+#pragma unroll
+                            for (int k = 0; k < 8; k++) {
+                                const int odd_k = (int)(((unsigned)row[k] * (unsigned)ps.P2o + (unsigned)c0) & 1u);
+                                const uint32_t size_k = 8u * (uint32_t)((cnt - odd_k) & ~1);
+                                if (row[k] >= 0 && size_k)
+                                    tc_reduce(ps.dst + (long long)row[k] * ps.P2o + (c0 + odd_k), st0 + (uint32_t)((k0 + k) * es) + 16 * odd_k, size_k);
+                            }
+                        }
                     }
                 }
                 if (elect_one()) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -649,7 +700,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_dense_kernel(const __grid_co
                     if (odd + whole < cnt) atomicAdd(o + cnt - 1, st[odd + cnt - 1]);
                 }
             }
-            if (((eh ? s.second : ~s.second) & ((1u << s.ngrp) - 1)) == 0) {  // no group of this range is the warp's
+            if (mine == 0) {  // no group of this range is the warp's
                 asm volatile("tcgen05.fence::before_thread_sync;");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(acce + a));
