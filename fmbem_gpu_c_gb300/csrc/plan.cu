@@ -973,7 +973,8 @@ extern "C" int fmm_far_field(fmm_plan *plan, const cuDoubleComplex *p, const dou
     double2 *pd = nullptr, *od = nullptr;
     double *ptd = nullptr;
     FMM_CUDA_TRY(cudaMalloc(&pd, sizeof(double2) * P->nf));
-    FMM_CUDA_TRY(cudaMalloc(&od, sizeof(double2) * (size_t)std::max(1, npts) * (1 + far_slices(P->nf, std::max(1, npts)))));
+    const int slices = far_slices(P->nf, std::max(1, npts));
+    FMM_CUDA_TRY(cudaMalloc(&od, sizeof(double2) * (size_t)std::max(1, npts) * (slices > 1 ? 1 + slices : 1)));
     FMM_CUDA_TRY(cudaMalloc(&ptd, sizeof(double) * 3 * std::max(1, npts)));
     FMM_CUDA_TRY(cudaMemcpy(pd, p, sizeof(double2) * P->nf, cudaMemcpyDefault));
     FMM_CUDA_TRY(cudaMemcpy(ptd, pts, sizeof(double) * 3 * npts, cudaMemcpyDefault));

@@ -1071,6 +1071,7 @@ __global__ void __launch_bounds__(32 * FAR_P) far_field_kernel(const double *V, 
             for (int a = 0; a < 3; a++) sx[q][a][lane] = nod[a] * b[0] + nod[3 + a] * b[1] + nod[6 + a] * b[2];
         }
         __syncthreads();
+        if (t >= npts) continue;  // (a whole warp)
         double2 L = make_double2(0.0, 0.0), M = make_double2(0.0, 0.0);
         double dn = 0.0;
         for (int a = 0; a < 3; a++) dn += (sx[0][a][lane] - y[a]) * sn[a][lane];
@@ -1106,21 +1107,28 @@ __global__ void __launch_bounds__(32 * FAR_P) far_field_kernel(const double *V, 
     if (lane == 0 && t < npts) out[(size_t)blockIdx.y * npts + t] = acc;
 }
 
+// out[t] = the sum of point t's slices, a warp each
 __global__ void far_sum_kernel(const double2 *part, int npts, int slices, double2 *out)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npts; t += gridDim.x * blockDim.x) {
-        double2 a = part[t];
-        for (int s = 1; s < slices; s++) a = cadd(a, part[(size_t)s * npts + t]);
-        out[t] = a;
+    const int lane = threadIdx.x & 31;
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < npts; t += (gridDim.x * blockDim.x) >> 5) {
+        double2 a = make_double2(0.0, 0.0);
+        for (int s = lane; s < slices; s += 32) a = cadd(a, part[(size_t)s * npts + t]);
+        for (int o = 16; o > 0; o >>= 1) {
+            a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+            a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+        }
+        if (lane == 0) out[t] = a;
     }
 }
 
-// Slices of the elements: enough blocks for eight on each of 152 SMs, a slice of at least 128 elements
-// (few points against many elements leave SMs idle otherwise).
+// Slices of the elements: enough blocks for eight on each of 152 SMs, down to the 32 elements that a block takes at
+// a time (with at least 128, 320 triangles and up to 33 points were two to five blocks: 190 us against 97 with a
+// block per point).
 int far_slices(int nf, int npts)
 {
     const int blocks = (npts + FAR_P - 1) / FAR_P;
-    return std::max(1, std::min((8 * 152 + blocks - 1) / blocks, nf / 128));
+    return std::max(1, std::min((8 * 152 + blocks - 1) / blocks, (nf + FAR_E - 1) / FAR_E));
 }
 
 // out: npts values, and behind them the sums of far_slices() slices where there are several
@@ -1132,7 +1140,7 @@ int launch_far_field(Plan *P, const double2 *p, const double *pts, int npts, dou
     double2 *part = slices > 1 ? out + npts : out;
     far_field_kernel<<<dim3((npts + FAR_P - 1) / FAR_P, slices), 32 * FAR_P, 0, P->stream>>>(
         P->V_dev, P->F_dev, P->nf, P->opt.k, bco, cco, P->opt.rule, p, pts, npts, per, part);
-    if (slices > 1) far_sum_kernel<<<std::min((npts + 127) / 128, 152 * 8), 128, 0, P->stream>>>(part, npts, slices, out);
+    if (slices > 1) far_sum_kernel<<<std::min((npts + 3) / 4, 152 * 8), 128, 0, P->stream>>>(part, npts, slices, out);
     FMM_CUDA_TRY(cudaGetLastError());
     return FMM_OK;
 }
