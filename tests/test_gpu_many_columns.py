@@ -45,3 +45,27 @@ def test_whole_rotations_match_fp64(fm, p2, p3, monkeypatch):
         # a few columns of the same plan take the folded form
         assert np.linalg.norm(plan.matvec(X[1], fm.FMM_MIXED) - Y[1]) < 1e-5 * np.linalg.norm(Y[1])
         plan.close()
+
+
+def test_small_orders_keep_wide_tiles(fm):
+    """Orders of 3 to 5 on 5,120 triangles: 33 columns cost 0.42 ms in tiles of 64 columns, 0.62 in tiles of 32; 15
+    columns, in the other form of the tiles, 0.22."""
+    import time
+
+    import torch
+
+    plan = fm.Plan(*fm.geodesic_sphere(16, 0.1), k=25.0, depth=4, p_levels={2: 5, 3: 4, 4: 3}, rule=1, a=0.5, b=0.0, c=-1.0)
+
+    def best(nrhs):
+        x = torch.ones(plan.nf * nrhs, dtype=torch.complex128, device="cuda")
+        y = torch.empty_like(x)
+        t = []
+        for _ in range(30):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            plan.matvec(x, fm.FMM_MIXED, out=y)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    assert best(33) < 2.4 * best(15)
+    plan.close()
