@@ -47,12 +47,11 @@ __device__ __forceinline__ ff operator+(ff a, ff b)
     return ff(s, e);
 }
 
-// nearest float-float to a double, and back
+// nearest float-float to a double
 __device__ __forceinline__ ff ff_from(double d)
 {
     const float h = (float)d;
     return ff(h, (float)(d - (double)h));
 }
-__device__ __forceinline__ double ff_to(ff a) { return (double)a.hi + (double)a.lo; }
 
 } // namespace fmm

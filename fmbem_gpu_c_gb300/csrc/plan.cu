@@ -787,8 +787,9 @@ struct PlanOps {
         baxpy_kernel<<<dim3(blas_grid(P->nf) / 2 + 1, 1, R), 256, 0, P->stream>>>(P->gm_V, vj(), P->nf, nvec, P->gm_dev_h,
                                                                                   nvec, W, P->nf, P->nf);
     }
-    // One column of up to 65,536 unknowns: a block's share of W is at most 432 entries; larger ones are
-    // bound by reading the vectors (81,920 unknowns, 30 vectors: 39 MB a pass), not by launches.
+    // One column of up to 65,536 unknowns: a block's share of W is at most 432 entries.  60 steps on a matvec of
+    // order 2, in one launch each against step by step: 5,120 unknowns 10.9 against 13.3 ms, 64,980 27.9 against 31.8;
+    // beyond, the vectors' reading takes over (81,920 34.7 against 38.4, 200,000 58.5 against 59.5).
     bool step_fits() const { return P->nf <= 65536; }
     int step(int nvec, double2 *W, double2 *next, std::vector<double2> &h1, std::vector<double2> &h2, std::vector<double> &hn)
     {
