@@ -534,8 +534,8 @@ static int ensure_classes(RcrList &Lst)
     cudaError_t ce = cudaMalloc(&cs, sizeof(int) * n);
     if (ce == cudaSuccess) ce = cudaMalloc(&Lst.cdst, sizeof(int) * n);
     if (ce == cudaSuccess) ce = cudaMalloc(&Lst.cdir, sizeof(short) * n);
-    if (ce == cudaSuccess) ce = cudaMemcpy(tmp, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaMemcpy(tmp + n, Lst.key_beg.data(), sizeof(int) * (nkeys + 1), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = upload(tmp, perm.data(), sizeof(int) * n);
+    if (ce == cudaSuccess) ce = upload(tmp + n, Lst.key_beg.data(), sizeof(int) * (nkeys + 1));
     if (ce == cudaSuccess) {
         class_order_kernel<<<std::min((n + 255) / 256, 152 * 16), 256>>>(n, tmp, Lst.src, Lst.dst, tmp + n, nkeys, Lst.key0, cs,
                                                                         Lst.cdst, Lst.cdir);
@@ -575,7 +575,7 @@ static int ensure_items(RcrList &Lst, int form, int nrhs, size_t ws_bytes)
         FMM_CUDA_TRY(cudaMalloc(&f.items, sizeof(int4) * items.size()));
         f.items_cap = items.size();
     }
-    if (!items.empty()) FMM_CUDA_TRY(cudaMemcpy(f.items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice));
+    if (!items.empty()) FMM_CUDA_TRY(upload(f.items, items.data(), sizeof(int4) * items.size()));
     f.n_items = (int)items.size();
     f.items_nrhs = nrhs;
     return FMM_OK;
@@ -730,7 +730,7 @@ static int build_tile_tables(Plan *P)
     for (int n = 0; n < pmax; n++)
         for (int m = 0; m <= n; m++) pairs.push_back((n * n + n) | m << 16);
     FMM_CUDA_TRY(dev_alloc(P, (void **)&P->pairs, sizeof(int) * pairs.size()));
-    FMM_CUDA_TRY(cudaMemcpy(P->pairs, pairs.data(), sizeof(int) * pairs.size(), cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(P->pairs, pairs.data(), sizeof(int) * pairs.size()));
     return FMM_OK;
 }
 
@@ -823,8 +823,8 @@ static int ensure_units(const std::vector<int> &rot_off, TileForm &f, bool fold,
     f.units_tc = 0;
     FMM_CUDA_TRY(cudaMalloc(&f.urot, sizeof(int2) * ur.size()));
     FMM_CUDA_TRY(cudaMalloc(&f.ucoax, sizeof(int) * uc.size()));
-    FMM_CUDA_TRY(cudaMemcpy(f.urot, ur.data(), sizeof(int2) * ur.size(), cudaMemcpyHostToDevice));
-    FMM_CUDA_TRY(cudaMemcpy(f.ucoax, uc.data(), sizeof(int) * uc.size(), cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(f.urot, ur.data(), sizeof(int2) * ur.size()));
+    FMM_CUDA_TRY(upload(f.ucoax, uc.data(), sizeof(int) * uc.size()));
     f.units_tc = f.tc;
     f.units_bal = f.bal;
     return FMM_OK;
@@ -898,8 +898,8 @@ static int upload_list(Plan *P, RcrList &Lst, int which, const std::vector<int> 
     if (T == 0) return FMM_OK;
     FMM_CUDA_TRY(dev_alloc(P, (void **)&Lst.src, sizeof(int) * T));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&Lst.dst, sizeof(int) * T));
-    FMM_CUDA_TRY(cudaMemcpy(Lst.src, gs.data(), sizeof(int) * T, cudaMemcpyHostToDevice));
-    FMM_CUDA_TRY(cudaMemcpy(Lst.dst, gd.data(), sizeof(int) * T, cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(Lst.src, gs.data(), sizeof(int) * T));
+    FMM_CUDA_TRY(upload(Lst.dst, gd.data(), sizeof(int) * T));
     return FMM_OK;
 }
 

@@ -426,7 +426,7 @@ static int ensure_ff(Plan *P)
     if (P->scaled) {
         const std::vector<double> &d = P->dsc[P->lmax];
         FMM_CUDA_TRY(dev_alloc(P, (void **)&P->dsc_leaf_dev, sizeof(double) * d.size()));
-        FMM_CUDA_TRY(cudaMemcpy(P->dsc_leaf_dev, d.data(), sizeof(double) * d.size(), cudaMemcpyHostToDevice));
+        FMM_CUDA_TRY(upload(P->dsc_leaf_dev, d.data(), sizeof(double) * d.size()));
     }
     FMM_CUDA_TRY(cudaGetLastError());
     P->ff_ready = 1;
@@ -845,7 +845,7 @@ int near_transpose_values(Plan *P, const double2 *vals, double2 *valsT)
     long long nnz = P->num_near;
     long long *perm_dev = nullptr;
     FMM_CUDA_TRY(cudaMalloc(&perm_dev, sizeof(long long) * std::max<long long>(1, nnz)));
-    FMM_CUDA_TRY(cudaMemcpy(perm_dev, perm.data(), sizeof(long long) * nnz, cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(perm_dev, perm.data(), sizeof(long long) * nnz));
     gather_kernel<<<152 * 8, 256, 0, P->stream>>>(vals, perm_dev, nnz, valsT);
     FMM_CUDA_TRY(cudaGetLastError());
     FMM_CUDA_TRY(cudaStreamSynchronize(P->stream));
@@ -863,12 +863,12 @@ int build_transpose(Plan *P)
     if (st) return st;
     long long *perm_dev = nullptr;
     FMM_CUDA_TRY(cudaMalloc(&perm_dev, sizeof(long long) * std::max<long long>(1, nnz)));
-    FMM_CUDA_TRY(cudaMemcpy(perm_dev, perm.data(), sizeof(long long) * nnz, cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(perm_dev, perm.data(), sizeof(long long) * nnz));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&P->nearT_beg, sizeof(int) * (P->nf + 1)));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&P->nearT_col, sizeof(int) * std::max<long long>(1, nnz)));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&P->nearT64, sizeof(double2) * std::max<long long>(1, nnz)));
-    FMM_CUDA_TRY(cudaMemcpy(P->nearT_beg, tb.data(), sizeof(int) * (P->nf + 1), cudaMemcpyHostToDevice));
-    FMM_CUDA_TRY(cudaMemcpy(P->nearT_col, tc.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(P->nearT_beg, tb.data(), sizeof(int) * (P->nf + 1)));
+    FMM_CUDA_TRY(upload(P->nearT_col, tc.data(), sizeof(int) * nnz));
     gather_kernel<<<152 * 8, 256, 0, P->stream>>>(P->near64, perm_dev, nnz, P->nearT64);
     FMM_CUDA_TRY(cudaGetLastError());
     if (P->U32) {

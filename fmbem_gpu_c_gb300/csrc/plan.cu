@@ -977,8 +977,14 @@ extern "C" int fmm_far_field(fmm_plan *plan, const cuDoubleComplex *p, const dou
     const int slices = far_slices(P->nf, std::max(1, npts));
     FMM_CUDA_TRY(cudaMalloc(&od, sizeof(double2) * (size_t)std::max(1, npts) * (slices > 1 ? 1 + slices : 1)));
     FMM_CUDA_TRY(cudaMalloc(&ptd, sizeof(double) * 3 * std::max(1, npts)));
-    FMM_CUDA_TRY(cudaMemcpy(pd, p, sizeof(double2) * P->nf, cudaMemcpyDefault));
-    FMM_CUDA_TRY(cudaMemcpy(ptd, pts, sizeof(double) * 3 * npts, cudaMemcpyDefault));
+    // (host memory on the plan's own stream; device memory after what the default stream has before it)
+    auto copy_in = [&](void *to, const void *from, size_t n) {
+        if (!is_device_ptr(from)) return cudaMemcpyAsync(to, from, n, cudaMemcpyHostToDevice, P->stream);
+        const cudaError_t e = cudaMemcpy(to, from, n, cudaMemcpyDeviceToDevice);
+        return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+    };
+    FMM_CUDA_TRY(copy_in(pd, p, sizeof(double2) * P->nf));
+    FMM_CUDA_TRY(copy_in(ptd, pts, sizeof(double) * 3 * npts));
     int st = launch_far_field(P, pd, ptd, npts, od);
     if (st == FMM_OK) {
         FMM_CUDA_TRY(cudaStreamSynchronize(P->stream));

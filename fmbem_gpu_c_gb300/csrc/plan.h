@@ -8,6 +8,14 @@
 
 namespace fmm {
 
+// Host to device, complete on return.  cudaMemcpy may return while the last of a copy from pageable memory is still on
+// its way, and the plans' streams are non-blocking: they do not wait for the default stream that it is on.
+inline cudaError_t upload(void *dst, const void *src, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 constexpr int NDIR = 316;      // M2L offsets (dx,dy,dz) in [-3,3]^3 with max |d| >= 2
 constexpr int NDIST = 15;      // distinct squared lengths of those offsets
 constexpr int TABLE_PAD = 4;   // entries readable past the last one of the rotation and coaxial tables of

@@ -121,7 +121,7 @@ template <typename Tp>
 static int upload(Scene *S, Tp **dst, const std::vector<Tp> &src)
 {
     FMM_CUDA_TRY(salloc(S, dst, sizeof(Tp) * src.size()));
-    if (!src.empty()) FMM_CUDA_TRY(cudaMemcpy(*dst, src.data(), sizeof(Tp) * src.size(), cudaMemcpyHostToDevice));
+    if (!src.empty()) FMM_CUDA_TRY(fmm::upload(*dst, src.data(), sizeof(Tp) * src.size()));
     return FMM_OK;
 }
 

@@ -819,7 +819,7 @@ static int build_tc_dense(Plan *P, int l, int which)
     };
     cudaError_t e = cudaMalloc(&T, sizeof(double2) * (size_t)g.ncls * P2o * P2i);
     if (e == cudaSuccess) e = cudaMalloc(&rep_dev, sizeof(int) * rep.size());
-    if (e == cudaSuccess) e = cudaMemcpy(rep_dev, rep.data(), sizeof(int) * rep.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(rep_dev, rep.data(), sizeof(int) * rep.size());
     if (e != cudaSuccess) return fail(e);
     int st = gen_dense_rcr(P, l, which, rep_dev, g.ncls, T);
     if (st) {
@@ -839,7 +839,7 @@ static int build_tc_dense(Plan *P, int l, int which)
             h[pm + n] = which == PASS_L2L ? par : inv;      // in
         }
         e = cudaMalloc(&fdev, sizeof(double) * h.size());
-        if (e == cudaSuccess) e = cudaMemcpy(fdev, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = upload(fdev, h.data(), sizeof(double) * h.size());
         if (e != cudaSuccess) return fail(e);
         fo = fdev;
         fi = fdev + pm;
@@ -921,8 +921,8 @@ static int ensure_td_items(RcrList &Lst, size_t ws, int nrhs, cudaStream_t st)
     if (T > 0) {
         int *perm_dev = nullptr;
         FMM_CUDA_TRY(cudaMalloc(&perm_dev, sizeof(int) * T));
-        cudaError_t e = cudaMemcpy(perm_dev, perm.data(), sizeof(int) * T, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(g.dir, pdir.data(), sizeof(int) * T, cudaMemcpyHostToDevice);
+        cudaError_t e = upload(perm_dev, perm.data(), sizeof(int) * T);
+        if (e == cudaSuccess) e = upload(g.dir, pdir.data(), sizeof(int) * T);
         if (e == cudaSuccess) {
             tc_permute_kernel<<<(T + 255) / 256, 256, 0, st>>>(T, perm_dev, Lst.src, Lst.dst, g.src, g.dst);
             e = cudaGetLastError();
@@ -937,7 +937,7 @@ static int ensure_td_items(RcrList &Lst, size_t ws, int nrhs, cudaStream_t st)
         FMM_CUDA_TRY(cudaMalloc(&g.items, sizeof(int4) * items.size()));
         g.items_cap = items.size();
     }
-    if (!items.empty()) FMM_CUDA_TRY(cudaMemcpy(g.items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice));
+    if (!items.empty()) FMM_CUDA_TRY(upload(g.items, items.data(), sizeof(int4) * items.size()));
     g.n_items = (int)items.size();
     g.items_nrhs = nrhs;
     return FMM_OK;

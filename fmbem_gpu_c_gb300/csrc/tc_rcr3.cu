@@ -623,15 +623,15 @@ int build_tc3(Plan *P, int l, int which)
     }
     FMM_CUDA_TRY(dev_alloc(P, (void **)&t.opsR, sizeof(float) * tabR.size()));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&t.opsC, sizeof(float) * std::max<size_t>(1, tabC.size())));
-    FMM_CUDA_TRY(cudaMemcpy(t.opsR, tabR.data(), sizeof(float) * tabR.size(), cudaMemcpyHostToDevice));
-    if (!tabC.empty()) FMM_CUDA_TRY(cudaMemcpy(t.opsC, tabC.data(), sizeof(float) * tabC.size(), cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(t.opsR, tabR.data(), sizeof(float) * tabR.size()));
+    if (!tabC.empty()) FMM_CUDA_TRY(upload(t.opsC, tabC.data(), sizeof(float) * tabC.size()));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&t.blkR, sizeof(int4) * t.hblkR.size()));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&t.blkC, sizeof(int4) * std::max<size_t>(1, t.hblkC.size())));
-    FMM_CUDA_TRY(cudaMemcpy(t.blkR, t.hblkR.data(), sizeof(int4) * t.hblkR.size(), cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(t.blkR, t.hblkR.data(), sizeof(int4) * t.hblkR.size()));
     if (!t.hblkC.empty())
-        FMM_CUDA_TRY(cudaMemcpy(t.blkC, t.hblkC.data(), sizeof(int4) * t.hblkC.size(), cudaMemcpyHostToDevice));
+        FMM_CUDA_TRY(upload(t.blkC, t.hblkC.data(), sizeof(int4) * t.hblkC.size()));
     FMM_CUDA_TRY(dev_alloc(P, (void **)&t.t_dir, sizeof(int) * t.T));
-    FMM_CUDA_TRY(cudaMemcpy(t.t_dir, tdir.data(), sizeof(int) * t.T, cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(upload(t.t_dir, tdir.data(), sizeof(int) * t.T));
     t.built = 1;
     return FMM_OK;
 }
@@ -713,7 +713,7 @@ static int t3_prepare(Plan *P, Tc3 &t, int nrhs)
             FMM_CUDA_TRY(cudaMalloc(&ptr, sizeof(int4) * v.size()));
             cap = v.size();
         }
-        if (!v.empty()) FMM_CUDA_TRY(cudaMemcpy(ptr, v.data(), sizeof(int4) * v.size(), cudaMemcpyHostToDevice));
+        if (!v.empty()) FMM_CUDA_TRY(fmm::upload(ptr, v.data(), sizeof(int4) * v.size()));
         return FMM_OK;
     };
     int e = upload(itR1, t.itR1, t.capR1);
@@ -724,8 +724,8 @@ static int t3_prepare(Plan *P, Tc3 &t, int nrhs)
         FMM_CUDA_TRY(dev_alloc(P, (void **)&t.listR, sizeof(int) * t.T));
         FMM_CUDA_TRY(dev_alloc(P, (void **)&t.listC, sizeof(int) * t.T));
     }
-    FMM_CUDA_TRY(cudaMemcpy(t.listR, listR.data(), sizeof(int) * t.T, cudaMemcpyHostToDevice));
-    FMM_CUDA_TRY(cudaMemcpy(t.listC, listC.data(), sizeof(int) * t.T, cudaMemcpyHostToDevice));
+    FMM_CUDA_TRY(fmm::upload(t.listR, listR.data(), sizeof(int) * t.T));
+    FMM_CUDA_TRY(fmm::upload(t.listC, listC.data(), sizeof(int) * t.T));
     const size_t need = (size_t)ct * nrhs * t.p * t.p;
     if (need > t.scratch_cap) {
         if (t.W) cudaFree(t.W);
