@@ -1074,7 +1074,8 @@ __global__ void __launch_bounds__(32 * FAR_P) far_field_kernel(const double *V, 
         if (t >= npts) continue;  // (a whole warp)
         double2 L = make_double2(0.0, 0.0), M = make_double2(0.0, 0.0);
         double dn = 0.0;
-        for (int a = 0; a < 3; a++) dn += (sx[0][a][lane] - y[a]) * sn[a][lane];
+        if (hc)
+            for (int a = 0; a < 3; a++) dn += (sx[0][a][lane] - y[a]) * sn[a][lane];
         for (int q = 0; q < nq; q++) {
             const double d0 = sx[q][0][lane] - y[0], d1 = sx[q][1][lane] - y[1], d2 = sx[q][2][lane] - y[2];
             const double rr = d0 * d0 + d1 * d1 + d2 * d2, inv = rsqrt(rr);
