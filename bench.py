@@ -329,8 +329,10 @@ def gpu_arm(args, world, rank, local):
     bf16_peak, hbm_peak, peak_kind = peaks()
     achieved_tflops = rcr_flops / (rcr_ms / 1e3) / 1e12
     # the M2L levels on the tensor cores (tc_dense_kernel): split-TF32 GEMMs over dense operators, three
-    # products per input and output, re and im.  From 100,000 translations on two blocks, sums and
-    # differences of m and -m; below, the whole operator in four.  (Padding left out.)
+    # products per input and output, re and im.  From 100,000 translations on (or as FMMBEM_TENSOR_FOLD says, the same
+    # rule as the library's) two blocks, sums and differences of m and -m; below, the whole operator in four.
+    # (Padding left out.)
+    fold = os.environ.get("FMMBEM_TENSOR_FOLD")
     tc_levels = [l for l in range(info.lmin, info.lmax + 1) if info.m2l_tensor[l]]
     tc = None
     if tc_levels:
@@ -338,7 +340,8 @@ def gpu_arm(args, world, rank, local):
         for l in tc_levels:
             p, t = info.p_level[l], info.num_m2l[l]
             sums, diffs = p * (p + 1), p * (p - 1)  # real inputs and outputs of the two blocks
-            ex += 6.0 * t * (sums ** 2 + diffs ** 2 if t >= 100000 else (sums + diffs) ** 2)
+            folded = t >= 100000 if fold is None else fold not in ("", "0")
+            ex += 6.0 * t * (sums ** 2 + diffs ** 2 if folded else (sums + diffs) ** 2)
         tc_ms = sum(float(np.mean(kernel_ms["m2l_l%d" % l])) for l in tc_levels)
         tc_alg = sum(info.num_m2l[l] * f_rcr(info.p_level[l]) for l in tc_levels)
         tc = {"kernel": "tc_dense_kernel (tcgen05.mma kind::tf32, split TF32, TMEM accumulators)", "levels": tc_levels,

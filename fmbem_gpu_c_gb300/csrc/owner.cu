@@ -91,8 +91,7 @@ template <> struct Ops<double> {
 
 // Float-float: the pairs (re, im) of the high and of the low parts side by side, so that the packed
 // FP32 instructions (two FP32 operations each, at the FP32 pipes' rate but half the issue slots)
-// work on re and im together.  Each operation rounds as its scalar form: ff_mac is ff_fma
-// (ff.cuh) on both parts.
+// work on re and im together.  Each half rounds as the scalar operation would.
 struct __align__(16) ffv {
     f2 hi, lo;
 };

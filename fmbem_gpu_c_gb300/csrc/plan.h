@@ -47,7 +47,7 @@ struct Tc3 {
 // A batched pass on the tensor cores as dense operators (tc_dense.cu).  M2L: one operator per
 // class of the 316 directions with equal (dz, dx^2 + dy^2) -- equal polar angle and distance,
 // so the class's directions differ only by their azimuthal phases, which the kernel applies
-// to each row.  M2M / L2L: one operator per octant.  Real-embedded and split into TF32 hi/lo
+// to each row.  M2M / L2L: one operator per z bit of the octant.  Real-embedded and split into TF32 hi/lo
 // parts in the layout the MMA reads.
 constexpr int TC_MAXCH = 40, TC_MAXPIECE = 12, TC_MAXSUB = 4;
 constexpr int TC_PAD = 256;

@@ -35,17 +35,17 @@
 //              not lie on 16 bytes), overlapping the next tile's MMAs where there are two sets.
 // Every wait has a time limit, after which the thread sets the plan's error flag and stops.
 //
-// What bounds it: 16 columns on the 81,920-triangle sphere, p = 14 (192,528 translations) 2.78 ms and
-// p = 10 (650,304) 3.21 ms.  At p = 10 a tile takes 10,000 cycles, of which the MMAs need 4,400 (52 cycles
+// What bounds it: 16 columns on the 81,920-triangle sphere, p = 14 (192,528 translations) 2.77 ms and
+// p = 10 (650,304) 2.82 ms.  At p = 10 a tile takes 8,900 cycles, of which the MMAs need 4,400 (52 cycles
 // each at N = 112 / 96, the full TF32 rate) and the reductions into L2 4,900 (20 bytes a cycle and SM is
-// what the L2 takes from all of them); the issue slots are 63 % busy, a third of them with A's phases
-// and splits.  At p = 14 (one set of accumulators) reading them out, 10,000 of 36,000 cycles, is not hidden.  An earlier
+// what the L2 takes from all of them); the issue slots are 71 % busy, a third of them with A's phases
+// and splits.  At p = 14 (one set of accumulators) reading them out, 10,000 of 36,000 cycles, is not hidden.  Through L2
+// go 10 and 14 TB/s, half of it at p = 14 and a third at p = 10 the operator, streamed again for every tile.  An earlier
 // form, with the whole operator, A in shared memory and one atomic per 16 bytes of output, took 5.96
 // and 5.58 ms (its load/store unit 80 % busy with rows read 16 bytes a lane, A's stores and the atomics).
 // Orders up to 5 are bound by the epilogue's work per row: one group of all degrees, a tile each for the two warps of
 // a quarter in turn, and rows on odd coefficients (odd p^2) as many at a time as the others (649,008 translations, one
-// column: p = 4 115 -> 95 us, p = 5 216 -> 138, p = 9 414 -> 309, p = 10 274 -> 256; the
-// times above are from before).
+// column: p = 4 115 -> 95 us, p = 5 216 -> 138, p = 9 414 -> 309, p = 10 274 -> 256).
 // What made the difference: half the products; A through TMEM; source rows by cp.async, a row per
 // instruction; outputs by bulk reductions, a row's group per instruction; the MMA's issue by one
 // elected thread with operands in uniform registers (500 instead of 950 cycles per six MMAs).
@@ -1052,7 +1052,7 @@ int check_tc_error(Plan *P)
 }
 
 // M2L levels that run dense (order p <= 16, T translations, nb boxes).  Large levels: the dense form is the faster
-// one (16 columns on the 81,920-triangle sphere: p = 10, 650,304 translations 3.2 ms against 9.3 on the SIMT
+// one (16 columns on the 81,920-triangle sphere: p = 10, 650,304 translations 2.8 ms against 9.3 on the SIMT
 // tiles; p = 14, 192,528 translations 2.8 against 6.0).  Small ones: the SIMT tiles are, by little (one column, tiles
 // against dense: T = 2,504 p = 9 12 against 18 us, p = 14 18 against 24; T = 10,592 p = 9 18 against 20, p = 14 37
 // against 41, p = 16 45 against 59).  The line lies where slower tiles used to lose: a level keeps
