@@ -618,15 +618,16 @@ int pick_cols(int rows, size_t elem, size_t most)
 constexpr size_t PART_CAP = 128u << 20;
 
 // ---- scratch, shared by the plans of a device.  A plan takes a buffer while it enqueues its translations and gives it
-// back with an event behind them: the next one to take it waits for that event on its own stream (or finds it
-// passed).  Buffers are added while they stay under POOL_CAP in all, so that plans on several streams run side by
-// side; the last plan of the device to go frees them.  (128 MB in each plan for its life: 256 bodies of a scene
-// would have held 32 GB.)
+// back with an event behind them: the next plan to take it waits for that event on its own stream (or finds it
+// passed).  A plan prefers the buffer that it used last, if no other has since: its own stream orders that.  Buffers
+// are added while they stay under POOL_CAP in all, so that plans on several streams run side by side; the last plan
+// of the device to go frees them.  (128 MB in each plan for its life: 256 bodies of a scene would have held 32 GB.)
 constexpr size_t POOL_CAP = 512u << 20, SMALL_PART = 16u << 20;
 struct Scratch {
     void *ptr = nullptr;
     size_t bytes = 0;
     cudaEvent_t done = nullptr;
+    const Plan *owner = nullptr;  // who used it last (null: gone)
     bool busy = false;
 };
 struct Pool {
@@ -648,16 +649,19 @@ int pool_take(Plan *P, size_t bytes, void **ptr)
     for (;;) {
         int mine = -1, idle = -1, behind = -1, small = -1, room = -1;
         size_t all = 0;
+        bool busy = false;
         for (int i = 0; i < (int)pool.buf.size(); i++) {
             Scratch &s = pool.buf[i];
             all += s.bytes;
-            if (!s.ptr) room = i;
-            if (s.busy) continue;
-            if (s.bytes < bytes) {
-                if (s.ptr) small = i;
+            if (!s.ptr) {
+                if (!s.busy) room = i;
                 continue;
             }
-            if (i == P->own_scratch) {
+            busy = busy || s.busy;
+            if (s.busy) continue;
+            if (s.bytes < bytes) {
+                small = i;
+            } else if (s.owner == P) {
                 mine = i;
             } else if (cudaEventQuery(s.done) == cudaSuccess) {
                 idle = i;
@@ -673,11 +677,10 @@ int pool_take(Plan *P, size_t bytes, void **ptr)
                 Scratch &s = pool.buf[small];
                 FMM_CUDA_TRY(cudaEventSynchronize(s.done));
                 cudaFree(s.ptr);
-                s.ptr = nullptr;
-                s.bytes = 0;
+                s = Scratch{nullptr, 0, s.done};
                 continue;
             }
-            if (take < 0) {  // all are being handed out by other threads
+            if (take < 0 && busy) {  // all are being handed to kernels by other threads
                 pool_free.wait(lock);
                 continue;
             }
@@ -690,7 +693,10 @@ int pool_take(Plan *P, size_t bytes, void **ptr)
             Scratch &s = pool.buf[room];
             if (!s.done) FMM_CUDA_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
             const cudaError_t ce = cudaMalloc(&s.ptr, bytes);
-            if (ce != cudaSuccess && behind < 0) FMM_CUDA_TRY(ce);
+            if (ce != cudaSuccess && behind < 0) {
+                s.ptr = nullptr;
+                FMM_CUDA_TRY(ce);
+            }
             if (ce == cudaSuccess) {
                 s.bytes = bytes;
                 take = room;
@@ -701,8 +707,9 @@ int pool_take(Plan *P, size_t bytes, void **ptr)
             }
         }
         Scratch &s = pool.buf[take];
-        FMM_CUDA_TRY(cudaStreamWaitEvent(P->stream, s.done, 0));
+        if (s.owner != P) FMM_CUDA_TRY(cudaStreamWaitEvent(P->stream, s.done, 0));
         s.busy = true;
+        s.owner = P;
         P->own_scratch = take;
         *ptr = s.ptr;
         return FMM_OK;
@@ -725,7 +732,10 @@ void pool_leave(Plan *P)
     std::lock_guard<std::mutex> lock(pool_mutex);
     Pool &pool = pools[P->opt.device];
     P->own_scratch = Plan::NO_POOL;
-    if (--pool.users > 0) return;
+    pool.users--;
+    for (Scratch &s : pool.buf)
+        if (s.owner == P) s.owner = nullptr;
+    if (pool.users > 0) return;
     for (Scratch &s : pool.buf) {
         cudaFree(s.ptr);
         if (s.done) cudaEventDestroy(s.done);
